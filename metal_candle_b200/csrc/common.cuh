@@ -23,6 +23,7 @@ struct DeviceState {
   int sm_count = 0;
   int* status_word = nullptr;  // device int: 0, or the code of a bounded wait that gave up
   long long* selftest_out = nullptr;  // three device words behind the status word (mcb_selftest_wait_timeout)
+  bool f32_tile_smem = false;  // the float32 tile kernel's shared-memory limit has been raised
   void* encode_tiled = nullptr;  // cuTensorMapEncodeTiled resolved through the runtime
 };
 DeviceState* current_device_state();  // null (and error set) when mcb_init was not called

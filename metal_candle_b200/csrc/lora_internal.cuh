@@ -50,6 +50,11 @@ inline int64_t h_pitch(int64_t M) { return ((M + 63) / 64) * 64; }
 namespace f32path {
 size_t workspace_bytes(int64_t M, int64_t K, int64_t N, int64_t r);
 int delta_fwd(const LoraArgs& a);
+// The delta of few tokens in one cluster launch, float32 arithmetic for either dtype of x and out.  Up to 512 tokens it
+// beats the two float32 launches (400 x 4096 -> 4096 r64: 52 us against 91).
+constexpr int64_t kDeltaMaxTokens = 512;
+bool delta_small(int64_t M, int64_t r);
+int delta_cluster(const LoraArgs& a, int dtype);
 int linear_fwd(const LoraArgs& a);
 int linear_bwd(const LoraArgs& a);
 // out[M,N] = a[M,K] b[K,N]

@@ -767,6 +767,11 @@ size_t workspace_bytes(int64_t M, int64_t K, int64_t N, int64_t r) {
 
 int delta_fwd(const LoraArgs& a, const DeviceState* ds) {
   if (int rc = check_ws(a, "lora_delta_fwd")) return rc;
+  // Few tokens: one cluster launch in float32 arithmetic instead of the operand pack and a GEMM of one or two 128-row
+  // tiles.  64 x 1024 -> 1024 r16: 4.8 us against 14.2; 256 x 4096 -> 4096 r64: 33 against 38.  Beyond that the tensor
+  // cores win.  (Sizes and alignment that the GEMM refuses are still refused, below.)
+  if (a.M <= 256 && f32path::delta_small(a.M, a.r) && a.K % 8 == 0 && a.N % 8 == 0 && aligned16(a.x) && aligned16(a.y))
+    return f32path::delta_cluster(a, MCB_BF16);
   Workspace w = carve(a.ws, a.M, a.K, a.N, a.r);
   if (int rc = pack(a, w, 0)) return rc;
   GemmCall c;
