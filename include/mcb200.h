@@ -420,6 +420,15 @@ int mcb_add(const void* a, const void* b, void* out, int64_t n, int dtype, void*
  * d loss / d logits. */
 int mcb_cross_entropy(void* logits, const int32_t* targets, float* nll, int32_t* count, float* loss,
                       int64_t M, int64_t V, int write_grad, int dtype, void* stream);
+/* The same loss with the logits left as they are: the gradient goes to dlogits [M,V] (null: loss only), in the same pass.
+ * targets [M] are int32 or int64 (target_bytes 4 or 8); with has_ignore, ignore_index is ignored as well as -1.  Scratch:
+ * t32 [M], nll [M].  info[0] = targets that count, info[1] = targets that are neither ignored nor in [0,V) (they count as
+ * ignored), info[2] is scratch; info_host, if not null, is page-locked host memory (device-accessible) that gets
+ * info[0] and info[1] before the row kernel runs, and info_event (a cudaEvent_t or null) is recorded at that point: a
+ * caller can check the targets without waiting for the loss. */
+int mcb_cross_entropy_out(const void* logits, void* dlogits, const void* targets, int target_bytes, int has_ignore,
+                          int64_t ignore_index, int32_t* t32, int32_t* info, int32_t* info_host, void* info_event, float* nll,
+                          float* loss, int64_t M, int64_t V, int dtype, void* stream);
 /* The same loss a chunk of tokens at a time, for a caller that produces the logits chunk by chunk (lm_head on a
  * slice of the tokens), turns each chunk into its gradient in place and feeds that straight to the lm_head backward,
  * so that the [tokens, vocabulary] matrix of the whole batch never exists (the reference materialises it, and walks

@@ -137,6 +137,7 @@ SIGNATURES = {
     "mcb_swiglu_bwd": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _i32, _vp]),
     "mcb_add": (_i32, [_vp, _vp, _vp, _i64, _i32, _vp]),
     "mcb_cross_entropy": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _i32, _vp]),
+    "mcb_cross_entropy_out": (_i32, [_vp, _vp, _vp, _i32, _i32, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _vp]),
     "mcb_cross_entropy_count": (_i32, [_vp, _vp, _i64, _i64, _vp]),
     "mcb_cross_entropy_chunk": (_i32, [_vp, _vp, _vp, _vp, _i64, _i64, _i32, _i32, _vp]),
     "mcb_cross_entropy_finish": (_i32, [_vp, _vp, _vp, _i64, _vp]),

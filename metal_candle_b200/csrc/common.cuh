@@ -24,6 +24,8 @@ struct DeviceState {
   int* status_word = nullptr;  // device int: 0, or the code of a bounded wait that gave up
   long long* selftest_out = nullptr;  // three device words behind the status word (mcb_selftest_wait_timeout)
   bool f32_tile_smem = false;  // the float32 tile kernel's shared-memory limit has been raised
+  bool ce_smem[2] = {false, false};  // the same of the cross-entropy cluster kernel (bf16, float32)
+  int ce_clusters[2][9] = {};  // its resident clusters, by dtype and cluster size; 0 = not asked yet
   void* encode_tiled = nullptr;  // cuTensorMapEncodeTiled resolved through the runtime
 };
 DeviceState* current_device_state();  // null (and error set) when mcb_init was not called

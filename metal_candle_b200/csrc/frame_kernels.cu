@@ -1,7 +1,6 @@
 // The element-wise "frame" of the Qwen-shaped training step around the LoRA hot path: embedding
-// gather, rotary embedding with the head-major re-layout attention wants, SwiGLU, residual add, and a
-// fused cross-entropy forward+backward.  All are HBM-bound streaming kernels; float32 or bfloat16
-// storage, float32 arithmetic.
+// gather, rotary embedding with the head-major re-layout attention wants, SwiGLU and residual add.  All
+// are HBM-bound streaming kernels; float32 or bfloat16 storage, float32 arithmetic.
 #include "common.cuh"
 
 namespace mcb {
@@ -254,143 +253,6 @@ __global__ void mul_kernel(const T* __restrict__ a, const T* __restrict__ b, T* 
     out[i] = from_f32<T>(to_f32(a[i]) * (mode == 0 ? to_f32(b[i]) : scalar));
 }
 
-// ---- cross-entropy forward + backward (src/training/loss.rs:97-146) ----------------------------------------
-// One block per row of logits [M,V].  Sweep 1: online max / sum-exp (HBM read).  Sweep 2 (the row is in
-// L2 by now): overwrite the row with d loss / d logits = (softmax - onehot) * inv_count; ignored rows get
-// zeros.  nll[row] = logsumexp - logit[target] (0 for ignored rows); a second tiny kernel sums nll in
-// row order, so the loss is deterministic.
-constexpr float kLog2e = 1.4426950408889634f;
-// 2^x with denormal results flushed to zero: one instruction, where __expf's denormal handling takes several
-// (relative error about 2^-22; the long-row loops below are bound by their instruction count)
-__device__ __forceinline__ float ex2_ftz(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ void online_combine(float& m, float& s, float m2, float s2) {
-  const float mm = fmaxf(m, m2);
-  if (mm == -INFINITY) { m = mm; s = 0.0f; return; }
-  s = s * __expf(m - mm) + s2 * __expf(m2 - mm);
-  m = mm;
-}
-
-// Persistent: block b takes rows b, b + gridDim.x, ...  Measured on [8192, 151936] bf16: how many rows are in flight
-// (148 blocks of 1024 threads = 45 MB, inside the L2, up to 1184 blocks of 256 threads = 360 MB) moves the time by
-// 10 % at most, smaller blocks ahead: the loops are bound by their instructions (two exponentials per element over
-// the two sweeps), not by where sweep 2 finds the row.
-template <typename T>
-__global__ void __launch_bounds__(1024)
-cross_entropy_kernel(T* __restrict__ logits, const int32_t* __restrict__ targets, float* __restrict__ nll,
-                     const int32_t* __restrict__ count_ptr, int64_t M, int V, int write_grad) {
-  __shared__ float sm[32], ss[32];
-  const float inv_count = 1.0f / static_cast<float>(max(1, *count_ptr));
-  using VT = Vec16<T>;
-  constexpr int NV = VT::N;
-  const int bd = blockDim.x;
-  for (int64_t row = blockIdx.x; row < M; row += gridDim.x) {
-    T* lr = logits + row * V;
-    const int32_t tgt = targets[row];
-    const bool ignored = tgt < 0 || tgt >= V;  // u32::MAX (src/training/trainer.rs:385) reads as -1
-    if (ignored) {   // the same for every thread of the block
-      if (threadIdx.x == 0) nll[row] = 0.0f;
-      if (write_grad)
-        for (int c = threadIdx.x; c < V; c += bd) lr[c] = from_f32<T>(0.0f);
-      continue;
-    }
-    const bool vec = (V % NV == 0) && ((reinterpret_cast<uintptr_t>(lr) & 15u) == 0);
-    float m = -INFINITY, s = 0.0f;
-    if (vec) {
-      const int nvec = V / NV;
-      const auto* src = reinterpret_cast<const decltype(VT::raw)*>(lr);
-      auto absorb = [&](const VT& t) {
-        float f[NV];
-        t.to_float(f);
-        float vm = f[0];
-#pragma unroll
-        for (int j = 1; j < NV; ++j) vm = fmaxf(vm, f[j]);
-        if (vm == -INFINITY) return;  // a wholly masked vector adds nothing (and exp(-inf - -inf) would be NaN)
-        if (vm > m) { s *= __expf(m - vm); m = vm; }
-        const float m2 = -m * kLog2e;   // exp(f - m) = 2^(f log2e - m log2e): one fused multiply-add and one special function
-#pragma unroll
-        for (int j = 0; j < NV; ++j) s += ex2_ftz(fmaf(f[j], kLog2e, m2));
-      };
-      int c = threadIdx.x;
-      for (; c + 3 * bd < nvec; c += 4 * bd) {   // four loads in flight per thread
-        VT t0, t1, t2, t3;
-        t0.raw = src[c]; t1.raw = src[c + bd]; t2.raw = src[c + 2 * bd]; t3.raw = src[c + 3 * bd];
-        absorb(t0); absorb(t1); absorb(t2); absorb(t3);
-      }
-      for (; c < nvec; c += bd) {
-        VT t; t.raw = src[c];
-        absorb(t);
-      }
-    } else {
-      for (int c = threadIdx.x; c < V; c += bd) {
-        const float v = to_f32(lr[c]);
-        if (v > m) { s = s * __expf(m - v) + 1.0f; m = v; } else if (v != -INFINITY) { s += __expf(v - m); }
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float m2 = __shfl_xor_sync(0xffffffffu, m, o), s2 = __shfl_xor_sync(0xffffffffu, s, o);
-      online_combine(m, s, m2, s2);
-    }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = bd >> 5;
-    if (lane == 0) { sm[warp] = m; ss[warp] = s; }
-    __syncthreads();
-    m = sm[0]; s = ss[0];
-    for (int w = 1; w < nw; ++w) online_combine(m, s, sm[w], ss[w]);
-    const float lse = m + logf(s);
-    if (threadIdx.x == 0) nll[row] = lse - to_f32(lr[tgt]);
-    __syncthreads();  // thread 0 has read lr[tgt] before anyone overwrites it; sm / ss are free for the next row
-    if (write_grad) {
-      if (vec) {
-        const int nvec = V / NV;
-        auto* dst = reinterpret_cast<decltype(VT::raw)*>(lr);
-        const float lse2 = -lse * kLog2e;
-        auto grad = [&](VT& t, int c) {
-          float f[NV];
-          t.to_float(f);
-#pragma unroll
-          for (int j = 0; j < NV; ++j) {
-            float p = ex2_ftz(fmaf(f[j], kLog2e, lse2));
-            if (c * NV + j == tgt) p -= 1.0f;
-            f[j] = p * inv_count;
-          }
-          t.from_float(f);
-          dst[c] = t.raw;
-        };
-        int c = threadIdx.x;
-        for (; c + 3 * bd < nvec; c += 4 * bd) {
-          VT t0, t1, t2, t3;
-          t0.raw = dst[c]; t1.raw = dst[c + bd]; t2.raw = dst[c + 2 * bd]; t3.raw = dst[c + 3 * bd];
-          grad(t0, c); grad(t1, c + bd); grad(t2, c + 2 * bd); grad(t3, c + 3 * bd);
-        }
-        for (; c < nvec; c += bd) {
-          VT t; t.raw = dst[c];
-          grad(t, c);
-        }
-      } else {
-        for (int c = threadIdx.x; c < V; c += bd) {
-          float p = __expf(to_f32(lr[c]) - lse);
-          if (c == tgt) p -= 1.0f;
-          lr[c] = from_f32<T>(p * inv_count);
-        }
-      }
-    }
-  }
-}
-
-// Launch shape of cross_entropy_kernel: eight blocks of 256 threads per SM, fewer when there are fewer rows.
-static void cross_entropy_launch_shape(int64_t rows, int64_t V, unsigned* grid, unsigned* block) {
-  const DeviceState* ds = current_device_state();
-  const int sms = ds ? ds->sm_count : 148;
-  const int threads = 256, per_sm = 8;
-  const int64_t blocks = static_cast<int64_t>(sms) * per_sm;
-  *block = static_cast<unsigned>(threads);
-  *grid = static_cast<unsigned>(rows < blocks ? rows : blocks);
-}
-
 // out[n,k] = W[n,k] + scale * sum_j A[k,j] B[j,n]   (LoRAAdapter::merge_weights, src/training/adapter.rs:315-354:
 // base + scaling * (A B)^T for a base weight stored [out, in]).  One thread per 4 consecutive k of one n; A rows
 // and the B column are read through the read-only cache, the product is accumulated in float32.
@@ -419,38 +281,6 @@ __global__ void merge_weights_kernel(const T* __restrict__ W, const float* __res
         out[o] = from_f32<T>(to_f32(W[o]) + scale * acc[e]);
       }
     }
-  }
-}
-
-__global__ void count_valid_kernel(const int32_t* __restrict__ targets, int64_t M, int V, int32_t* __restrict__ count) {
-  __shared__ int red[32];
-  int c = 0;
-  for (int64_t i = threadIdx.x; i < M; i += blockDim.x) c += (targets[i] >= 0 && targets[i] < V) ? 1 : 0;
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int w = 0; w < (blockDim.x >> 5); ++w) t += red[w];
-    *count = t;
-  }
-}
-
-// loss[0] = sum(nll) / count, loss[1] = sum(nll); serial tree in fixed order (one block).
-__global__ void reduce_nll_kernel(const float* __restrict__ nll, int64_t M, const int32_t* __restrict__ count,
-                                  float* __restrict__ loss) {
-  __shared__ double red[1024];
-  double acc = 0.0;
-  for (int64_t i = threadIdx.x; i < M; i += blockDim.x) acc += static_cast<double>(nll[i]);
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    loss[1] = static_cast<float>(red[0]);
-    loss[0] = static_cast<float>(red[0] / static_cast<double>(max(1, *count)));
   }
 }
 
@@ -655,60 +485,6 @@ extern "C" int mcb_mul_scalar(const void* a, void* out, int64_t n, float value, 
   const int grid = grid_for(n, 256, ds->sm_count);
   MCB_DTYPE_SWITCH(dtype, (mul_kernel<T><<<grid, 256, 0, st>>>((const T*)a, (const T*)a, (T*)out, n, value, 1)));
   MCB_CHECK_LAUNCH("mul_scalar");
-  return MCB_OK;
-}
-
-extern "C" int mcb_cross_entropy(void* logits, const int32_t* targets, float* nll, int32_t* count, float* loss,
-                                 int64_t M, int64_t V, int write_grad, int dtype, void* stream) {
-  MCB_NVTX_RANGE("mcb_cross_entropy");
-  if (!logits || !targets || !nll || !count || !loss) return fail(MCB_ERR_NULL, "cross_entropy: null pointer");
-  if (M <= 0 || V <= 0 || M > 0x7fffffff || V > 0x7fffffff) return fail(MCB_ERR_SHAPE, "cross_entropy: bad shape");
-  if (!current_device_state()) return MCB_ERR_NOT_INIT;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  count_valid_kernel<<<1, 1024, 0, st>>>(targets, M, (int)V, count);
-  MCB_CHECK_LAUNCH("count_valid");
-  unsigned grid = 0, block = 0;
-  cross_entropy_launch_shape(M, V, &grid, &block);
-  MCB_DTYPE_SWITCH(dtype, (cross_entropy_kernel<T><<<grid, block, 0, st>>>((T*)logits, targets, nll, count, M, (int)V, write_grad)));
-  MCB_CHECK_LAUNCH("cross_entropy");
-  reduce_nll_kernel<<<1, 1024, 0, st>>>(nll, M, count, loss);
-  MCB_CHECK_LAUNCH("reduce_nll");
-  return MCB_OK;
-}
-
-// The three stages of mcb_cross_entropy as separate calls, so that the logits can be produced, consumed and
-// discarded a chunk of tokens at a time (the [tokens, vocabulary] matrix of the whole batch never exists).
-extern "C" int mcb_cross_entropy_count(const int32_t* targets, int32_t* count, int64_t M, int64_t V, void* stream) {
-  MCB_NVTX_RANGE("mcb_cross_entropy_count");
-  if (!targets || !count) return fail(MCB_ERR_NULL, "cross_entropy_count: null pointer");
-  if (M <= 0 || V <= 0 || M > 0x7fffffff || V > 0x7fffffff) return fail(MCB_ERR_SHAPE, "cross_entropy_count: bad shape");
-  if (!current_device_state()) return MCB_ERR_NOT_INIT;
-  count_valid_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(targets, M, (int)V, count);
-  MCB_CHECK_LAUNCH("count_valid");
-  return MCB_OK;
-}
-
-extern "C" int mcb_cross_entropy_chunk(void* logits, const int32_t* targets, float* nll, const int32_t* count, int64_t rows,
-                                       int64_t V, int write_grad, int dtype, void* stream) {
-  MCB_NVTX_RANGE("mcb_cross_entropy_chunk");
-  if (!logits || !targets || !nll || !count) return fail(MCB_ERR_NULL, "cross_entropy_chunk: null pointer");
-  if (rows <= 0 || V <= 0 || rows > 0x7fffffff || V > 0x7fffffff) return fail(MCB_ERR_SHAPE, "cross_entropy_chunk: bad shape");
-  if (!current_device_state()) return MCB_ERR_NOT_INIT;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  unsigned grid = 0, block = 0;
-  cross_entropy_launch_shape(rows, V, &grid, &block);
-  MCB_DTYPE_SWITCH(dtype, (cross_entropy_kernel<T><<<grid, block, 0, st>>>((T*)logits, targets, nll, count, rows, (int)V, write_grad)));
-  MCB_CHECK_LAUNCH("cross_entropy");
-  return MCB_OK;
-}
-
-extern "C" int mcb_cross_entropy_finish(const float* nll, const int32_t* count, float* loss, int64_t M, void* stream) {
-  MCB_NVTX_RANGE("mcb_cross_entropy_finish");
-  if (!nll || !count || !loss) return fail(MCB_ERR_NULL, "cross_entropy_finish: null pointer");
-  if (M <= 0 || M > 0x7fffffff) return fail(MCB_ERR_SHAPE, "cross_entropy_finish: bad shape");
-  if (!current_device_state()) return MCB_ERR_NOT_INIT;
-  reduce_nll_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(nll, M, count, loss);
-  MCB_CHECK_LAUNCH("reduce_nll");
   return MCB_OK;
 }
 

@@ -44,6 +44,8 @@ struct Params {
   float eps, scale;
   int* status;
   uint32_t stage_bytes, bar_off;
+  int mis;           // ragged rows: elements from the 16-byte boundary below `in0` to it (the same for in1 and out)
+  uint32_t stream_bytes;  // bytes of one input stream per stage
   uint32_t w_off;    // float32 copy of the rmsnorm weight in shared memory, 0 = none (no weight, or streamed forward)
 };
 
@@ -66,7 +68,7 @@ __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b
 // This lane's vectors lane, lane+32, ... of a row in shared memory, kept as they are (16 bytes each); vectors
 // at or beyond nv read as `fill`.
 template <typename T, int KMAX>
-__device__ __forceinline__ void load_row(const uint8_t* s0, int lane, int nv, Vec16<T> (&v)[KMAX], float fill) {
+__device__ __forceinline__ void load_row(const uint8_t* s0, int lane, int nv, Vec16<T> (&v)[KMAX], float fill, int first = 0) {
   using V = Vec16<T>;
   float ff[V::N];
 #pragma unroll
@@ -76,7 +78,7 @@ __device__ __forceinline__ void load_row(const uint8_t* s0, int lane, int nv, Ve
 #pragma unroll
   for (int k = 0; k < KMAX; ++k) {
     const int vi = lane + 32 * k;
-    if (vi < nv) v[k].raw = reinterpret_cast<const decltype(fv.raw)*>(s0)[vi];
+    if (vi < nv && vi >= first) v[k].raw = reinterpret_cast<const decltype(fv.raw)*>(s0)[vi];
     else v[k].raw = fv.raw;
   }
 }
@@ -96,10 +98,14 @@ __host__ __device__ constexpr int rowpipe_min_blocks(int op, int w, int elems_pe
   return w <= 8 ? 2 : 1;
 }
 
+// RAG: rows that are not whole 16-byte vectors, or not aligned to them (softmax only).  Rows lie back to back, so a tile of
+// them is one bulk copy of the 16-byte granules that cover it.  The whole granules of a row take the same code as an
+// aligned row; its elements in the first and last granule, which it shares with its neighbours, are taken one per lane
+// (masking them inside the vector code made every vector pay: 150 instead of 94 us for the backward of 8 x 14 x 777 x 777).
 // KMAX > 0: a lane owns vectors lane, lane+32, ... (KMAX of them) of every row and keeps them in registers —
 // the row itself (forward ops) or the dw sums (rmsnorm backward with dw).  KMAX == 0: rows of any width,
 // streamed from shared memory twice.
-template <typename T, int OP, int W, int KMAX>
+template <typename T, int OP, int W, int KMAX, bool RAG>
 __global__ void __launch_bounds__((W + 1) * 32, rowpipe_min_blocks(OP, W, KMAX * Vec16<T>::N))
 rowpipe_kernel(const Params p) {
   using V = Vec16<T>;
@@ -131,7 +137,7 @@ rowpipe_kernel(const Params p) {
 
   const int R = W / p.wpr;   // rows per tile
   const int64_t n_tiles = (p.rows + R - 1) / R;
-  const uint32_t stream_bytes = static_cast<uint32_t>(R) * p.row_bytes;
+  const uint32_t stream_bytes = p.stream_bytes;
 
   constexpr bool kDw = (OP == kRmsBwd && KMAX > 0);  // per-lane dw sums kept in registers
   float dwa[kDw ? KMAX : 1][N];
@@ -155,7 +161,16 @@ rowpipe_kernel(const Params p) {
       const uint32_t fb = full0 + 8 * stage, sb = base + stage * p.stage_bytes;
       const char* g0 = static_cast<const char*>(p.in0) + row0 * p.row_bytes;
       const char* g1 = kTwoIn ? static_cast<const char*>(p.in1) + row0 * p.row_bytes : nullptr;
-      if (p.causal_seq > 0) {
+      if constexpr (RAG) {
+        if (lane == 0) {
+          const int64_t e0 = row0 * p.D + p.mis, e1 = e0 + static_cast<int64_t>(nrows) * p.D;   // elements from the boundary on
+          const int64_t v0 = e0 / N, v1 = (e1 + N - 1) / N;
+          const uint32_t b = static_cast<uint32_t>(v1 - v0) * 16;
+          mbar_expect_tx(fb, b * (kTwoIn ? 2u : 1u));
+          bulk_load(sb, static_cast<const T*>(p.in0) - p.mis + v0 * N, b, fb);
+          if (kTwoIn) bulk_load(sb + stream_bytes, static_cast<const T*>(p.in1) - p.mis + v0 * N, b, fb);
+        }
+      } else if (p.causal_seq > 0) {
         // lane r copies row r of the tile, only up to its query position
         const int q0 = static_cast<int>(row0 % p.causal_seq);  // one division per tile
         int q = q0 + lane;
@@ -183,15 +198,29 @@ rowpipe_kernel(const Params p) {
     int stage = 0;
     uint32_t phase = 0;
     const float inv_d = 1.0f / static_cast<float>(p.D);
-    const int nvec = p.nvec;
+    int nvec = p.nvec;
     for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
       if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * stage, phase, abort_flag, 52, p.status))) break;
       const int rit = warp / p.wpr, seg = warp - rit * p.wpr;   // row of the tile, segment of the row
       const int64_t row = t * R + rit;
       if (row < p.rows) {
         const uint8_t* s0 = gen_base + stage * p.stage_bytes + rit * p.row_bytes;
-        const uint8_t* s1 = s0 + stream_bytes;
         T* orow = static_cast<T*>(p.out) + row * p.D;
+        // ragged rows: elements [lo, end) of the covering granules, whole granules [fa, nvec); the first 2N lanes each take
+        // one of the elements before or behind them (edge < 0: none)
+        int lo = 0, fa = 0, edge = -1;
+        if constexpr (RAG) {
+          const int64_t e0 = t * R * p.D + p.mis, e = row * p.D + p.mis;
+          s0 = gen_base + stage * p.stage_bytes + (e / N - e0 / N) * 16;
+          lo = static_cast<int>(e % N);
+          const int end = lo + p.D;
+          fa = (lo + N - 1) / N;
+          nvec = end / N;                      // fa <= nvec: D >= 2N is checked on the host
+          edge = lane < N ? lo + lane : nvec * N + lane - N;
+          if (edge >= (lane < N ? fa * N : end) || lane >= 2 * N) edge = -1;
+          orow -= lo;
+        }
+        const uint8_t* s1 = s0 + stream_bytes;
         if constexpr (OP == kRmsFwd && KMAX > 0) {
           V v[KMAX];
           load_row<T, KMAX>(s0, lane, nvec, v, 0.0f);
@@ -363,40 +392,41 @@ rowpipe_kernel(const Params p) {
           }
         } else if constexpr (OP == kSmFwd && KMAX > 0) {
           const bool causal = p.causal_seq > 0;
-          const int q = causal ? static_cast<int>(row % p.causal_seq) : p.D;  // last kept column
+          const int q = causal ? static_cast<int>(row % p.causal_seq) + lo : p.D + lo;  // last kept element
           const int nv_keep = causal ? min(nvec, q / N + 1) : nvec;
           const int vq = causal ? q / N : -1;  // only the vector that holds column q has masked elements behind it
           const float sc = p.scale * kLog2e;   // work in base-2 logits
           V v[KMAX];
-          load_row<T, KMAX>(s0, lane, nv_keep, v, -INFINITY);
+          load_row<T, KMAX>(s0, lane, nv_keep, v, -INFINITY, fa);
+          auto mask = [&](int vi, float (&f)[N]) {
+            if (vi == vq) {
+#pragma unroll
+              for (int j = 0; j < N; ++j)
+                if (vq * N + j > q) f[j] = -INFINITY;
+            }
+          };
+          const float xe = RAG && edge >= 0 && edge <= q ? to_f32(reinterpret_cast<const T*>(s0)[edge]) : -INFINITY;
           float m = -INFINITY;
 #pragma unroll
           for (int k = 0; k < KMAX; ++k) {
             float f[N];
             v[k].to_float(f);
-            if (lane + 32 * k == vq) {
-#pragma unroll
-              for (int j = 0; j < N; ++j)
-                if (vq * N + j > q) f[j] = -INFINITY;
-            }
+            mask(lane + 32 * k, f);
 #pragma unroll
             for (int j = 0; j < N; ++j) m = fmaxf(m, f[j]);
           }
+          if constexpr (RAG) m = fmaxf(m, xe);
           m = warp_max(m) * sc;  // sc > 0: max commutes with the scaling
           // Up to 32 elements per lane keep their exponentials in registers; wider rows compute them twice
           // (once for the sum, once for the output) rather than spill.
           constexpr bool kKeep = KMAX * N <= 32;
           float e[kKeep ? KMAX : 1][N];
-          float inv = 0.0f;
+          float inv = 0.0f, ee = 0.0f;   // ee: the edge element's exponential
           const float2 sc2 = f2(sc, sc), nm2 = f2(-m, -m);
           auto exps = [&](int k, float (&o)[N]) {
             float f[N];
             v[k].to_float(f);
-            if (lane + 32 * k == vq) {
-#pragma unroll
-              for (int j = 0; j < N; ++j)
-                if (vq * N + j > q) f[j] = -INFINITY;
-            }
+            mask(lane + 32 * k, f);
 #pragma unroll
             for (int j = 0; j < N; j += 2) {
               const float2 a = __ffma2_rn(f2(f[j], f[j + 1]), sc2, nm2);
@@ -420,6 +450,7 @@ rowpipe_kernel(const Params p) {
                 for (int j = 0; j < N; ++j) e[k][j] = t[j];
               }
             }
+            if constexpr (RAG) { ee = fast_exp2(fmaf(xe, sc, -m)); acc0.x += ee; }
             const float ssum = warp_sum((acc0.x + acc0.y) + (acc1.x + acc1.y));
             inv = ssum > 0.0f ? 1.0f / ssum : 0.0f;
           }
@@ -427,7 +458,7 @@ rowpipe_kernel(const Params p) {
 #pragma unroll
           for (int k = 0; k < KMAX; ++k) {
             const int vi = lane + 32 * k;
-            if (vi < nvec) {
+            if (vi < nvec && vi >= fa) {
               float t[N], o[N];
               if (m == -INFINITY) {
 #pragma unroll
@@ -448,38 +479,44 @@ rowpipe_kernel(const Params p) {
               __stcs(reinterpret_cast<decltype(a.raw)*>(orow) + vi, a.raw);
             }
           }
+          if constexpr (RAG) {
+            if (edge >= 0) orow[edge] = from_f32<T>(ee * inv);
+          }
         } else if constexpr (OP == kSmFwd) {
-          const int q = p.causal_seq > 0 ? static_cast<int>(row % p.causal_seq) : p.D;  // last kept column (one division per row per warp)
+          const int q = p.causal_seq > 0 ? static_cast<int>(row % p.causal_seq) + lo : p.D + lo;  // last kept element
           const int nv_keep = p.causal_seq > 0 ? min(nvec, q / N + 1) : nvec;
+          const float xe = RAG && edge >= 0 && edge <= q ? to_f32(reinterpret_cast<const T*>(s0)[edge]) : -INFINITY;
           const float sc = p.scale * kLog2e;  // work in base-2 logits
           // pass 1: row maximum (cheap), pass 2: sum of 2^(x - max) with independent partial sums
           float m = -INFINITY;
 #pragma unroll 4
-          for (int vi = lane; vi < nv_keep; vi += 32) {
+          for (int vi = fa + lane; vi < nv_keep; vi += 32) {
             V a; a.raw = reinterpret_cast<const decltype(a.raw)*>(s0)[vi];
             float f[N]; a.to_float(f);
 #pragma unroll
             for (int j = 0; j < N; ++j) m = fmaxf(m, (vi * N + j <= q) ? f[j] : -INFINITY);
           }
+          if constexpr (RAG) m = fmaxf(m, xe);
           m = warp_max(m) * sc;  // sc > 0: max commutes with the scaling
           float s = 0.0f;
           if (m != -INFINITY) {
             float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll 4
-            for (int vi = lane; vi < nv_keep; vi += 32) {
+            for (int vi = fa + lane; vi < nv_keep; vi += 32) {
               V a; a.raw = reinterpret_cast<const decltype(a.raw)*>(s0)[vi];
               float f[N]; a.to_float(f);
 #pragma unroll
               for (int j = 0; j < N; ++j)
                 part[j & 3] += (vi * N + j <= q) ? fast_exp2(fmaf(f[j], sc, -m)) : 0.0f;
             }
+            if constexpr (RAG) part[0] += fast_exp2(fmaf(xe, sc, -m));
             s = (part[0] + part[1]) + (part[2] + part[3]);
           }
           s = warp_sum(s);
           const float inv = s > 0.0f ? 1.0f / s : 0.0f;
           const float mref = (m == -INFINITY) ? 0.0f : m;
 #pragma unroll 4
-          for (int vi = lane; vi < nvec; vi += 32) {
+          for (int vi = fa + lane; vi < nvec; vi += 32) {
             float f[N];
             if (vi < nv_keep) {
               V a; a.raw = reinterpret_cast<const decltype(a.raw)*>(s0)[vi];
@@ -493,21 +530,30 @@ rowpipe_kernel(const Params p) {
             V a; a.from_float(f);
             __stcs(reinterpret_cast<decltype(a.raw)*>(orow) + vi, a.raw);
           }
+          if constexpr (RAG) {
+            if (edge >= 0) orow[edge] = from_f32<T>(fast_exp2(fmaf(xe, sc, -mref)) * inv);
+          }
         } else {  // kSmBwd
-          const int q = p.causal_seq > 0 ? static_cast<int>(row % p.causal_seq) : p.D;
+          const int q = p.causal_seq > 0 ? static_cast<int>(row % p.causal_seq) + lo : p.D + lo;
           const int nv_keep = p.causal_seq > 0 ? min(nvec, q / N + 1) : nvec;
+          float ye = 0.0f, ge = 0.0f;
+          if (RAG && edge >= 0 && edge <= q) {
+            ye = to_f32(reinterpret_cast<const T*>(s0)[edge]);
+            ge = to_f32(reinterpret_cast<const T*>(s1)[edge]);
+          }
           float dot = 0.0f;
 #pragma unroll 4
-          for (int vi = lane; vi < nv_keep; vi += 32) {
+          for (int vi = fa + lane; vi < nv_keep; vi += 32) {
             V a, b; a.raw = reinterpret_cast<const decltype(a.raw)*>(s0)[vi];
             b.raw = reinterpret_cast<const decltype(b.raw)*>(s1)[vi];
             float y[N], g[N]; a.to_float(y); b.to_float(g);
 #pragma unroll
             for (int j = 0; j < N; ++j) dot = fmaf((vi * N + j <= q) ? y[j] : 0.0f, g[j], dot);
           }
+          if constexpr (RAG) dot = fmaf(ye, ge, dot);
           dot = warp_sum(dot);
 #pragma unroll 4
-          for (int vi = lane; vi < nvec; vi += 32) {
+          for (int vi = fa + lane; vi < nvec; vi += 32) {
             float o[N];
             if (vi < nv_keep) {
               V a, b; a.raw = reinterpret_cast<const decltype(a.raw)*>(s0)[vi];
@@ -521,6 +567,9 @@ rowpipe_kernel(const Params p) {
             }
             V a; a.from_float(o);
             __stcs(reinterpret_cast<decltype(a.raw)*>(orow) + vi, a.raw);
+          }
+          if constexpr (RAG) {
+            if (edge >= 0) orow[edge] = from_f32<T>(ye * (ge - dot) * p.scale);
           }
         }
       }
@@ -559,33 +608,33 @@ rowpipe_kernel(const Params p) {
   }
 }
 
-template <typename T, int OP, int W, int KMAX>
+template <typename T, int OP, int W, int KMAX, bool RAG>
 int launch_one(const Params& p, int grid, size_t smem, cudaStream_t st) {
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(rowpipe_kernel<T, OP, W, KMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(rowpipe_kernel<T, OP, W, KMAX, RAG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (227 * 1024) / 2 - 1024);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(rowpipe_kernel)");
     // ask for the largest shared-memory carve-out so that two CTAs of ~100 KB fit an SM
-    e = cudaFuncSetAttribute(rowpipe_kernel<T, OP, W, KMAX>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    e = cudaFuncSetAttribute(rowpipe_kernel<T, OP, W, KMAX, RAG>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(rowpipe_kernel carve-out)");
     attr_set[dev] = true;
   }
-  rowpipe_kernel<T, OP, W, KMAX><<<grid, (W + 1) * 32, smem, st>>>(p);
+  rowpipe_kernel<T, OP, W, KMAX, RAG><<<grid, (W + 1) * 32, smem, st>>>(p);
   MCB_CHECK_LAUNCH("rowpipe_kernel");
   return MCB_OK;
 }
 
-template <typename T, int OP, int KMAX>
+template <typename T, int OP, int KMAX, bool RAG = false>
 int launch_w(int W, const Params& p, int grid, size_t smem, cudaStream_t st) {
   switch (W) {
-    case 16: return launch_one<T, OP, 16, KMAX>(p, grid, smem, st);
-    case 8: return launch_one<T, OP, 8, KMAX>(p, grid, smem, st);
-    case 4: return launch_one<T, OP, 4, KMAX>(p, grid, smem, st);
-    case 2: return launch_one<T, OP, 2, KMAX>(p, grid, smem, st);
+    case 16: return launch_one<T, OP, 16, KMAX, RAG>(p, grid, smem, st);
+    case 8: return launch_one<T, OP, 8, KMAX, RAG>(p, grid, smem, st);
+    case 4: return launch_one<T, OP, 4, KMAX, RAG>(p, grid, smem, st);
+    case 2: return launch_one<T, OP, 2, KMAX, RAG>(p, grid, smem, st);
   }
   return fail(MCB_ERR_UNSUPPORTED, "rowpipe: W=%d", W);
 }
@@ -597,9 +646,13 @@ int try_launch(int op, const void* in0, const void* in1, const void* w, void* ou
                int* dw_blocks, int64_t rows, int64_t D, float eps, int causal_seq, float scale, const DeviceState* ds,
                cudaStream_t st, const void* res) {
   constexpr int N = Vec16<T>::N;
-  if (D % N != 0 || D > (1 << 20)) return 1;
+  const bool softmax = op == kSmFwd || op == kSmBwd;
+  if (D > (1 << 20)) return 1;
+  const uintptr_t at0 = reinterpret_cast<uintptr_t>(in0), at1 = reinterpret_cast<uintptr_t>(in1 ? in1 : in0), ato = reinterpret_cast<uintptr_t>(out);
+  const bool rag = D % N != 0 || ((at0 | at1 | ato) & 15u) != 0;
+  if (rag && !(softmax && ((at0 ^ at1) & 15u) == 0 && ((at0 ^ ato) & 15u) == 0 && at0 % sizeof(T) == 0 && D >= 2 * N)) return 1;
   if (res != nullptr && (op != kRmsBwd || !aligned16(res))) return 1;
-  if (!aligned16(in0) || !aligned16(out) || (in1 && !aligned16(in1)) || (w && !aligned16(w))) return 1;
+  if (w && !aligned16(w)) return 1;
   const int n_streams = (op == kRmsBwd || op == kSmBwd) ? 2 : 1;
   const int64_t row_bytes = D * static_cast<int64_t>(sizeof(T));
   // RMSNorm with a weight keeps a float32 copy of it in shared memory, taken out of the stage budget
@@ -609,8 +662,10 @@ int try_launch(int op, const void* in0, const void* in1, const void* w, void* ou
   const int64_t budget = w_bytes + kSmemBudget <= per_cta ? kSmemBudget : per_cta - w_bytes;
   if (budget < kSmemBudget / 2) return 1;
   int W = 0, stages = 0;
+  // a tile's bytes per stream: its rows, or for ragged ones the granules that cover them
+  auto tile_bytes = [&](int rows_) { return rag ? (rows_ * row_bytes + 30) / 16 * 16 + 16 : rows_ * row_bytes; };
   for (int cand : {16, 8, 4, 2}) {
-    const int64_t stage_bytes = cand * row_bytes * n_streams;
+    const int64_t stage_bytes = tile_bytes(cand) * n_streams;
     const int s = static_cast<int>(budget / stage_bytes);
     if (s >= 3) { W = cand; stages = s > kMaxStages ? kMaxStages : s; break; }
   }
@@ -621,7 +676,7 @@ int try_launch(int op, const void* in0, const void* in1, const void* w, void* ou
   }
   // One warp per row only pays while enough warps fit: forward ops (one input stream, more arithmetic per
   // byte) want at least 8 rows per tile, backward ops at least 4; wider rows go to the register kernels.
-  const int nvec = static_cast<int>(D / N);
+  const int nvec = static_cast<int>(rag ? (D + 2 * N - 2) / N : D / N);
   // The RMSNorm backward of very wide rows (only 2 rows fit a stage) gives every row 4 warps, each with a
   // contiguous segment of the row; the warps of a row exchange their two sums through shared memory.
   // (Measured: at 4 rows per stage, 2 warps per row are slower than one.)
@@ -639,7 +694,7 @@ int try_launch(int op, const void* in0, const void* in1, const void* w, void* ou
     if (kmax * N >= 32 && W > 8) {
       // 32 or more elements per lane: eight rows per tile and two CTAs per SM keep the register file from spilling
       W = 8;
-      const int sN = static_cast<int>(budget / (W * row_bytes * n_streams));
+      const int sN = static_cast<int>(budget / (tile_bytes(W) * n_streams));
       stages = sN > kMaxStages ? kMaxStages : sN;
     }
   }
@@ -655,7 +710,9 @@ int try_launch(int op, const void* in0, const void* in1, const void* w, void* ou
   p.rows = rows; p.D = static_cast<int>(D); p.nvec = nvec; p.row_bytes = static_cast<int>(row_bytes);
   p.stages = stages; p.n_streams = n_streams; p.wpr = wpr; p.causal_seq = causal_seq; p.eps = eps; p.scale = scale;
   p.status = ds->status_word;
-  p.stage_bytes = static_cast<uint32_t>(R * row_bytes * n_streams);
+  p.mis = rag ? static_cast<int>((at0 & 15u) / sizeof(T)) : 0;
+  p.stream_bytes = static_cast<uint32_t>(tile_bytes(R));
+  p.stage_bytes = p.stream_bytes * n_streams;
   p.bar_off = (static_cast<uint32_t>(stages) * p.stage_bytes + 127u) & ~127u;
   size_t smem = p.bar_off + 16 * kMaxStages + 16 + 128;
   p.w_off = 0;
@@ -667,6 +724,17 @@ int try_launch(int op, const void* in0, const void* in1, const void* w, void* ou
   int grid = 2 * ds->sm_count;
   if (grid > n_tiles) grid = static_cast<int>(n_tiles);
   if (dw_blocks) *dw_blocks = grid;
+  if (rag) {
+    if (op == kSmBwd) return launch_w<T, kSmBwd, 0, true>(W, p, grid, smem, st);
+    switch (kmax) {
+      case 0: return launch_w<T, kSmFwd, 0, true>(W, p, grid, smem, st);
+      case 1: return launch_w<T, kSmFwd, 1, true>(W, p, grid, smem, st);
+      case 2: return launch_w<T, kSmFwd, 2, true>(W, p, grid, smem, st);
+      case 4: return launch_w<T, kSmFwd, 4, true>(W, p, grid, smem, st);
+      case 8: return launch_w<T, kSmFwd, 8, true>(W, p, grid, smem, st);
+    }
+    return 1;
+  }
 #define MCB_RP(OPC, KM) return launch_w<T, OPC, KM>(W, p, grid, smem, st)
   switch (op) {
     case kRmsFwd:

@@ -181,6 +181,7 @@ extern "C" {
     pub fn mcb_swiglu_bwd(gate: *const c_void, up: *const c_void, dout: *const c_void, dgate: *mut c_void, dup: *mut c_void, n: i64, dtype: c_int, stream: *mut c_void) -> c_int;
     pub fn mcb_add(a: *const c_void, b: *const c_void, out: *mut c_void, n: i64, dtype: c_int, stream: *mut c_void) -> c_int;
     pub fn mcb_cross_entropy(logits: *mut c_void, targets: *const i32, nll: *mut f32, count: *mut i32, loss: *mut f32, M: i64, V: i64, write_grad: c_int, dtype: c_int, stream: *mut c_void) -> c_int;
+    pub fn mcb_cross_entropy_out(logits: *const c_void, dlogits: *mut c_void, targets: *const c_void, target_bytes: c_int, has_ignore: c_int, ignore_index: i64, t32: *mut i32, info: *mut i32, info_host: *mut i32, info_event: *mut c_void, nll: *mut f32, loss: *mut f32, M: i64, V: i64, dtype: c_int, stream: *mut c_void) -> c_int;
     pub fn mcb_cross_entropy_count(targets: *const i32, count: *mut i32, M: i64, V: i64, stream: *mut c_void) -> c_int;
     pub fn mcb_cross_entropy_chunk(logits: *mut c_void, targets: *const i32, nll: *mut f32, count: *const i32, rows: i64, V: i64, write_grad: c_int, dtype: c_int, stream: *mut c_void) -> c_int;
     pub fn mcb_cross_entropy_finish(nll: *const f32, count: *const i32, loss: *mut f32, M: i64, stream: *mut c_void) -> c_int;

@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+import threading
 from dataclasses import dataclass, field
 from enum import Enum
 from typing import Callable, Dict, Iterable, List, Optional, Tuple
@@ -433,6 +434,21 @@ class StepMetrics:
 IGNORE_INDEX = 0xFFFFFFFF  # u32::MAX, what TrainingStep passes (src/training/trainer.rs:385)
 
 
+_check_slots = threading.local()
+
+
+def _target_check(device):
+    """Page-locked room for the two target counts of a loss and an event behind their copy, one pair per thread and
+    device: a call waits for its own counts before it returns, so the pair is free again for the next one."""
+    slots = _check_slots.__dict__
+    got = slots.get(device.index)
+    if got is None:
+        event = torch.cuda.Event()
+        event.record(torch.cuda.current_stream(device))
+        got = slots[device.index] = (torch.zeros(2, dtype=torch.int32, pin_memory=True), event)
+    return got
+
+
 def cross_entropy_loss(logits: torch.Tensor, targets: torch.Tensor, ignore_index: Optional[int] = None,
                        return_grad: bool = False):
     """cross_entropy_loss (src/training/loss.rs:58-147): mean over non-ignored tokens of
@@ -445,24 +461,28 @@ def cross_entropy_loss(logits: torch.Tensor, targets: torch.Tensor, ignore_index
         raise InvalidConfig(f"targets must be 2D (batch, seq_len), got shape {list(ts)}")
     if ls[0] != ts[0] or ls[1] != ts[1]:
         raise InvalidConfig(f"logits and targets batch/seq_len mismatch: logits {list(ls[:2])} vs targets {list(ts)}")
-    backend._require_cuda(logits.contiguous(), targets.contiguous())
+    work, t = logits.contiguous(), targets.contiguous()
+    backend._require_cuda(work, t)
+    if t.dtype not in (torch.int64, torch.int32):
+        t = t.to(torch.int64)
     M, V = ls[0] * ls[1], ls[2]
-    t = targets.contiguous().view(-1).to(torch.int64)
-    if ignore_index is not None:
-        t = torch.where(t == ignore_index, torch.full_like(t, -1), t)
-    if bool(((t >= V) | ((t < 0) & (t != -1))).any()):
+    lib, dt, dev = backend._lib_for(work), backend._dtype_code(work), work.device
+    grad = torch.empty_like(work) if return_grad else None
+    scratch = torch.empty(2 * M + 3, dtype=torch.int32, device=dev)   # targets as int32, their counts, the rows' losses
+    t32, info, nll = scratch[:M], scratch[M:M + 3], scratch[M + 3:]
+    loss = torch.empty(2, dtype=torch.float32, device=dev)
+    host, checked = _target_check(dev)
+    _lib.check(lib.mcb_cross_entropy_out(work.data_ptr(), backend._ptr(grad), t.data_ptr(), t.element_size(), int(ignore_index is not None),
+                                         int(ignore_index or 0), t32.data_ptr(), info.data_ptr(), host.data_ptr(),
+                                         checked.cuda_event, nll.data_ptr(), loss.data_ptr(), M, V, dt, backend._stream()))
+    # the counts arrive ahead of the loss itself: wait for them alone
+    checked.synchronize()
+    kept, bad = host.tolist()
+    if bad:
         raise TrainingError(f"target index out of range for vocab size {V}")
-    t32 = t.to(torch.int32)
-    work = logits.contiguous().clone() if return_grad else logits.contiguous()
-    lib = backend._lib_for(work)
-    nll = torch.empty(M, dtype=torch.float32, device=work.device)
-    count = torch.empty(1, dtype=torch.int32, device=work.device)
-    loss = torch.empty(2, dtype=torch.float32, device=work.device)
-    _lib.check(lib.mcb_cross_entropy(work.data_ptr(), t32.data_ptr(), nll.data_ptr(), count.data_ptr(), loss.data_ptr(),
-                                     M, V, int(return_grad), backend._dtype_code(work), backend._stream()))
-    if int(count.item()) == 0:
+    if kept == 0:
         raise InvalidConfig("all tokens are ignored, cannot compute loss")
-    return (loss[:1], work) if return_grad else loss[:1]
+    return (loss[:1], grad) if return_grad else loss[:1]
 
 
 class TrainingStep:

@@ -63,3 +63,84 @@ def test_delta_edges(cuda_device, dtype, M, K, N, r):
     got = B.lora_forward_fused(dev_t(x, dtype, cuda_device), dev_t(c["A"], torch.float32, cuda_device), dev_t(c["B"], torch.float32, cuda_device), 2.0)
     want, _ = R.lora_forward(x, rounded(c["A"], dtype), rounded(c["B"], dtype), 2.0)
     assert R.max_abs_normalised(back(got), want) <= TOL[dtype]
+
+
+# rows that are no whole 16-byte vectors (one bulk copy of the granules that cover a tile, edge elements one per lane): every
+# misalignment, register-resident and streamed widths, the causal form, tensors that start off a 16-byte boundary
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,D", [(64, 17), (70, 63), (333, 257), (130, 777), (90, 1023), (66, 2049), (3, 777), (64, 5001)])
+@pytest.mark.parametrize("shift", [0, 3])
+def test_softmax_ragged_rows(cuda_device, dtype, rows, D, shift):
+    from metal_candle_b200 import backend as B
+
+    def put(a):   # the values of `a` in a tensor that starts `shift` elements into an allocation
+        buf = torch.full((a.size + shift + 8,), float("nan"), dtype=dtype, device=cuda_device)
+        view = buf[shift:shift + a.size].view(a.shape)
+        view.copy_(torch.from_numpy(np.ascontiguousarray(a)).to(cuda_device).to(dtype))
+        return view, buf
+
+    x, dy = rounded(S.normal(41, "x", (rows, D)) * 3, dtype), rounded(S.normal(41, "dy", (rows, D)), dtype)
+    (xt, _), (dyt, _), (yt, ybuf), (dxt, dxbuf) = put(x), put(dy), put(x * 0), put(x * 0)
+    want = R.softmax_stable(x.astype(np.float64))
+    B.softmax_fused(xt, out=yt)
+    assert R.max_abs_normalised(back(yt), want) <= TOL[dtype]
+    B.softmax_backward(yt, dyt, out=dxt)
+    y = back(yt).astype(np.float64)
+    assert R.max_abs_normalised(back(dxt), y * (dy - (dy * y).sum(-1, keepdims=True))) <= TOL[dtype]
+    for buf in (ybuf, dxbuf):   # nothing outside the rows was written
+        assert torch.isnan(buf[:shift]).all() and torch.isnan(buf[shift + rows * D:]).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("seq", [65, 777, 1031, 2049])
+def test_softmax_causal_ragged_rows(cuda_device, dtype, seq):
+    from metal_candle_b200 import _lib, backend as B
+
+    x, dy = (rounded(S.normal(42, n, (2, seq, seq)), dtype) for n in ("x", "dy"))
+    mask = np.triu(np.full((seq, seq), -np.inf), 1)
+    xt, dyt = dev_t(x, dtype, cuda_device), dev_t(dy, dtype, cuda_device)
+    y, dx = torch.full_like(xt, float("nan")), torch.full_like(xt, float("nan"))
+    lib = _lib.load()
+    code, st = B._dtype_code(xt), torch.cuda.current_stream().cuda_stream
+    _lib.check(lib.mcb_softmax_causal_fwd(xt.data_ptr(), y.data_ptr(), 2 * seq, seq, seq, 0.5, code, st))
+    want = R.softmax_stable(0.5 * x.astype(np.float64) + mask)
+    assert R.max_abs_normalised(back(y), want) <= TOL[dtype]
+    _lib.check(lib.mcb_softmax_causal_bwd(y.data_ptr(), dyt.data_ptr(), dx.data_ptr(), 2 * seq, seq, seq, 0.5, code, st))
+    yf = back(y).astype(np.float64)
+    assert R.max_abs_normalised(back(dx), 0.5 * yf * (dy - (dy * yf).sum(-1, keepdims=True))) <= TOL[dtype]
+    assert np.all(back(dx)[:, np.triu_indices(seq, 1)[0], np.triu_indices(seq, 1)[1]] == 0)
+
+
+# the loss: short rows (block kernel), rows over 1, 2, 4 and 8 CTAs, rows that are no whole vectors, more rows than clusters,
+# ignored targets, int32 and int64 targets
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,V,tdtype", [(5, 50, torch.int64), (3, 8192, torch.int32), (700, 8193, torch.int64), (90, 50257, torch.int32),
+                                           (160, 60001, torch.int64), (40, 151936, torch.int64)])
+def test_cross_entropy_rows(cuda_device, dtype, rows, V, tdtype):
+    from metal_candle_b200 import _lib
+    from metal_candle_b200.training import cross_entropy_loss
+
+    x = rounded(S.normal(43, "x", (1, rows, V)) * 2, dtype)
+    t = np.random.default_rng(7).integers(0, V, (1, rows))
+    t[0, 0], t[0, -1], t[0, 1] = 0, V - 1, -1
+    if rows > 20:
+        t[0, 7:12] = -1
+    xt = dev_t(x, dtype, cuda_device)
+    before = xt.clone()
+    loss, grad = cross_entropy_loss(xt, torch.from_numpy(t).to(cuda_device).to(tdtype), ignore_index=-1, return_grad=True)
+    assert torch.equal(xt, before)
+    x64 = x[0].astype(np.float64)
+    lse = np.log(np.exp(x64 - x64.max(-1, keepdims=True)).sum(-1)) + x64.max(-1)
+    keep = t[0] >= 0
+    nll = lse[keep] - x64[keep, t[0][keep]]
+    assert abs(float(loss) - nll.mean()) <= 1e-5 * abs(nll.mean())   # float32 sums of exponentials of 2^-22 each
+    want = np.where(keep[:, None], np.exp(x64 - lse[:, None]), 0.0)
+    want[np.nonzero(keep)[0], t[0][keep]] -= 1.0
+    assert R.max_abs_normalised(back(grad)[0], want / keep.sum()) <= TOL[dtype]
+    # the in-place form of the training step
+    tg = torch.from_numpy(t[0].astype(np.int32)).to(cuda_device)
+    nl, cnt, ls = torch.empty(rows, device=cuda_device), torch.empty(1, dtype=torch.int32, device=cuda_device), torch.empty(2, device=cuda_device)
+    _lib.check(_lib.load().mcb_cross_entropy(xt.data_ptr(), tg.data_ptr(), nl.data_ptr(), cnt.data_ptr(), ls.data_ptr(), rows, V, 1,
+                                             0 if dtype == torch.float32 else 1, torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(xt, grad) and float(ls[0]) == float(loss) and int(cnt) == int(keep.sum())
+    assert _lib.device_status() == 0
