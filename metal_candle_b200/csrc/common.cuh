@@ -26,6 +26,7 @@ struct DeviceState {
   bool f32_tile_smem = false;  // the float32 tile kernel's shared-memory limit has been raised
   bool ce_smem[2] = {false, false};  // the same of the cross-entropy cluster kernel (bf16, float32)
   int ce_clusters[2][9] = {};  // its resident clusters, by dtype and cluster size; 0 = not asked yet
+  int split_clusters[9] = {};  // clusters of the split GEMM kernel the device runs at once, by cluster size
   void* encode_tiled = nullptr;  // cuTensorMapEncodeTiled resolved through the runtime
 };
 DeviceState* current_device_state();  // null (and error set) when mcb_init was not called

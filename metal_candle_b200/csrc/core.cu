@@ -51,7 +51,7 @@ DeviceState* current_device_state() {
   return &g_dev[dev];
 }
 
-int init_gemm_kernels();  // umma_gemm.cu: raises dynamic shared-memory limits
+int init_gemm_kernels(DeviceState* ds);  // umma_gemm.cu: raises dynamic shared-memory limits
 
 // ---- per-kernel timing -----------------------------------------------------------------------------
 namespace {
@@ -123,7 +123,7 @@ extern "C" int mcb_init(int device) {
   if (fn == nullptr || qres != cudaDriverEntryPointSuccess)
     return fail(MCB_ERR_UNSUPPORTED, "mcb_init: driver does not export cuTensorMapEncodeTiled");
   st.encode_tiled = fn;
-  if (int rc = init_gemm_kernels()) return rc;
+  if (int rc = init_gemm_kernels(&st)) return rc;
   st.ready = true;
   std::lock_guard<std::mutex> lk(g_mu);
   g_dev[device] = st;

@@ -228,7 +228,7 @@ cross_entropy_cluster_kernel(const CeParams p) {
   cl.sync();   // every CTA's barriers exist before a peer arrives on them
   const float inv_count = 1.0f / static_cast<float>(max(1, *p.count));
   const T* in = static_cast<const T*>(p.in) - p.mis;    // 16-byte boundaries
-  T* out = static_cast<T*>(p.out) - p.mis;
+  T* out = static_cast<T*>(p.out) - p.mis;              // (not touched without write_grad)
   // this CTA's share of a row: vectors [v_begin, v_end) counted from the boundary
   auto share = [&](int64_t row, int64_t& v_begin, int& n) {
     const int64_t e0 = row * p.V + p.mis, v0 = e0 / N, v1 = (e0 + p.V + N - 1) / N;
@@ -479,18 +479,20 @@ prepare_targets_kernel(const I* __restrict__ targets, int32_t* __restrict__ t32,
   if (threadIdx.x == 2) info[2] = 0;   // the row kernel's count of finished CTAs
 }
 
-// Row kernel launch: in -> out (which may be the same tensor).
+// Row kernel launch: in -> out (which may be the same tensor); out is null when no gradient is wanted.
 template <typename T>
 int launch_rows(const void* in, void* out, const int32_t* targets, float* nll, const int32_t* count, int64_t M, int64_t V, int write_grad,
                 float* loss, int* done, DeviceState* ds, cudaStream_t st) {
   constexpr int N = Vec16<T>::N;
-  const uintptr_t ai = reinterpret_cast<uintptr_t>(in), ao = reinterpret_cast<uintptr_t>(out);
+  const uintptr_t ai = reinterpret_cast<uintptr_t>(in), ao = reinterpret_cast<uintptr_t>(out ? out : in);
   const int64_t row_vecs = (V + 2 * N - 2) / N;   // vectors that cover a row at most
   int ctas = 1;
   while (ctas < 8 && (row_vecs + ctas - 1) / ctas * 16 > kCeGoodBytes) ctas *= 2;
   const int64_t cta_vecs = (row_vecs + ctas - 1) / ctas;
+  // In place (the training step, a chunk of tokens at a time) the block kernel stays, although it is 12 % slower there: its
+  // order of summation is what the step's losses and gradients have been reproducible with.
   // 16 KB: below that a CTA's 384 lanes have two or three vectors each and the per-row exchanges dominate
-  if (row_vecs * 16 >= 16 * 1024 && cta_vecs * 16 <= kCeMaxBytes && ((ai ^ ao) & 15u) == 0 && ai % sizeof(T) == 0) {
+  if (in != out && row_vecs * 16 >= 16 * 1024 && cta_vecs * 16 <= kCeMaxBytes && ((ai ^ ao) & 15u) == 0 && ai % sizeof(T) == 0) {
     CeParams p;
     p.in = in; p.out = out; p.targets = targets; p.nll = nll; p.count = count;
     p.M = M; p.V = static_cast<int>(V); p.write_grad = write_grad; p.mis = static_cast<int>((ai & 15u) / sizeof(T));
@@ -612,6 +614,6 @@ extern "C" int mcb_cross_entropy_out(const void* logits, void* dlogits, const vo
   MCB_CHECK_LAUNCH("prepare_targets");
   if (info_event != nullptr) MCB_CHECK_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(info_event), st));
   const bool grad = dlogits != nullptr;
-  if (int rc = launch_rows(logits, grad ? dlogits : const_cast<void*>(logits), t32, nll, info, M, V, grad ? 1 : 0, dtype, loss, info + 2, ds, st)) return rc;
+  if (int rc = launch_rows(logits, dlogits, t32, nll, info, M, V, grad ? 1 : 0, dtype, loss, info + 2, ds, st)) return rc;
   return MCB_OK;
 }

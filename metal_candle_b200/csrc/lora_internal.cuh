@@ -88,6 +88,14 @@ struct GemmCall {
   // up by d gate and d up instead of storing it (pair kernel only).
   __nv_bfloat16* swiglu_up = nullptr;
 };
+// Tile width and reduction parts of the split-reduction kernel (umma_split.cu); bn == 0: the persistent kernels run.
+struct SplitPlan {
+  int bn = 0, splits = 1;
+};
+SplitPlan split_plan(int64_t M, int64_t N, int64_t K, int rp, bool pair_kernel, const DeviceState* ds);
+// Runs the call with that plan; with act != null its columns are blocks of 128 gate and 128 up features (bn 256) and c.Y,
+// up, act receive gate, up and silu(gate) * up.
+int launch_split(const SplitPlan& plan, const GemmCall& c, __nv_bfloat16* up, __nv_bfloat16* act, const DeviceState* ds, cudaStream_t st);
 size_t workspace_bytes(int64_t M, int64_t K, int64_t N, int64_t r);
 int delta_fwd(const LoraArgs& a, const DeviceState* ds);
 int linear_fwd(const LoraArgs& a, const DeviceState* ds);

@@ -41,6 +41,7 @@ using namespace umma;
 
 int init_grad_kernel();
 int init_gemm2_kernel();
+int init_split_kernel(DeviceState* ds);
 bool gemm2_eligible(const GemmCall& c);
 int launch_gemm2(const GemmCall& c, const DeviceState* ds, cudaStream_t st);
 size_t grad_partial_bytes(int64_t M, int64_t K, int64_t N, int rp);
@@ -594,6 +595,17 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
                 (long long)c.K, (long long)c.N);
   if (!aligned16(c.X) || (c.W && !aligned16(c.W)) || (c.Y && !aligned16(c.Y)) || (c.H && !aligned16(c.H)) || (c.R && !aligned16(c.R)))
     return fail(MCB_ERR_ALIGN, "bf16 path needs 16-byte aligned matrices");
+  // shapes with too few tiles to fill the chip: narrower tiles, reduction in parts (umma_split.cu)
+  if (c.W != nullptr && c.Y != nullptr && c.swiglu_up == nullptr) {
+    const SplitPlan sp = split_plan(c.M, c.N, c.K, c.rp, gemm2_eligible(c), ds);
+    if (sp.bn > 0) {
+      if (int rc = launch_split(sp, c, nullptr, nullptr, ds, st)) return rc;
+      if (c.grads == nullptr) return MCB_OK;
+      const GradRequest& q = *c.grads;
+      return launch_grad2(q.X[0], q.Ht[0], q.C[0], q.out[0], q.transposed[0], q.X[1], q.Ht[1], q.C[1], q.out[1], q.transposed[1],
+                          q.h_pitch, q.part, c.M, q.r, c.rp, q.accumulate, ds, st);
+    }
+  }
   // linears of useful size (with or without the rank path) run on CTA pairs (umma_gemm2.cu)
   if (gemm2_eligible(c)) return launch_gemm2(c, ds, st);
   GemmParams p;
@@ -753,10 +765,11 @@ int check_ws(const LoraArgs& a, const char* op) {
 
 }  // namespace
 
-int init_kernels() {
+int init_kernels(DeviceState* ds) {
   cudaError_t e = cudaFuncSetAttribute(lora_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget + 1024);
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(lora_gemm_kernel)");
   if (int rc = init_gemm2_kernel()) return rc;
+  if (int rc = init_split_kernel(ds)) return rc;
   return init_grad_kernel();
 }
 
@@ -1049,6 +1062,6 @@ int matmul_nt(const void* a, const void* bt, void* out, int64_t M, int64_t K, in
 
 }  // namespace bf16path
 
-int init_gemm_kernels() { return bf16path::init_kernels(); }
+int init_gemm_kernels(DeviceState* ds) { return bf16path::init_kernels(ds); }
 
 }  // namespace mcb

@@ -138,14 +138,6 @@ __device__ __forceinline__ void swiglu_bwd_pair(float2 d, float2 g, float2 u, fl
   dgate = __ffma2_rn(tu, q, tu);
 }
 
-// silu(g) * u with the same two flushing special functions (5 instructions)
-__device__ __forceinline__ float silu_mul(float g, float u) {
-  float e, s;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-1.4426950408889634f * g));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(1.0f + e));
-  return g * s * u;
-}
-
 __device__ __forceinline__ void tile_coords2(const Gemm2Params& p, int t, int& mt, int& nt) {
   const int per_band = p.group_m * p.num_n_tiles;
   const int band = t / per_band;
@@ -720,6 +712,14 @@ int launch_gemm2_swiglu(const __nv_bfloat16* X, const __nv_bfloat16* Wgu, __nv_b
                         __nv_bfloat16* Act, int64_t M, int64_t K, int64_t F, const DeviceState* ds, cudaStream_t st) {
   if (F % 128 != 0 || K % 8 != 0) return fail(MCB_ERR_ALIGN, "linear_swiglu: features %lld must be a multiple of 128, reduction %lld of 8", (long long)F, (long long)K);
   if (M > 0x7fffff00ll || 2 * F > 0x7fffff00ll || K > 0x7fffff00ll) return fail(MCB_ERR_SHAPE, "linear_swiglu: dimension exceeds 2^31");
+  // up to one round of 128-token tiles over the SMs, one-CTA tiles (umma_split.cu) end earlier than 256-token pairs
+  if ((M + 127) / 128 * (F / 128) <= ds->sm_count) {
+    GemmCall c;
+    c.X = X; c.W = Wgu; c.Y = G; c.M = M; c.N = 2 * F; c.K = K;
+    SplitPlan sp;
+    sp.bn = 256;
+    return launch_split(sp, c, U, Act, ds, st);
+  }
   Gemm2Params p;
   memset(&p, 0, sizeof(p));
   p.M = static_cast<int>(M); p.N = static_cast<int>(2 * F); p.K = static_cast<int>(K);

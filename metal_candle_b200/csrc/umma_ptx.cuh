@@ -172,6 +172,14 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
+// silu(g) * u with flushing approximate special functions (5 instructions; relative error about 2^-22)
+__device__ __forceinline__ float silu_mul(float g, float u) {
+  float e, s;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-1.4426950408889634f * g));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(1.0f + e));
+  return g * s * u;
+}
+
 // Output staging of the GEMM epilogues: per epilogue warp, up to kEpiBufsMax buffers of 32 rows x 64 bytes
 // (32 bf16 columns), rows swizzled in 16-byte units as CU_TENSOR_MAP_SWIZZLE_64B expects.
 constexpr int kEpiBufsMax = 3;
