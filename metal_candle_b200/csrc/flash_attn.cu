@@ -31,8 +31,12 @@
 #include <cuda.h>
 #include <string.h>
 
+#include <cooperative_groups.h>
+
 #include "lora_internal.cuh"
 #include "umma_ptx.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace mcb {
 namespace attn {
@@ -405,6 +409,7 @@ struct BwdParams {
   __nv_bfloat16* dQ;
   __nv_bfloat16* dK;
   __nv_bfloat16* dV;
+  int kv_parts;   // CTAs of a cluster that share the query steps of one key block (dK / dV kernel)
   int* status;
 };
 
@@ -665,12 +670,14 @@ attn_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 // ---------------------------------------------------------------------------------------------------------
 // backward, part 2: dK, dV
 // ---------------------------------------------------------------------------------------------------------
-// One CTA per SM: 2 control warps + 8 element-wise warps (two per tensor-memory lane quadrant, 32 of the 64 query
-// columns each; no row reductions are needed here because the log-sum-exp is known).  Loads are double-buffered,
-// S^T / dP^T are double-buffered in tensor memory and so are P^T / dS^T (bf16 pairs, handed to the dV / dK products
-// as tensor-memory A operands), so the tensor core computes the next step's S^T, dP^T while the element-wise
-// warps work on the current one.
-constexpr int kKvThreads = 320;
+// One CTA per SM: 2 control warps + two groups of 8 element-wise warps (two per tensor-memory lane quadrant, 32 of the
+// 64 query columns each; no row reductions are needed here because the log-sum-exp is known).  S^T / dP^T are
+// double-buffered in tensor memory and so are P^T / dS^T (bf16 pairs, handed to the dV / dK products as tensor-memory A
+// operands); the groups take the steps in turn, one buffer each.  A step is a chain (wait, tensor-memory loads,
+// exponentials, tensor-memory stores, wait); with one group every second of its links was exposed: 16 kv heads x 7
+// query heads x 1024 positions, whole kernel: 117 us with one group, 109 with two.  (K and V as tensor-memory operands
+// instead of shared-memory ones made no difference: 167 against 169 us for the whole backward pass.)
+constexpr int kKvThreads = 576;
 constexpr uint32_t kKvOffK = 0;                       // K block [128 keys x 64]
 constexpr uint32_t kKvOffV = kKvOffK + kQBytes;
 constexpr int kKvStages = 4;
@@ -679,6 +686,7 @@ constexpr uint32_t kKvStageBytes = 2 * kKBytes + 512;
 constexpr uint32_t kKvStageStride = 2 * kKBytes + 1024;
 constexpr uint32_t kKvOffBar = kKvOffStage + kKvStages * kKvStageStride;
 constexpr uint32_t kKvSmem = kKvOffBar + 256 + 1024;
+static_assert(2 * kBQ * kD * 4 <= kKvStages * kKvStageStride, "the parts' sums reuse the load ring");
 
 __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -721,20 +729,24 @@ attn_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
   // of bf16 pairs) and dS^T (32): 384 / 416 and 448 / 480
   const uint32_t tDV = tmem_base + 256, tDK = tmem_base + 320, tPT0 = tmem_base + 384;
 
-  const int kb = blockIdx.y, nb = blockIdx.x;   // all kv heads of key block 0 (the most query steps) start first
+  // all kv heads of key block 0 (the most query steps) start first
+  const int kb = blockIdx.y, part = blockIdx.x % p.kv_parts, nb = blockIdx.x / p.kv_parts;
   const int nq = p.S / kBK;                      // query steps of 64 per head
   const int i0 = 2 * kb;                         // first query step that sees this key block
   const int per_head = nq - i0;
-  const int nsteps = p.G * per_head;
+  // this CTA's steps [t0, t0 + nsteps) of the key block's G * per_head; a part may be empty
+  const int all_steps = p.G * per_head;
+  const int t0 = static_cast<int>(static_cast<int64_t>(all_steps) * part / p.kv_parts);
+  const int nsteps = static_cast<int>(static_cast<int64_t>(all_steps) * (part + 1) / p.kv_parts) - t0;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (lane == 0 && nsteps > 0) {
       mbar_expect_tx(kv_full, 2 * kQBytes);
       tma_load_2d(base + kKvOffK, &tmK, kv_full, 0, nb * p.S + kb * kBQ);
       tma_load_2d(base + kKvOffV, &tmV, kv_full, 0, nb * p.S + kb * kBQ);
       for (int t = 0; t < nsteps; ++t) {
         const int st = t % kKvStages;
-        const int g = t / per_head, i = i0 + t % per_head;
+        const int g = (t0 + t) / per_head, i = i0 + (t0 + t) % per_head;
         if (!mbar_wait(ld_empty0 + 8 * st, ((t / kKvStages) & 1) ^ 1, abort_flag, 91, p.status)) break;
         const int64_t qrow = (static_cast<int64_t>(nb) * p.G + g) * p.S + static_cast<int64_t>(i) * kBK;
         const uint32_t sb = base + kKvOffStage + st * kKvStageStride, fb = ld_full0 + 8 * st;
@@ -767,7 +779,7 @@ attn_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
         }
         umma_commit(sdp_full0 + 8 * st);
       };
-      bool ok = mbar_wait(kv_full, 0, abort_flag, 92, p.status);
+      bool ok = nsteps > 0 && mbar_wait(kv_full, 0, abort_flag, 92, p.status);
       if (ok) ok = mbar_wait(ld_full0, 0, abort_flag, 93, p.status);
       if (ok) {
         tcgen05_fence_after();
@@ -805,14 +817,15 @@ attn_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     }
   } else {
     const int quad = warp & 3;            // tensor-memory lane quadrant of this warp
-    const int half = (warp - 2) >> 2;     // which 32 of the 64 query columns
+    const int half = ((warp - 2) >> 2) & 1;   // which 32 of the 64 query columns
+    const int group = (warp - 2) >> 3;        // which steps: even or odd
     const int row = quad * 32 + lane;
     const int key = kb * kBQ + row;
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
     bool ok = true;
-    for (int t = 0; t < nsteps; ++t) {
-      const int st = t & 1;
-      const int i = i0 + t % per_head;
+    for (int t = group; t < nsteps; t += 2) {
+      const int st = group;
+      const int i = i0 + (t0 + t) % per_head;
       ok = __all_sync(0xffffffffu, mbar_wait(sdp_full0 + 8 * st, (t >> 1) & 1, abort_flag, 95, p.status));
       if (!ok) break;
       tcgen05_fence_after();
@@ -858,20 +871,23 @@ attn_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
       __syncwarp();
       if (lane == 0) mbar_arrive(pds_ready0 + 8 * (t & 1));
     }
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(out_full, 0, abort_flag, 96, p.status));
+    if (ok && nsteps > 0) ok = __all_sync(0xffffffffu, mbar_wait(out_full, 0, abort_flag, 96, p.status));
     if (ok) {
       tcgen05_fence_after();
-      const int64_t krow = static_cast<int64_t>(nb) * p.S + key;
+      __nv_bfloat16* orow = (group == 0 ? p.dV : p.dK) + (static_cast<int64_t>(nb) * p.S + key) * kD;   // group 0 writes dV, 1 dK
+      const float f = group == 0 ? 1.0f : p.scale;
 #pragma unroll
-      for (int which = 0; which < 2; ++which) {
-        __nv_bfloat16* orow = (which == 0 ? p.dV : p.dK) + krow * kD;
-        const float f = which == 0 ? 1.0f : p.scale;
+      for (int cb = 0; cb < 32; cb += 16) {
+        const int c = half * 32 + cb;
+        uint32_t v[16];
+        tmem_ld_x16((group == 0 ? tDV : tDK) + lane_addr + c, v);
+        tmem_ld_wait();
+        if (p.kv_parts > 1) {
+          // this part's sums, column by column, into the load ring (every step's tiles have been read)
+          float* at = reinterpret_cast<float*>(gen_base + kKvOffStage) + (group * kD + c) * kBQ + row;
 #pragma unroll
-        for (int cb = 0; cb < 32; cb += 16) {
-          const int c = half * 32 + cb;
-          uint32_t v[16];
-          tmem_ld_x16((which == 0 ? tDV : tDK) + lane_addr + c, v);
-          tmem_ld_wait();
+          for (int e = 0; e < 16; ++e) at[e * kBQ] = nsteps > 0 ? __uint_as_float(v[e]) : 0.0f;
+        } else {
           uint32_t w[8];
 #pragma unroll
           for (int e = 0; e < 16; e += 2) w[e >> 1] = pack_bf16(__uint_as_float(v[e]) * f, __uint_as_float(v[e + 1]) * f);
@@ -880,6 +896,31 @@ attn_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
         }
       }
     }
+  }
+
+  if (p.kv_parts > 1) {
+    // each CTA of the cluster adds up its share of the key rows from all parts, in their order
+    __syncwarp();
+    cg::cluster_group cl = cg::this_cluster();
+    cl.sync();
+    if (warp >= 2) {
+      const int rows = kBQ / p.kv_parts, cols = kD / p.kv_parts / 2;   // rows of this CTA, columns of a thread
+      const int e = threadIdx.x - 64;
+      const int row = part * rows + e % rows, c0 = e / rows * cols;    // columns 0..63 are dV, 64..127 dK
+      const float* src = reinterpret_cast<const float*>(gen_base + kKvOffStage) + c0 * kBQ + row;
+      const float f = c0 < kD ? 1.0f : p.scale;
+      __nv_bfloat16* orow = (c0 < kD ? p.dV : p.dK) + (static_cast<int64_t>(nb) * p.S + kb * kBQ + row) * kD + (c0 & (kD - 1));
+      for (int c = 0; c < cols; c += 4) {
+        float a[4] = {};
+        for (int q = 0; q < p.kv_parts; ++q) {
+          const float* peer = cl.map_shared_rank(src, q) + c * kBQ;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) a[k] += peer[k * kBQ];
+        }
+        *reinterpret_cast<uint2*>(orow + c) = make_uint2(pack_bf16(a[0] * f, a[1] * f), pack_bf16(a[2] * f, a[3] * f));
+      }
+    }
+    cl.sync();   // no CTA leaves while another reads its sums
   }
 
   __syncwarp();
@@ -920,6 +961,28 @@ int check_shape(const char* who, int64_t nb, int64_t groups, int64_t seq, int64_
   if (nb <= 0 || groups <= 0 || nb > 65535 || groups > 65535) return fail(MCB_ERR_SHAPE, "%s: nb=%lld groups=%lld", who, (long long)nb, (long long)groups);
   if (nb * groups * seq > 0x7fffff00ll) return fail(MCB_ERR_SHAPE, "%s: more than 2^31 query rows", who);
   return MCB_OK;
+}
+
+// How many CTAs of a cluster share a key block's query steps.  One CTA per key block ends with the CTAs of the first key
+// block, which have all G * nq steps; parts shorten that chain, but each costs a CTA's start, its exchange and the wait for
+// a cluster's worth of free SMs.  The launch takes about the longer of one part and an SM's share of all steps and parts.
+// Whole backward pass with 1 / 2 / 4 / 8 parts, us (kv heads x query heads each x positions):
+//   16 x 7 x 1024: 169 / 126 / 147 / 203    8 x 7 x 512: 76 / 53 / 40 / 56    2 x 7 x 2048: 258 / 154 / 101 / 98
+//   32 x 7 x 2048: 709 / 744 / 856 / 1103   64 x 7 x 256: 69 / 72 / 84 / 137  4 x 7 x 4096: 579 / 366 / 391 / 464
+// the rule takes the fastest of each.
+int dkv_parts(int64_t nb, int64_t groups, int64_t seq, int sms) {
+  const double cost[4] = {3.0, 8.0, 10.0, 13.0};   // of a CTA with 1, 2, 4, 8 parts, in steps
+  const double nq = static_cast<double>((seq + kBK - 1) / kBK), blocks = static_cast<double>((seq + kBQ - 1) / kBQ);
+  const double longest = groups * nq, all = static_cast<double>(nb) * groups * blocks * (nq - blocks + 1.0);
+  int best = 1;
+  double best_t = 0.0;
+  for (int i = 0; i < 4; ++i) {
+    const double parts = 1 << i;
+    const double one = longest / parts + cost[i], share = (all + nb * blocks * parts * cost[i]) / sms;
+    const double t = one > share ? one : share;
+    if (i == 0 || t < best_t) { best = 1 << i; best_t = t; }
+  }
+  return best;
 }
 
 }  // namespace
@@ -1049,8 +1112,16 @@ extern "C" int mcb_attention_causal_bwd_ex(const void* q, const void* k, const v
   const unsigned gq = static_cast<unsigned>(n_tiles < slots ? n_tiles : slots);
   attn_dq_kernel<<<gq, kThreads, kDqSmem, st>>>(tmQ128, tmdO128, tmK64, tmV64, p);
   MCB_CHECK_LAUNCH("attn_dq_kernel");
-  dim3 gk(static_cast<unsigned>(nb), static_cast<unsigned>(seq / kBQ));
-  attn_dkv_kernel<<<gk, kKvThreads, kKvSmem, st>>>(tmK128, tmV128, tmQ64, tmdO64, p);
+  p.kv_parts = dkv_parts(nb, groups, seq, ds->sm_count);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(nb * p.kv_parts), static_cast<unsigned>(seq / kBQ));
+  cfg.blockDim = dim3(kKvThreads);
+  cfg.dynamicSmemBytes = kKvSmem; cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(p.kv_parts); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = p.kv_parts > 1 ? 1 : 0;
+  MCB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_dkv_kernel, tmK128, tmV128, tmQ64, tmdO64, p));
   MCB_CHECK_LAUNCH("attn_dkv_kernel");
   return MCB_OK;
 }

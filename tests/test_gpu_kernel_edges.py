@@ -185,3 +185,22 @@ def test_gate_up_swiglu_few_tokens(cuda_device, M, K, F):
     g, u = (x.astype(np.float64) @ w.astype(np.float64).T for w in (wg, wu))
     for got, want in ((gate, g), (up, u), (act, g / (1 + np.exp(-g)) * u)):
         assert R.max_abs_normalised(back(got), want) <= 2e-2
+
+
+# key blocks x kv heads from one to more than the SMs, so that every number of CTAs sharing a key block occurs; (1, 1, 128)
+# has fewer query steps than the CTAs that share its key block
+@pytest.mark.parametrize("nb,G,seq", [(1, 1, 128), (1, 7, 128), (4, 7, 256), (16, 3, 512), (40, 2, 512)])
+def test_attention_backward_shared_key_blocks(cuda_device, nb, G, seq):
+    from metal_candle_b200 import backend as B
+
+    q, k, v, do = (S.bf16_round(S.normal(92, n, s)) for n, s in (("q", (nb, G, seq, 64)), ("k", (nb, seq, 64)), ("v", (nb, seq, 64)),
+                                                                 ("do", (nb, G, seq, 64))))
+    bf = torch.bfloat16
+    qd, dod = (dev_t(t.reshape(nb, G * seq, 64), bf, cuda_device) for t in (q, do))
+    kd, vd = dev_t(k, bf, cuda_device), dev_t(v, bf, cuda_device)
+    o, lse = B.attention_causal_forward(qd, kd, vd, G, 0.125)
+    first = B.attention_causal_backward(qd, kd, vd, o, lse, dod, G, 0.125)
+    again = B.attention_causal_backward(qd, kd, vd, o, lse, dod, G, 0.125)
+    for got, rep, want in zip(first, again, R.causal_gqa_attention_backward(q, k, v, 0.125, do)):
+        assert torch.equal(got, rep)
+        assert np.abs(back(got).reshape(want.shape) - want).max() <= 2e-2 * np.abs(want).max()
