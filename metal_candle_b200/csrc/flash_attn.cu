@@ -20,7 +20,7 @@
 //               S = Q K^T (double-buffered, ahead) and dP = dO V^T into tensor memory, P = exp(scale*S - lse),
 //               dS = P (dP - delta) with delta = rowsum(dO * O), dS (bf16 pairs) written over the half of dP already
 //               read, dQ += dS K accumulated in tensor memory with dS as a tensor-memory A operand.
-//               It also writes delta and lse*log2(e) for the second kernel.
+//               It also writes -delta and -lse*log2(e) for the second kernel.
 //   dkv kernel  one CTA per (128 keys, kv head), steps of 64 queries over the heads of the group, one key row
 //               per thread pair: S^T = K Q^T, dP^T = V dO^T, P^T and dS^T back into tensor memory (A operands),
 //               dV += P^T dO and dK += dS^T Q accumulated in tensor memory over all steps (which also sums over
@@ -404,8 +404,8 @@ struct BwdParams {
   const __nv_bfloat16* O;
   const __nv_bfloat16* dO;
   const float* lse;
-  float* delta;   // [nb, G*S]
-  float* lse2;    // [nb, G*S]: lse * log2(e)
+  float* ndelta;  // [nb, G*S]: -delta, as the dK / dV kernel adds it
+  float* nlse2;   // [nb, G*S]: -lse * log2(e)
   __nv_bfloat16* dQ;
   __nv_bfloat16* dK;
   __nv_bfloat16* dV;
@@ -572,8 +572,8 @@ attn_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         }
       }
       const float lse2 = p.lse[w.qrow0 + row] * kLog2e;
-      p.delta[w.qrow0 + row] = delta;
-      p.lse2[w.qrow0 + row] = lse2;
+      p.ndelta[w.qrow0 + row] = -delta;
+      p.nlse2[w.qrow0 + row] = -lse2;
       const float2 sc2 = f2(p.sc, p.sc), nl2 = f2(-lse2, -lse2), nd2 = f2(-delta, -delta);
       for (int j = 0; j < w.nkb; ++j) {
         const uint32_t n = n0 + j;
@@ -677,6 +677,9 @@ attn_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 // exponentials, tensor-memory stores, wait); with one group every second of its links was exposed: 16 kv heads x 7
 // query heads x 1024 positions, whole kernel: 117 us with one group, 109 with two.  (K and V as tensor-memory operands
 // instead of shared-memory ones made no difference: 167 against 169 us for the whole backward pass.)
+// A warp issued 840 instructions a step and scheduler, a third of them waits: S^T is read in one 32-column load and its
+// exponentials are taken under the load of dP^T, and the arithmetic runs on packed pairs (which have no operand negation,
+// so the first kernel leaves -lse and -delta).  Backward pass of 16 x 7 x 1024: 126 -> 120 us, 32 x 7 x 2048: 708 -> 671.
 constexpr int kKvThreads = 576;
 constexpr uint32_t kKvOffK = 0;                       // K block [128 keys x 64]
 constexpr uint32_t kKvOffV = kKvOffK + kQBytes;
@@ -755,8 +758,8 @@ attn_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
         int dcol, drow;
         o_coords(p.S, p.G, p.HKV, p.o_tok, nb, g, i * kBK, dcol, drow);
         tma_load_2d(sb + kKBytes, &tmdO, fb, dcol, drow);
-        bulk_load_1d(sb + 2 * kKBytes, p.lse2 + qrow, 256, fb);
-        bulk_load_1d(sb + 2 * kKBytes + 256, p.delta + qrow, 256, fb);
+        bulk_load_1d(sb + 2 * kKBytes, p.nlse2 + qrow, 256, fb);
+        bulk_load_1d(sb + 2 * kKBytes + 256, p.ndelta + qrow, 256, fb);
       }
     }
   } else if (warp == 1) {
@@ -832,37 +835,40 @@ attn_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
       const uint32_t tS = tmem_base + st * 128 + lane_addr, tDP = tS + 64;
       // this warp's 32 query columns are 16 packed columns of each of P^T and dS^T
       const uint32_t tPT = tPT0 + st * 64 + lane_addr + half * 16;
+      const float* st_nl2 = reinterpret_cast<const float*>(gen_base + kKvOffStage + (t % kKvStages) * kKvStageStride + 2 * kKBytes) + half * 32;
+      const float* st_nd = st_nl2 + 64;
+      const int q0 = i * kBK + half * 32;
+      const bool diag = i * kBK < (kb + 1) * kBQ;   // some query of this step lies before some key of the block
+      const float2 sc2 = f2(p.sc, p.sc);
+      // the exponentials are taken while dP^T is still on its way from tensor memory
+      uint32_t vs[32], vd[32];
+      tmem_ld_x32(tS + half * 32, vs);
+      tmem_ld_wait_on(vs);
+      tmem_ld_x32(tDP + half * 32, vd);
+#pragma unroll
+      for (int e = 0; e < 32; e += 4) {
+        const float4 nl = *reinterpret_cast<const float4*>(st_nl2 + e);
+        const float2 ta = __ffma2_rn(f2(__uint_as_float(vs[e]), __uint_as_float(vs[e + 1])), sc2, f2(nl.x, nl.y));
+        const float2 tb = __ffma2_rn(f2(__uint_as_float(vs[e + 2]), __uint_as_float(vs[e + 3])), sc2, f2(nl.z, nl.w));
+        float pr[4] = {ex2(ta.x), ex2(ta.y), ex2(tb.x), ex2(tb.y)};
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          if (diag && key > q0 + e + x) pr[x] = 0.0f;
+          vs[e + x] = __float_as_uint(pr[x]);
+        }
+      }
+      tmem_ld_wait_on(vd);
       uint32_t wp[16], wd[16];
-      const float* st_lse2 = reinterpret_cast<const float*>(gen_base + kKvOffStage + (t % kKvStages) * kKvStageStride + 2 * kKBytes);
-      const float* st_delta = st_lse2 + 64;
-      const int q0 = i * kBK;
-      const bool diag = q0 < (kb + 1) * kBQ;   // some query of this step lies before some key of the block
 #pragma unroll
-      for (int cb = 0; cb < 32; cb += 16) {
-        const int c = half * 32 + cb;
-        uint32_t vs[16], vd[16];
-        tmem_ld_x16(tS + c, vs);
-        tmem_ld_x16(tDP + c, vd);
-        float l2[16], dl[16];
-#pragma unroll
-        for (int e = 0; e < 16; e += 4) {
-          const float4 a = *reinterpret_cast<const float4*>(st_lse2 + c + e);
-          const float4 b = *reinterpret_cast<const float4*>(st_delta + c + e);
-          l2[e] = a.x; l2[e + 1] = a.y; l2[e + 2] = a.z; l2[e + 3] = a.w;
-          dl[e] = b.x; dl[e + 1] = b.y; dl[e + 2] = b.z; dl[e + 3] = b.w;
-        }
-        tmem_ld_wait();
-#pragma unroll
-        for (int e = 0; e < 16; e += 2) {
-          float p0 = ex2(fmaf(__uint_as_float(vs[e]), p.sc, -l2[e]));
-          float p1 = ex2(fmaf(__uint_as_float(vs[e + 1]), p.sc, -l2[e + 1]));
-          if (diag) {
-            if (key > q0 + c + e) p0 = 0.0f;
-            if (key > q0 + c + e + 1) p1 = 0.0f;
-          }
-          wp[(cb + e) >> 1] = pack_bf16(p0, p1);
-          wd[(cb + e) >> 1] = pack_bf16(p0 * (__uint_as_float(vd[e]) - dl[e]), p1 * (__uint_as_float(vd[e + 1]) - dl[e + 1]));
-        }
+      for (int e = 0; e < 32; e += 4) {
+        const float4 nd = *reinterpret_cast<const float4*>(st_nd + e);
+        const float2 pa = f2(__uint_as_float(vs[e]), __uint_as_float(vs[e + 1])), pb = f2(__uint_as_float(vs[e + 2]), __uint_as_float(vs[e + 3]));
+        const float2 da = __fmul2_rn(pa, __fadd2_rn(f2(__uint_as_float(vd[e]), __uint_as_float(vd[e + 1])), f2(nd.x, nd.y)));
+        const float2 db = __fmul2_rn(pb, __fadd2_rn(f2(__uint_as_float(vd[e + 2]), __uint_as_float(vd[e + 3])), f2(nd.z, nd.w)));
+        wp[e >> 1] = pack_bf16(pa.x, pa.y);
+        wp[(e >> 1) + 1] = pack_bf16(pb.x, pb.y);
+        wd[e >> 1] = pack_bf16(da.x, da.y);
+        wd[(e >> 1) + 1] = pack_bf16(db.x, db.y);
       }
       tmem_st_x16(tPT, wp);
       tmem_st_x16(tPT + 32, wd);
@@ -966,7 +972,7 @@ int check_shape(const char* who, int64_t nb, int64_t groups, int64_t seq, int64_
 // How many CTAs of a cluster share a key block's query steps.  One CTA per key block ends with the CTAs of the first key
 // block, which have all G * nq steps; parts shorten that chain, but each costs a CTA's start, its exchange and the wait for
 // a cluster's worth of free SMs.  The launch takes about the longer of one part and an SM's share of all steps and parts.
-// Whole backward pass with 1 / 2 / 4 / 8 parts, us (kv heads x query heads each x positions):
+// Whole backward pass with 1 / 2 / 4 / 8 parts, us (kv heads x query heads each x positions; with today's step a twentieth less):
 //   16 x 7 x 1024: 169 / 126 / 147 / 203    8 x 7 x 512: 76 / 53 / 40 / 56    2 x 7 x 2048: 258 / 154 / 101 / 98
 //   32 x 7 x 2048: 709 / 744 / 856 / 1103   64 x 7 x 256: 69 / 72 / 84 / 137  4 x 7 x 4096: 579 / 366 / 391 / 464
 // the rule takes the fastest of each.
@@ -1084,8 +1090,8 @@ extern "C" int mcb_attention_causal_bwd_ex(const void* q, const void* k, const v
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const size_t rows = static_cast<size_t>(nb) * groups * seq * 4;
   uint8_t* w = static_cast<uint8_t*>(workspace);
-  float* delta = reinterpret_cast<float*>(w); w += up1k(rows);
-  float* lse2 = reinterpret_cast<float*>(w);
+  float* ndelta = reinterpret_cast<float*>(w); w += up1k(rows);
+  float* nlse2 = reinterpret_cast<float*>(w);
   CUtensorMap tmQ128, tmdO128, tmK64, tmV64, tmK128, tmV128, tmQ64, tmdO64;
   if (int rc = encode(ds, &tmQ128, q, kD, nb * groups * seq, kBQ, "Q")) return rc;
   // dO either like Q ([rows, 64]) or token-major ([batch*S, heads*64]: a head's tile is a column offset)
@@ -1103,7 +1109,7 @@ extern "C" int mcb_attention_causal_bwd_ex(const void* q, const void* k, const v
   p.HKV = o_token_major ? static_cast<int>(kv_heads) : 1; p.o_tok = o_token_major ? 1 : 0;
   p.sc = scale * kLog2e; p.scale = scale;
   p.O = static_cast<const __nv_bfloat16*>(o); p.dO = static_cast<const __nv_bfloat16*>(dout); p.lse = lse;
-  p.delta = delta; p.lse2 = lse2;
+  p.ndelta = ndelta; p.nlse2 = nlse2;
   p.dQ = static_cast<__nv_bfloat16*>(dq); p.dK = static_cast<__nv_bfloat16*>(dk); p.dV = static_cast<__nv_bfloat16*>(dv);
   p.status = ds->status_word;
   // persistent: two CTAs per SM walk over the (query block, head, batch) items, heavy ones first
