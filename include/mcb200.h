@@ -333,6 +333,17 @@ int mcb_attention_causal_bwd_ex(const void* q, const void* k, const void* v, con
                                 int64_t seq, int64_t head_dim, float scale, int dtype, int64_t kv_heads,
                                 int o_token_major, void* workspace, size_t workspace_bytes, void* stream);
 
+/* The same two calls for a sequence of any length from 1 on (the tiles are filled up with zeros on chip; no operand is
+ * padded).  The calls above keep refusing a length that is no multiple of 128. */
+int mcb_attention_causal_fwd_ragged(const void* q, const void* k, const void* v, void* o, float* lse, int64_t nb,
+                                    int64_t groups, int64_t seq, int64_t head_dim, float scale, int dtype,
+                                    int64_t kv_heads, int o_token_major, void* workspace, size_t workspace_bytes,
+                                    void* stream);
+int mcb_attention_causal_bwd_ragged(const void* q, const void* k, const void* v, const void* o, const void* dout,
+                                    const float* lse, void* dq, void* dk, void* dv, int64_t nb, int64_t groups,
+                                    int64_t seq, int64_t head_dim, float scale, int dtype, int64_t kv_heads,
+                                    int o_token_major, void* workspace, size_t workspace_bytes, void* stream);
+
 /* ---- data-parallel exchange ------------------------------------------------------------------- */
 
 /* The reference trains on one device and has no communication layer; these calls are the one exchange step of the

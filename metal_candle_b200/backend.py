@@ -371,14 +371,28 @@ def linear_swiglu_forward(x: torch.Tensor, w_gate_up: torch.Tensor):
 # ---------------------------------------------------------------------------------------------
 
 def attention_supported(q: torch.Tensor, seq: int) -> bool:
-    """Shapes the fused attention kernels are built for (others use the unfused sequence)."""
+    """Shapes `attention_causal_forward` and `_backward` take."""
     return q.dtype == torch.bfloat16 and q.shape[-1] == 64 and seq % 128 == 0
+
+
+def attention_ragged_supported(q: torch.Tensor) -> bool:
+    """Tensors `attention_causal_ragged_forward` and `_backward` take, whatever the sequence length."""
+    return q.dtype == torch.bfloat16 and q.shape[-1] == 64
 
 
 def attention_causal_forward(q, k, v, groups: int, scale: float, kv_heads: int = 0):
     """Attention::forward's core (src/models/transformer.rs:257-285) in one kernel.  q [nb, groups*S, d]
     (row g*S + s), k and v [nb, S, d].  Returns (o, lse [nb, groups*S] float32); o is laid out like q, or, with
     kv_heads > 0 (nb = batch*kv_heads), token-major [batch*S, kv_heads*groups*d] - the o_proj input as it is."""
+    return _attention_forward("mcb_attention_causal_fwd_ex", q, k, v, groups, scale, kv_heads)
+
+
+def attention_causal_ragged_forward(q, k, v, groups: int, scale: float, kv_heads: int = 0):
+    """`attention_causal_forward` for a sequence of any length."""
+    return _attention_forward("mcb_attention_causal_fwd_ragged", q, k, v, groups, scale, kv_heads)
+
+
+def _attention_forward(entry: str, q, k, v, groups: int, scale: float, kv_heads: int):
     _require_cuda(q, k, v)
     nb, S, d = k.shape
     if q.shape != (nb, groups * S, d) or v.shape != k.shape:
@@ -389,16 +403,23 @@ def attention_causal_forward(q, k, v, groups: int, scale: float, kv_heads: int =
     o = (torch.empty((nb // kv_heads) * S, kv_heads * groups * d, dtype=q.dtype, device=q.device) if kv_heads
          else torch.empty_like(q))
     lse = torch.empty(nb, groups * S, dtype=torch.float32, device=q.device)
-    ws = workspace(q.device, lib.mcb_attention_workspace_bytes(nb, groups, S, d))
-    _lib.check(lib.mcb_attention_causal_fwd_ex(_ptr(q), _ptr(k), _ptr(v), _ptr(o), _ptr(lse), nb, groups, S, d, float(scale),
-                                               _dtype_code(q), int(kv_heads), int(bool(kv_heads)), _ptr(ws), ws.numel(),
-                                               _stream()))
+    _lib.check(getattr(lib, entry)(_ptr(q), _ptr(k), _ptr(v), _ptr(o), _ptr(lse), nb, groups, S, d, float(scale), _dtype_code(q),
+                                   int(kv_heads), int(bool(kv_heads)), None, 0, _stream()))   # the forward needs no workspace
     return o, lse
 
 
 def attention_causal_backward(q, k, v, o, lse, dout, groups: int, scale: float, kv_heads: int = 0):
     """Gradients of `attention_causal_forward`: (dq like q, dk and dv like k, summed over the group).  With
     kv_heads > 0, o and dout are token-major as returned by the forward."""
+    return _attention_backward("mcb_attention_causal_bwd_ex", q, k, v, o, lse, dout, groups, scale, kv_heads)
+
+
+def attention_causal_ragged_backward(q, k, v, o, lse, dout, groups: int, scale: float, kv_heads: int = 0):
+    """`attention_causal_backward` for a sequence of any length."""
+    return _attention_backward("mcb_attention_causal_bwd_ragged", q, k, v, o, lse, dout, groups, scale, kv_heads)
+
+
+def _attention_backward(entry: str, q, k, v, o, lse, dout, groups: int, scale: float, kv_heads: int):
     _require_cuda(q, k, v, o, lse, dout)
     nb, S, d = k.shape
     want = ((nb // kv_heads) * S, kv_heads * groups * d) if kv_heads else tuple(q.shape)
@@ -407,9 +428,9 @@ def attention_causal_backward(q, k, v, o, lse, dout, groups: int, scale: float, 
     lib = _lib_for(q)
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
     ws = workspace(q.device, lib.mcb_attention_workspace_bytes(nb, groups, S, d))
-    _lib.check(lib.mcb_attention_causal_bwd_ex(_ptr(q), _ptr(k), _ptr(v), _ptr(o), _ptr(dout), _ptr(lse), _ptr(dq), _ptr(dk),
-                                               _ptr(dv), nb, groups, S, d, float(scale), _dtype_code(q), int(kv_heads),
-                                               int(bool(kv_heads)), _ptr(ws), ws.numel(), _stream()))
+    _lib.check(getattr(lib, entry)(_ptr(q), _ptr(k), _ptr(v), _ptr(o), _ptr(dout), _ptr(lse), _ptr(dq), _ptr(dk), _ptr(dv), nb,
+                                   groups, S, d, float(scale), _dtype_code(q), int(kv_heads), int(bool(kv_heads)), _ptr(ws),
+                                   ws.numel(), _stream()))
     return dq, dk, dv
 
 

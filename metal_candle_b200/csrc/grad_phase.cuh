@@ -47,13 +47,6 @@ struct GradShared {
   volatile int* abort_flag;
 };
 
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
-
 // Bounded wait until *flag >= target (written by other CTAs with a release at gpu scope).
 __device__ __forceinline__ bool flag_wait(const int* flag, int target, volatile int* abort_flag, int code, int* status) {
   const unsigned long long t0 = umma::globaltimer_ns();

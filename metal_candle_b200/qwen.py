@@ -10,7 +10,7 @@ library's own kernels; the frozen weights get no gradients.
 
 Everything with arithmetic in it is a kernel of libmetal_candle_b200 except the six batched attention
 contractions (Q K^T, P V and their reverses): the fused attention kernels of csrc/flash_attn.cu where they apply
-(bf16, head_dim 64, sequence a multiple of 128), otherwise plain library GEMMs (torch.bmm -> cuBLAS).
+(bf16, head_dim 64), otherwise plain library GEMMs (torch.bmm -> cuBLAS).
 """
 from __future__ import annotations
 
@@ -284,14 +284,14 @@ class Qwen:
 
     # -- attention core on [B,H,S,d] tensors; grouped-query heads are folded into the row dimension --
     def _attention_fwd(self, Qr, Kr, Vr, B, S):
-        """Returns (P, O, lse): the fused kernel (bf16, head_dim 64, S a multiple of 128) keeps only the
-        log-sum-exp of each row; other shapes materialise the probabilities P as the reference does."""
+        """Returns (P, O, lse): the fused kernel (bf16, head_dim 64) keeps only the log-sum-exp of each row; other
+        dtypes and head sizes materialise the probabilities P as the reference does."""
         c = self.config
         Hk, G, d = c.num_key_value_heads, c.num_attention_heads // c.num_key_value_heads, c.head_dim
-        if backend.attention_supported(Qr, S):
+        if backend.attention_ragged_supported(Qr):
             # the fused kernel writes its output token-major, [B*S, hidden]: the o_proj input as it is
-            O, lse = backend.attention_causal_forward(Qr.view(B * Hk, G * S, d), Kr.view(B * Hk, S, d),
-                                                      Vr.view(B * Hk, S, d), G, 1.0 / math.sqrt(d), kv_heads=Hk)
+            O, lse = backend.attention_causal_ragged_forward(Qr.view(B * Hk, G * S, d), Kr.view(B * Hk, S, d),
+                                                             Vr.view(B * Hk, S, d), G, 1.0 / math.sqrt(d), kv_heads=Hk)
             return None, O, lse
         scores = torch.bmm(Qr.view(B * Hk, G * S, d), Kr.view(B * Hk, S, d).transpose(1, 2))  # [B*Hk, G*S, S]
         rows = scores.numel() // S
@@ -305,9 +305,9 @@ class Qwen:
         Hk, G, d = c.num_key_value_heads, c.num_attention_heads // c.num_key_value_heads, c.head_dim
         if P is None:
             # fused: O and dO are token-major [B*S, hidden] (o_proj's input and its gradient as they are)
-            return backend.attention_causal_backward(Qr.view(B * Hk, G * S, d), Kr.view(B * Hk, S, d),
-                                                     Vr.view(B * Hk, S, d), O, lse, dO, G, 1.0 / math.sqrt(d),
-                                                     kv_heads=Hk)
+            return backend.attention_causal_ragged_backward(Qr.view(B * Hk, G * S, d), Kr.view(B * Hk, S, d),
+                                                            Vr.view(B * Hk, S, d), O, lse, dO, G, 1.0 / math.sqrt(d),
+                                                            kv_heads=Hk)
         dO3 = dO.view(B * Hk, G * S, d)
         dV = torch.bmm(P.transpose(1, 2), dO3)                       # [B*Hk, S, d], summed over the group
         dP = torch.bmm(dO3, Vr.view(B * Hk, S, d).transpose(1, 2))   # [B*Hk, G*S, S]

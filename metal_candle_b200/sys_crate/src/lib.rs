@@ -165,6 +165,8 @@ extern "C" {
     pub fn mcb_attention_causal_bwd(q: *const c_void, k: *const c_void, v: *const c_void, o: *const c_void, dout: *const c_void, lse: *const f32, dq: *mut c_void, dk: *mut c_void, dv: *mut c_void, nb: i64, groups: i64, seq: i64, head_dim: i64, scale: f32, dtype: c_int, workspace: *mut c_void, workspace_bytes: usize, stream: *mut c_void) -> c_int;
     pub fn mcb_attention_causal_fwd_ex(q: *const c_void, k: *const c_void, v: *const c_void, o: *mut c_void, lse: *mut f32, nb: i64, groups: i64, seq: i64, head_dim: i64, scale: f32, dtype: c_int, kv_heads: i64, o_token_major: c_int, workspace: *mut c_void, workspace_bytes: usize, stream: *mut c_void) -> c_int;
     pub fn mcb_attention_causal_bwd_ex(q: *const c_void, k: *const c_void, v: *const c_void, o: *const c_void, dout: *const c_void, lse: *const f32, dq: *mut c_void, dk: *mut c_void, dv: *mut c_void, nb: i64, groups: i64, seq: i64, head_dim: i64, scale: f32, dtype: c_int, kv_heads: i64, o_token_major: c_int, workspace: *mut c_void, workspace_bytes: usize, stream: *mut c_void) -> c_int;
+    pub fn mcb_attention_causal_fwd_ragged(q: *const c_void, k: *const c_void, v: *const c_void, o: *mut c_void, lse: *mut f32, nb: i64, groups: i64, seq: i64, head_dim: i64, scale: f32, dtype: c_int, kv_heads: i64, o_token_major: c_int, workspace: *mut c_void, workspace_bytes: usize, stream: *mut c_void) -> c_int;
+    pub fn mcb_attention_causal_bwd_ragged(q: *const c_void, k: *const c_void, v: *const c_void, o: *const c_void, dout: *const c_void, lse: *const f32, dq: *mut c_void, dk: *mut c_void, dv: *mut c_void, nb: i64, groups: i64, seq: i64, head_dim: i64, scale: f32, dtype: c_int, kv_heads: i64, o_token_major: c_int, workspace: *mut c_void, workspace_bytes: usize, stream: *mut c_void) -> c_int;
     pub fn mcb_comm_unique_id(id_out: *mut c_void) -> c_int;
     pub fn mcb_comm_init_rank(comm_out: *mut *mut mcb_comm, nranks: c_int, rank: c_int, id: *const c_void, timeout_ms: c_int, flags: c_int) -> c_int;
     pub fn mcb_comm_allreduce_bucket(comm: *mut mcb_comm, buf: *mut f32, count: i64, stream: *mut c_void) -> c_int;

@@ -204,3 +204,56 @@ def test_attention_backward_shared_key_blocks(cuda_device, nb, G, seq):
     for got, rep, want in zip(first, again, R.causal_gqa_attention_backward(q, k, v, 0.125, do)):
         assert torch.equal(got, rep)
         assert np.abs(back(got).reshape(want.shape) - want).max() <= 2e-2 * np.abs(want).max()
+
+
+# nb kv heads, G query heads each, S positions: one row, the edges of the 64-key blocks and 128-query tiles, remainders;
+# (2, 1, 64) and (1, 1, 1) have fewer query steps than the CTAs that share a key block
+RAGGED_ATTENTION = [(1, 1, 1), (2, 3, 5), (1, 7, 63), (2, 1, 64), (2, 7, 65), (4, 2, 111), (2, 1, 127), (1, 2, 129), (2, 2, 193), (1, 7, 333)]
+
+
+@pytest.mark.parametrize("nb,G,seq", RAGGED_ATTENTION)
+@pytest.mark.parametrize("token_major", [False, True])
+def test_attention_of_any_length(cuda_device, nb, G, seq, token_major):
+    from metal_candle_b200 import _lib, backend as B
+
+    q, k, v, do = (S.bf16_round(S.normal(91, n, s)) for n, s in (("q", (nb, G, seq, 64)), ("k", (nb, seq, 64)), ("v", (nb, seq, 64)),
+                                                                 ("do", (nb, G, seq, 64))))
+    want_o, want_lse, _ = R.causal_gqa_attention(q, k, v, 0.125)
+    wdq, wdk, wdv = R.causal_gqa_attention_backward(q, k, v, 0.125, do)
+    kvh = nb if token_major else 0
+
+    def layout(a):   # one batch of nb kv heads: [nb, G, S, d] -> [S, nb * G * d]
+        return a.transpose(2, 0, 1, 3).reshape(seq, nb * G * 64) if token_major else a.reshape(nb, G * seq, 64)
+
+    bf = torch.bfloat16
+    qd, kd, vd = dev_t(q.reshape(nb, G * seq, 64), bf, cuda_device), dev_t(k, bf, cuda_device), dev_t(v, bf, cuda_device)
+    o, lse = B.attention_causal_ragged_forward(qd, kd, vd, G, 0.125, kv_heads=kvh)
+    dq, dk, dv = B.attention_causal_ragged_backward(qd, kd, vd, o, lse, dev_t(layout(do), bf, cuda_device), G, 0.125, kv_heads=kvh)
+    assert _lib.device_status() == 0
+    assert np.abs(back(lse).reshape(nb, G, seq) - want_lse).max() <= 2e-2
+    # one position attends to itself alone: P = 1 and dS = 0, so dq and dk are the rounding of dP - delta around zero
+    # (a sum of 64 products of size 1 in float32, times |k| / 8: below 1e-4)
+    floor = 1e-2 if seq == 1 else 0.0
+    for got, want in ((o, layout(want_o)), (dq, wdq.reshape(nb, G * seq, 64)), (dk, wdk), (dv, wdv)):
+        assert np.abs(back(got) - want).max() <= 2e-2 * max(np.abs(want).max(), floor)
+
+
+def test_attention_of_any_length_reads_no_other_head(cuda_device):
+    """Tiles that reach past the end of a sequence: what lies there (the next head, inf and NaN in it) must not matter."""
+    from metal_candle_b200 import backend as B
+
+    seq, G = 77, 2
+    g = torch.Generator(device=cuda_device).manual_seed(3)
+    q, k, v, do = (torch.randn(3, rows, 64, device=cuda_device, generator=g).to(torch.bfloat16) for rows in (G * seq, seq, seq, G * seq))
+    alone = [t[:1].contiguous() for t in (q, k, v, do)]
+    for t, bad in ((q, float("nan")), (k, float("inf")), (v, float("nan")), (do, float("inf"))):
+        t[1:] = bad
+
+    def run(q, k, v, do):
+        o, lse = B.attention_causal_ragged_forward(q, k, v, G, 0.125)
+        return (o, lse) + B.attention_causal_ragged_backward(q, k, v, o, lse, do, G, 0.125)
+
+    # the number of CTAs that share a key block depends on the number of heads, so sums may be ordered differently
+    for a, b in zip(run(*alone), run(q, k, v, do)):
+        assert torch.isfinite(b[0].float()).all()
+        torch.testing.assert_close(a[0].float(), b[0].float(), rtol=2e-2, atol=1e-3)
