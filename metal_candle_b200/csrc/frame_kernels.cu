@@ -80,9 +80,11 @@ __global__ void rope_relayout_kernel(const T* __restrict__ src, T* __restrict__ 
   }
 }
 
-// Scalar variant for head sizes whose half is not a multiple of the vector width.
 // The same for the query, key and value heads of a fused q/k/v row in one launch: the sines and cosines of a
-// (position, chunk) are computed once and used for the rotated segments (q and k); v is only re-laid out.
+// (position, chunk) are computed once and used for the rotated segments (q and k); v is only re-laid out.  grid.y shares
+// the heads: at 333 tokens one thread per (token, chunk) is 11 blocks, each thread working through 18 heads one after the
+// other (10.4 us); with the heads spread over as many blocks as fill the chip the launch takes 6.3 us, although
+// every share computes the sines again.  Many tokens keep one share: 32768 x 18 heads move 151 MB and are HBM-bound.
 template <typename T>
 struct RopeSegment {
   T* head_major;    // [B, H, S, d]
@@ -98,6 +100,9 @@ __global__ void rope_relayout_qkv_kernel(T* __restrict__ fused, RopeSegment<T> s
   const int half = d / 2;
   const int chunks = half / N;
   const int64_t total = static_cast<int64_t>(B) * S * chunks;
+  const int heads = s0.H + s1.H + s2.H;
+  const int h_begin = static_cast<int>(static_cast<int64_t>(heads) * blockIdx.y / gridDim.y);
+  const int h_end = static_cast<int>(static_cast<int64_t>(heads) * (blockIdx.y + 1) / gridDim.y);
   for (int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
        idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int c = static_cast<int>(idx % chunks);
@@ -115,7 +120,8 @@ __global__ void rope_relayout_qkv_kernel(T* __restrict__ fused, RopeSegment<T> s
 #pragma unroll
     for (int g = 0; g < 3; ++g) {
       const RopeSegment<T>& sg = g == 0 ? s0 : g == 1 ? s1 : s2;
-      for (int h = 0; h < sg.H; ++h) {
+      const int first = g == 0 ? 0 : g == 1 ? s0.H : s0.H + s1.H;   // the segment's part of heads [h_begin, h_end)
+      for (int h = max(0, h_begin - first); h < min(sg.H, h_end - first); ++h) {
         const int64_t tok = (static_cast<int64_t>(b) * S + s) * pitch + sg.offset + static_cast<int64_t>(h) * d;
         const int64_t hm = ((static_cast<int64_t>(b) * sg.H + h) * S + s) * d;
         const T* in = inverse ? sg.head_major + hm : fused + tok;
@@ -140,6 +146,7 @@ __global__ void rope_relayout_qkv_kernel(T* __restrict__ fused, RopeSegment<T> s
   }
 }
 
+// Scalar variant for head sizes whose half is not a multiple of the vector width.
 template <typename T>
 __global__ void rope_relayout_scalar_kernel(const T* __restrict__ src, T* __restrict__ dst, int B, int S, int H, int d,
                                             float theta, int rotate, int inverse, int64_t pitch, int64_t offset) {
@@ -341,7 +348,12 @@ extern "C" int mcb_rope_relayout_qkv(void* fused, void* q, void* k, void* v, int
     return MCB_OK;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int grid = grid_for(B * S * (half / vec_n), 128, ds->sm_count);
+  const int64_t heads = Hq + 2 * Hk;
+  const int blocks = grid_for(B * S * (half / vec_n), 128, ds->sm_count);
+  int64_t shares = (4 * static_cast<int64_t>(ds->sm_count) + blocks - 1) / blocks;   // four blocks per SM
+  if (shares > heads) shares = heads;
+  if (shares > 65535) shares = 65535;
+  const dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>(shares));
   MCB_DTYPE_SWITCH(dtype, ({
     RopeSegment<T> s0{static_cast<T*>(q), static_cast<int>(Hq), 0, 1};
     RopeSegment<T> s1{static_cast<T*>(k), static_cast<int>(Hk), Hq * d, 1};

@@ -257,3 +257,27 @@ def test_attention_of_any_length_reads_no_other_head(cuda_device):
     for a, b in zip(run(*alone), run(q, k, v, do)):
         assert torch.isfinite(b[0].float()).all()
         torch.testing.assert_close(a[0].float(), b[0].float(), rtol=2e-2, atol=1e-3)
+
+
+# tokens of one share of the heads per block (many) and of several, down to one head each (few)
+@pytest.mark.parametrize("batch,seq", [(1, 1), (3, 111), (2, 1500), (1, 20000)])
+@pytest.mark.parametrize("inverse", [0, 1])
+def test_rope_qkv_shares_heads(cuda_device, batch, seq, inverse):
+    """The merged launch against the three single ones, whose results it has to repeat to the bit."""
+    from metal_candle_b200 import _lib
+    from metal_candle_b200.backend import MCB_BF16, _ptr, _stream
+
+    lib = _lib.init(0)
+    g = torch.Generator(device=cuda_device).manual_seed(5)
+    heads, width = (14, 2, 2), 18 * 64
+    fused = torch.randn(batch * seq, width, device=cuda_device, generator=g).to(torch.bfloat16)
+    major = [torch.randn(batch, h, seq, 64, device=cuda_device, generator=g).to(torch.bfloat16) for h in heads]
+    want_fused, want_major = fused.clone(), [m.clone() for m in major]
+    _lib.check(lib.mcb_rope_relayout_qkv(_ptr(fused), *(_ptr(m) for m in major), batch, seq, 14, 2, 64, 1e6, inverse, width, MCB_BF16, _stream()))
+    at = 0
+    for m, h, rotate in zip(want_major, heads, (1, 1, 0)):
+        src, dst = (m, want_fused) if inverse else (want_fused, m)
+        _lib.check(lib.mcb_rope_relayout_ex(_ptr(src), _ptr(dst), batch, seq, h, 64, 1e6, rotate, inverse, width, at, MCB_BF16, _stream()))
+        at += h * 64
+    assert torch.equal(fused, want_fused) and all(torch.equal(a, b) for a, b in zip(major, want_major))
+
