@@ -281,3 +281,21 @@ def test_rope_qkv_shares_heads(cuda_device, batch, seq, inverse):
         at += h * 64
     assert torch.equal(fused, want_fused) and all(torch.equal(a, b) for a, b in zip(major, want_major))
 
+
+@pytest.mark.parametrize("count", [1, 64, 65, 256, 257, 600])
+def test_adamw_many_tensors(cuda_device, count):
+    """One launch holds 64 or 256 descriptors; the update itself is elementwise, so it equals that of one tensor at a time."""
+    from metal_candle_b200.training import AdamW, AdamWConfig
+
+    g = torch.Generator(device=cuda_device).manual_seed(9)
+    sizes = [1 + (37 * i) % 203 for i in range(count)]
+    together = [torch.randn(n, device=cuda_device, generator=g) for n in sizes]
+    grads = [torch.randn(n, device=cuda_device, generator=g) for n in sizes]
+    single = [p.clone() for p in together]
+    a, b = AdamW(AdamWConfig()), AdamW(AdamWConfig())
+    for _ in range(2):
+        a.step_vars(together, grads)
+        for p, gr in zip(single, grads):
+            b.step_var(p, gr)
+    assert a.step_count == b.step_count == 2 * count
+    assert all(torch.equal(p, q) for p, q in zip(together, single))
