@@ -98,7 +98,7 @@ __device__ __forceinline__ void load_tile(uint32_t dst, const Operand& o, int ro
 
 // Bound: the FMA pipe, with shared-memory reads next.  A thread owns 16 x 8 outputs: 6 LDS.128 feed 128 FMAs, which keeps
 // the reads below the 128 bytes per cycle an SM has; the FMAs are packed pairs (fma.rn.f32x2), which leaves issue slots
-// for the copies.  2048 x 1536 x 1536: 272 us (35 TFLOP/s; 64 x 64 tiles of 4 x 4 outputs took 480), 512 x 768 x 768: 33
+// for the copies.  2048 x 1536 x 1536: 262 us (37 TFLOP/s; 64 x 64 tiles of 4 x 4 outputs took 480), 512 x 768 x 768: 29
 // us (240).  A shape with few tiles (512 x 768 x 768: 48) leaves SMs idle, so up to 8 CTAs of a cluster share a tile's
 // reduction and add their partial tiles through distributed shared memory, in rank order: deterministic, no workspace.
 __global__ void __launch_bounds__(kTileThreads, 4) tile_kernel(const TileParams p) {
@@ -138,8 +138,12 @@ __global__ void __launch_bounds__(kTileThreads, 4) tile_kernel(const TileParams 
     load_step(s + kStages - 1);
     const float* sa = smem + (s % kStages) * kStageFloats + 4 * ty;
     const float* sb = smem + (s % kStages) * kStageFloats + kStep * kPitchA + 4 * tx;
+    // a step's indices behind the end are zeros: a rank of 8 is a quarter of a step, and that step is the last CTA's fourth
+    // at 512 x 768 x 768 (forward 39.0 -> 34.9 us, 1024 x 768 -> 768 59.5 -> 55.4)
+    const int left = s < main_steps ? p.K - (s_begin + s) * kStep : p.R - (s - main_steps) * kStep;
+    const int kn = left < kStep ? left : kStep;
 #pragma unroll 2
-    for (int k = 0; k < kStep; ++k) {
+    for (int k = 0; k < kn; ++k) {
       float a[16];
       float4 b[2];
 #pragma unroll
