@@ -22,10 +22,17 @@ __device__ __forceinline__ float ex2_ftz(float x) {
 }
 __device__ __forceinline__ void online_combine(float& m, float& s, float m2, float s2) {
   const float mm = fmaxf(m, m2);
-  if (mm == -INFINITY) { m = mm; s = 0.0f; return; }
+  if (mm == -INFINITY) { m = mm; s += s2; return; }   // nothing kept yet: both sums are 0, or NaN from a NaN logit
   s = s * __expf(m - mm) + s2 * __expf(m2 - mm);
   m = mm;
 }
+
+// Beyond this magnitude a maximum times log2(e) may overflow: -m log2(e) is then infinite and the fused form
+// 2^(x log2e - m log2e) is inf or 0 where x equals m (a row, or a share of one, masked with the type's lowest value).  Such
+// maxima take differences first, 2^((x - m) log2e), in loops of their own; no logit in earnest gets there.
+constexpr float kFusedMax = 8.507059e37f;   // 2^126
+__device__ __forceinline__ bool beyond_fused(float m) { return fabsf(m) > kFusedMax && fabsf(m) != INFINITY; }
+__device__ __forceinline__ float exp_diff(float x, float m) { return ex2_ftz((x - m) * kLog2e); }
 
 // Rows that do not fit the cluster kernel below: short ones, whose share of a CTA would be a few vectors, and rows of more
 // than 800 KB.  Persistent: block b takes rows b, b + gridDim.x, ...; sweep 1 takes the maximum and the sum, sweep 2 reads the
@@ -53,6 +60,7 @@ cross_entropy_kernel(const T* in, T* out, const int32_t* __restrict__ targets, f
     const bool vec = (V % NV == 0) && (((reinterpret_cast<uintptr_t>(lr) | reinterpret_cast<uintptr_t>(gr)) & 15u) == 0);
     float m = -INFINITY, s = 0.0f;
     if (vec) {
+      float m2 = 0.0f;   // -m log2(e), finite also for the lowest values (a row whose maximum is one is summed again below)
       const int nvec = V / NV;
       const auto* src = reinterpret_cast<const decltype(VT::raw)*>(lr);
       auto absorb = [&](const VT& t) {
@@ -61,9 +69,9 @@ cross_entropy_kernel(const T* in, T* out, const int32_t* __restrict__ targets, f
         float vm = f[0];
 #pragma unroll
         for (int j = 1; j < NV; ++j) vm = fmaxf(vm, f[j]);
-        if (vm == -INFINITY) return;  // a wholly masked vector adds nothing (and exp(-inf - -inf) would be NaN)
-        if (vm > m) { s *= __expf(m - vm); m = vm; }
-        const float m2 = -m * kLog2e;   // exp(f - m) = 2^(f log2e - m log2e): one fused multiply-add and one special function
+        if (vm > m) { s *= __expf(m - vm); m = vm; m2 = -fmaxf(m, -kFusedMax) * kLog2e; }
+        // exp(f - m) = 2^(f log2e - m log2e): one fused multiply-add and one special function; masked logits add 0, with
+        // nothing kept yet (m2 = 0) as well, and a NaN among them reaches the sum
 #pragma unroll
         for (int j = 0; j < NV; ++j) s += ex2_ftz(fmaf(f[j], kLog2e, m2));
       };
@@ -85,14 +93,30 @@ cross_entropy_kernel(const T* in, T* out, const int32_t* __restrict__ targets, f
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-      const float m2 = __shfl_xor_sync(0xffffffffu, m, o), s2 = __shfl_xor_sync(0xffffffffu, s, o);
-      online_combine(m, s, m2, s2);
+      const float mo = __shfl_xor_sync(0xffffffffu, m, o), so = __shfl_xor_sync(0xffffffffu, s, o);
+      online_combine(m, s, mo, so);
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = bd >> 5;
     if (lane == 0) { sm[warp] = m; ss[warp] = s; }
     __syncthreads();
     m = sm[0]; s = ss[0];
     for (int w = 1; w < nw; ++w) online_combine(m, s, sm[w], ss[w]);
+    if (beyond_fused(m)) {   // the same for every thread of the block
+      float d = 0.0f;
+      for (int c = threadIdx.x; c < V; c += bd) d += exp_diff(to_f32(lr[c]), m);
+      d = warp_sum(d);
+      __syncthreads();   // everyone has read ss
+      if (lane == 0) ss[warp] = d;
+      __syncthreads();
+      s = 0.0f;
+      for (int w = 0; w < nw; ++w) s += ss[w];
+      if (threadIdx.x == 0) nll[row] = (m - to_f32(lr[tgt])) + logf(s);   // (m + log s would lose the logarithm)
+      __syncthreads();
+      if (write_grad)
+        for (int c = threadIdx.x; c < V; c += bd)
+          gr[c] = from_f32<T>((exp_diff(to_f32(lr[c]), m) / s - (c == tgt ? 1.0f : 0.0f)) * inv_count);
+      continue;
+    }
     const float lse = m + logf(s);
     if (threadIdx.x == 0) nll[row] = lse - to_f32(lr[tgt]);
     __syncthreads();  // thread 0 has read lr[tgt] before anyone overwrites it; sm / ss are free for the next row
@@ -311,8 +335,9 @@ cross_entropy_cluster_kernel(const CeParams p) {
       // pass 2: sum of 2^((x - m) log2 e), two lanes at a time
       const float2 l2 = make_float2(kLog2e, kLog2e);
       float2 s2 = make_float2(0.0f, 0.0f);
-      if (m != -INFINITY) {
-        const float2 nm = make_float2(-m * kLog2e, -m * kLog2e);
+      if (!beyond_fused(m)) {
+        const float nm1 = m == -INFINITY ? 0.0f : -m * kLog2e;   // a wholly masked share adds 0, or NaN if it holds one
+        const float2 nm = make_float2(nm1, nm1);
 #pragma unroll 4
         for (int vi = fa + tid; vi < fb; vi += kLanes) {
           VT t;
@@ -326,6 +351,8 @@ cross_entropy_cluster_kernel(const CeParams p) {
           }
         }
         for (int e = edge_b; e < edge_e; ++e) s2.x += ex2_ftz(fmaf(to_f32(selem[e]), kLog2e, nm.x));
+      } else {
+        for (int e = lo + tid; e < hi; e += kLanes) s2.x += exp_diff(to_f32(selem[e]), m);
       }
       const float sw = warp_sum(s2.x + s2.y);
       if (lane == 0) red[1][warp] = sw;
@@ -351,20 +378,22 @@ cross_entropy_cluster_kernel(const CeParams p) {
         par ^= 1;
       }
       const float lse = m + logf(s);
-      if (tid == 0 && tgt >= lo && tgt < hi) p.nll[row] = lse - to_f32(selem[tgt]);
+      const bool diff = beyond_fused(m);   // the same in every CTA of the cluster
+      if (tid == 0 && tgt >= lo && tgt < hi) p.nll[row] = diff ? (m - to_f32(selem[tgt])) + logf(s) : lse - to_f32(selem[tgt]);
       // pass 3: the gradient
       const float2 nl = make_float2(-lse * kLog2e, -lse * kLog2e), ic = make_float2(inv_count, inv_count);
       auto grad_one = [&](float x, bool is_target) { return from_f32<T>((ex2_ftz(fmaf(x, kLog2e, nl.x)) - (is_target ? 1.0f : 0.0f)) * inv_count); };
       float x_target = 0.0f;
       bool owner = false;   // this thread writes the target's vector below, and that element once more behind the loop
-      if (p.write_grad) {
+      if (p.write_grad && diff) {
+        for (int e = lo + tid; e < hi; e += kLanes)
+          orow[e] = from_f32<T>((exp_diff(to_f32(selem[e]), m) / s - (e == tgt ? 1.0f : 0.0f)) * inv_count);
+      } else if (p.write_grad) {
         if (tgt >= fa * N && tgt < fb * N) {
           owner = (tgt / N - fa) % kLanes == tid;
           x_target = to_f32(selem[tgt]);
         }
         for (int e = edge_b; e < edge_e; ++e) orow[e] = grad_one(to_f32(selem[e]), e == tgt);
-      }
-      if (p.write_grad) {
 #pragma unroll 4
         for (int vi = fa + tid; vi < fb; vi += kLanes) {
           VT t;

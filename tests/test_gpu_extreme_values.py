@@ -1,0 +1,65 @@
+"""GPU: rows that hold the lowest finite values, -inf or NaN, against the same operation in float64.
+
+A masked position is either -inf or the type's lowest finite value; both must act as "contributes nothing" wherever any
+other value is larger, and a NaN must not vanish.
+"""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def masked_logits(V, dtype, dev):
+    """One row per kind of masking, [rows, V]; the target of every row is column 1."""
+    x = torch.randn(8, V, device=dev, generator=torch.Generator(device=dev).manual_seed(V)).mul_(2).to(dtype)
+    low = torch.finfo(dtype).min
+    x[0, V // 2:] = low            # whole shares and whole vectors of the lowest value, behind and before the kept ones
+    x[1, 2:V // 2] = low
+    x[2, V // 2:] = -math.inf
+    x[3, 3 * V // 4:] = math.nan   # a share that holds nothing but NaN
+    x[4, 2:V // 2] = -math.inf
+    x[4, V // 4] = math.nan        # one NaN among masked logits
+    x[5] = low                     # nothing but the lowest value: uniform
+    x[6] = 3e38                    # so large that x * log2(e) overflows: uniform
+    x[7, 2:] = -math.inf           # two logits are left
+    return x
+
+
+# block kernel: short rows and rows of more than 800 KB; cluster kernel: 1, 2, 4 and 8 CTAs per row, rows of whole and of
+# partial vectors; in place (the training step's form) always the block kernel
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("V", [50, 5000, 5001, 9000, 32000, 50257, 151936, 420001])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_cross_entropy_of_masked_logits(cuda_device, dtype, V, in_place):
+    from metal_candle_b200 import _lib, backend
+    from metal_candle_b200.training import cross_entropy_loss
+
+    x = masked_logits(V, dtype, cuda_device)
+    lib = _lib.load()
+    for row in range(x.shape[0]):
+        r64 = x[row].double()
+        # log_softmax by hand: the largest logit first, so that nothing overflows
+        d = r64 - r64[~r64.isnan()].max()
+        logp = d - d.exp().sum().log()
+        want, want_g = -logp[1], logp.exp()
+        want_g[1] -= 1.0
+        if in_place:
+            g = x[row].clone()
+            t = torch.ones(1, dtype=torch.int32, device=cuda_device)
+            nll, count, loss = torch.empty(1, device=cuda_device), torch.empty_like(t), torch.empty(2, device=cuda_device)
+            _lib.check(lib.mcb_cross_entropy(g.data_ptr(), t.data_ptr(), nll.data_ptr(), count.data_ptr(), loss.data_ptr(), 1, V, 1,
+                                             backend._dtype_code(g), backend._stream()))
+        else:
+            t = torch.ones(1, 1, dtype=torch.int64, device=cuda_device)
+            loss, g = cross_entropy_loss(x[row].clone().view(1, 1, V), t, return_grad=True)
+            g = g.view(-1)
+        if want.isnan():
+            assert loss[0].isnan() and g.isnan().all(), row
+            continue
+        # float32 sums of exponentials of 2^-22 each; a gradient element is rounded to its type once
+        assert abs(float(loss[0]) - float(want)) <= 1e-5 * abs(float(want)) + 1e-6, (row, float(loss[0]), float(want))
+        rel = 2.0 ** -8 if dtype == torch.bfloat16 else 2e-5
+        assert ((g.double() - want_g).abs() <= rel * want_g.abs() + 1e-7).all(), row
+    assert _lib.device_status() == 0
