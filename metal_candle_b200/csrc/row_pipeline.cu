@@ -678,6 +678,9 @@ int try_launch(int op, const void* in0, const void* in1, const void* w, void* ou
   constexpr int N = Vec16<T>::N;
   const bool softmax = op == kSmFwd || op == kSmBwd;
   if (D > (1 << 20)) return 1;
+  // The forward scales the maximum instead of every score, which needs a positive finite scale: with scale <= 0 the largest
+  // score is not the largest product, and 0 * -inf of a masked score is NaN.  The register kernels scale first.
+  if (op == kSmFwd && !(scale > 0.0f && scale < INFINITY)) return 1;
   const uintptr_t at0 = reinterpret_cast<uintptr_t>(in0), at1 = reinterpret_cast<uintptr_t>(in1 ? in1 : in0), ato = reinterpret_cast<uintptr_t>(out);
   const bool rag = D % N != 0 || ((at0 | at1 | ato) & 15u) != 0;
   if (rag && !(softmax && ((at0 ^ at1) & 15u) == 0 && ((at0 ^ ato) & 15u) == 0 && at0 % sizeof(T) == 0 && D >= 2 * N)) return 1;

@@ -63,3 +63,21 @@ def test_cross_entropy_of_masked_logits(cuda_device, dtype, V, in_place):
         rel = 2.0 ** -8 if dtype == torch.bfloat16 else 2e-5
         assert ((g.double() - want_g).abs() <= rel * want_g.abs() + 1e-7).all(), row
     assert _lib.device_status() == 0
+
+
+# rows of whole and of partial 16-byte vectors, held in registers and streamed
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("seq", [64, 65, 776, 777, 1030, 2100])
+@pytest.mark.parametrize("scale", [0.125, 0.0, -0.5])
+def test_causal_softmax_of_any_scale(cuda_device, dtype, seq, scale):
+    from metal_candle_b200 import _lib, backend
+
+    rows = 2 * seq
+    x = torch.randn(rows, seq, device=cuda_device, generator=torch.Generator(device=cuda_device).manual_seed(seq)).mul_(4).to(dtype)
+    y = torch.full_like(x, math.nan)
+    _lib.check(_lib.load().mcb_softmax_causal_fwd(x.data_ptr(), y.data_ptr(), rows, seq, seq, scale, backend._dtype_code(x), backend._stream()))
+    mask = torch.ones(seq, seq, dtype=torch.bool, device=cuda_device).triu(1).repeat(2, 1)
+    want = torch.softmax((x.double() * scale).masked_fill(mask, -math.inf), -1)
+    # bfloat16: rounded to its type once; float32: exponents up to 40, each product and difference rounded to 2^-24 of that
+    rel = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-5
+    assert ((y.double() - want).abs() <= rel * want + 1e-30).all()
