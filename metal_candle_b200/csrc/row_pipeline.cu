@@ -83,6 +83,24 @@ __device__ __forceinline__ void load_row(const uint8_t* s0, int lane, int nv, Ve
   }
 }
 
+// Softmax of a row whose scaled maximum is not finite, elements [lo, end) of `in`, those behind `last` masked.  Either the
+// maximum itself is finite and its product with the scale overflows (a row masked with the type's lowest value, or of values
+// near the largest): the fused form 2^(x scale - m) would be 0 or NaN where x equals the maximum, so differences come first.
+// Or it is -inf (nothing kept: all 0, but a NaN stays one) or +inf (NaN where x is +inf, 0 elsewhere).
+template <typename T>
+__device__ __forceinline__ void softmax_row_of_extremes(const T* in, T* out, int lo, int end, int last, float row_max, float sc, int lane) {
+  const float ref = row_max == -INFINITY ? 0.0f : row_max;
+  float s = 0.0f;
+#pragma unroll 1
+  for (int e = lo + lane; e < end; e += 32)
+    if (e <= last) s += fast_exp2((to_f32(in[e]) - ref) * sc);
+  s = warp_sum(s);
+  const float inv = s > 0.0f ? 1.0f / s : 0.0f;
+#pragma unroll 1
+  for (int e = lo + lane; e < end; e += 32)
+    out[e] = from_f32<T>(e <= last ? fast_exp2((to_f32(in[e]) - ref) * sc) * inv : 0.0f);
+}
+
 // bytes of a causal row that are needed: columns 0..q, rounded up to 16 bytes
 __device__ __forceinline__ uint32_t causal_bytes(int q, int elem_bytes, int row_bytes) {
   uint32_t b = (static_cast<uint32_t>(q + 1) * elem_bytes + 15u) & ~15u;
@@ -446,25 +464,28 @@ rowpipe_kernel(const Params p) {
             for (int j = 0; j < N; ++j) m = fmaxf(m, f[j]);
           }
           if constexpr (RAG) m = fmaxf(m, xe);
-          m = warp_max(m) * sc;  // sc > 0: max commutes with the scaling
-          // Up to 32 elements per lane keep their exponentials in registers; wider rows compute them twice
-          // (once for the sum, once for the output) rather than spill.
-          constexpr bool kKeep = KMAX * N <= 32;
-          float e[kKeep ? KMAX : 1][N];
-          float inv = 0.0f, ee = 0.0f;   // ee: the edge element's exponential
-          const float2 sc2 = f2(sc, sc), nm2 = f2(-m, -m);
-          auto exps = [&](int k, float (&o)[N]) {
-            float f[N];
-            v[k].to_float(f);
-            mask(lane + 32 * k, f);
+          const float row_max = warp_max(m);
+          m = row_max * sc;  // sc > 0: max commutes with the scaling
+          if (__builtin_expect(!(fabsf(m) < INFINITY), 0)) {
+            softmax_row_of_extremes(reinterpret_cast<const T*>(s0), orow, lo, lo + p.D, q, row_max, sc, lane);
+          } else {
+            // Up to 32 elements per lane keep their exponentials in registers; wider rows compute them twice
+            // (once for the sum, once for the output) rather than spill.
+            constexpr bool kKeep = KMAX * N <= 32;
+            float e[kKeep ? KMAX : 1][N];
+            float ee = 0.0f;   // the edge element's exponential
+            const float2 sc2 = f2(sc, sc), nm2 = f2(-m, -m);
+            auto exps = [&](int k, float (&o)[N]) {
+              float f[N];
+              v[k].to_float(f);
+              mask(lane + 32 * k, f);
 #pragma unroll
-            for (int j = 0; j < N; j += 2) {
-              const float2 a = __ffma2_rn(f2(f[j], f[j + 1]), sc2, nm2);
-              o[j] = fast_exp2(a.x);
-              o[j + 1] = fast_exp2(a.y);
-            }
-          };
-          if (m != -INFINITY) {
+              for (int j = 0; j < N; j += 2) {
+                const float2 a = __ffma2_rn(f2(f[j], f[j + 1]), sc2, nm2);
+                o[j] = fast_exp2(a.x);
+                o[j + 1] = fast_exp2(a.y);
+              }
+            };
             float2 acc0 = f2(0.0f, 0.0f), acc1 = f2(0.0f, 0.0f);
 #pragma unroll
             for (int k = 0; k < KMAX; ++k) {
@@ -482,35 +503,32 @@ rowpipe_kernel(const Params p) {
             }
             if constexpr (RAG) { ee = fast_exp2(fmaf(xe, sc, -m)); acc0.x += ee; }
             const float ssum = warp_sum((acc0.x + acc0.y) + (acc1.x + acc1.y));
-            inv = ssum > 0.0f ? 1.0f / ssum : 0.0f;
-          }
-          const float2 i2 = f2(inv, inv);
+            const float inv = ssum > 0.0f ? 1.0f / ssum : 0.0f;
+            const float2 i2 = f2(inv, inv);
 #pragma unroll
-          for (int k = 0; k < KMAX; ++k) {
-            const int vi = lane + 32 * k;
-            if (vi < nvec && vi >= fa) {
-              float t[N], o[N];
-              if (m == -INFINITY) {
+            for (int k = 0; k < KMAX; ++k) {
+              const int vi = lane + 32 * k;
+              if (vi < nvec && vi >= fa) {
+                float t[N], o[N];
+                if constexpr (kKeep) {
 #pragma unroll
-                for (int j = 0; j < N; ++j) t[j] = 0.0f;
-              } else if constexpr (kKeep) {
+                  for (int j = 0; j < N; ++j) t[j] = e[k][j];
+                } else {
+                  exps(k, t);
+                }
 #pragma unroll
-                for (int j = 0; j < N; ++j) t[j] = e[k][j];
-              } else {
-                exps(k, t);
+                for (int j = 0; j < N; j += 2) {
+                  const float2 a = __fmul2_rn(f2(t[j], t[j + 1]), i2);
+                  o[j] = a.x; o[j + 1] = a.y;
+                }
+                V a;
+                a.from_float(o);
+                __stcs(reinterpret_cast<decltype(a.raw)*>(orow) + vi, a.raw);
               }
-#pragma unroll
-              for (int j = 0; j < N; j += 2) {
-                const float2 a = __fmul2_rn(f2(t[j], t[j + 1]), i2);
-                o[j] = a.x; o[j + 1] = a.y;
-              }
-              V a;
-              a.from_float(o);
-              __stcs(reinterpret_cast<decltype(a.raw)*>(orow) + vi, a.raw);
             }
-          }
-          if constexpr (RAG) {
-            if (edge >= 0) orow[edge] = from_f32<T>(ee * inv);
+            if constexpr (RAG) {
+              if (edge >= 0) orow[edge] = from_f32<T>(ee * inv);
+            }
           }
         } else if constexpr (OP == kSmFwd) {
           const int q = p.causal_seq > 0 ? static_cast<int>(row % p.causal_seq) + lo : p.D + lo;  // last kept element
@@ -527,9 +545,11 @@ rowpipe_kernel(const Params p) {
             for (int j = 0; j < N; ++j) m = fmaxf(m, (vi * N + j <= q) ? f[j] : -INFINITY);
           }
           if constexpr (RAG) m = fmaxf(m, xe);
-          m = warp_max(m) * sc;  // sc > 0: max commutes with the scaling
-          float s = 0.0f;
-          if (m != -INFINITY) {
+          const float row_max = warp_max(m);
+          m = row_max * sc;  // sc > 0: max commutes with the scaling
+          if (__builtin_expect(!(fabsf(m) < INFINITY), 0)) {
+            softmax_row_of_extremes(reinterpret_cast<const T*>(s0), orow, lo, lo + p.D, q, row_max, sc, lane);
+          } else {
             float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll 4
             for (int vi = fa + lane; vi < nv_keep; vi += 32) {
@@ -540,28 +560,26 @@ rowpipe_kernel(const Params p) {
                 part[j & 3] += (vi * N + j <= q) ? fast_exp2(fmaf(f[j], sc, -m)) : 0.0f;
             }
             if constexpr (RAG) part[0] += fast_exp2(fmaf(xe, sc, -m));
-            s = (part[0] + part[1]) + (part[2] + part[3]);
-          }
-          s = warp_sum(s);
-          const float inv = s > 0.0f ? 1.0f / s : 0.0f;
-          const float mref = (m == -INFINITY) ? 0.0f : m;
+            const float s = warp_sum((part[0] + part[1]) + (part[2] + part[3]));
+            const float inv = s > 0.0f ? 1.0f / s : 0.0f;
 #pragma unroll 4
-          for (int vi = fa + lane; vi < nvec; vi += 32) {
-            float f[N];
-            if (vi < nv_keep) {
-              V a; a.raw = reinterpret_cast<const decltype(a.raw)*>(s0)[vi];
-              a.to_float(f);
+            for (int vi = fa + lane; vi < nvec; vi += 32) {
+              float f[N];
+              if (vi < nv_keep) {
+                V a; a.raw = reinterpret_cast<const decltype(a.raw)*>(s0)[vi];
+                a.to_float(f);
 #pragma unroll
-              for (int j = 0; j < N; ++j) f[j] = (vi * N + j <= q) ? fast_exp2(fmaf(f[j], sc, -mref)) * inv : 0.0f;
-            } else {
+                for (int j = 0; j < N; ++j) f[j] = (vi * N + j <= q) ? fast_exp2(fmaf(f[j], sc, -m)) * inv : 0.0f;
+              } else {
 #pragma unroll
-              for (int j = 0; j < N; ++j) f[j] = 0.0f;
+                for (int j = 0; j < N; ++j) f[j] = 0.0f;
+              }
+              V a; a.from_float(f);
+              __stcs(reinterpret_cast<decltype(a.raw)*>(orow) + vi, a.raw);
             }
-            V a; a.from_float(f);
-            __stcs(reinterpret_cast<decltype(a.raw)*>(orow) + vi, a.raw);
-          }
-          if constexpr (RAG) {
-            if (edge >= 0) orow[edge] = from_f32<T>(fast_exp2(fmaf(xe, sc, -mref)) * inv);
+            if constexpr (RAG) {
+              if (edge >= 0) orow[edge] = from_f32<T>(fast_exp2(fmaf(xe, sc, -m)) * inv);
+            }
           }
         } else {  // kSmBwd
           const int q = p.causal_seq > 0 ? static_cast<int>(row % p.causal_seq) + lo : p.D + lo;

@@ -81,3 +81,51 @@ def test_causal_softmax_of_any_scale(cuda_device, dtype, seq, scale):
     # bfloat16: rounded to its type once; float32: exponents up to 40, each product and difference rounded to 2^-24 of that
     rel = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-5
     assert ((y.double() - want).abs() <= rel * want + 1e-30).all()
+
+
+# rows held in registers (1 to 8 vectors per lane), streamed rows, register kernels; whole and partial vectors
+SOFTMAX_WIDTHS = [64, 65, 300, 776, 777, 1040, 1041, 2050, 2104, 4097]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D", SOFTMAX_WIDTHS)
+@pytest.mark.parametrize("causal", [False, True])
+def test_softmax_of_the_largest_values(cuda_device, dtype, D, causal):
+    """Scores whose product with log2(e) overflows: rows masked with the lowest value, wholly and in part."""
+    from metal_candle_b200 import _lib, backend
+
+    low, rows = torch.finfo(dtype).min, D if causal else 96
+    x = torch.randn(rows, D, device=cuda_device, generator=torch.Generator(device=cuda_device).manual_seed(D)).to(dtype)
+    kinds = [low, 3e38, -2.5e38]
+    for i, value in enumerate(kinds):
+        x[i::8] = value
+    x[3::8, :D // 2] = low
+    x[4::8, 1:] = low
+    x[5::8, D // 3] = 3e38
+    y = torch.full_like(x, math.nan)
+    x64 = x.double()
+    if causal:
+        _lib.check(_lib.load().mcb_softmax_causal_fwd(x.data_ptr(), y.data_ptr(), rows, D, D, 1.0, backend._dtype_code(x), backend._stream()))
+        x64 = x64.masked_fill(torch.ones(D, D, dtype=torch.bool, device=cuda_device).triu(1), -math.inf)
+    else:
+        backend.softmax_fused(x, out=y)
+    want = torch.softmax(x64, -1)
+    rel = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-5
+    assert ((y.double() - want).abs() <= rel * want + 1e-30).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D", SOFTMAX_WIDTHS)
+def test_softmax_keeps_nan_and_clears_masked_rows(cuda_device, dtype, D):
+    from metal_candle_b200 import backend
+
+    x = torch.randn(96, D, device=cuda_device, generator=torch.Generator(device=cuda_device).manual_seed(D)).to(dtype)
+    x[0::4] = math.nan
+    x[1::4] = -math.inf
+    x[2::4] = -math.inf
+    x[2::4, D // 2] = math.nan
+    y = backend.softmax_fused(x)
+    assert y[0::4].isnan().all()
+    assert (y[1::4] == 0).all()                     # nothing kept: zeros
+    assert y[2::4, D // 2].isnan().all()
+    torch.testing.assert_close(y[3::4].double(), torch.softmax(x[3::4].double(), -1), rtol=2.0 ** -8 if dtype == torch.bfloat16 else 1e-5, atol=1e-30)
