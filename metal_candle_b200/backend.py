@@ -12,6 +12,8 @@ back to it: a tensor that is not on a CUDA device is an error.
 """
 from __future__ import annotations
 
+import threading
+
 import torch
 
 from . import _lib
@@ -49,30 +51,53 @@ def _stream():
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
+def _capturing() -> bool:
+    return torch._C._cuda_isCurrentStreamCapturing()
+
+
 def _lib_for(t: torch.Tensor):
     return _lib.init(t.device.index if t.device.index is not None else torch.cuda.current_device())
 
 
-_ws_cache = {}
+class _Scratch(threading.local):
+    """This thread's scratch buffers by (device index, stream handle), the least recently made first."""
+
+    def __init__(self):
+        self.buffers = {}
+
+
+_scratch = _Scratch()
+_SCRATCH_STREAMS = 8   # buffers a thread keeps; a program that uses more streams than that allocates again
+
+
+def _new_scratch(device: torch.device, nbytes: int) -> torch.Tensor:
+    raw = torch.empty(max(nbytes, 1 << 20) + 1024, dtype=torch.uint8, device=device)
+    off = (-raw.data_ptr()) % 1024
+    return raw[off:off + max(nbytes, 1 << 20)]
 
 
 def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    """A per-device scratch buffer that only grows.  The returned view starts on a 1024-byte boundary (the
-    bf16 GEMM requires it; torch's allocator only promises 512)."""
-    key = (device.type, device.index)
-    buf = _ws_cache.get(key)
+    """Scratch memory for one call on the current stream, starting on a 1024-byte boundary (the bf16 GEMM requires it;
+    torch's allocator only promises 512).  A call's kernels write it and read it back, so whatever else uses the same
+    bytes has to come before or after all of them in stream order: each stream has a buffer of its own, which only grows,
+    and each thread (whose launches can fall between another's) its own set.  A buffer is made on the stream it serves, so
+    one that is replaced goes back to that stream's pool, behind the kernels that still read it.  While a CUDA graph is
+    being captured the memory comes from the graph's pool: its address is part of the graph, and nothing outgrows it."""
+    if _capturing():
+        return _new_scratch(device, nbytes)
+    buffers, key = _scratch.buffers, (device.index, _stream())
+    buf = buffers.get(key)
     if buf is None or buf.numel() < nbytes:
-        raw = torch.empty(max(nbytes, 1 << 20) + 1024, dtype=torch.uint8, device=device)
-        off = (-raw.data_ptr()) % 1024
-        buf = raw[off:off + max(nbytes, 1 << 20)]
-        _ws_cache[key] = buf
+        buffers.pop(key, None)
+        while len(buffers) >= _SCRATCH_STREAMS:
+            del buffers[next(iter(buffers))]
+        buf = buffers[key] = _new_scratch(device, nbytes)
     return buf
 
 
 def workspace_refs(device: torch.device):
-    """The scratch buffer currently cached for `device` (a list of zero or one tensors).  Whoever bakes its address
-    into something replayable (a CUDA graph) keeps these references for as long as that thing lives."""
-    buf = _ws_cache.get((device.type, device.index))
+    """The scratch buffer this thread has for the current stream of `device` (a list of zero or one tensors)."""
+    buf = _scratch.buffers.get((device.index, _stream()))
     return [] if buf is None else [buf]
 
 

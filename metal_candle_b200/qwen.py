@@ -79,14 +79,9 @@ class _Linear:
 class CapturedStep:
     """forward_backward of a fixed shape as a CUDA graph (Qwen.capture_forward_backward)."""
 
-    def __init__(self, graph, ids, targets, loss, grads, keepalive=(), count=None):
+    def __init__(self, graph, ids, targets, loss, grads, count=None):
         self.graph, self.ids, self.targets, self.loss, self.grads = graph, ids, targets, loss, grads
         self.count = count   # int32 [1]: targets of the last replayed batch that were not ignored
-        # The graph's kernels carry the ADDRESSES of the scratch buffers that were current at capture time (GEMM
-        # operand packs, partial sums, attention and RMSNorm scratch).  The per-device scratch buffer is replaced
-        # when a later call needs a larger one; holding the captured ones here keeps their memory from being handed
-        # to another tensor while this graph can still be replayed.
-        self._keepalive = list(keepalive)
 
     def __call__(self, input_ids: torch.Tensor, target_ids: torch.Tensor):
         """Copies the batch into the graph's input buffers (device to device, or from pinned host memory) and
@@ -434,7 +429,7 @@ class Qwen:
     def capture_forward_backward(self, batch: int, seq: int, keep_hooks: bool = False, pool=None) -> "CapturedStep":
         """Records forward_backward for one (batch, seq) shape into a CUDA graph.  The step is some thousand
         short launches; replayed from a graph they run back to back without the host in the loop.  Call it
-        after at least one eager forward_backward of the same shape (kernel attributes and cached workspaces
+        after at least one eager forward_backward of the same shape (kernel attributes and the re-laid weights
         are set up on first use, which must not happen during capture).  The adapter's tensors are read in
         place, so optimizer updates between replays are seen; inputs go into the returned object's `ids` and
         `targets` buffers.  `keep_hooks` leaves `layer_done_hook` / `backward_done_hook` installed during the
@@ -451,7 +446,6 @@ class Qwen:
         was_profiling = _lib.profile_enabled()
         _lib.profile_enable(False)                                # per-launch events cannot be recorded either
         graph = torch.cuda.CUDAGraph()
-        keep = backend.workspace_refs(self.device)   # the scratch buffer the first captured kernels will point at
         try:
             torch.cuda.synchronize(self.device)
             with torch.cuda.graph(graph, pool=pool, capture_error_mode="thread_local"):
@@ -459,8 +453,7 @@ class Qwen:
         finally:
             self.layer_done_hook, self.backward_done_hook = hook, done_hook
             _lib.profile_enable(was_profiling)
-        return CapturedStep(graph, ids, targets, loss, grads, keepalive=keep + backend.workspace_refs(self.device),
-                            count=self.last_count)
+        return CapturedStep(graph, ids, targets, loss, grads, count=self.last_count)
 
     def _layer_bwd(self, dh3, L, sv, idx, B, S, accumulate):
         c = self.config

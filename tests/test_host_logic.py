@@ -157,3 +157,41 @@ def test_oracle_dropout_mask_is_a_pure_function_of_seed_and_position():
     y = R.lora_forward_dropout(x, A, B, 2.0, 0.5, 11, 0)
     keep = R.dropout_mask(8, 0.5, 11, 0).reshape(4, 2)
     assert np.allclose(y, (np.where(keep, 3.0 / 0.5, 0.0) @ B) * 2.0)
+
+
+def test_scratch_belongs_to_one_thread_and_stream(monkeypatch):
+    """A call's kernels write their scratch memory and read it back: no two streams and no two threads share it, a buffer
+    that is outgrown is replaced for its own stream alone, and a capture takes none of them."""
+    import threading
+
+    from metal_candle_b200 import backend
+
+    now = {"stream": 1, "capturing": False}
+    monkeypatch.setattr(backend, "_stream", lambda: now["stream"])
+    monkeypatch.setattr(backend, "_capturing", lambda: now["capturing"])
+    monkeypatch.setattr(backend, "_scratch", backend._Scratch())
+    cpu = torch.device("cpu")
+    a = backend.workspace(cpu, 100)
+    assert a.data_ptr() % 1024 == 0 and a.numel() >= 1 << 20
+    assert backend.workspace(cpu, 1 << 20) is a and backend.workspace_refs(cpu)[0] is a
+    now["stream"] = 2
+    assert backend.workspace_refs(cpu) == []
+    b = backend.workspace(cpu, 100)
+    assert b is not a
+    big = backend.workspace(cpu, 3 << 20)
+    assert big.numel() >= 3 << 20 and backend.workspace(cpu, 100) is big
+    now["stream"] = 1
+    assert backend.workspace(cpu, 100) is a
+    other = []
+    t = threading.Thread(target=lambda: other.append(backend.workspace(cpu, 100)))
+    t.start()
+    t.join()
+    assert other[0] is not a and backend.workspace(cpu, 100) is a
+    now["capturing"] = True
+    c = backend.workspace(cpu, 100)
+    assert c is not a and backend.workspace(cpu, 100) is not c
+    now["capturing"] = False
+    for s in range(3, 40):   # however many streams a program uses, a thread keeps a few buffers
+        now["stream"] = s
+        backend.workspace(cpu, 100)
+    assert len(backend._scratch.buffers) <= backend._SCRATCH_STREAMS
