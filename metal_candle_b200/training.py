@@ -265,38 +265,48 @@ class StateError(TrainingError):
 class AdamW:
     """AdamW with decoupled weight decay.  ONE step counter is shared by all parameters and advances
     once per tensor update, as in the reference (src/training/optimizer.rs:172-176,236-238).  Parameters
-    are float32 CUDA tensors updated in place (`Var::set`, optimizer.rs:313)."""
+    are float32 CUDA tensors updated in place (`Var::set`, optimizer.rs:313).
+
+    A variable is known by where its elements lie, address and count (a buffer and a view of its first part are two
+    variables).  Its memory is held as long as its moments are, so that no other tensor can turn up at its address and be
+    taken for it; `zero_state` lets go of both."""
 
     def __init__(self, config: Optional[AdamWConfig] = None):
         self.config = AdamWConfig() if config is None else AdamWConfig(**config.__dict__)
         self.config.validate()
         self.state: Dict[object, Tuple[torch.Tensor, torch.Tensor]] = {}
+        self._held: Dict[object, torch.Tensor] = {}
         self.step_count = 0
 
     def add_parameter(self, name, param: torch.Tensor) -> None:
         self.state[name] = (torch.zeros_like(param, dtype=torch.float32), torch.zeros_like(param, dtype=torch.float32))
+        if name == self._key(param):
+            self._held[name] = param.detach()
 
     def _key(self, var: torch.Tensor):
-        return ("var", var.data_ptr())
+        return ("var", var.data_ptr(), var.numel())
 
     def state_of(self, var: torch.Tensor):
         return self.state[self._key(var)]
 
     def _launch(self, items, grad_scale: float = 1.0) -> None:
         # This loop is most of an update's time on the host: one attribute read per fact and tensor, and the descriptors
-        # packed in one go instead of as one ctypes structure per tensor (192 tensors, one update: 416 -> 237 us).
+        # packed in one go instead of as one ctypes structure per tensor (192 tensors, one update: 416 -> 237 us, 267 with the
+        # check of the moments).
         f32, words = torch.float32, []
-        for address, p, g, m, v, t in items:
+        for address, n, p, g, m, v, t in items:
             if p.dtype is not f32 or g.dtype is not f32:
                 raise TrainingError("AdamW parameters and gradients must be float32")
             if g.shape != p.shape:
                 raise TrainingError(f"gradient shape {list(g.shape)} does not match parameter {list(p.shape)}")
             if not (p.is_cuda and g.is_cuda and p.is_contiguous()):
                 backend._require_cuda(p, g)
-            words += (address, g.data_ptr(), m.data_ptr(), v.data_ptr(), p.numel(), t, 0)
+            if m.numel() != n or v.numel() != n:   # (the kernel reads and writes n elements of each)
+                raise StateError(f"moments of {m.numel()} and {v.numel()} elements do not match a parameter of {n}")
+            words += (address, g.data_ptr(), m.data_ptr(), v.data_ptr(), n, t, 0)
         table = (_lib.AdamWTensor * len(items))()
         struct.pack_into("=" + "QQQQqii" * len(items), table, 0, *words)
-        lib = backend._lib_for(items[0][1])
+        lib = backend._lib_for(items[0][2])
         c = self.config
         _lib.check(lib.mcb_adamw_multi(table, len(items), c.learning_rate, c.beta1, c.beta2, c.epsilon, c.weight_decay,
                                        float(grad_scale), backend._stream()))
@@ -307,7 +317,7 @@ class AdamW:
             raise StateError(f"parameter '{name}' not found in optimizer")
         self.step_count += 1
         m, v = self.state[name]
-        self._launch([(param.data_ptr(), param, grad.contiguous(), m, v, self.step_count)])
+        self._launch([(param.data_ptr(), param.numel(), param, grad.contiguous(), m, v, self.step_count)])
         return param
 
     def step_var(self, var: torch.Tensor, grad: torch.Tensor) -> None:
@@ -322,13 +332,13 @@ class AdamW:
         multi-tensor launch: tensor j of this call gets step number step_count + j + 1."""
         items, state = [], self.state
         for var, g in zip(variables, grads):
-            address = var.data_ptr()
-            mv = state.get(("var", address))
+            address, n = var.data_ptr(), var.numel()
+            mv = state.get(("var", address, n))
             if mv is None:
-                self.add_parameter(("var", address), var)
-                mv = state["var", address]
+                self.add_parameter(("var", address, n), var)
+                mv = state["var", address, n]
             self.step_count += 1
-            items.append((address, var, g.contiguous(), mv[0], mv[1], self.step_count))
+            items.append((address, n, var, g.contiguous(), mv[0], mv[1], self.step_count))
         if items:
             self._launch(items, grad_scale)
 
@@ -340,6 +350,7 @@ class AdamW:
 
     def zero_state(self) -> None:
         self.state.clear()
+        self._held.clear()
         self.step_count = 0
 
 

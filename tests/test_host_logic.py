@@ -195,3 +195,70 @@ def test_scratch_belongs_to_one_thread_and_stream(monkeypatch):
         now["stream"] = s
         backend.workspace(cpu, 100)
     assert len(backend._scratch.buffers) <= backend._SCRATCH_STREAMS
+
+
+class _LaunchLog:
+    """Stands in for the library: notes the descriptors of each launch instead of making it."""
+
+    def __init__(self):
+        self.launches = []
+
+    def mcb_adamw_multi(self, table, n, *rest):
+        self.launches.append([(t.p, t.g, t.m, t.v, t.n, t.t) for t in table[:n]])
+        return 0
+
+
+@pytest.fixture
+def launch_log(monkeypatch):
+    from metal_candle_b200 import backend
+
+    log = _LaunchLog()
+    monkeypatch.setattr(backend, "_lib_for", lambda t: log if torch.is_tensor(t) else None)
+    monkeypatch.setattr(backend, "_stream", lambda: 0)
+    monkeypatch.setattr(backend, "_require_cuda", lambda *t: None)
+    return log
+
+
+def test_adamw_moments_belong_to_the_elements(launch_log):
+    """A flat buffer and the view of its first elements start at one address: their moments are not the same, and neither
+    is read or written past its end."""
+    flat = torch.zeros(100)
+    first = flat[:10]
+    opt = AdamW(AdamWConfig())
+    for order in ([first, flat], [flat, first], [flat[:10].view(2, 5)]):
+        opt.step_vars(order, [torch.ones_like(t) for t in order])
+        for (p, _, m, v, n, _), t in zip(launch_log.launches[-1], order):
+            em, ev = opt.state_of(t)
+            assert p == flat.data_ptr() and n == t.numel() == em.numel() == ev.numel() and (m, v) == (em.data_ptr(), ev.data_ptr())
+    assert len(opt.state) == 2
+    opt.step_var(flat, torch.ones(100))
+    assert launch_log.launches[-1][0][4] == 100 and opt.step_count == 6
+
+
+def test_adamw_refuses_moments_of_another_size(launch_log):
+    from metal_candle_b200.training import StateError
+
+    opt, p = AdamW(AdamWConfig()), torch.zeros(8)
+    opt.add_parameter("w", torch.zeros(4))
+    with pytest.raises(StateError):
+        opt.step("w", p, torch.zeros(8))
+    opt.step_vars([p], [torch.zeros(8)])
+    opt.state[opt._key(p)] = (torch.zeros(8), torch.zeros(7))
+    with pytest.raises(StateError):
+        opt.step_vars([p], [torch.zeros(8)])
+    assert len(launch_log.launches) == 1
+
+
+def test_adamw_state_is_not_inherited_through_a_reused_address(launch_log):
+    """While moments are kept, so is the memory they are known by: a later tensor cannot lie at the same address."""
+    opt = AdamW(AdamWConfig())
+    seen = set()
+    for _ in range(50):
+        p = torch.zeros(1000)
+        assert p.data_ptr() not in seen
+        seen.add(p.data_ptr())
+        opt.step_vars([p], [torch.ones(1000)])
+        del p
+    assert len(opt.state) == 50
+    opt.zero_state()
+    assert opt.state == {} and opt._held == {}
