@@ -390,7 +390,8 @@ typedef struct {
 
 /* Replaces AdamW::step / step_var (src/training/optimizer.rs:227-316) for a list of float32 tensors
  * in a few launches:  m=b1 m+(1-b1)g; v=b2 v+(1-b2)g^2; p -= lr*(m/(1-b1^t))/(sqrt(v/(1-b2^t))+eps)
- * + (wd*lr)*p.  `tensors` is a HOST array.  g is multiplied by grad_scale first (1/world size in the
+ * + (wd*lr)*p.  `tensors` is a HOST array; tensors whose p overlap (one listed twice, a buffer and a view of
+ * it) are updated one after the other, in the order of the list.  g is multiplied by grad_scale first (1/world size in the
  * data-parallel step; 1 otherwise). */
 int mcb_adamw_multi(const mcb_adamw_tensor* tensors, int n_tensors, float lr, float beta1, float beta2,
                     float eps, float weight_decay, float grad_scale, void* stream);

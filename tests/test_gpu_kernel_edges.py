@@ -299,3 +299,25 @@ def test_adamw_many_tensors(cuda_device, count):
             b.step_var(p, gr)
     assert a.step_count == b.step_count == 2 * count
     assert all(torch.equal(p, q) for p, q in zip(together, single))
+
+
+@pytest.mark.parametrize("count", [2, 70, 200, 300])
+def test_adamw_of_overlapping_tensors(cuda_device, count):
+    """A parameter listed twice, and a buffer next to views of it: the update is that of one tensor after the other."""
+    from metal_candle_b200.training import AdamW, AdamWConfig
+
+    def lists(seed):
+        g = torch.Generator(device=cuda_device).manual_seed(seed)
+        flat = torch.randn(5000, device=cuda_device, generator=g)
+        others = [torch.randn(1000 + i, device=cuda_device, generator=g) for i in range(count - 2)]
+        variables = [flat[100:3000]] + others + [flat]
+        variables[count // 2:count // 2] = [flat[100:3000], flat[:200]]
+        return flat, variables, [torch.randn(v.shape, device=cuda_device, generator=g) for v in variables]
+
+    (flat_a, vars_a, grads), (flat_b, vars_b, _) = lists(1), lists(1)
+    a, b = AdamW(AdamWConfig()), AdamW(AdamWConfig())
+    for _ in range(3):
+        a.step_vars(vars_a, grads)
+        for p, gr in zip(vars_b, grads):
+            b.step_var(p, gr)
+    assert torch.equal(flat_a, flat_b) and all(torch.equal(p, q) for p, q in zip(vars_a, vars_b))
