@@ -25,7 +25,11 @@ struct DeviceState {
   long long* selftest_out = nullptr;  // three device words behind the status word (mcb_selftest_wait_timeout)
   bool f32_tile_smem = false;  // the float32 tile kernel's shared-memory limit has been raised
   bool ce_smem[2] = {false, false};  // the same of the cross-entropy cluster kernel (bf16, float32)
-  int ce_clusters[2][9] = {};  // its resident clusters, by dtype and cluster size; 0 = not asked yet
+  struct ResidentClusters {
+    size_t smem = 0;  // shared memory of a CTA the answer holds for; 0 = no answer yet
+    int count = 0;
+  };
+  ResidentClusters ce_clusters[2][9][4];  // its resident clusters, by dtype and cluster size: the last four shared-memory sizes
   int split_clusters[9] = {};  // clusters of the split GEMM kernel the device runs at once, by cluster size
   void* encode_tiled = nullptr;  // cuTensorMapEncodeTiled resolved through the runtime
 };

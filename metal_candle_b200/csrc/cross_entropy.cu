@@ -3,6 +3,8 @@
 // over the logits or into a tensor of its own.  A second tiny kernel sums nll in row order, so the loss is deterministic.
 #include <cooperative_groups.h>
 
+#include <mutex>
+
 #include "common.cuh"
 #include "umma_ptx.cuh"
 
@@ -508,6 +510,23 @@ prepare_targets_kernel(const I* __restrict__ targets, int32_t* __restrict__ t32,
   if (threadIdx.x == 2) info[2] = 0;   // the row kernel's count of finished CTAs
 }
 
+// Clusters of the launch `cfg` describes that the device runs at once.  The answer depends on the vocabulary through the
+// CTAs' shared memory (float32, 8 CTAs a row: 25 KB at 50257 columns, 76 KB at 151936, 688 and 384 CTAs); the query
+// takes microseconds, so the last few answers are kept.
+template <typename T>
+int resident_clusters(const cudaLaunchConfig_t& cfg, DeviceState::ResidentClusters (&kept)[4], int* count) {
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lock(mu);
+  for (const auto& k : kept)
+    if (k.smem == cfg.dynamicSmemBytes) { *count = k.count; return MCB_OK; }
+  int n = 0;
+  MCB_CHECK_CUDA(cudaOccupancyMaxActiveClusters(&n, cross_entropy_cluster_kernel<T>, &cfg));
+  for (int i = 3; i > 0; --i) kept[i] = kept[i - 1];
+  kept[0].smem = cfg.dynamicSmemBytes;
+  kept[0].count = *count = n > 0 ? n : 1;
+  return MCB_OK;
+}
+
 // Row kernel launch: in -> out (which may be the same tensor); out is null when no gradient is wanted.
 template <typename T>
 int launch_rows(const void* in, void* out, const int32_t* targets, float* nll, const int32_t* count, int64_t M, int64_t V, int write_grad,
@@ -542,12 +561,8 @@ int launch_rows(const void* in, void* out, const int32_t* targets, float* nll, c
     attr[0].val.clusterDim.x = static_cast<unsigned>(ctas); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
     // as many clusters as are resident together: a later one would start its share of the rows when the others are done
-    int& resident = ds->ce_clusters[sizeof(T) == 4][ctas];
-    if (resident == 0) {
-      int n = 0;
-      MCB_CHECK_CUDA(cudaOccupancyMaxActiveClusters(&n, cross_entropy_cluster_kernel<T>, &cfg));
-      resident = n > 0 ? n : 1;
-    }
+    int resident = 0;
+    if (int rc = resident_clusters<T>(cfg, ds->ce_clusters[sizeof(T) == 4][ctas], &resident)) return rc;
     cfg.gridDim = dim3(static_cast<unsigned>((M < resident ? M : resident) * ctas));
     const cudaError_t e = cudaLaunchKernelEx(&cfg, cross_entropy_cluster_kernel<T>, p);
     if (e != cudaSuccess) return cuda_fail(e, "cross_entropy_cluster_kernel launch");

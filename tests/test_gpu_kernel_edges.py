@@ -321,3 +321,42 @@ def test_adamw_of_overlapping_tensors(cuda_device, count):
         for p, gr in zip(vars_b, grads):
             b.step_var(p, gr)
     assert torch.equal(flat_a, flat_b) and all(torch.equal(p, q) for p, q in zip(vars_a, vars_b))
+
+
+def test_loss_grid_does_not_depend_on_earlier_vocabularies(cuda_device, tmp_path):
+    """Two vocabularies whose rows take the same number of CTAs but other amounts of shared memory: the grid of either is the
+    same whichever a process meets first."""
+    import json
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    child = """
+import json, sys
+import torch
+from torch.profiler import ProfilerActivity, profile
+from metal_candle_b200.training import cross_entropy_loss
+t = torch.zeros(1, 400, dtype=torch.int64, device="cuda")
+vocabularies = [int(v) for v in sys.argv[2:]]
+for v in vocabularies:
+    cross_entropy_loss(torch.zeros(1, 400, v, device="cuda"), t, return_grad=True)
+grids = {}
+for v in vocabularies:
+    x = torch.zeros(1, 400, v, device="cuda")
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        cross_entropy_loss(x, t, return_grad=True)
+        torch.cuda.synchronize()
+    p.export_chrome_trace(sys.argv[1])
+    grids[v] = [e["args"]["grid"] for e in json.load(open(sys.argv[1]))["traceEvents"] if "cluster_kernel" in e.get("name", "")]
+print(json.dumps(grids))
+"""
+    runs = []
+    for order in (("50257", "151936"), ("151936", "50257")):
+        r = subprocess.run([sys.executable, "-c", child, str(tmp_path / "trace.json"), *order], capture_output=True, text=True,
+                           cwd=Path(__file__).resolve().parent.parent, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        runs.append(json.loads(r.stdout.splitlines()[-1]))
+    if not all(runs[0].values()):
+        pytest.skip("no kernel records from the profiler")
+    assert runs[0] == runs[1]
+    assert runs[0]["50257"] != runs[0]["151936"]
