@@ -506,7 +506,7 @@ int rank_product(cudaStream_t st, const float* x, const float* F, int64_t fk, in
 }
 
 int check_sizes(const LoraArgs& a) {
-  if (a.M > 0x7fffff00ll || a.N > 0x7fffff00ll || a.K > 0x7fffff00ll) return fail(MCB_ERR_SHAPE, "f32 path: dimension exceeds 2^31");
+  if (a.M > 0x7fffff00ll || a.N > 0x7fffff00ll || a.K > 0x7fffff00ll) return fail(MCB_ERR_SHAPE, "LoRA kernels: dimension exceeds 2^31");
   return MCB_OK;
 }
 
@@ -525,6 +525,7 @@ size_t workspace_bytes(int64_t M, int64_t K, int64_t N, int64_t r) {
 bool delta_small(int64_t M, int64_t r) { return M <= kDeltaMaxTokens && r <= kDeltaMaxRank; }
 
 int delta_cluster(const LoraArgs& a, int dtype) {
+  if (int rc = check_sizes(a)) return rc;
   // one token per cluster is the quicker form while a thread's share of A is a few words
   const bool one = a.M <= 18 && a.r * a.K <= 8192;
   if (dtype == MCB_F32) return one ? launch_delta<float, 1>(a) : launch_delta<float, 4>(a);
@@ -532,6 +533,7 @@ int delta_cluster(const LoraArgs& a, int dtype) {
 }
 
 int delta_fwd(const LoraArgs& a) {
+  if (int rc = check_sizes(a)) return rc;
   const int64_t rp = rank_padded(a.r);
   if (a.ws_bytes < workspace_bytes(a.M, a.K, a.N, a.r) || !a.ws)
     return fail(MCB_ERR_WORKSPACE, "lora_delta_fwd(f32): workspace too small");

@@ -753,7 +753,14 @@ int pack(const LoraArgs& a, const Workspace& w, int mode) {
   return MCB_OK;
 }
 
+// ahead of the operand pack, which counts in 32 bits like the GEMM behind it
+int check_extents(const LoraArgs& a, const char* op) {
+  if (a.M > 0x7fffff00ll || a.N > 0x7fffff00ll || a.K > 0x7fffff00ll) return fail(MCB_ERR_SHAPE, "%s(bf16): dimension exceeds 2^31", op);
+  return MCB_OK;
+}
+
 int check_ws(const LoraArgs& a, const char* op) {
+  if (int rc = check_extents(a, op)) return rc;
   if (a.r == 0) return MCB_OK;
   if (a.r > 64) return fail(MCB_ERR_UNSUPPORTED, "%s(bf16): rank %lld > 64", op, (long long)a.r);
   if (!a.ws || a.ws_bytes < workspace_bytes(a.M, a.K, a.N, a.r))
@@ -965,6 +972,7 @@ int check_fused(const LoraArgs& a, const LoraSegments& sg, const char* op) {
                   (long long)sg.n_off[i], (long long)(sg.n_off[i] + sg.n[i]), (long long)a.N);
     end = sg.n_off[i] + sg.n[i];
   }
+  if (int rc = check_extents(a, op)) return rc;
   const size_t need = fused_workspace_bytes(a.M, a.K, a.N, a.r, sg.count);
   if (!a.ws || a.ws_bytes < need) return fail(MCB_ERR_WORKSPACE, "%s: workspace %zu < %zu bytes", op, a.ws_bytes, need);
   if ((reinterpret_cast<uintptr_t>(a.ws) & 1023u) != 0) return fail(MCB_ERR_ALIGN, "%s: workspace must be 1024-byte aligned", op);

@@ -360,3 +360,20 @@ print(json.dumps(grids))
         pytest.skip("no kernel records from the profiler")
     assert runs[0] == runs[1]
     assert runs[0]["50257"] != runs[0]["151936"]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("M", [1, 64, 1000])
+@pytest.mark.parametrize("K,N", [(1 << 31, 64), (64, 1 << 31), ((1 << 32) - 8, 64)])
+def test_lora_refuses_dimensions_beyond_31_bits(cuda_device, dtype, M, K, N):
+    """The kernels count in 32 bits; the ABI admits dimensions of u32.  (The buffers are small: nothing may be launched.)"""
+    from metal_candle_b200 import _lib, backend as B
+
+    small = torch.empty(1 << 20, dtype=torch.uint8, device=cuda_device)
+    at = small.data_ptr() + (-small.data_ptr()) % 1024
+    lib, code = _lib.load(), B._dtype_code(torch.empty(0, dtype=dtype))
+    before = lib.mcb_launch_count()
+    calls = (lambda: lib.mcb_lora_delta_fwd(at, at, at, at, M, K, N, 8, 2.0, code, at, 1 << 62, B._stream()),
+             lambda: lib.mcb_lora_linear_fwd(at, at, None, at, at, at, at, M, K, N, 8, 2.0, code, 0, at, 1 << 62, B._stream()))
+    for call in calls:
+        assert call() == -2 and b"2^31" in lib.mcb_last_error() and lib.mcb_launch_count() == before
