@@ -975,16 +975,17 @@ int encode(const DeviceState* ds, CUtensorMap* map, const void* ptr, int64_t inn
   return MCB_OK;
 }
 
-int check_shape(const char* who, int64_t nb, int64_t groups, int64_t seq, int64_t head_dim, int dtype, bool ragged) {
+int check_shape(const char* who, int64_t nb, int64_t groups, int64_t seq, int64_t head_dim, int dtype, bool ragged, bool backward) {
   if (dtype != MCB_BF16) return fail(MCB_ERR_UNSUPPORTED, "%s: bfloat16 only", who);
   if (head_dim != kD) return fail(MCB_ERR_UNSUPPORTED, "%s: head dimension %lld (only 64 is built)", who, (long long)head_dim);
   if (seq <= 0 || (!ragged && seq % kBQ != 0)) return fail(MCB_ERR_UNSUPPORTED, "%s: sequence length %lld is not a multiple of 128", who, (long long)seq);
   if (nb <= 0 || groups <= 0 || (!ragged && (nb > 65535 || groups > 65535)))
     return fail(MCB_ERR_SHAPE, "%s: nb=%lld groups=%lld", who, (long long)nb, (long long)groups);
   if (!ragged && nb * groups * seq > 0x7fffff00ll) return fail(MCB_ERR_SHAPE, "%s: more than 2^31 query rows", who);
-  // work items and the grids of the kernels are counted in 32 bits
-  if (seq > 65535ll * kBQ || nb > 0x0fffffffll || groups > 0x7fffffffll / nb ||
-      nb * groups > 0x7fffffffll / ((seq + kBQ - 1) / kBQ))
+  // positions and work items are counted in 32 bits; the dK / dV kernel's grid has a key block per y and up to 8 CTAs per
+  // kv head in x
+  if (seq > 0x7fffff00ll || groups > 0x7fffffffll / nb || nb * groups > 0x7fffffffll / ((seq + kBQ - 1) / kBQ) ||
+      (backward && (seq > 65535ll * kBQ || nb > 0x0fffffffll)))
     return fail(MCB_ERR_SHAPE, "%s: nb=%lld groups=%lld seq=%lld", who, (long long)nb, (long long)groups, (long long)seq);
   return MCB_OK;
 }
@@ -1041,7 +1042,7 @@ int attention_fwd(const void* q, const void* k, const void* v, void* o, float* l
                   int64_t head_dim, float scale, int dtype, int64_t kv_heads, int o_token_major, bool ragged, void* stream) {
   using namespace mcb::attn;
   if (!q || !k || !v || !o) return fail(MCB_ERR_NULL, "attention_causal_fwd: q, k, v or o is null");
-  if (int rc = check_shape("attention_causal_fwd", nb, groups, seq, head_dim, dtype, ragged)) return rc;
+  if (int rc = check_shape("attention_causal_fwd", nb, groups, seq, head_dim, dtype, ragged, false)) return rc;
   if (o_token_major && (kv_heads <= 0 || nb % kv_heads != 0))
     return fail(MCB_ERR_SHAPE, "attention_causal_fwd: nb=%lld is not a multiple of kv_heads=%lld", (long long)nb, (long long)kv_heads);
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o)) return fail(MCB_ERR_ALIGN, "attention_causal_fwd: 16-byte alignment");
@@ -1106,7 +1107,7 @@ int attention_bwd(const void* q, const void* k, const void* v, const void* o, co
     return fail(MCB_ERR_SHAPE, "attention_causal_bwd: nb=%lld is not a multiple of kv_heads=%lld", (long long)nb, (long long)kv_heads);
   if (!q || !k || !v || !o || !dout || !lse || !dq || !dk || !dv)
     return fail(MCB_ERR_NULL, "attention_causal_bwd: a required pointer is null");
-  if (int rc = check_shape("attention_causal_bwd", nb, groups, seq, head_dim, dtype, ragged)) return rc;
+  if (int rc = check_shape("attention_causal_bwd", nb, groups, seq, head_dim, dtype, ragged, true)) return rc;
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o) || !aligned16(dout) || !aligned16(dq) ||
       !aligned16(dk) || !aligned16(dv))
     return fail(MCB_ERR_ALIGN, "attention_causal_bwd: 16-byte alignment");

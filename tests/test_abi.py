@@ -111,3 +111,28 @@ def test_host_only_entry_points_work_without_a_gpu():
     bad = _lib.QwenConfig(151936, 896, 4864, 24, 7, 1, 1e-6, 1e6)                      # head_dim 128
     assert lib.mcb_qwen_arena_bytes(C.byref(bad), entries, 96, 16, 1, 128) == 0
     assert b"head_dim" in lib.mcb_last_error()
+
+
+def test_attention_length_limits():
+    """The forward counts positions in 32 bits; only the backward's grid ends at 65535 key blocks of 128.  Pointers off a
+    16-byte boundary are refused behind the shape, so nothing is launched either way."""
+    from metal_candle_b200 import _lib
+
+    lib = _lib.load()
+    long, ws = 65536 * 128, 1 << 40
+
+    def fwd(nb, groups, seq, ragged):
+        f = lib.mcb_attention_causal_fwd_ragged if ragged else lib.mcb_attention_causal_fwd_ex
+        return f(8, 8, 8, 8, 8, nb, groups, seq, 64, 0.125, _lib.MCB_BF16, 0, 0, None, 0, None)
+
+    def bwd(nb, groups, seq, ragged):
+        f = lib.mcb_attention_causal_bwd_ragged if ragged else lib.mcb_attention_causal_bwd_ex
+        return f(8, 8, 8, 8, 8, 8, 8, 8, 8, nb, groups, seq, 64, 0.125, _lib.MCB_BF16, 0, 0, 1024, ws, None)
+
+    shape, align = -2, -3
+    for ragged in (False, True):
+        assert fwd(1, 1, long, ragged) == align and fwd(2, 7, long, ragged) == align
+        assert fwd(1, 1, 0x7fffff00, ragged) == align and fwd(1, 1, 0x7fffff80, ragged) == shape
+        assert bwd(1, 1, long - 128, ragged) == align and bwd(1, 1, long, ragged) == shape
+    assert fwd(1, 1, long + 1, True) == align and fwd(1 << 28, 1, 1, True) == align and fwd(1 << 28, 8, 1, True) == shape
+    assert bwd(1 << 28, 1, 1, True) == shape and fwd(65536, 1, 128, False) == shape
