@@ -790,8 +790,16 @@ int delta_fwd(const LoraArgs& a, const DeviceState* ds) {
   // Few tokens: one cluster launch in float32 arithmetic instead of the operand pack and a GEMM of one or two 128-row
   // tiles.  64 x 1024 -> 1024 r16: 4.8 us against 14.2; 256 x 4096 -> 4096 r64: 33 against 38.  Beyond that the tensor
   // cores win.  (Sizes and alignment that the GEMM refuses are still refused, below.)
-  if (a.M <= 256 && f32path::delta_small(a.M, a.r) && a.K % 8 == 0 && a.N % 8 == 0 && aligned16(a.x) && aligned16(a.y))
-    return f32path::delta_cluster(a, MCB_BF16);
+  if (a.M <= 256 && f32path::delta_small(a.M, a.r) && a.K % 8 == 0 && a.N % 8 == 0 && aligned16(a.x) && aligned16(a.y)) {
+    const bool prof = profile_on();
+    if (prof) {
+      const double m = static_cast<double>(a.M), kn = static_cast<double>(a.K + a.N), r = static_cast<double>(a.r);
+      profile_begin(kProfGemmLora, 2.0 * m * r * kn, 2.0 * m * kn + 4.0 * r * kn, a.stream);
+    }
+    const int rc = f32path::delta_cluster(a, MCB_BF16);
+    if (prof) profile_end(a.stream);
+    return rc;
+  }
   Workspace w = carve(a.ws, a.M, a.K, a.N, a.r);
   if (int rc = pack(a, w, 0)) return rc;
   GemmCall c;

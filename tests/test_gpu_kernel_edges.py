@@ -377,3 +377,21 @@ def test_lora_refuses_dimensions_beyond_31_bits(cuda_device, dtype, M, K, N):
              lambda: lib.mcb_lora_linear_fwd(at, at, None, at, at, at, at, M, K, N, 8, 2.0, code, 0, at, 1 << 62, B._stream()))
     for call in calls:
         assert call() == -2 and b"2^31" in lib.mcb_last_error() and lib.mcb_launch_count() == before
+
+
+@pytest.mark.parametrize("M", [1, 5, 256, 257])
+def test_bf16_delta_is_recorded_by_the_profile(cuda_device, M):
+    """Both forms of the delta (one cluster launch up to 256 tokens, the GEMM beyond) report to the per-kernel profile."""
+    from metal_candle_b200 import _lib, backend as B
+
+    K, N, r = 512, 384, 8
+    x = torch.zeros(M, K, dtype=torch.bfloat16, device=cuda_device)
+    A, Bm = torch.zeros(K, r, device=cuda_device), torch.zeros(r, N, device=cuda_device)
+    _lib.profile_enable(True)
+    try:
+        _lib.profile_summary(2)
+        B.lora_forward_fused(x, A, Bm, 2.0)
+        launches, ms, flops, _ = _lib.profile_summary(2)
+    finally:
+        _lib.profile_enable(False)
+    assert launches == 1 and ms > 0 and flops == 2.0 * M * r * (K + N)
