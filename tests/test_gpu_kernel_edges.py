@@ -111,10 +111,10 @@ def test_softmax_causal_ragged_rows(cuda_device, dtype, seq):
     assert np.all(back(dx)[:, np.triu_indices(seq, 1)[0], np.triu_indices(seq, 1)[1]] == 0)
 
 
-# the loss: short rows (block kernel), rows over 1, 2, 4 and 8 CTAs, rows that are no whole vectors, more rows than clusters,
-# ignored targets, int32 and int64 targets
+# the loss: short rows (block kernel), rows over 1, 2 (32000 bfloat16), 4 (32000 float32) and 8 CTAs, rows that are no whole
+# vectors, more rows than clusters, ignored targets, int32 and int64 targets
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("rows,V,tdtype", [(5, 50, torch.int64), (3, 8192, torch.int32), (700, 8193, torch.int64), (90, 50257, torch.int32),
+@pytest.mark.parametrize("rows,V,tdtype", [(5, 50, torch.int64), (3, 8192, torch.int32), (700, 8193, torch.int64), (30, 32000, torch.int32), (90, 50257, torch.int32),
                                            (160, 60001, torch.int64), (40, 151936, torch.int64)])
 def test_cross_entropy_rows(cuda_device, dtype, rows, V, tdtype):
     from metal_candle_b200 import _lib
@@ -144,6 +144,40 @@ def test_cross_entropy_rows(cuda_device, dtype, rows, V, tdtype):
                                              0 if dtype == torch.float32 else 1, torch.cuda.current_stream().cuda_stream))
     assert R.max_abs_normalised(back(xt), want / keep.sum()) <= TOL[dtype] and int(cnt) == int(keep.sum())
     assert abs(float(ls[0]) - nll.mean()) <= 1e-5 * abs(nll.mean())
+    assert _lib.device_status() == 0
+
+
+# logits and gradient that start off a 16-byte boundary: by the same amount (the cluster kernel, elements in front of the
+# first whole vector), by different ones (the block kernel); what surrounds the gradient is not written
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("V", [8193, 32000, 50257])
+@pytest.mark.parametrize("shift,out_shift", [(0, 0), (1, 1), (3, 3), (3, 0), (1, 2)])
+def test_cross_entropy_of_shifted_rows(cuda_device, dtype, V, shift, out_shift):
+    from metal_candle_b200 import _lib, backend as B
+
+    rows = 7
+    x = rounded(S.normal(44, "x", (rows, V)) * 2, dtype)
+    t = torch.tensor([0, V - 1, -1, 5, V // 2, 1, V - 2], device=cuda_device)
+    buf = torch.full((rows * V + shift + 8,), 100.0, dtype=dtype, device=cuda_device)   # a neighbour would win every maximum
+    buf[shift:shift + rows * V] = torch.from_numpy(np.ascontiguousarray(x)).to(cuda_device).to(dtype).view(-1)
+    out = torch.full((rows * V + out_shift + 8,), float("nan"), dtype=dtype, device=cuda_device)
+    t32, info = (torch.empty(n, dtype=torch.int32, device=cuda_device) for n in (rows, 3))
+    nll, loss = (torch.empty(n, device=cuda_device) for n in (rows, 2))
+    e = buf.element_size()
+    _lib.check(_lib.load().mcb_cross_entropy_out(buf.data_ptr() + shift * e, out.data_ptr() + out_shift * e, t.data_ptr(), 8, 0, 0, t32.data_ptr(),
+                                                 info.data_ptr(), None, None, nll.data_ptr(), loss.data_ptr(), rows, V,
+                                                 B._dtype_code(buf), B._stream()))
+    x64 = x.astype(np.float64)
+    p = np.exp(x64 - x64.max(-1, keepdims=True))
+    p /= p.sum(-1, keepdims=True)
+    keep, at = (t >= 0).cpu().numpy(), np.maximum(t.cpu().numpy(), 0)
+    want_nll = np.where(keep, -np.log(p[np.arange(rows), at]), 0.0)
+    p[np.arange(rows), at] -= 1.0
+    got = out[out_shift:out_shift + rows * V].view(rows, V)
+    assert np.abs(back(nll) - want_nll).max() <= 1e-5 * np.abs(want_nll).max()
+    assert abs(float(loss[0]) - want_nll.sum() / keep.sum()) <= 1e-5 * want_nll.mean()
+    assert R.max_abs_normalised(back(got), np.where(keep[:, None], p, 0.0) / keep.sum()) <= TOL[dtype]
+    assert torch.isnan(out[:out_shift]).all() and torch.isnan(out[out_shift + rows * V:]).all()
     assert _lib.device_status() == 0
 
 
@@ -187,9 +221,9 @@ def test_gate_up_swiglu_few_tokens(cuda_device, M, K, F):
         assert R.max_abs_normalised(back(got), want) <= 2e-2
 
 
-# key blocks x kv heads from one to more than the SMs, so that every number of CTAs sharing a key block occurs; (1, 1, 128)
-# has fewer query steps than the CTAs that share its key block
-@pytest.mark.parametrize("nb,G,seq", [(1, 1, 128), (1, 7, 128), (4, 7, 256), (16, 3, 512), (40, 2, 512)])
+# key blocks x kv heads from one to more than the SMs: 1, 4, 8, 2 and 1 CTAs share a key block, 4 and 8 in the last two, whose
+# last key block has 2 and 4 query steps, so that some of its CTAs have none
+@pytest.mark.parametrize("nb,G,seq", [(1, 1, 128), (1, 7, 128), (4, 7, 256), (16, 3, 512), (40, 2, 512), (1, 1, 1024), (1, 2, 1024)])
 def test_attention_backward_shared_key_blocks(cuda_device, nb, G, seq):
     from metal_candle_b200 import backend as B
 
@@ -206,9 +240,10 @@ def test_attention_backward_shared_key_blocks(cuda_device, nb, G, seq):
         assert np.abs(back(got).reshape(want.shape) - want).max() <= 2e-2 * np.abs(want).max()
 
 
-# nb kv heads, G query heads each, S positions: one row, the edges of the 64-key blocks and 128-query tiles, remainders;
-# (2, 1, 64) and (1, 1, 1) have fewer query steps than the CTAs that share a key block
-RAGGED_ATTENTION = [(1, 1, 1), (2, 3, 5), (1, 7, 63), (2, 1, 64), (2, 7, 65), (4, 2, 111), (2, 1, 127), (1, 2, 129), (2, 2, 193), (1, 7, 333)]
+# nb kv heads, G query heads each, S positions: one row, the edges of the 64-key blocks and 128-query tiles, remainders; in
+# the last two, 4 CTAs share a key block and the last one has a single query step
+RAGGED_ATTENTION = [(1, 1, 1), (2, 3, 5), (1, 7, 63), (2, 1, 64), (2, 7, 65), (4, 2, 111), (2, 1, 127), (1, 2, 129), (2, 2, 193), (1, 7, 333),
+                    (1, 1, 897), (2, 1, 700)]
 
 
 @pytest.mark.parametrize("nb,G,seq", RAGGED_ATTENTION)
