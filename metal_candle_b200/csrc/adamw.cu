@@ -4,8 +4,8 @@
 // be kept in step with the host; parameters may take 32764 bytes); grid.y selects the tensor, grid.x strides over its
 // elements four at a time.  The q, k, v, o adapters of 24 layers are 192 tensors: three launches of 64 took 14.5 us, one
 // launch of 192 takes 10.3 (in a graph).  Up to 64 tensors take the small table: the parameters are copied into every launch.
-// HBM-bound: 28 bytes per element (read p,g,m,v; write p,m,v).  The arithmetic keeps the reference's operation order and roundings -- each candle op in
-// src/training/optimizer.rs:243-272 is one float32 rounding, so products and sums are NOT contracted
+// HBM-bound: 28 bytes per element (read p,g,m,v; write p,m,v).  The arithmetic keeps the reference's operation order and
+// roundings -- each candle op in src/training/optimizer.rs:243-272 is one float32 rounding, so products and sums are NOT contracted
 // into FMAs, and "tensor / scalar" is a multiplication by the float32 reciprocal of the scalar, as
 // candle's scalar division is an affine by 1/rhs.
 #include <algorithm>

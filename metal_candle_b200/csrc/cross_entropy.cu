@@ -36,8 +36,8 @@ constexpr float kFusedMax = 8.507059e37f;   // 2^126
 __device__ __forceinline__ bool beyond_fused(float m) { return fabsf(m) > kFusedMax && fabsf(m) != INFINITY; }
 __device__ __forceinline__ float exp_diff(float x, float m) { return ex2_ftz((x - m) * kLog2e); }
 
-// Rows that do not fit the cluster kernel below: short ones, whose share of a CTA would be a few vectors, and rows of more
-// than 800 KB.  Persistent: block b takes rows b, b + gridDim.x, ...; sweep 1 takes the maximum and the sum, sweep 2 reads the
+// Every call in place (the training step's form), and the rows the cluster kernel below does not take: short ones, rows of
+// more than 800 KB, and input and output that start differently far from a 16-byte boundary.  Persistent: block b takes rows b, b + gridDim.x, ...; sweep 1 takes the maximum and the sum, sweep 2 reads the
 // row again (from L2 while the rows in flight fit it) and writes the gradient.
 template <typename T>
 __global__ void __launch_bounds__(1024)
@@ -168,7 +168,8 @@ cross_entropy_kernel(const T* in, T* out, const int32_t* __restrict__ targets, f
 // most 40 KB let five CTAs of different rows sit on an SM, so that one's loads and stores run under another's arithmetic;
 // only four warps work on a share, because with more of them a row's fixed costs (waits, reductions, the exchange) outweigh
 // its dozen vectors per lane.  (maximum, sum) are exchanged through distributed shared memory, once per row, in rank order.
-// 1000 x 151936 bf16: 129 us = 4.7 TB/s; 12 warps on 76 KB in 8 pieces 179, 7 warps on 38 KB in 2 pieces 137.
+// 1000 x 151936 bf16: 129 us = 4.7 TB/s; 12 warps on 76 KB in 8 pieces 179, 7 warps on 38 KB in 2 pieces 137.  With the
+// kernel that checks the targets in front, 137 us; 138 since rows of extreme values have loops of their own.
 //
 // Rows lie back to back and need not be whole 16-byte vectors: a row is the vectors that cover it (`mis` elements of
 // misalignment at the start of the tensor, the same in input and output); the neighbours' elements in its first and last
@@ -537,9 +538,11 @@ int launch_rows(const void* in, void* out, const int32_t* targets, float* nll, c
   int ctas = 1;
   while (ctas < 8 && (row_vecs + ctas - 1) / ctas * 16 > kCeGoodBytes) ctas *= 2;
   const int64_t cta_vecs = (row_vecs + ctas - 1) / ctas;
-  // In place (the training step, a chunk of tokens at a time) the block kernel stays, although it is 12 % slower there: its
-  // order of summation is what the step's losses and gradients have been reproducible with.
-  // 16 KB: below that a CTA's 384 lanes have two or three vectors each and the per-row exchanges dominate
+  // In place (the training step, a chunk of tokens at a time) the block kernel stays, although it is 12 % slower there: the
+  // step's losses and gradients keep its order of summation.
+  // From 16 KB on a CTA's 128 lanes have at least eight vectors each.  Measured with the line at 1 KB, block kernel / this
+  // one: 1000 rows of 2 KB 10.9 / 11.5 us, of 8 KB 16.3 / 15.3; 16000 rows of 2 KB 88 / 61 us, of 8 KB 131 / 84.  So it is
+  // only few and very short rows that the block kernel is quicker with.
   if (in != out && row_vecs * 16 >= 16 * 1024 && cta_vecs * 16 <= kCeMaxBytes && ((ai ^ ao) & 15u) == 0 && ai % sizeof(T) == 0) {
     CeParams p;
     p.in = in; p.out = out; p.targets = targets; p.nll = nll; p.count = count;

@@ -611,7 +611,7 @@ int linear_bwd(const LoraArgs& a) {
   GradProblemF32 qb = {dy, hs, 1, pitch, 1, a.N, a.dB, static_cast<int>(a.N), a.dB ? static_cast<int>((a.N + 31) / 32) : 0};
   const int64_t jb = (a.r + kGradCols - 1) / kGradCols;
   const int64_t blocks = (qa.blocks + qb.blocks) * jb;
-  // share the tokens out while that adds resident CTAs (8 per SM) and every warp keeps 8 tokens
+  // share the tokens out until there are four CTAs per SM (eight fit), as long as every warp keeps 8 tokens
   int splits = 1;
   while (splits < 8 && blocks * splits < 4ll * ds->sm_count && a.M >= 2ll * splits * kGradWarps * 8) splits *= 2;
   int M = static_cast<int>(a.M), r = static_cast<int>(a.r), acc = a.accumulate;

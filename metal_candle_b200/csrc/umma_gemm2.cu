@@ -120,8 +120,8 @@ __host__ __device__ constexpr uint32_t make_idesc2(int n) {
 
 // Two neighbouring elements of the SwiGLU backward: d gate = d u s (1 + g (1 - s)), d up = d g s with s = sigmoid(g).
 // The epilogue warps are bound by their instruction count, so: the two approximate special functions flush
-// denormals (the compiler then adds no range handling around them; relative error about 2^-22), products are shared
-// between the two results, and the multiplies and adds run as packed pairs (one instruction for two elements).
+// denormals (the compiler then adds no range handling around them; relative error of s about 2^-22 from the functions and
+// |g| 2^-24 from the rounded exponent), products are shared between the two results, and the multiplies and adds run as packed pairs (one instruction for two elements).
 // g -> -inf gives s = 0 and both results 0; g -> +inf gives s = 1, d gate = d u, d up = d g.
 __device__ __forceinline__ void swiglu_bwd_pair(float2 d, float2 g, float2 u, float2& dgate, float2& dup) {
   const float2 a = __fmul2_rn(g, make_float2(-1.4426950408889634f, -1.4426950408889634f));
@@ -712,7 +712,9 @@ int launch_gemm2_swiglu(const __nv_bfloat16* X, const __nv_bfloat16* Wgu, __nv_b
                         __nv_bfloat16* Act, int64_t M, int64_t K, int64_t F, const DeviceState* ds, cudaStream_t st) {
   if (F % 128 != 0 || K % 8 != 0) return fail(MCB_ERR_ALIGN, "linear_swiglu: features %lld must be a multiple of 128, reduction %lld of 8", (long long)F, (long long)K);
   if (M > 0x7fffff00ll || 2 * F > 0x7fffff00ll || K > 0x7fffff00ll) return fail(MCB_ERR_SHAPE, "linear_swiglu: dimension exceeds 2^31");
-  // up to one round of 128-token tiles over the SMs, one-CTA tiles (umma_split.cu) end earlier than 256-token pairs
+  // Up to one round of 128-token tiles over the SMs, one-CTA tiles (umma_split.cu) end earlier than 256-token pairs: pairs /
+  // one-CTA tiles in us, 896 -> 4864 at 64 tokens 12.5 / 10.6, at 384 (114 tiles) 18.8 / 12.3; 2048 -> 5632 at 256 20.1 /
+  // 19.3, at 384 (132 tiles) 31.7 / 19.5; 4096 -> 14336 at 128 (112 tiles) 58 / 46.  Beyond one round the pairs run.
   if ((M + 127) / 128 * (F / 128) <= ds->sm_count) {
     GemmCall c;
     c.X = X; c.W = Wgu; c.Y = G; c.M = M; c.N = 2 * F; c.K = K;

@@ -5,7 +5,7 @@
 // Bound: latency, and the L2 feed of the few SMs that have a tile.  333 tokens x 896 outputs are 12 tiles of 128 x 224: on
 // the persistent kernel 12 of 148 SMs stream the whole weight, and a down projection's 76 k-blocks (or the 2374 of the
 // lm_head backward) run one after the other.  Here the tile is narrowed and its reduction cut into up to 8 parts until the
-// chip is full (the choice is `pick` below); a CTA computes one part of one tile:
+// chip is full (the choice is `split_plan` below); a CTA computes one part of one tile:
 //   warp 0  TMA loads (128B swizzle) into a stage ring    warp 1  tcgen05.mma, accumulator in tensor memory
 //   warps 2-9  stage Q in shared memory meanwhile, then move the float32 accumulator into shared memory (over the ring)
 // and after the cluster barrier each CTA adds up its share of the tile's rows from all parts through distributed shared
