@@ -51,10 +51,6 @@ def _stream():
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
-def _capturing() -> bool:
-    return torch._C._cuda_isCurrentStreamCapturing()
-
-
 def _lib_for(t: torch.Tensor):
     return _lib.init(t.device.index if t.device.index is not None else torch.cuda.current_device())
 
@@ -76,6 +72,11 @@ def _new_scratch(device: torch.device, nbytes: int) -> torch.Tensor:
     return raw[off:off + max(nbytes, 1 << 20)]
 
 
+def _scratch_key(device: torch.device):
+    index = device.index   # None: the current device
+    return index, torch._C._cuda_getCurrentRawStream(index) if index is not None else _stream()
+
+
 def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     """Scratch memory for one call on the current stream, starting on a 1024-byte boundary (the bf16 GEMM requires it;
     torch's allocator only promises 512).  A call's kernels write it and read it back, so whatever else uses the same
@@ -83,9 +84,9 @@ def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     and each thread (whose launches can fall between another's) its own set.  A buffer is made on the stream it serves, so
     one that is replaced goes back to that stream's pool, behind the kernels that still read it.  While a CUDA graph is
     being captured the memory comes from the graph's pool: its address is part of the graph, and nothing outgrows it."""
-    if _capturing():
+    if torch._C._cuda_isCurrentStreamCapturing():
         return _new_scratch(device, nbytes)
-    buffers, key = _scratch.buffers, (device.index, _stream())
+    buffers, key = _scratch.buffers, _scratch_key(device)
     buf = buffers.get(key)
     if buf is None or buf.numel() < nbytes:
         buffers.pop(key, None)
@@ -97,7 +98,7 @@ def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
 
 def workspace_refs(device: torch.device):
     """The scratch buffer this thread has for the current stream of `device` (a list of zero or one tensors)."""
-    buf = _scratch.buffers.get((device.index, _stream()))
+    buf = _scratch.buffers.get(_scratch_key(device))
     return [] if buf is None else [buf]
 
 

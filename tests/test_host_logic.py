@@ -168,7 +168,7 @@ def test_scratch_belongs_to_one_thread_and_stream(monkeypatch):
 
     now = {"stream": 1, "capturing": False}
     monkeypatch.setattr(backend, "_stream", lambda: now["stream"])
-    monkeypatch.setattr(backend, "_capturing", lambda: now["capturing"])
+    monkeypatch.setattr(torch._C, "_cuda_isCurrentStreamCapturing", lambda: now["capturing"])
     monkeypatch.setattr(backend, "_scratch", backend._Scratch())
     cpu = torch.device("cpu")
     a = backend.workspace(cpu, 100)
