@@ -11,6 +11,8 @@
  *     workspaces included.  The library allocates no device memory in these calls (the one small
  *     per-device status word is created by mcb_init).  There is no CPU fallback.
  *   - `stream` is a cudaStream_t passed as void*; work is enqueued, never synchronised.
+ *   - a call's kernels write its workspace and read it back: calls that are not ordered one behind the other on a
+ *     stream (other streams, other threads that launch on the same one) need workspaces of their own.
  *   - matrices are dense row-major.  M = product of the leading dims (batch*seq tokens),
  *     K = in_features, N = out_features, r = LoRA rank.
  *
