@@ -430,3 +430,26 @@ def test_bf16_delta_is_recorded_by_the_profile(cuda_device, M):
     finally:
         _lib.profile_enable(False)
     assert launches == 1 and ms > 0 and flops == 2.0 * M * r * (K + N)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("seq", [32, 64, 255, 256, 512, 777, 1024, 1100])
+def test_causal_softmax_backward_in_registers(cuda_device, dtype, seq):
+    """One to eight vectors per lane, whole and ragged rows: exact zeros behind the query position, against the oracle."""
+    from metal_candle_b200 import _lib
+    from metal_candle_b200.backend import _dtype_code, _ptr, _stream
+
+    rng = np.random.default_rng(seq)
+    rows = 3 * seq
+    y = rng.random((rows, seq))
+    y[np.arange(seq)[None, :] > (np.arange(rows) % seq)[:, None]] = 0.0
+    y, dy = rounded(y / y.sum(1, keepdims=True), dtype), rounded(rng.standard_normal((rows, seq)), dtype)
+    yd, dyd = dev_t(y, dtype, cuda_device), dev_t(dy, dtype, cuda_device)
+    dx = torch.full_like(yd, 7.0)
+    lib = _lib.load()
+    _lib.check(lib.mcb_softmax_causal_bwd(_ptr(yd), _ptr(dyd), _ptr(dx), rows, seq, seq, 0.125, _dtype_code(yd), _stream()))
+    y64, dy64 = y.astype(np.float64), dy.astype(np.float64)
+    want = y64 * (dy64 - (y64 * dy64).sum(1, keepdims=True)) * 0.125
+    got = back(dx)
+    assert R.max_abs_normalised(got, want) <= TOL[dtype]
+    assert (got[np.arange(seq)[None, :] > (np.arange(rows) % seq)[:, None]] == 0.0).all()
