@@ -523,6 +523,40 @@ int mcb_qwen_train_step(mcb_qwen* q, const int32_t* ids, const int32_t* targets,
 int mcb_qwen_info(const mcb_qwen* q, int64_t* adamw_steps, int64_t* persistent_bytes, int32_t** kept_targets_dev);
 int mcb_qwen_destroy(mcb_qwen* q);
 
+/* One decoder layer (QwenDecoderLayer::forward, src/models/qwen.rs:95-143) and its reverse, for a host that keeps the
+ * model's tensors itself and walks over the layers: the same kernel launches as the engine's, in one call, for a sequence
+ * of any length.  Stateless: every pointer is read from `call`, nothing is kept.  `saved` is what the backward needs of
+ * the forward (the same block again), `scratch` is free after the call; both are 1024-byte aligned device memory whose
+ * sizes mcb_qwen_layer_bytes gives (adapted_modules: bit m set = module m has an adapter; backward = 0: scratch for the
+ * forward alone).  bfloat16, head_dim 64; all adapters of the layer share rank and scale. */
+typedef struct {
+  int64_t batch, seq;
+  int32_t rank;
+  float scale;
+  const void* input_layernorm;           /* [hidden] */
+  const void* post_attention_layernorm;  /* [hidden] */
+  const void* w_qkv;                     /* [hidden + 2 kv, hidden]: the q, k and v weights one below the other */
+  const void* w_qkv_t;                   /* the same [in, out] (backward) */
+  const void* b_qkv;                     /* [hidden + 2 kv] */
+  const void* w_gate_up;                 /* interleaved as mcb_linear_swiglu_fwd takes it, or null: weight[4], weight[5] */
+  const void* weight[7];                 /* by module, [out, in]; q, k and v are not read */
+  const void* weight_t[7];               /* by module, [in, out]; o, gate, up and down, backward only */
+  const float* A[7];                     /* by module, or null */
+  const float* B[7];
+  float* dA[7];                          /* backward only */
+  float* dB[7];
+  void* saved;
+  void* scratch;
+  size_t saved_bytes, scratch_bytes;
+} mcb_qwen_layer_call;
+int mcb_qwen_layer_bytes(const mcb_qwen_config* cfg, int adapted_modules, int rank, int64_t batch, int64_t seq, int backward,
+                         int64_t* saved_bytes, int64_t* scratch_bytes);
+/* h_in, h_out: [batch * seq, hidden]. */
+int mcb_qwen_layer_forward(const mcb_qwen_config* cfg, const mcb_qwen_layer_call* call, const void* h_in, void* h_out, void* stream);
+/* dh: gradient of h_out, dh_in: of h_in (another buffer). */
+int mcb_qwen_layer_backward(const mcb_qwen_config* cfg, const mcb_qwen_layer_call* call, const void* h_in, const void* dh, void* dh_in,
+                            int accumulate, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

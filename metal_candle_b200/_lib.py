@@ -61,6 +61,15 @@ class AdamWTensor(C.Structure):
                 ("n", C.c_int64), ("t", C.c_int32), ("pad_", C.c_int32)]
 
 
+class QwenLayerCall(C.Structure):
+    _fields_ = [("batch", C.c_int64), ("seq", C.c_int64), ("rank", C.c_int32), ("scale", C.c_float),
+                ("input_layernorm", C.c_void_p), ("post_attention_layernorm", C.c_void_p),
+                ("w_qkv", C.c_void_p), ("w_qkv_t", C.c_void_p), ("b_qkv", C.c_void_p), ("w_gate_up", C.c_void_p),
+                ("weight", C.c_void_p * 7), ("weight_t", C.c_void_p * 7),
+                ("A", C.c_void_p * 7), ("B", C.c_void_p * 7), ("dA", C.c_void_p * 7), ("dB", C.c_void_p * 7),
+                ("saved", C.c_void_p), ("scratch", C.c_void_p), ("saved_bytes", C.c_size_t), ("scratch_bytes", C.c_size_t)]
+
+
 _vp, _i64, _i32, _f32, _sz = C.c_void_p, C.c_int64, C.c_int, C.c_float, C.c_size_t
 
 # name -> (restype, argtypes); every symbol include/mcb200.h declares
@@ -156,6 +165,9 @@ SIGNATURES = {
     "mcb_qwen_train_step": (_i32, [_vp, _vp, _vp, _i64, _i64, _f32, _f32, _f32, _f32, _f32, _f32, _vp, _vp]),
     "mcb_qwen_info": (_i32, [_vp, C.POINTER(C.c_int64), C.POINTER(C.c_int64), C.POINTER(_vp)]),
     "mcb_qwen_destroy": (_i32, [_vp]),
+    "mcb_qwen_layer_bytes": (_i32, [C.POINTER(QwenConfig), _i32, _i32, _i64, _i64, _i32, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]),
+    "mcb_qwen_layer_forward": (_i32, [C.POINTER(QwenConfig), C.POINTER(QwenLayerCall), _vp, _vp, _vp]),
+    "mcb_qwen_layer_backward": (_i32, [C.POINTER(QwenConfig), C.POINTER(QwenLayerCall), _vp, _vp, _vp, _i32, _vp]),
     "mcb_adamw_multi": (_i32, [C.POINTER(AdamWTensor), _i32, _f32, _f32, _f32, _f32, _f32, _f32, _vp]),
 }
 

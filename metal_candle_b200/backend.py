@@ -66,10 +66,15 @@ _scratch = _Scratch()
 _SCRATCH_STREAMS = 8   # buffers a thread keeps; a program that uses more streams than that allocates again
 
 
-def _new_scratch(device: torch.device, nbytes: int) -> torch.Tensor:
-    raw = torch.empty(max(nbytes, 1 << 20) + 1024, dtype=torch.uint8, device=device)
+def aligned_block(device: torch.device, nbytes: int) -> torch.Tensor:
+    """`nbytes` of device memory from a 1024-byte boundary on."""
+    raw = torch.empty(nbytes + 1024, dtype=torch.uint8, device=device)
     off = (-raw.data_ptr()) % 1024
-    return raw[off:off + max(nbytes, 1 << 20)]
+    return raw[off:off + nbytes]
+
+
+def _new_scratch(device: torch.device, nbytes: int) -> torch.Tensor:
+    return aligned_block(device, max(nbytes, 1 << 20))
 
 
 def _scratch_key(device: torch.device):

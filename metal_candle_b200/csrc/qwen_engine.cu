@@ -65,15 +65,17 @@ struct Saved {   // what one layer's backward needs from its forward
   __nv_bfloat16 *hqkv, *ho, *hg, *hu, *hd;
 };
 
-}  // namespace
-
-struct mcb_qwen {
+struct Dims {
   mcb_qwen_config cfg;
-  int64_t max_tokens = 0;
   int rank = 0;
   float scale = 1.0f;
   int64_t H = 0, I = 0, KV = 0, V = 0, d = 0, W3 = 0;
   int G = 0;
+};
+
+}  // namespace
+
+struct mcb_qwen : Dims {
   const __nv_bfloat16 *embed = nullptr, *final_norm = nullptr, *lm_head = nullptr, *lm_head_t = nullptr;
   std::vector<LayerState> layers;
   std::vector<mcb_qwen_adapter_entry> order;   // adapters in the caller's order (AdamW visits them so)
@@ -93,7 +95,7 @@ struct mcb_qwen {
 
 namespace {
 
-size_t ws_bytes_for(const mcb_qwen* q, int64_t M) {
+size_t ws_bytes_for(const Dims* q, int64_t M) {
   size_t w = 0;
   auto mx = [&](size_t v) { if (v > w) w = v; };
   const int r = q->rank;
@@ -182,50 +184,63 @@ struct StepPlan {
   __nv_bfloat16 *dQ = nullptr, *dK = nullptr, *dV = nullptr, *logits = nullptr;
 };
 
-void plan_step(const mcb_qwen* q, Bump& b, int64_t M, int64_t B, int64_t S, StepPlan* p) {
+void plan_layer(const Dims* q, const LayerState& L, Bump& b, int64_t M, int64_t B, int64_t S, Saved* out) {
   const int64_t H = q->H, I = q->I, KV = q->KV;
   const int r = q->rank;
   const size_t hrow = static_cast<size_t>(mcb_lora_h_pitch(M));
+  Saved& s = *out;
+  s.n1 = b.take_n<__nv_bfloat16>(M * H);
+  s.Qr = b.take_n<__nv_bfloat16>(M * H);
+  s.Kr = b.take_n<__nv_bfloat16>(M * KV);
+  s.Vr = b.take_n<__nv_bfloat16>(M * KV);
+  s.lse = b.take_n<float>(static_cast<size_t>(B) * q->cfg.num_heads * S);
+  s.o = b.take_n<__nv_bfloat16>(M * H);
+  s.h2 = b.take_n<__nv_bfloat16>(M * H);
+  if (has(L, kGate) || has(L, kUp)) s.n2 = b.take_n<__nv_bfloat16>(M * H);
+  s.gate = b.take_n<__nv_bfloat16>(M * I);
+  s.up = b.take_n<__nv_bfloat16>(M * I);
+  if (has(L, kDown)) s.act = b.take_n<__nv_bfloat16>(M * I);
+  const int nq = (has(L, kQ) ? 1 : 0) + (has(L, kK) ? 1 : 0) + (has(L, kV) ? 1 : 0);
+  if (nq > 0) s.hqkv = b.take_n<__nv_bfloat16>(static_cast<size_t>(mcb_lora_rank_padded(static_cast<int64_t>(r) * nq)) * hrow);
+  const size_t h1 = static_cast<size_t>(mcb_lora_rank_padded(r)) * hrow;
+  if (has(L, kO)) s.ho = b.take_n<__nv_bfloat16>(h1);
+  if (has(L, kGate)) s.hg = b.take_n<__nv_bfloat16>(h1);
+  if (has(L, kUp)) s.hu = b.take_n<__nv_bfloat16>(h1);
+  if (has(L, kDown)) s.hd = b.take_n<__nv_bfloat16>(h1);
+}
+
+// scratch of one layer's calls; those of the forward alone come first
+void plan_scratch(const Dims* q, Bump& b, int64_t M, int64_t B, int64_t S, bool backward, StepPlan* p) {
+  const int64_t H = q->H, I = q->I, KV = q->KV;
+  p->ws_bytes = ws_bytes_for(q, M);
+  p->ws = b.take(p->ws_bytes);
+  p->qkv = b.take_n<__nv_bfloat16>(M * q->W3);
+  p->t_MH[0] = b.take_n<__nv_bfloat16>(M * H);
+  p->t_MI[0] = b.take_n<__nv_bfloat16>(M * I);
+  if (!backward) return;
+  p->attn_ws_bytes = mcb_attention_workspace_bytes(B * q->cfg.num_kv_heads, q->G, S, q->d);
+  p->attn_ws = b.take(p->attn_ws_bytes);
+  for (int i = 1; i < 4; ++i) p->t_MH[i] = b.take_n<__nv_bfloat16>(M * H);
+  p->t_MI[1] = b.take_n<__nv_bfloat16>(M * I);
+  p->dQ = b.take_n<__nv_bfloat16>(M * H);
+  p->dK = b.take_n<__nv_bfloat16>(M * KV);
+  p->dV = b.take_n<__nv_bfloat16>(M * KV);
+}
+
+void plan_step(const mcb_qwen* q, Bump& b, int64_t M, int64_t B, int64_t S, StepPlan* p) {
+  const int64_t H = q->H;
   p->saved.resize(q->layers.size());
   for (size_t li = 0; li < q->layers.size(); ++li) {
-    const LayerState& L = q->layers[li];
-    Saved& s = p->saved[li];
-    memset(&s, 0, sizeof(s));
-    s.h = b.take_n<__nv_bfloat16>(M * H);
-    s.n1 = b.take_n<__nv_bfloat16>(M * H);
-    s.Qr = b.take_n<__nv_bfloat16>(M * H);
-    s.Kr = b.take_n<__nv_bfloat16>(M * KV);
-    s.Vr = b.take_n<__nv_bfloat16>(M * KV);
-    s.lse = b.take_n<float>(static_cast<size_t>(B) * q->cfg.num_heads * S);
-    s.o = b.take_n<__nv_bfloat16>(M * H);
-    s.h2 = b.take_n<__nv_bfloat16>(M * H);
-    if (has(L, kGate) || has(L, kUp)) s.n2 = b.take_n<__nv_bfloat16>(M * H);
-    s.gate = b.take_n<__nv_bfloat16>(M * I);
-    s.up = b.take_n<__nv_bfloat16>(M * I);
-    if (has(L, kDown)) s.act = b.take_n<__nv_bfloat16>(M * I);
-    const int nq = (has(L, kQ) ? 1 : 0) + (has(L, kK) ? 1 : 0) + (has(L, kV) ? 1 : 0);
-    if (nq > 0) s.hqkv = b.take_n<__nv_bfloat16>(static_cast<size_t>(mcb_lora_rank_padded(static_cast<int64_t>(r) * nq)) * hrow);
-    const size_t h1 = static_cast<size_t>(mcb_lora_rank_padded(r)) * hrow;
-    if (has(L, kO)) s.ho = b.take_n<__nv_bfloat16>(h1);
-    if (has(L, kGate)) s.hg = b.take_n<__nv_bfloat16>(h1);
-    if (has(L, kUp)) s.hu = b.take_n<__nv_bfloat16>(h1);
-    if (has(L, kDown)) s.hd = b.take_n<__nv_bfloat16>(h1);
+    memset(&p->saved[li], 0, sizeof(Saved));
+    p->saved[li].h = b.take_n<__nv_bfloat16>(M * H);
+    plan_layer(q, q->layers[li], b, M, B, S, &p->saved[li]);
   }
   p->h_final = b.take_n<__nv_bfloat16>(M * H);
   p->nf = b.take_n<__nv_bfloat16>(M * H);
   p->dnf = b.take_n<__nv_bfloat16>(M * H);
   p->nll = b.take_n<float>(M);
   p->lossbuf = b.take_n<float>(256);
-  p->ws_bytes = ws_bytes_for(q, M);
-  p->ws = b.take(p->ws_bytes);
-  p->attn_ws_bytes = mcb_attention_workspace_bytes(B * q->cfg.num_kv_heads, q->G, S, q->d);
-  p->attn_ws = b.take(p->attn_ws_bytes);
-  p->qkv = b.take_n<__nv_bfloat16>(M * q->W3);
-  for (int i = 0; i < 4; ++i) p->t_MH[i] = b.take_n<__nv_bfloat16>(M * H);
-  for (int i = 0; i < 2; ++i) p->t_MI[i] = b.take_n<__nv_bfloat16>(M * I);
-  p->dQ = b.take_n<__nv_bfloat16>(M * H);
-  p->dK = b.take_n<__nv_bfloat16>(M * KV);
-  p->dV = b.take_n<__nv_bfloat16>(M * KV);
+  plan_scratch(q, b, M, B, S, true, p);
   const int64_t want = q->ce_chunk > 0 ? q->ce_chunk : mcb_ce_chunk_tokens(M, H);
   const int64_t chunk = want < M ? want : M;
   p->logits = b.take_n<__nv_bfloat16>(static_cast<size_t>(chunk) * q->V);
@@ -238,20 +253,20 @@ void plan_step(const mcb_qwen* q, Bump& b, int64_t M, int64_t B, int64_t S, Step
   } while (0)
 
 // y = x W^T (+bias) (+residual) + LoRA, one projection
-int lin_fwd(const mcb_qwen* q, const StepPlan& p, const void* x, const void* W, const void* bias, const Adapter& a, const void* residual,
+int lin_fwd(const Dims* q, const StepPlan& p, const void* x, const void* W, const void* bias, const Adapter& a, const void* residual,
             void* y, void* h_save, int64_t M, int64_t K, int64_t N, cudaStream_t st) {
   const int r = a.A ? q->rank : 0;
   return mcb_lora_linear_fwd_ex(x, W, bias, a.A, a.B, residual, y, r ? h_save : nullptr, M, K, N, r, q->scale, MCB_BF16, MCB_W_OUT_IN,
                                 p.ws, p.ws_bytes, st);
 }
-int lin_bwd(const mcb_qwen* q, const StepPlan& p, const void* x, const void* Wt, const Adapter& a, const void* dy, const void* h_save,
+int lin_bwd(const Dims* q, const StepPlan& p, const void* x, const void* Wt, const Adapter& a, const void* dy, const void* h_save,
             const void* dx_residual, void* dx, int accumulate, int64_t M, int64_t K, int64_t N, cudaStream_t st) {
   const int r = a.A ? q->rank : 0;
   return mcb_lora_linear_bwd_ex(r ? x : nullptr, Wt, a.A, a.B, dy, r ? h_save : nullptr, dx_residual, dx, r ? a.dA : nullptr,
                                 r ? a.dB : nullptr, accumulate, M, K, N, r, q->scale, MCB_BF16, MCB_W_IN_OUT, p.ws, p.ws_bytes, st);
 }
 
-int qkv_segments(const mcb_qwen* q, const LayerState& L, mcb_lora_segment* segs) {
+int qkv_segments(const Dims* q, const LayerState& L, mcb_lora_segment* segs) {
   const int64_t off[3] = {0, q->H, q->H + q->KV};
   const int64_t wid[3] = {q->H, q->KV, q->KV};
   int n = 0;
@@ -264,11 +279,9 @@ int qkv_segments(const mcb_qwen* q, const LayerState& L, mcb_lora_segment* segs)
   return n;
 }
 
-int layer_forward(const mcb_qwen* q, const StepPlan& p, size_t li, const __nv_bfloat16* h_in, __nv_bfloat16* h_out, int64_t B, int64_t S,
-                  cudaStream_t st) {
-  const LayerState& L = q->layers[li];
-  const Saved& s = p.saved[li];
-  const int64_t M = B * S, H = q->H, I = q->I, KV = q->KV, W3 = q->W3;
+int layer_forward(const Dims* q, const StepPlan& p, const LayerState& L, const Saved& s, const __nv_bfloat16* h_in, __nv_bfloat16* h_out,
+                  int64_t B, int64_t S, cudaStream_t st) {
+  const int64_t M = B * S, H = q->H, I = q->I, W3 = q->W3;
   const float eps = q->cfg.rms_norm_eps, theta = q->cfg.rope_theta;
   const int Hq = static_cast<int>(q->cfg.num_heads), Hk = static_cast<int>(q->cfg.num_kv_heads);
   QCHECK(mcb_rmsnorm_fwd(h_in, L.ln1, s.n1, nullptr, M, H, eps, MCB_BF16, st));
@@ -282,7 +295,7 @@ int layer_forward(const mcb_qwen* q, const StepPlan& p, size_t li, const __nv_bf
                                   MCB_W_OUT_IN, p.ws, p.ws_bytes, st));
   QCHECK(mcb_rope_relayout_qkv(p.qkv, s.Qr, s.Kr, s.Vr, B, S, Hq, Hk, q->d, theta, 0, W3, MCB_BF16, st));
   const float sc = 1.0f / sqrtf(static_cast<float>(q->d));
-  QCHECK(mcb_attention_causal_fwd_ex(s.Qr, s.Kr, s.Vr, s.o, s.lse, B * Hk, q->G, S, q->d, sc, MCB_BF16, Hk, 1, p.attn_ws, p.attn_ws_bytes,
+  QCHECK(mcb_attention_causal_fwd_ragged(s.Qr, s.Kr, s.Vr, s.o, s.lse, B * Hk, q->G, S, q->d, sc, MCB_BF16, Hk, 1, p.attn_ws, p.attn_ws_bytes,
                                      st));
   QCHECK(lin_fwd(q, p, s.o, L.w[kO], nullptr, L.ad[kO], h_in, s.h2, s.ho, M, H, H, st));
   __nv_bfloat16* n2 = s.n2 ? s.n2 : p.t_MH[0];
@@ -300,11 +313,9 @@ int layer_forward(const mcb_qwen* q, const StepPlan& p, size_t li, const __nv_bf
 }
 
 // dh_in: gradient of the layer's output [M,H]; dh_out: gradient of its input
-int layer_backward(const mcb_qwen* q, const StepPlan& p, size_t li, const __nv_bfloat16* dh3, __nv_bfloat16* dh_out, int64_t B, int64_t S,
-                   int accumulate, cudaStream_t st) {
-  const LayerState& L = q->layers[li];
-  const Saved& s = p.saved[li];
-  const int64_t M = B * S, H = q->H, I = q->I, KV = q->KV, W3 = q->W3;
+int layer_backward(const Dims* q, const StepPlan& p, const LayerState& L, const Saved& s, const __nv_bfloat16* dh3, __nv_bfloat16* dh_out,
+                   int64_t B, int64_t S, int accumulate, cudaStream_t st) {
+  const int64_t M = B * S, H = q->H, I = q->I, W3 = q->W3;
   const float eps = q->cfg.rms_norm_eps, theta = q->cfg.rope_theta;
   const int Hq = static_cast<int>(q->cfg.num_heads), Hk = static_cast<int>(q->cfg.num_kv_heads);
   // MLP
@@ -331,7 +342,7 @@ int layer_backward(const mcb_qwen* q, const StepPlan& p, size_t li, const __nv_b
   __nv_bfloat16* d_o = p.t_MH[1];
   QCHECK(lin_bwd(q, p, s.o, L.wt[kO], L.ad[kO], dh2, s.ho, nullptr, d_o, accumulate, M, H, H, st));
   const float sc = 1.0f / sqrtf(static_cast<float>(q->d));
-  QCHECK(mcb_attention_causal_bwd_ex(s.Qr, s.Kr, s.Vr, s.o, d_o, s.lse, p.dQ, p.dK, p.dV, B * Hk, q->G, S, q->d, sc, MCB_BF16, Hk, 1,
+  QCHECK(mcb_attention_causal_bwd_ragged(s.Qr, s.Kr, s.Vr, s.o, d_o, s.lse, p.dQ, p.dK, p.dV, B * Hk, q->G, S, q->d, sc, MCB_BF16, Hk, 1,
                                      p.attn_ws, p.attn_ws_bytes, st));
   __nv_bfloat16* dqkv = p.qkv;
   QCHECK(mcb_rope_relayout_qkv(dqkv, p.dQ, p.dK, p.dV, B, S, Hq, Hk, q->d, theta, 1, W3, MCB_BF16, st));
@@ -353,8 +364,7 @@ int layer_backward(const mcb_qwen* q, const StepPlan& p, size_t li, const __nv_b
 // ---- C ABI -------------------------------------------------------------------------------------------------------
 
 namespace {
-int fill(mcb_qwen* q, const mcb_qwen_config* cfg, const mcb_qwen_weights* w, const mcb_qwen_adapter_entry* adapters, int n_adapters,
-         int rank, float scale) {
+int fill_dims(Dims* q, const mcb_qwen_config* cfg, int rank, float scale) {
   q->cfg = *cfg;
   q->H = cfg->hidden_size; q->I = cfg->intermediate_size; q->V = cfg->vocab_size;
   if (cfg->num_heads <= 0 || cfg->num_kv_heads <= 0 || cfg->hidden_size % cfg->num_heads != 0 || cfg->num_heads % cfg->num_kv_heads != 0)
@@ -369,6 +379,11 @@ int fill(mcb_qwen* q, const mcb_qwen_config* cfg, const mcb_qwen_weights* w, con
   if (rank < 0 || rank > 21 * 3) return fail(MCB_ERR_SHAPE, "mcb_qwen: rank %d", rank);
   if (rank * 3 > 64) return fail(MCB_ERR_UNSUPPORTED, "mcb_qwen: rank %d x 3 fused projections exceeds 64 rank columns", rank);
   q->rank = rank; q->scale = scale;
+  return MCB_OK;
+}
+int fill(mcb_qwen* q, const mcb_qwen_config* cfg, const mcb_qwen_weights* w, const mcb_qwen_adapter_entry* adapters, int n_adapters,
+         int rank, float scale) {
+  if (int rc = fill_dims(q, cfg, rank, scale)) return rc;
   q->layers.resize(static_cast<size_t>(cfg->num_layers));
   for (size_t li = 0; li < q->layers.size(); ++li) {
     LayerState& L = q->layers[li];
@@ -497,7 +512,7 @@ extern "C" int mcb_qwen_forward_backward(mcb_qwen* q, const int32_t* ids, const 
   QCHECK(mcb_embedding_fwd(ids, q->embed, p.saved[0].h, M, H, V, MCB_BF16, st));
   for (size_t li = 0; li < nl; ++li) {
     __nv_bfloat16* h_out = li + 1 < nl ? p.saved[li + 1].h : p.h_final;
-    QCHECK(layer_forward(q, p, li, p.saved[li].h, h_out, batch, seq, st));
+    QCHECK(layer_forward(q, p, q->layers[li], p.saved[li], p.saved[li].h, h_out, batch, seq, st));
   }
   QCHECK(mcb_rmsnorm_fwd(p.h_final, q->final_norm, p.nf, nullptr, M, H, q->cfg.rms_norm_eps, MCB_BF16, st));
   // lm_head, loss and lm_head backward, a chunk of tokens at a time
@@ -518,7 +533,7 @@ extern "C" int mcb_qwen_forward_backward(mcb_qwen* q, const int32_t* ids, const 
   QCHECK(mcb_rmsnorm_bwd_ex(p.h_final, q->final_norm, p.dnf, nullptr, dh, nullptr, 0, M, H, q->cfg.rms_norm_eps, MCB_BF16, nullptr, 0, st));
   bool forked = false;
   for (size_t k = nl; k-- > 0;) {
-    QCHECK(layer_backward(q, p, k, dh, dh_next, batch, seq, accumulate, st));
+    QCHECK(layer_backward(q, p, q->layers[k], p.saved[k], dh, dh_next, batch, seq, accumulate, st));
     __nv_bfloat16* t = dh; dh = dh_next; dh_next = t;
     if (q->comm != nullptr) {
       for (size_t bi = 0; bi < q->bucket_layer.size(); ++bi) {
@@ -581,4 +596,98 @@ extern "C" int mcb_qwen_destroy(mcb_qwen* q) {
   if (q->ev_join) cudaEventDestroy(q->ev_join);
   delete q;
   return MCB_OK;
+}
+
+// ---- one decoder layer -------------------------------------------------------------------------------------------
+namespace {
+int layer_from_call(const mcb_qwen_config* cfg, const mcb_qwen_layer_call* c, bool backward, Dims* q, LayerState* L, Saved* s, StepPlan* p,
+                    const char* op) {
+  if (!cfg || !c || !c->saved || !c->scratch) return fail(MCB_ERR_NULL, "%s: null pointer", op);
+  if (c->batch <= 0 || c->seq <= 0) return fail(MCB_ERR_SHAPE, "%s: batch %lld x seq %lld", op, (long long)c->batch, (long long)c->seq);
+  if (((reinterpret_cast<uintptr_t>(c->saved) | reinterpret_cast<uintptr_t>(c->scratch)) & 1023u) != 0)
+    return fail(MCB_ERR_ALIGN, "%s: saved and scratch must be 1024-byte aligned", op);
+  if (int rc = fill_dims(q, cfg, c->rank, c->scale)) return rc;
+  const void* need[] = {c->input_layernorm, c->post_attention_layernorm, c->w_qkv, c->b_qkv, c->weight[kO], c->weight[kDown]};
+  for (const void* w : need)
+    if (!w) return fail(MCB_ERR_NULL, "%s: a weight is null", op);
+  if (!c->w_gate_up && (!c->weight[kGate] || !c->weight[kUp])) return fail(MCB_ERR_NULL, "%s: no gate and up weights", op);
+  *L = LayerState();
+  L->ln1 = static_cast<const __nv_bfloat16*>(c->input_layernorm);
+  L->ln2 = static_cast<const __nv_bfloat16*>(c->post_attention_layernorm);
+  L->wqkv = static_cast<const __nv_bfloat16*>(c->w_qkv);
+  L->wqkv_t = static_cast<const __nv_bfloat16*>(c->w_qkv_t);
+  L->bqkv = static_cast<const __nv_bfloat16*>(c->b_qkv);
+  L->wgu = static_cast<const __nv_bfloat16*>(c->w_gate_up);
+  for (int m = 0; m < kModules; ++m) {
+    L->w[m] = static_cast<const __nv_bfloat16*>(c->weight[m]);
+    L->wt[m] = static_cast<const __nv_bfloat16*>(c->weight_t[m]);
+    Adapter& a = L->ad[m];
+    a.A = c->A[m]; a.B = c->B[m]; a.dA = c->dA[m]; a.dB = c->dB[m];
+    if (a.A != nullptr && (c->rank <= 0 || !a.B || (backward && (!a.dA || !a.dB)))) return fail(MCB_ERR_NULL, "%s: adapter of module %d is incomplete", op, m);
+  }
+  if (L->wgu != nullptr && (has(*L, kGate) || has(*L, kUp)))
+    return fail(MCB_ERR_UNSUPPORTED, "%s: the interleaved gate/up weight takes no adapter on either", op);
+  if (backward) {
+    if (!L->wqkv_t) return fail(MCB_ERR_NULL, "%s: a transposed weight is null", op);
+    for (int m = kO; m <= kDown; ++m)
+      if (!L->wt[m]) return fail(MCB_ERR_NULL, "%s: a transposed weight is null", op);
+  }
+  const int64_t M = c->batch * c->seq;
+  memset(s, 0, sizeof(*s));
+  Bump bs;
+  bs.base = static_cast<uint8_t*>(c->saved); bs.size = c->saved_bytes;
+  plan_layer(q, *L, bs, M, c->batch, c->seq, s);
+  Bump bt;
+  bt.base = static_cast<uint8_t*>(c->scratch); bt.size = c->scratch_bytes;
+  plan_scratch(q, bt, M, c->batch, c->seq, backward, p);
+  if (bs.overflow || bt.overflow)
+    return fail(MCB_ERR_WORKSPACE, "%s: saved %zu of %zu bytes, scratch %zu of %zu", op, c->saved_bytes, bs.peak, c->scratch_bytes, bt.peak);
+  return MCB_OK;
+}
+}  // namespace
+
+extern "C" int mcb_qwen_layer_bytes(const mcb_qwen_config* cfg, int adapted_modules, int rank, int64_t batch, int64_t seq, int backward,
+                                    int64_t* saved_bytes, int64_t* scratch_bytes) {
+  if (!cfg || !saved_bytes || !scratch_bytes) return fail(MCB_ERR_NULL, "mcb_qwen_layer_bytes: null pointer");
+  if (batch <= 0 || seq <= 0) return fail(MCB_ERR_SHAPE, "mcb_qwen_layer_bytes: batch %lld x seq %lld", (long long)batch, (long long)seq);
+  Dims q;
+  if (int rc = fill_dims(&q, cfg, rank, 1.0f)) return rc;
+  LayerState L = LayerState();
+  for (int m = 0; m < kModules; ++m)
+    if (adapted_modules & (1 << m)) L.ad[m].A = reinterpret_cast<const float*>(1);   // only its presence is looked at
+  Saved s;
+  memset(&s, 0, sizeof(s));
+  Bump bs, bt;
+  StepPlan p;
+  plan_layer(&q, L, bs, batch * seq, batch, seq, &s);
+  plan_scratch(&q, bt, batch * seq, batch, seq, backward != 0, &p);
+  *saved_bytes = static_cast<int64_t>(bs.peak);
+  *scratch_bytes = static_cast<int64_t>(bt.peak);
+  return MCB_OK;
+}
+
+extern "C" int mcb_qwen_layer_forward(const mcb_qwen_config* cfg, const mcb_qwen_layer_call* call, const void* h_in, void* h_out, void* stream) {
+  MCB_NVTX_RANGE("mcb_qwen_layer_forward");
+  Dims q;
+  LayerState L;
+  Saved s;
+  StepPlan p;
+  if (int rc = layer_from_call(cfg, call, false, &q, &L, &s, &p, "mcb_qwen_layer_forward")) return rc;
+  if (!h_in || !h_out) return fail(MCB_ERR_NULL, "mcb_qwen_layer_forward: null pointer");
+  return layer_forward(&q, p, L, s, static_cast<const __nv_bfloat16*>(h_in), static_cast<__nv_bfloat16*>(h_out), call->batch, call->seq,
+                       static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int mcb_qwen_layer_backward(const mcb_qwen_config* cfg, const mcb_qwen_layer_call* call, const void* h_in, const void* dh, void* dh_in,
+                                       int accumulate, void* stream) {
+  MCB_NVTX_RANGE("mcb_qwen_layer_backward");
+  Dims q;
+  LayerState L;
+  Saved s;
+  StepPlan p;
+  if (int rc = layer_from_call(cfg, call, true, &q, &L, &s, &p, "mcb_qwen_layer_backward")) return rc;
+  if (!h_in || !dh || !dh_in) return fail(MCB_ERR_NULL, "mcb_qwen_layer_backward: null pointer");
+  s.h = static_cast<__nv_bfloat16*>(const_cast<void*>(h_in));   // only read
+  return layer_backward(&q, p, L, s, static_cast<const __nv_bfloat16*>(dh), static_cast<__nv_bfloat16*>(dh_in), call->batch, call->seq,
+                        accumulate, static_cast<cudaStream_t>(stream));
 }

@@ -14,6 +14,7 @@ contractions (Q K^T, P V and their reverses): the fused attention kernels of csr
 """
 from __future__ import annotations
 
+import ctypes
 import math
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Tuple
@@ -90,6 +91,104 @@ class CapturedStep:
         self.targets.copy_(target_ids, non_blocking=True)
         self.graph.replay()
         return self.loss, self.grads
+
+
+class _LayerCalls:
+    """The decoder layers of one pass as one library call each (mcb_qwen_layer_forward / _backward) instead of one per
+    kernel: a forward of 24 layers over 3 x 111 tokens is some 220 launches, which cost the host 3.5 ms as calls from here
+    and 1.8 ms this way.  The launches and their results are the same.  Lives for one pass: it holds the scratch memory,
+    and reads the model's tensors anew for every call."""
+
+    def __init__(self, model: "Qwen", batch: int, seq: int, backward: bool):
+        c = model.config
+        self.model, self.batch, self.seq, self.backward = model, batch, seq, backward
+        self.cfg = ctypes.byref(_lib.QwenConfig(c.vocab_size, c.hidden_size, c.intermediate_size, c.num_hidden_layers,
+                                                c.num_attention_heads, c.num_key_value_heads, c.rms_norm_eps, c.rope_theta))
+        # what the library's layer takes; other models and settings run kernel by kernel
+        self.usable = (model.dtype == torch.bfloat16 and c.head_dim == 64 and c.intermediate_size % 8 == 0 and c.vocab_size % 8 == 0
+                       and model.fuse_swiglu_bwd)
+        self.sizes: Dict[Tuple[int, int], Tuple[int, int]] = {}
+        self.scratch = None
+        self.shared = None    # without a backward to come, every layer uses the same block
+
+    def _tensors_ok(self, L, names) -> bool:
+        """The shapes and layouts the library's layer assumes (the call per kernel checks its own and reports)."""
+        c, dt = self.model.config, self.model.dtype
+        for name in ("input_layernorm", "post_attention_layernorm"):
+            if L[name].shape != (c.hidden_size,) or L[name].dtype != dt or not L[name].is_contiguous():
+                return False
+        for name in names:
+            lin = L[name]
+            for w, shape in ((lin.weight, (lin.out_f, lin.in_f)), (lin.weight_t, (lin.in_f, lin.out_f))):
+                if w.shape != shape or w.dtype != dt or not w.is_contiguous() or not w.is_cuda:
+                    return False
+            if lin.bias is not None and name not in ("q_proj", "k_proj", "v_proj"):
+                return False
+        return True
+
+    def prepare(self, idx: int, saved=None):
+        """(call, block) for layer `idx`, its block of saved tensors newly made unless given, or None where the layer has to
+        run kernel by kernel."""
+        m = self.model
+        L = m.layers[idx]
+        fq = m._qkv_fused(L) if self.usable else None
+        if fq is None:
+            return None
+        rank = next(l.lora for l in fq["lins"] if l.lora is not None).config.rank
+        w_gu = m._gate_up_weight(L)
+        if rank * 3 > 64 or not self._tensors_ok(L, ("o_proj", "gate_proj", "up_proj", "down_proj")):
+            return None
+        call = _lib.QwenLayerCall()
+        mask = 0
+        for i, name in enumerate(m.MODULES):
+            lin = L[name]
+            if i >= 3:
+                call.weight[i], call.weight_t[i] = lin.weight.data_ptr(), lin.weight_t.data_ptr()
+            lora = lin.lora
+            if lora is None:
+                continue
+            a, b = lora.lora_a, lora.lora_b
+            if (lora.config.scaling() != fq["scale"] or a.shape != (lin.in_f, rank) or b.shape != (rank, lin.out_f)
+                    or a.dtype != torch.float32 or b.dtype != torch.float32 or not (a.is_cuda and b.is_cuda)
+                    or not (a.is_contiguous() and b.is_contiguous())):
+                return None
+            mask |= 1 << i
+            call.A[i], call.B[i] = a.data_ptr(), b.data_ptr()
+            if self.backward:
+                ga, gb = m._grad_slices[f"layers.{idx}.{name}"]
+                call.dA[i], call.dB[i] = ga.data_ptr(), gb.data_ptr()
+        size = self.sizes.get((mask, rank))
+        if size is None:
+            sv, sc = ctypes.c_int64(0), ctypes.c_int64(0)
+            _lib.check(m.lib.mcb_qwen_layer_bytes(self.cfg, mask, rank, self.batch, self.seq, int(self.backward), ctypes.byref(sv),
+                                                  ctypes.byref(sc)))
+            size = self.sizes[(mask, rank)] = (sv.value, sc.value)
+        if self.scratch is None or self.scratch.numel() < size[1]:
+            self.scratch = backend.aligned_block(m.device, size[1])
+        if saved is None:
+            if not self.backward and self.shared is not None and self.shared.numel() >= size[0]:
+                saved = self.shared
+            else:
+                saved = self.shared = backend.aligned_block(m.device, size[0])
+        call.batch, call.seq, call.rank, call.scale = self.batch, self.seq, rank, fq["scale"]
+        call.input_layernorm, call.post_attention_layernorm = L["input_layernorm"].data_ptr(), L["post_attention_layernorm"].data_ptr()
+        call.w_qkv, call.w_qkv_t, call.b_qkv = fq["w"].data_ptr(), fq["wt"].data_ptr(), fq["bias"].data_ptr()
+        if w_gu is not None:
+            call.w_gate_up = w_gu.data_ptr()
+        call.saved, call.saved_bytes = saved.data_ptr(), saved.numel()
+        call.scratch, call.scratch_bytes = self.scratch.data_ptr(), self.scratch.numel()
+        return call, saved
+
+    def forward(self, prepared, h: torch.Tensor) -> torch.Tensor:
+        out = torch.empty_like(h)
+        _lib.check(self.model.lib.mcb_qwen_layer_forward(self.cfg, ctypes.byref(prepared[0]), h.data_ptr(), out.data_ptr(), _stream()))
+        return out
+
+    def layer_backward(self, prepared, h: torch.Tensor, dh: torch.Tensor, accumulate: bool) -> torch.Tensor:
+        out = torch.empty_like(dh)
+        _lib.check(self.model.lib.mcb_qwen_layer_backward(self.cfg, ctypes.byref(prepared[0]), h.data_ptr(), dh.data_ptr(), out.data_ptr(),
+                                                          int(bool(accumulate)), _stream()))
+        return out
 
 
 class Qwen:
@@ -314,8 +413,12 @@ class Qwen:
         return dQ, dK, dV
 
     # -- forward --
-    def _layer_fwd(self, h, L, B, S, save: bool):
+    def _layer_fwd(self, h, idx, B, S, save: bool, calls: _LayerCalls):
         c = self.config
+        prepared = calls.prepare(idx)
+        if prepared is not None:
+            return calls.forward(prepared, h), (dict(block=prepared[1], h=h) if save else None)
+        L = self.layers[idx]
         n1 = self._norm(h, L["input_layernorm"])
         fq = self._qkv_fused(L)
         hqkv = None
@@ -363,8 +466,9 @@ class Qwen:
         """Qwen::forward (src/models/qwen.rs:236-251) with a causal mask: logits [B, S, vocab]."""
         B, S = input_ids.shape
         h = self._embed(input_ids.to(torch.int32).contiguous().view(-1))
-        for L in self.layers:
-            h, _ = self._layer_fwd(h, L, B, S, save=False)
+        calls = _LayerCalls(self, B, S, backward=False)
+        for idx in range(len(self.layers)):
+            h, _ = self._layer_fwd(h, idx, B, S, False, calls)
         nf = self._norm(h, self.norm)
         logits, _ = self._lin(nf, self.lm_head, False)
         return logits.view(B, S, -1)
@@ -384,8 +488,9 @@ class Qwen:
         tgt32 = target_ids.to(torch.int32).contiguous().view(-1)  # u32::MAX wraps to -1 = ignored
         h = self._embed(ids32)
         saved = []
-        for L in self.layers:
-            h, sv = self._layer_fwd(h, L, B, S, save=True)
+        calls = _LayerCalls(self, B, S, backward=True)
+        for idx in range(len(self.layers)):
+            h, sv = self._layer_fwd(h, idx, B, S, True, calls)
             saved.append(sv)
         nf = self._norm(h, self.norm)
         nll = torch.empty(M, dtype=torch.float32, device=self.device)
@@ -418,7 +523,7 @@ class Qwen:
         dh, _ = backend.rms_norm_backward(h, self.norm, dnf, c.rms_norm_eps, need_dw=False)
         del dnf
         for idx in range(len(self.layers) - 1, -1, -1):
-            dh = self._layer_bwd(dh, self.layers[idx], saved[idx], idx, B, S, accumulate)
+            dh = self._layer_bwd(dh, saved[idx], idx, B, S, accumulate, calls)
             saved[idx] = None
             if self.layer_done_hook is not None:
                 self.layer_done_hook(idx)
@@ -455,8 +560,11 @@ class Qwen:
             _lib.profile_enable(was_profiling)
         return CapturedStep(graph, ids, targets, loss, grads, count=self.last_count)
 
-    def _layer_bwd(self, dh3, L, sv, idx, B, S, accumulate):
+    def _layer_bwd(self, dh3, sv, idx, B, S, accumulate, calls: _LayerCalls):
         c = self.config
+        if "block" in sv:
+            return calls.layer_backward(calls.prepare(idx, sv["block"]), sv["h"], dh3, accumulate)
+        L = self.layers[idx]
         key = lambda m: f"layers.{idx}.{m}"
         # MLP
         gt, up = sv["gate"], sv["up"]

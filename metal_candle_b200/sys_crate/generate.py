@@ -23,6 +23,7 @@ TYPES = {
     "size_t": "usize", "char": "c_char", "mcb_adamw_tensor": "mcb_adamw_tensor", "mcb_comm": "mcb_comm",
     "mcb_lora_segment": "mcb_lora_segment", "mcb_qwen": "mcb_qwen", "mcb_qwen_config": "mcb_qwen_config",
     "mcb_qwen_weights": "mcb_qwen_weights", "mcb_qwen_adapter_entry": "mcb_qwen_adapter_entry",
+    "mcb_qwen_layer_call": "mcb_qwen_layer_call",
 }
 
 
@@ -161,6 +162,32 @@ def render(consts, funcs) -> str:
         "    pub B: *const f32,",
         "    pub dA: *mut f32,",
         "    pub dB: *mut f32,",
+        "}",
+        "",
+        "/// One call of `mcb_qwen_layer_forward` / `_backward`: a layer's tensors, by module where there are seven.",
+        "#[repr(C)]",
+        "#[derive(Debug, Clone, Copy)]",
+        "pub struct mcb_qwen_layer_call {",
+        "    pub batch: i64,",
+        "    pub seq: i64,",
+        "    pub rank: i32,",
+        "    pub scale: f32,",
+        "    pub input_layernorm: *const c_void,",
+        "    pub post_attention_layernorm: *const c_void,",
+        "    pub w_qkv: *const c_void,",
+        "    pub w_qkv_t: *const c_void,",
+        "    pub b_qkv: *const c_void,",
+        "    pub w_gate_up: *const c_void,",
+        "    pub weight: [*const c_void; 7],",
+        "    pub weight_t: [*const c_void; 7],",
+        "    pub A: [*const f32; 7],",
+        "    pub B: [*const f32; 7],",
+        "    pub dA: [*mut f32; 7],",
+        "    pub dB: [*mut f32; 7],",
+        "    pub saved: *mut c_void,",
+        "    pub scratch: *mut c_void,",
+        "    pub saved_bytes: usize,",
+        "    pub scratch_bytes: usize,",
         "}",
         "",
         "/// Opaque training-step engine (`mcb_qwen_*`).",

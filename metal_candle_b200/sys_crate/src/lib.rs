@@ -105,6 +105,32 @@ pub struct mcb_qwen_adapter_entry {
     pub dB: *mut f32,
 }
 
+/// One call of `mcb_qwen_layer_forward` / `_backward`: a layer's tensors, by module where there are seven.
+#[repr(C)]
+#[derive(Debug, Clone, Copy)]
+pub struct mcb_qwen_layer_call {
+    pub batch: i64,
+    pub seq: i64,
+    pub rank: i32,
+    pub scale: f32,
+    pub input_layernorm: *const c_void,
+    pub post_attention_layernorm: *const c_void,
+    pub w_qkv: *const c_void,
+    pub w_qkv_t: *const c_void,
+    pub b_qkv: *const c_void,
+    pub w_gate_up: *const c_void,
+    pub weight: [*const c_void; 7],
+    pub weight_t: [*const c_void; 7],
+    pub A: [*const f32; 7],
+    pub B: [*const f32; 7],
+    pub dA: [*mut f32; 7],
+    pub dB: [*mut f32; 7],
+    pub saved: *mut c_void,
+    pub scratch: *mut c_void,
+    pub saved_bytes: usize,
+    pub scratch_bytes: usize,
+}
+
 /// Opaque training-step engine (`mcb_qwen_*`).
 #[repr(C)]
 pub struct mcb_qwen {
@@ -197,4 +223,7 @@ extern "C" {
     pub fn mcb_qwen_train_step(q: *mut mcb_qwen, ids: *const i32, targets: *const i32, batch: i64, seq: i64, lr: f32, beta1: f32, beta2: f32, eps: f32, weight_decay: f32, grad_scale: f32, loss_out: *mut f32, stream: *mut c_void) -> c_int;
     pub fn mcb_qwen_info(q: *const mcb_qwen, adamw_steps: *mut i64, persistent_bytes: *mut i64, kept_targets_dev: *mut *mut i32) -> c_int;
     pub fn mcb_qwen_destroy(q: *mut mcb_qwen) -> c_int;
+    pub fn mcb_qwen_layer_bytes(cfg: *const mcb_qwen_config, adapted_modules: c_int, rank: c_int, batch: i64, seq: i64, backward: c_int, saved_bytes: *mut i64, scratch_bytes: *mut i64) -> c_int;
+    pub fn mcb_qwen_layer_forward(cfg: *const mcb_qwen_config, call: *const mcb_qwen_layer_call, h_in: *const c_void, h_out: *mut c_void, stream: *mut c_void) -> c_int;
+    pub fn mcb_qwen_layer_backward(cfg: *const mcb_qwen_config, call: *const mcb_qwen_layer_call, h_in: *const c_void, dh: *const c_void, dh_in: *mut c_void, accumulate: c_int, stream: *mut c_void) -> c_int;
 }

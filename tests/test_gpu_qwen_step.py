@@ -279,3 +279,58 @@ def test_fused_qkv_step_equals_the_separate_projections(cuda_device):
     for a, b in zip(g1, g0):
         assert R.max_abs_normalised(a.cpu().numpy(), b.cpu().numpy().astype(np.float64)) <= 2e-2
     model.fuse_qkv = True
+
+
+@pytest.mark.parametrize("which,nb,seq", [("qv", 3, 37), ("all", 2, 128), ("qv", 8, 128)])
+def test_layer_calls_equal_kernel_by_kernel(cuda_device, monkeypatch, which, nb, seq):
+    """A layer as one library call against its kernels called one by one: the same launches, so logits, loss and gradients
+    agree bit for bit, also where gradients accumulate and inside a captured step; 8 x 128 tokens take the pair kernels."""
+    from metal_candle_b200 import qwen
+    from metal_candle_b200.training import TargetModule
+
+    targets = all_targets() if which == "all" else [TargetModule.QProj, TargetModule.VProj]
+    cfg, model, adapter = build(cuda_device, torch.bfloat16, targets, cfg=fused_attention_config())
+    ids, tg = batch(51, nb, seq, cfg.vocab_size)
+    ids_d, tg_d = torch.from_numpy(ids).to(cuda_device), torch.from_numpy(tg).to(cuda_device)
+    used = []
+    prepare = qwen._LayerCalls.prepare
+
+    def run():
+        logits = model.forward(ids_d).clone()
+        loss, g = model.forward_backward(ids_d, tg_d)
+        loss, g = loss.clone(), [t.clone() for t in g]
+        model.forward_backward(ids_d, tg_d, accumulate=True)
+        return [logits, loss] + g + [t.clone() for t in g]
+
+    monkeypatch.setattr(qwen._LayerCalls, "prepare", lambda self, *a: used.append(prepare(self, *a)) or used[-1])
+    got = run()
+    assert used and all(u is not None for u in used)
+    step = model.capture_forward_backward(nb, seq)
+    loss_c, g_c = step(ids_d, tg_d)
+    torch.cuda.synchronize()
+    captured = [loss_c.clone()] + [t.clone() for t in g_c]
+    monkeypatch.setattr(qwen._LayerCalls, "prepare", lambda self, *a: None)
+    want = run()
+    assert len(got) == len(want) and all(torch.equal(a, b) for a, b in zip(got, want))
+    assert all(torch.equal(a, b) for a, b in zip(captured, want[1:]))
+
+
+def test_layer_calls_leave_other_layers_to_the_kernels(cuda_device):
+    """Adapters of two ranks, or of more rank columns than the library's layer takes, and adapter tensors that are not laid
+    out as it expects, go kernel by kernel (the last of these reports it)."""
+    from metal_candle_b200 import qwen
+    from metal_candle_b200.backend import TrainingError
+    from metal_candle_b200.training import TargetModule
+
+    cfg, model, adapter = build(cuda_device, torch.bfloat16, [TargetModule.QProj, TargetModule.VProj, TargetModule.OProj], cfg=fused_attention_config())
+    calls = qwen._LayerCalls(model, 2, 16, backward=False)
+    assert calls.prepare(0) is not None
+    o = model.layers[0]["o_proj"].lora
+    a, b = o.lora_a, o.lora_b
+    o.lora_a = a.t().contiguous().t()
+    assert calls.prepare(0) is None
+    with pytest.raises(TrainingError, match="contiguous"):
+        model.forward(torch.zeros(2, 16, dtype=torch.int32, device=cuda_device))
+    o.lora_a, o.lora_b = torch.cat([a, a], 1).contiguous(), torch.cat([b, b], 0).contiguous()
+    assert calls.prepare(0) is None and calls.prepare(1) is not None
+    assert torch.isfinite(model.forward(torch.zeros(2, 16, dtype=torch.int32, device=cuda_device)).float()).all()
