@@ -85,8 +85,8 @@ int mcb_selftest_wait_timeout(int64_t limit_cycles, int64_t* waited_cycles_out, 
 /* Smallest reduction length (in features) from which a linear WITH a rank path runs on CTA pairs instead of the
  * one-CTA kernel (default 1536; linears without a rank path always take the pair kernel when large enough). */
 #define MCB_OPT_PAIR_MIN_K 1
-/* 1 (default): the small operand-pack and partial-sum kernels around the fused LoRA GEMM are chained to it by
- * programmatic dependent launch, so that each kernel's launch and set-up run under its predecessor's tail; 0: plain
+/* 1 (default): the library's kernels are launched as programmatic dependents of the kernel before them in their stream, so that
+ * a kernel's launch and set-up run under its predecessor's tail (it touches no memory before that has finished); 0: plain
  * stream order. */
 #define MCB_OPT_PDL 2
 #define MCB_OPT_COUNT_ 3

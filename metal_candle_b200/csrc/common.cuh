@@ -70,7 +70,13 @@ void note_launch();
     mcb::note_launch();                                        \
   } while (0)
 
-// Kernel launch with or without the programmatic-serialization attribute (see umma_ptx.cuh).
+// Whether kernels are launched as programmatic dependents of the kernel before them in their stream (MCB_OPT_PDL; not while
+// launches are timed one by one): the launch and the kernel's set-up then pass under the tail of that kernel.  Every kernel
+// launched so lets its own dependents start at once and waits (grid_dependency_wait) before it touches memory: the wait ends
+// when the kernel before it, which has waited likewise, is complete.
+inline bool chained_launch() { return !profile_on() && option(MCB_OPT_PDL) != 0; }
+
+// Kernel launch with or without the programmatic-serialization attribute.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl,
                                  Args&&... args) {
@@ -87,6 +93,20 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // ---- device-side helpers -----------------------------------------------------------------
+
+// Programmatic dependent launch.  A kernel launched with the programmatic-serialization attribute may start while
+// its predecessor in the stream is still running; `grid_dependency_wait` blocks until the predecessor grid has
+// completed and its writes are visible.  `grid_launch_dependents` lets a dependent grid launched with that attribute
+// start early (it has no effect otherwise).  Both are no-ops for kernels launched the ordinary way.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The pointer again, as a value that is not known before this point: a load that may be taken for one of constant memory
+// (const __restrict__, __ldg) cannot be moved up over the wait before it.
+template <typename T>
+__device__ __forceinline__ T* from_here(T* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
 
 template <typename T>
 struct Vec16;  // a 16-byte vector of T, convertible to/from floats

@@ -44,7 +44,10 @@ __global__ void __launch_bounds__(1024)
 cross_entropy_kernel(const T* in, T* out, const int32_t* __restrict__ targets, float* __restrict__ nll,
                      const int32_t* __restrict__ count_ptr, int64_t M, int V, int write_grad) {
   __shared__ float sm[32], ss[32];
-  const float inv_count = 1.0f / static_cast<float>(max(1, *count_ptr));
+  grid_launch_dependents();
+  grid_dependency_wait();
+  targets = from_here(targets);
+  const float inv_count = 1.0f / static_cast<float>(max(1, *from_here(count_ptr)));
   using VT = Vec16<T>;
   constexpr int NV = VT::N;
   const int bd = blockDim.x;
@@ -253,6 +256,8 @@ cross_entropy_cluster_kernel(const CeParams p) {
     fence_proxy_async_smem();
   }
   cl.sync();   // every CTA's barriers exist before a peer arrives on them
+  grid_launch_dependents();
+  grid_dependency_wait();
   const float inv_count = 1.0f / static_cast<float>(max(1, *p.count));
   const T* in = static_cast<const T*>(p.in) - p.mis;    // 16-byte boundaries
   T* out = static_cast<T*>(p.out) - p.mis;              // (not touched without write_grad)
@@ -452,6 +457,9 @@ cross_entropy_cluster_kernel(const CeParams p) {
 __global__ void count_valid_kernel(const int32_t* __restrict__ targets, int64_t M, int V, int32_t* __restrict__ count) {
   __shared__ int red[32];
   int c = 0;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  targets = from_here(targets);
   for (int64_t i = threadIdx.x; i < M; i += blockDim.x) c += (targets[i] >= 0 && targets[i] < V) ? 1 : 0;
   for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
@@ -468,6 +476,10 @@ __global__ void reduce_nll_kernel(const float* __restrict__ nll, int64_t M, cons
                                   float* __restrict__ loss) {
   __shared__ double red[1024];
   double acc = 0.0;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  nll = from_here(nll);
+  count = from_here(count);
   for (int64_t i = threadIdx.x; i < M; i += blockDim.x) acc += static_cast<double>(nll[i]);
   red[threadIdx.x] = acc;
   __syncthreads();
@@ -490,6 +502,9 @@ prepare_targets_kernel(const I* __restrict__ targets, int32_t* __restrict__ t32,
                        int32_t* __restrict__ info, int32_t* info_host) {
   __shared__ int red[2][32];
   int good = 0, bad = 0;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  targets = from_here(targets);
   for (int64_t i = threadIdx.x; i < M; i += blockDim.x) {
     int64_t t = targets[i];
     if (has_ignore && t == ignore) t = -1;
@@ -559,14 +574,17 @@ int launch_rows(const void* in, void* out, const int32_t* targets, float* nll, c
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(ctas)); cfg.blockDim = dim3(kCeThreads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = static_cast<unsigned>(ctas); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
     // as many clusters as are resident together: a later one would start its share of the rows when the others are done
     int resident = 0;
     if (int rc = resident_clusters<T>(cfg, ds->ce_clusters[sizeof(T) == 4][ctas], &resident)) return rc;
     cfg.gridDim = dim3(static_cast<unsigned>((M < resident ? M : resident) * ctas));
+    if (chained_launch()) cfg.numAttrs = 2;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, cross_entropy_cluster_kernel<T>, p);
     if (e != cudaSuccess) return cuda_fail(e, "cross_entropy_cluster_kernel launch");
     MCB_CHECK_LAUNCH("cross_entropy_cluster_kernel");
@@ -574,11 +592,11 @@ int launch_rows(const void* in, void* out, const int32_t* targets, float* nll, c
   }
   // eight blocks of 256 threads per SM, fewer when there are fewer rows
   const int64_t blocks = static_cast<int64_t>(ds->sm_count) * 8;
-  cross_entropy_kernel<T><<<static_cast<unsigned>(M < blocks ? M : blocks), 256, 0, st>>>(static_cast<const T*>(in), static_cast<T*>(out),
-                                                                                          targets, nll, count, M, static_cast<int>(V), write_grad);
+  MCB_CHECK_CUDA(launch_kernel(cross_entropy_kernel<T>, dim3(static_cast<unsigned>(M < blocks ? M : blocks)), dim3(256), 0, st, chained_launch(),
+                               static_cast<const T*>(in), static_cast<T*>(out), targets, nll, count, M, static_cast<int>(V), write_grad));
   MCB_CHECK_LAUNCH("cross_entropy");
   if (loss != nullptr) {
-    reduce_nll_kernel<<<1, 1024, 0, st>>>(nll, M, count, loss);
+    MCB_CHECK_CUDA(launch_kernel(reduce_nll_kernel, dim3(1), dim3(1024), 0, st, chained_launch(), nll, M, count, loss));
     MCB_CHECK_LAUNCH("reduce_nll");
   }
   return MCB_OK;
@@ -603,10 +621,10 @@ extern "C" int mcb_cross_entropy(void* logits, const int32_t* targets, float* nl
   DeviceState* ds = current_device_state();
   if (!ds) return MCB_ERR_NOT_INIT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  count_valid_kernel<<<1, 1024, 0, st>>>(targets, M, (int)V, count);
+  MCB_CHECK_CUDA(launch_kernel(count_valid_kernel, dim3(1), dim3(1024), 0, st, chained_launch(), targets, M, (int)V, count));
   MCB_CHECK_LAUNCH("count_valid");
   if (int rc = launch_rows(logits, logits, targets, nll, count, M, V, write_grad, dtype, nullptr, nullptr, ds, st)) return rc;
-  reduce_nll_kernel<<<1, 1024, 0, st>>>(nll, M, count, loss);
+  MCB_CHECK_CUDA(launch_kernel(reduce_nll_kernel, dim3(1), dim3(1024), 0, st, chained_launch(), nll, M, count, loss));
   MCB_CHECK_LAUNCH("reduce_nll");
   return MCB_OK;
 }
@@ -618,7 +636,7 @@ extern "C" int mcb_cross_entropy_count(const int32_t* targets, int32_t* count, i
   if (!targets || !count) return fail(MCB_ERR_NULL, "cross_entropy_count: null pointer");
   if (M <= 0 || V <= 0 || M > 0x7fffffff || V > 0x7fffffff) return fail(MCB_ERR_SHAPE, "cross_entropy_count: bad shape");
   if (!current_device_state()) return MCB_ERR_NOT_INIT;
-  count_valid_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(targets, M, (int)V, count);
+  MCB_CHECK_CUDA(launch_kernel(count_valid_kernel, dim3(1), dim3(1024), 0, static_cast<cudaStream_t>(stream), chained_launch(), targets, M, (int)V, count));
   MCB_CHECK_LAUNCH("count_valid");
   return MCB_OK;
 }
@@ -638,7 +656,7 @@ extern "C" int mcb_cross_entropy_finish(const float* nll, const int32_t* count, 
   if (!nll || !count || !loss) return fail(MCB_ERR_NULL, "cross_entropy_finish: null pointer");
   if (M <= 0 || M > 0x7fffffff) return fail(MCB_ERR_SHAPE, "cross_entropy_finish: bad shape");
   if (!current_device_state()) return MCB_ERR_NOT_INIT;
-  reduce_nll_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(nll, M, count, loss);
+  MCB_CHECK_CUDA(launch_kernel(reduce_nll_kernel, dim3(1), dim3(1024), 0, static_cast<cudaStream_t>(stream), chained_launch(), nll, M, count, loss));
   MCB_CHECK_LAUNCH("reduce_nll");
   return MCB_OK;
 }
@@ -654,10 +672,13 @@ extern "C" int mcb_cross_entropy_out(const void* logits, void* dlogits, const vo
   DeviceState* ds = current_device_state();
   if (!ds) return MCB_ERR_NOT_INIT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (target_bytes == 8)
-    prepare_targets_kernel<int64_t><<<1, 1024, 0, st>>>(static_cast<const int64_t*>(targets), t32, M, V, has_ignore, ignore_index, info, info_host);
-  else
-    prepare_targets_kernel<int32_t><<<1, 1024, 0, st>>>(static_cast<const int32_t*>(targets), t32, M, V, has_ignore, ignore_index, info, info_host);
+  if (target_bytes == 8) {
+    MCB_CHECK_CUDA(launch_kernel(prepare_targets_kernel<int64_t>, dim3(1), dim3(1024), 0, st, chained_launch(), static_cast<const int64_t*>(targets), t32, M, V,
+                                 has_ignore, ignore_index, info, info_host));
+  } else {
+    MCB_CHECK_CUDA(launch_kernel(prepare_targets_kernel<int32_t>, dim3(1), dim3(1024), 0, st, chained_launch(), static_cast<const int32_t*>(targets), t32, M, V,
+                                 has_ignore, ignore_index, info, info_host));
+  }
   MCB_CHECK_LAUNCH("prepare_targets");
   if (info_event != nullptr) MCB_CHECK_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(info_event), st));
   const bool grad = dlogits != nullptr;

@@ -169,6 +169,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  grid_launch_dependents();
+  grid_dependency_wait();   // the set-up above ran under the tail of the kernel before
   // S buffers at columns 0 and 64, O at 128, the two P buffers (bf16 pairs: 32 columns each) at 192 and 224
   const uint32_t tO = tmem_base + 128, tP0 = tmem_base + 192;
   const int n_tiles = q_blocks(p.S) * p.G * p.NB;
@@ -466,6 +468,8 @@ attn_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  grid_launch_dependents();
+  grid_dependency_wait();   // the set-up above ran under the tail of the kernel before
   const uint32_t tDP = tmem_base + 128, tDQ = tmem_base + 192;
   FwdParams tp;   // the item order of the forward
   tp.S = p.S; tp.G = p.G; tp.NB = p.NB;
@@ -743,6 +747,8 @@ attn_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  grid_launch_dependents();
+  grid_dependency_wait();   // the set-up above ran under the tail of the kernel before
   // columns: S^T buffers at 0 and 128, dP^T at 64 and 192, dV at 256, dK at 320, then per buffer P^T (32 columns
   // of bf16 pairs) and dS^T (32): 384 / 416 and 448 / 480
   const uint32_t tDV = tmem_base + 256, tDK = tmem_base + 320, tPT0 = tmem_base + 384;
@@ -1067,7 +1073,7 @@ int attention_fwd(const void* q, const void* k, const void* v, void* o, float* l
   const int64_t n_tiles = q_blocks(static_cast<int>(seq)) * groups * nb;
   const int64_t slots = 2 * static_cast<int64_t>(ds->sm_count);
   const unsigned grid = static_cast<unsigned>(n_tiles < slots ? n_tiles : slots);
-  attn_fwd_kernel<<<grid, kThreads, kFwdSmem, st>>>(tmQ, tmK, tmVt, p);
+  MCB_CHECK_CUDA(launch_kernel(attn_fwd_kernel, dim3(grid), dim3(kThreads), kFwdSmem, st, chained_launch(), tmQ, tmK, tmVt, p));
   MCB_CHECK_LAUNCH("attn_fwd_kernel");
   return MCB_OK;
 }
@@ -1152,17 +1158,19 @@ int attention_bwd(const void* q, const void* k, const void* v, const void* o, co
   const int64_t n_tiles = q_blocks(static_cast<int>(seq)) * groups * nb;
   const int64_t slots = 2 * static_cast<int64_t>(ds->sm_count);
   const unsigned gq = static_cast<unsigned>(n_tiles < slots ? n_tiles : slots);
-  attn_dq_kernel<<<gq, kThreads, kDqSmem, st>>>(tmQ128, tmdO128, tmK64, tmV64, p);
+  MCB_CHECK_CUDA(launch_kernel(attn_dq_kernel, dim3(gq), dim3(kThreads), kDqSmem, st, chained_launch(), tmQ128, tmdO128, tmK64, tmV64, p));
   MCB_CHECK_LAUNCH("attn_dq_kernel");
   p.kv_parts = dkv_parts(nb, groups, seq, ds->sm_count);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(nb * p.kv_parts), static_cast<unsigned>(q_blocks(static_cast<int>(seq))));
   cfg.blockDim = dim3(kKvThreads);
   cfg.dynamicSmemBytes = kKvSmem; cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(p.kv_parts); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = p.kv_parts > 1 ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = chained_launch() ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(p.kv_parts); attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = p.kv_parts > 1 ? 2 : 1;
   MCB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_dkv_kernel, tmK128, tmV128, tmQ64, tmdO64, p));
   MCB_CHECK_LAUNCH("attn_dkv_kernel");
   return MCB_OK;

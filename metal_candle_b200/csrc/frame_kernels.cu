@@ -11,6 +11,10 @@ template <typename T>
 __global__ void embedding_fwd_kernel(const int32_t* __restrict__ ids, const T* __restrict__ table, T* __restrict__ out,
                                      int64_t M, int H, int vocab) {
   const int64_t row = blockIdx.x;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  ids = from_here(ids);
+  table = from_here(table);
   if (row >= M) return;
   int32_t id = ids[row];
   if (id < 0 || id >= vocab) id = 0;  // ids are validated on the host; never read out of range
@@ -97,6 +101,12 @@ __global__ void rope_relayout_qkv_kernel(T* __restrict__ fused, RopeSegment<T> s
                                          int d, float theta, int inverse, int64_t pitch) {
   using V = Vec16<T>;
   constexpr int N = V::N;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  fused = from_here(fused);
+  s0.head_major = from_here(s0.head_major);
+  s1.head_major = from_here(s1.head_major);
+  s2.head_major = from_here(s2.head_major);
   const int half = d / 2;
   const int chunks = half / N;
   const int64_t total = static_cast<int64_t>(B) * S * chunks;
@@ -182,6 +192,11 @@ template <typename T>
 __global__ void swiglu_fwd_kernel(const T* __restrict__ gate, const T* __restrict__ up, T* __restrict__ out, int64_t n) {
   using V = Vec16<T>;
   constexpr int N = V::N;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  gate = from_here(gate);
+  up = from_here(up);
+  out = from_here(out);
   const int64_t nv = n / N;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < nv;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -203,6 +218,13 @@ __global__ void swiglu_bwd_kernel(const T* __restrict__ gate, const T* __restric
                                   T* __restrict__ dgate, T* __restrict__ dup, int64_t n) {
   using V = Vec16<T>;
   constexpr int N = V::N;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  gate = from_here(gate);
+  up = from_here(up);
+  dout = from_here(dout);
+  dgate = from_here(dgate);
+  dup = from_here(dup);
   const int64_t nv = n / N;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < nv;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -316,7 +338,9 @@ extern "C" int mcb_embedding_fwd(const int32_t* ids, const void* table, void* ou
   if (M <= 0 || H <= 0 || vocab <= 0 || M > 0x7fffffff) return fail(MCB_ERR_SHAPE, "embedding_fwd: bad shape");
   if (!current_device_state()) return MCB_ERR_NOT_INIT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  MCB_DTYPE_SWITCH(dtype, (embedding_fwd_kernel<T><<<(unsigned)M, 128, 0, st>>>(ids, (const T*)table, (T*)out, M, (int)H, (int)vocab)));
+  cudaError_t le = cudaSuccess;
+  MCB_DTYPE_SWITCH(dtype, (le = launch_kernel(embedding_fwd_kernel<T>, dim3((unsigned)M), dim3(128), 0, st, chained_launch(), ids, (const T*)table, (T*)out, M, (int)H, (int)vocab)));
+  if (le != cudaSuccess) return cuda_fail(le, "embedding_fwd launch");
   MCB_CHECK_LAUNCH("embedding_fwd");
   return MCB_OK;
 }
@@ -358,7 +382,9 @@ extern "C" int mcb_rope_relayout_qkv(void* fused, void* q, void* k, void* v, int
     RopeSegment<T> s0{static_cast<T*>(q), static_cast<int>(Hq), 0, 1};
     RopeSegment<T> s1{static_cast<T*>(k), static_cast<int>(Hk), Hq * d, 1};
     RopeSegment<T> s2{static_cast<T*>(v), static_cast<int>(Hk), (Hq + Hk) * d, 0};
-    rope_relayout_qkv_kernel<T><<<grid, 128, 0, st>>>(static_cast<T*>(fused), s0, s1, s2, (int)B, (int)S, (int)d, theta, inverse, token_pitch);
+    const cudaError_t le = launch_kernel(rope_relayout_qkv_kernel<T>, grid, dim3(128), 0, st, chained_launch(), static_cast<T*>(fused), s0, s1, s2,
+                                         (int)B, (int)S, (int)d, theta, inverse, token_pitch);
+    if (le != cudaSuccess) return cuda_fail(le, "rope_relayout_qkv launch");
   }));
   MCB_CHECK_LAUNCH("rope_relayout_qkv");
   return MCB_OK;
@@ -403,7 +429,9 @@ extern "C" int mcb_swiglu_fwd(const void* gate, const void* up, void* out, int64
   if (!ds) return MCB_ERR_NOT_INIT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int grid = grid_for(n / 4, 256, ds->sm_count);
-  MCB_DTYPE_SWITCH(dtype, (swiglu_fwd_kernel<T><<<grid, 256, 0, st>>>((const T*)gate, (const T*)up, (T*)out, n)));
+  cudaError_t le = cudaSuccess;
+  MCB_DTYPE_SWITCH(dtype, (le = launch_kernel(swiglu_fwd_kernel<T>, dim3(grid), dim3(256), 0, st, chained_launch(), (const T*)gate, (const T*)up, (T*)out, n)));
+  if (le != cudaSuccess) return cuda_fail(le, "swiglu_fwd launch");
   MCB_CHECK_LAUNCH("swiglu_fwd");
   return MCB_OK;
 }
@@ -419,7 +447,9 @@ extern "C" int mcb_swiglu_bwd(const void* gate, const void* up, const void* dout
   if (!ds) return MCB_ERR_NOT_INIT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int grid = grid_for(n / 4, 256, ds->sm_count);
-  MCB_DTYPE_SWITCH(dtype, (swiglu_bwd_kernel<T><<<grid, 256, 0, st>>>((const T*)gate, (const T*)up, (const T*)dout, (T*)dgate, (T*)dup, n)));
+  cudaError_t le = cudaSuccess;
+  MCB_DTYPE_SWITCH(dtype, (le = launch_kernel(swiglu_bwd_kernel<T>, dim3(grid), dim3(256), 0, st, chained_launch(), (const T*)gate, (const T*)up, (const T*)dout, (T*)dgate, (T*)dup, n)));
+  if (le != cudaSuccess) return cuda_fail(le, "swiglu_bwd launch");
   MCB_CHECK_LAUNCH("swiglu_bwd");
   return MCB_OK;
 }

@@ -81,9 +81,6 @@ struct GemmCall {
   // Weight-gradient problems to run as a tail phase of the same launch (one-CTA kernel only), or null.  Problem 0
   // reads the H this call writes.
   const GradRequest* grads = nullptr;
-  // The launch directly before this call's GEMM on the same stream is the operand-pack kernel of this call (the
-  // GEMM may then be launched as its programmatic dependent).
-  bool after_pack = false;
   // Y is the gate buffer of a SwiGLU and this its up buffer: the product is d act, and the epilogue replaces gate and
   // up by d gate and d up instead of storing it (pair kernel only).
   __nv_bfloat16* swiglu_up = nullptr;

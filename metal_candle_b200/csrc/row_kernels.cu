@@ -257,6 +257,9 @@ colsum_partials_kernel(const float* __restrict__ partial, float* __restrict__ dw
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = blockIdx.x * 32 + lane;
   float s = 0.0f;
+  grid_launch_dependents();
+  grid_dependency_wait();
+  partial = from_here(partial);
   if (c < D) {
 #pragma unroll 8
     for (int b = warp; b < nblocks; b += 8) s += partial[static_cast<int64_t>(b) * D + c];
@@ -583,7 +586,9 @@ int rmsnorm_bwd_t(const void* x, const void* w, const void* dy, void* dx, float*
     const int rc = rowpipe::try_launch<T>(rowpipe::kRmsBwd, x, dy, w, dx, nullptr, dw ? (float*)ws : nullptr, &blocks, rows, D,
                                           eps, 0, 1.0f, ds, st, res);
     if (rc == MCB_OK && dw != nullptr) {
-      colsum_partials_kernel<<<(unsigned)((D + 31) / 32), 256, 0, st>>>((const float*)ws, dw, blocks, (int)D, accumulate);
+      const cudaError_t le = launch_kernel(colsum_partials_kernel, dim3((unsigned)((D + 31) / 32)), dim3(256), 0, st, chained_launch(),
+                                           (const float*)ws, dw, blocks, (int)D, accumulate);
+      if (le != cudaSuccess) return cuda_fail(le, "rmsnorm_dw_reduce launch");
       MCB_CHECK_LAUNCH("rmsnorm_dw_reduce");
     }
     if (rc != 1) return rc;

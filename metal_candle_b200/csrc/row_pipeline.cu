@@ -164,6 +164,8 @@ rowpipe_kernel(const Params p) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async_smem();
   }
+  grid_launch_dependents();
+  grid_dependency_wait();
   // The weight as float32, in planes of four columns per vector: column vi * N + j is at (j / 4) * w_plane + vi * 4 + j % 4,
   // so that the lanes of a warp, one vector each, read 16 bytes next to each other.  Column after column a bf16 vector's
   // eight weights are 32 bytes from its neighbour's, and every read of four (two) of them cost twice (four times) its
@@ -175,7 +177,7 @@ rowpipe_kernel(const Params p) {
     if (p.w_off != 0) {
       float* wd = reinterpret_cast<float*>(gen_base + p.w_off);
       for (int c = threadIdx.x; c < p.D; c += blockDim.x)
-        wd[c % N / 4 * w_plane + c / N * 4 + c % 4] = to_f32(static_cast<const T*>(p.w)[c]);
+        wd[c % N / 4 * w_plane + c / N * 4 + c % 4] = to_f32(from_here(static_cast<const T*>(p.w))[c]);
       wsm = wd;
     }
   }
@@ -755,7 +757,8 @@ int launch_one(const Params& p, int grid, size_t smem, cudaStream_t st) {
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(rowpipe_kernel carve-out)");
     attr_set[dev] = true;
   }
-  rowpipe_kernel<T, OP, W, KMAX, RAG><<<grid, (W + 1) * 32, smem, st>>>(p);
+  const cudaError_t le = launch_kernel(rowpipe_kernel<T, OP, W, KMAX, RAG>, dim3(grid), dim3((W + 1) * 32), smem, st, chained_launch(), p);
+  if (le != cudaSuccess) return cuda_fail(le, "rowpipe_kernel launch");
   MCB_CHECK_LAUNCH("rowpipe_kernel");
   return MCB_OK;
 }

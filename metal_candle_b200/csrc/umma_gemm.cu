@@ -62,7 +62,6 @@ struct GemmParams {
   int M, N, K;
   int BN, rp, has_w, stages;
   int num_m_tiles, num_n_tiles, num_tiles, num_k_blocks, group_m;
-  int pdl_wait;       // 1: launched as a programmatic dependent of the operand-pack kernel: wait for it before loading
   float scale;
   __nv_bfloat16* Y;
   const __nv_bfloat16* bias;
@@ -144,8 +143,9 @@ lora_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
-  // a partial-sum kernel chained behind this launch may be set up now; it waits for this grid before it reads
-  if (threadIdx.x == 0) grid_launch_dependents();
+  // everything up to here (barriers, tensor memory) ran under the tail of the kernel before
+  grid_launch_dependents();
+  grid_dependency_wait();
 
   const int nkb = p.num_k_blocks;
 
@@ -156,8 +156,6 @@ lora_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       uint32_t phase = 0;
       bool ok = true;
       int i = 0;
-      // everything up to here (barriers, tensor memory) ran under the tail of the operand-pack kernel
-      if (p.pdl_wait) grid_dependency_wait();
       for (int t = blockIdx.x; ok && t < p.num_tiles; t += gridDim.x, ++i) {
         int mt, nt;
         tile_coords(p, t, mt, nt);
@@ -456,6 +454,9 @@ __global__ void pack_lora_kernel(const float* __restrict__ A, const float* __res
                                  __nv_bfloat16* __restrict__ P, __nv_bfloat16* __restrict__ Q, int K, int N, int r,
                                  int rp, int mode, int* __restrict__ flags, int n_flags) {
   grid_launch_dependents();   // the GEMM chained behind this kernel may start its set-up; it waits before it loads P / Q
+  grid_dependency_wait();     // P, Q and the counters may still be in use, A and B in the making
+  A = from_here(A);
+  B = from_here(B);
   const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   // the per-tile counters of the backward kernel's tail phase start from zero in every call
   for (int64_t i = tid; i < n_flags; i += static_cast<int64_t>(gridDim.x) * blockDim.x) flags[i] = 0;
@@ -493,6 +494,7 @@ struct SegTable {
 __global__ void pack_lora_fused_kernel(const SegTable t, __nv_bfloat16* __restrict__ P, __nv_bfloat16* __restrict__ Q, int K,
                                        int N, int r, int rp, int mode, int* __restrict__ flags, int n_flags) {
   grid_launch_dependents();
+  grid_dependency_wait();
   const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   for (int64_t i = tid; i < n_flags; i += static_cast<int64_t>(gridDim.x) * blockDim.x) flags[i] = 0;
   const int64_t nP = static_cast<int64_t>(rp) * (mode == 0 ? K : N);
@@ -530,6 +532,10 @@ struct ScatterTable {
 };
 __global__ void scatter_fused_grads_kernel(const ScatterTable t, const float* __restrict__ dA_cat, const float* __restrict__ dB_cat,
                                            int K, int N, int r, int accumulate) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  dA_cat = from_here(dA_cat);
+  dB_cat = from_here(dB_cat);
   const int r_tot = t.count * r;
   const int64_t nA = static_cast<int64_t>(K) * r_tot;
   int64_t nB = 0;
@@ -701,11 +707,8 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
     }
     profile_begin(c.rp > 0 ? kProfGemmLora : kProfGemm, flops, bytes, st);
   }
-  // with a rank path the launch directly before this one is the operand-pack kernel
-  const bool pdl = c.after_pack && !prof && option(MCB_OPT_PDL) != 0;
-  p.pdl_wait = pdl ? 1 : 0;
   {
-    const cudaError_t le = launch_kernel(lora_gemm_kernel, dim3(grid), dim3(kThreads), kSmemBudget + 1024, st, pdl, tmX, tmW, tmP, tmQ,
+    const cudaError_t le = launch_kernel(lora_gemm_kernel, dim3(grid), dim3(kThreads), kSmemBudget + 1024, st, chained_launch(), tmX, tmW, tmP, tmQ,
                                          tmY, tail.tmX[0], tail.tmH[0], tail.tmX[1], tail.tmH[1], p, tail.p);
     if (le != cudaSuccess) return cuda_fail(le, "lora_gemm_kernel launch");
   }
@@ -746,9 +749,10 @@ Workspace carve(void* ws, int64_t M, int64_t K, int64_t N, int64_t r) {
 int pack(const LoraArgs& a, const Workspace& w, int mode) {
   const int rp = static_cast<int>(rank_padded(a.r));
   const int64_t n = static_cast<int64_t>(rp) * (a.K + a.N);
-  pack_lora_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, a.stream>>>(
-      a.A, a.B, w.P, w.Q, static_cast<int>(a.K), static_cast<int>(a.N), static_cast<int>(a.r), rp, mode,
-      mode == 1 ? w.flags : nullptr, mode == 1 ? static_cast<int>((a.M + BM - 1) / BM) : 0);
+  const cudaError_t le = launch_kernel(pack_lora_kernel, dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, a.stream, chained_launch(), a.A,
+                                       a.B, w.P, w.Q, static_cast<int>(a.K), static_cast<int>(a.N), static_cast<int>(a.r), rp, mode,
+                                       mode == 1 ? w.flags : nullptr, mode == 1 ? static_cast<int>((a.M + BM - 1) / BM) : 0);
+  if (le != cudaSuccess) return cuda_fail(le, "pack_lora launch");
   MCB_CHECK_LAUNCH("pack_lora");
   return MCB_OK;
 }
@@ -803,7 +807,6 @@ int delta_fwd(const LoraArgs& a, const DeviceState* ds) {
   Workspace w = carve(a.ws, a.M, a.K, a.N, a.r);
   if (int rc = pack(a, w, 0)) return rc;
   GemmCall c;
-  c.after_pack = true;
   c.X = static_cast<const __nv_bfloat16*>(a.x);
   c.P = w.P; c.Q = w.Q;
   c.Y = static_cast<__nv_bfloat16*>(a.y);
@@ -828,7 +831,6 @@ int linear_fwd(const LoraArgs& a, const DeviceState* ds) {
   if (a.r > 0) {
     Workspace w = carve(a.ws, a.M, a.K, a.N, a.r);
     if (int rc = pack(a, w, 0)) return rc;
-    c.after_pack = true;
     c.P = w.P; c.Q = w.Q;
     c.H = static_cast<__nv_bfloat16*>(a.h_save);
     c.h_pitch = h_pitch(a.M);
@@ -877,7 +879,6 @@ int linear_bwd(const LoraArgs& a, const DeviceState* ds) {
     c.swiglu_up = static_cast<__nv_bfloat16*>(a.swiglu_up);
     c.M = a.M; c.N = a.K; c.K = a.N;
     if (a.r > 0) {
-      c.after_pack = true;   // pack(a, w, 1) above is the launch directly before the GEMM
       c.P = w.P; c.Q = w.Q;
       c.H = (a.dA != nullptr) ? w.H1 : nullptr;
       c.h_pitch = h_pitch(a.M);
@@ -910,7 +911,6 @@ int linear_bwd(const LoraArgs& a, const DeviceState* ds) {
       // P/Q of the backward are still needed by nothing after the GEMM above, so they can be repacked
       if (int rc = pack(f, wf, 0)) return rc;
       GemmCall c;
-      c.after_pack = true;
       c.X = static_cast<const __nv_bfloat16*>(a.x);
       c.P = wf.P; c.Q = wf.Q;
       c.H = w.H2;
@@ -963,9 +963,10 @@ int pack_fused(const LoraArgs& a, const LoraSegments& sg, const Workspace& w, in
     t.n_off[i] = static_cast<int>(sg.n_off[i]); t.n[i] = static_cast<int>(sg.n[i]);
   }
   const int64_t n = static_cast<int64_t>(rp) * (a.K + a.N);
-  pack_lora_fused_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, a.stream>>>(
-      t, w.P, w.Q, static_cast<int>(a.K), static_cast<int>(a.N), static_cast<int>(a.r), rp, mode,
-      mode == 1 ? w.flags : nullptr, mode == 1 ? static_cast<int>((a.M + BM - 1) / BM) : 0);
+  const cudaError_t le = launch_kernel(pack_lora_fused_kernel, dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, a.stream,
+                                       chained_launch(), t, w.P, w.Q, static_cast<int>(a.K), static_cast<int>(a.N), static_cast<int>(a.r), rp, mode,
+                                       mode == 1 ? w.flags : nullptr, mode == 1 ? static_cast<int>((a.M + BM - 1) / BM) : 0);
+  if (le != cudaSuccess) return cuda_fail(le, "pack_lora_fused launch");
   MCB_CHECK_LAUNCH("pack_lora_fused");
   return MCB_OK;
 }
@@ -1001,7 +1002,6 @@ int linear_fused_fwd(const LoraArgs& a, const LoraSegments& sg, const DeviceStat
   FusedWorkspace f = carve_fused(a.ws, a.M, a.K, a.N, r_tot);
   if (int rc = pack_fused(a, sg, f.w, rp, 0)) return rc;
   GemmCall c;
-  c.after_pack = true;
   c.X = static_cast<const __nv_bfloat16*>(a.x);
   c.W = static_cast<const __nv_bfloat16*>(a.W);
   c.bias = static_cast<const __nv_bfloat16*>(a.bias);
@@ -1032,7 +1032,6 @@ int linear_fused_bwd(const LoraArgs& a, const LoraSegments& sg, const DeviceStat
   FusedWorkspace f = carve_fused(a.ws, a.M, a.K, a.N, r_tot);
   if (int rc = pack_fused(a, sg, f.w, rp, 1)) return rc;
   GemmCall c;
-  c.after_pack = true;
   c.X = static_cast<const __nv_bfloat16*>(a.dy);
   c.W = a.dx != nullptr ? static_cast<const __nv_bfloat16*>(a.W) : nullptr;
   c.Y = static_cast<__nv_bfloat16*>(a.dx);
@@ -1060,8 +1059,10 @@ int linear_fused_bwd(const LoraArgs& a, const LoraSegments& sg, const DeviceStat
     t.n_off[i] = static_cast<int>(sg.n_off[i]); t.n[i] = static_cast<int>(sg.n[i]);
     elems += a.r * sg.n[i];
   }
-  scatter_fused_grads_kernel<<<static_cast<unsigned>((elems + 255) / 256), 256, 0, a.stream>>>(
-      t, f.dA_cat, f.dB_cat, static_cast<int>(a.K), static_cast<int>(a.N), static_cast<int>(a.r), a.accumulate);
+  const cudaError_t le = launch_kernel(scatter_fused_grads_kernel, dim3(static_cast<unsigned>((elems + 255) / 256)), dim3(256), 0, a.stream,
+                                       chained_launch(), t, f.dA_cat, f.dB_cat, static_cast<int>(a.K), static_cast<int>(a.N),
+                                       static_cast<int>(a.r), a.accumulate);
+  if (le != cudaSuccess) return cuda_fail(le, "scatter_fused_grads launch");
   MCB_CHECK_LAUNCH("scatter_fused_grads");
   return MCB_OK;
 }

@@ -51,7 +51,6 @@ constexpr int kEpiBufs = kEpiBufsMax;
 struct Gemm2Params {
   int M, N, K;
   int BN, stages, rp;
-  int pdl_wait; // 1: launched as a programmatic dependent of the operand-pack kernel
   int swiglu;   // 1: the tile is [128 gate columns | 128 up columns]; the epilogue also writes silu(gate) * up
                 // 2: the product is d act of a SwiGLU; the epilogue turns it into d gate and d up (see U) and stores those
   int epi_bufs; // 2-KB staging buffers per 32 rows of the tile (kEpiBufs; 12 in the SwiGLU-backward form)
@@ -198,6 +197,8 @@ lora_gemm2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   cluster_sync_all();  // both CTAs' barriers exist before anything arrives on them remotely
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  grid_launch_dependents();
+  grid_dependency_wait();   // the set-up above ran under the tail of the kernel before
   const int nkb = p.num_k_blocks;
   const int half_n = p.BN / 2, half_r = p.rp / 2, quarter_n = p.BN / 4;
 
@@ -208,7 +209,6 @@ lora_gemm2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       uint32_t phase = 0;
       bool ok = true;
       int i = 0;
-      if (p.pdl_wait) grid_dependency_wait();   // the operand-pack kernel has finished
       for (int t = pair; ok && t < p.num_tiles; t += npairs, ++i) {
         int mt, nt;
         tile_coords2(p, t, mt, nt);
@@ -370,7 +370,6 @@ lora_gemm2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       if (++pf_k == cset) { pf_k = 0; pf_t += npairs; pf_tile(); }
     };
     if (p.swiglu == 2 && lane == 0 && !helper) {
-      if (p.pdl_wait) grid_dependency_wait();   // gate and up may come from the kernel before the operand pack
       pf_tile();
       for (int j = 0; j < ahead; ++j) gu_issue_next();
     }
@@ -694,10 +693,8 @@ int launch_gemm2(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
                   2.0 * m * n * k + 2.0 * m * c.r_true * (k + n),
                   2.0 * (m * k + n * k + (c.swiglu_up != nullptr ? 4.0 : 1.0) * m * n) + 2.0 * c.rp * (k + n), st);
   }
-  const bool pdl = c.after_pack && c.rp > 0 && !prof && option(MCB_OPT_PDL) != 0;
-  p.pdl_wait = pdl ? 1 : 0;
   {
-    const cudaError_t le = launch_kernel(lora_gemm2_kernel, dim3(2 * pairs), dim3(helpers ? kThreads2Wide : kThreads2), kSmem2 + 1024, st, pdl, tmX, tmW, tmP,
+    const cudaError_t le = launch_kernel(lora_gemm2_kernel, dim3(2 * pairs), dim3(helpers ? kThreads2Wide : kThreads2), kSmem2 + 1024, st, chained_launch(), tmX, tmW, tmP,
                                          tmQ, tmY, tmU, tmY, tmY64, tmU64, p);
     if (le != cudaSuccess) return cuda_fail(le, "lora_gemm2_kernel launch");
   }
@@ -759,7 +756,11 @@ int launch_gemm2_swiglu(const __nv_bfloat16* X, const __nv_bfloat16* Wgu, __nv_b
     const double m = static_cast<double>(M), n = static_cast<double>(2 * F), k = static_cast<double>(K);
     profile_begin(kProfGemm, 2.0 * m * n * k, 2.0 * (m * k + n * k + 1.5 * m * n), st);
   }
-  lora_gemm2_kernel<<<2 * pairs, kThreads2, kSmem2 + 1024, st>>>(tmX, tmW, tmX, tmX, tmG, tmU, tmA, tmG, tmG, p);
+  {
+    const cudaError_t le = launch_kernel(lora_gemm2_kernel, dim3(2 * pairs), dim3(kThreads2), kSmem2 + 1024, st, chained_launch(), tmX, tmW, tmX, tmX,
+                                         tmG, tmU, tmA, tmG, tmG, p);
+    if (le != cudaSuccess) return cuda_fail(le, "lora_gemm2_kernel launch");
+  }
   if (prof) profile_end(st);
   MCB_CHECK_LAUNCH("lora_gemm2_kernel");
   return MCB_OK;

@@ -64,7 +64,8 @@ lora_grad_umma_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_con
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
 
-  if (threadIdx.x == 0) grid_launch_dependents();   // the partial-sum kernel may be set up; it waits for this grid
+  grid_launch_dependents();   // the partial-sum kernel may be set up; it waits for this grid
+  grid_dependency_wait();
   GradShared sh;
   sh.base = base; sh.full0 = full0; sh.empty0 = empty0; sh.done_bar = done_bar; sh.tmem_base = tmem_base;
   sh.abort_flag = abort_flag;
@@ -93,7 +94,8 @@ struct ReduceProblem {
 __global__ void __launch_bounds__(256)
 lora_grad_reduce_kernel(ReduceProblem a, ReduceProblem b, int blocks_a, int r, int rp, int accumulate) {
   __shared__ float red[8][32];
-  grid_dependency_wait();   // launched as a programmatic dependent of the kernel that writes the partials
+  grid_launch_dependents();
+  grid_dependency_wait();   // for the kernel that writes the partials
   const bool second = static_cast<int>(blockIdx.x) >= blocks_a;
   const ReduceProblem q = second ? b : a;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -468,7 +470,7 @@ int launch_grad_reduce(const GradPlan& plan, cudaStream_t st) {
   const int blocks_b = two ? static_cast<int>((rq.C[1] * p.rp + 31) / 32) : 0;
   {
     const cudaError_t le = launch_kernel(lora_grad_reduce_kernel, dim3(static_cast<unsigned>(blocks_a + blocks_b)), dim3(256), 0, st,
-                                         option(MCB_OPT_PDL) != 0 && !profile_on(), ra, rb, blocks_a, rq.r, p.rp, rq.accumulate);
+                                         chained_launch(), ra, rb, blocks_a, rq.r, p.rp, rq.accumulate);
     if (le != cudaSuccess) return cuda_fail(le, "lora_grad_reduce launch");
   }
   MCB_CHECK_LAUNCH("lora_grad_reduce");
@@ -501,7 +503,9 @@ int launch_grad2(const __nv_bfloat16* X0, const __nv_bfloat16* Ht0, int64_t C0, 
   if (int rc = plan_grad2(rq, M, rp, ds->sm_count, kGradSmemBudget, ds, &plan)) return rc;
   const bool prof = profile_on();
   if (prof) profile_begin(kProfGrad, 2.0 * M * (rq.C[0] + rq.C[1]) * r, 2.0 * M * (rq.C[0] + rq.C[1]) + 2.0 * np * M * rp, st);
-  lora_grad_umma_kernel<<<plan.p.n_cta, kGradThreads, kGradSmem, st>>>(plan.tmX[0], plan.tmH[0], plan.tmX[1], plan.tmH[1], plan.p);
+  const cudaError_t le = launch_kernel(lora_grad_umma_kernel, dim3(plan.p.n_cta), dim3(kGradThreads), kGradSmem, st, chained_launch(), plan.tmX[0],
+                                       plan.tmH[0], plan.tmX[1], plan.tmH[1], plan.p);
+  if (le != cudaSuccess) return cuda_fail(le, "lora_grad_umma_kernel launch");
   if (prof) profile_end(st);
   MCB_CHECK_LAUNCH("lora_grad_umma_kernel");
   return launch_grad_reduce(plan, st);

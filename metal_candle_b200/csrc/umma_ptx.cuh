@@ -71,12 +71,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1)
       : "memory");
 }
-// Programmatic dependent launch.  A kernel launched with the programmatic-serialization attribute may start while
-// its predecessor in the stream is still running; `grid_dependency_wait` blocks until the predecessor grid has
-// completed and its writes are visible.  `grid_launch_dependents` lets a dependent grid launched with that attribute
-// start early (it has no effect otherwise).  Both are no-ops for kernels launched the ordinary way.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"

@@ -405,7 +405,7 @@ int launch_split(const SplitPlan& plan, const GemmCall& c, __nv_bfloat16* up, __
     attr[na].val.clusterDim.x = static_cast<unsigned>(p.splits); attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = 1;
     ++na;
   }
-  if (c.after_pack && !prof && option(MCB_OPT_PDL) != 0) {
+  if (chained_launch()) {
     attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;

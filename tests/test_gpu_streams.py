@@ -91,3 +91,54 @@ def test_calls_captured_by_the_caller_outlive_the_scratch_buffer(cuda_device):
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(out, want))
     del junk
+
+
+def test_chained_launches_change_nothing(cuda_device):
+    """Kernels launched while the one before still runs (MCB_OPT_PDL), against launches that wait for it: a chain in which every
+    call reads what the last one wrote or writes over what it reads, in eager form and captured."""
+    from metal_candle_b200 import _lib, backend as B
+
+    lib = _lib.load()
+    g = torch.Generator(device=cuda_device).manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, device=cuda_device, generator=g)  # noqa: E731
+    M, H, r = 1100, 896, 16
+    A, Bm = rnd(H, r) * 0.05, rnd(r, H) * 0.05
+    lin = {dt: (rnd(M, H).to(dt), (rnd(H, H) / 30).to(dt), (1 + 0.1 * rnd(H)).to(dt)) for dt in (torch.bfloat16, torch.float32)}
+    wt = {dt: B.transpose_2d(t[1]) for dt, t in lin.items()}
+    targets = torch.randint(0, H, (M,), device=cuda_device, generator=g, dtype=torch.int32)
+
+    def chain():
+        out = []
+        for dt, (x, w, gain) in lin.items():
+            h, grad_a = x, torch.zeros(H, r, device=cuda_device)
+            grad_b = torch.zeros(r, H, device=cuda_device)
+            for _ in range(4):
+                n = B.rms_norm_fused(h, 1e-6, weight=gain)
+                h2, hs = B.lora_linear_forward(n, w, None, A, Bm, 2.0, residual=h)
+                p = B.softmax_fused(h2, out=h2)
+                p = B.softmax_backward(p, n, out=p)
+                dx, _, _ = B.lora_linear_backward(n, wt[dt], A, Bm, 2.0, p, h_save=hs, grad_a=grad_a, grad_b=grad_b, accumulate=True)
+                h, dw = B.rms_norm_backward(h, gain, dx, 1e-6, dx_residual=n)
+                out += [dw]
+            logits, nll, count, loss = h.clone(), torch.empty(M, device=cuda_device), torch.empty(1, dtype=torch.int32, device=cuda_device), torch.empty(2, device=cuda_device)
+            _lib.check(lib.mcb_cross_entropy(logits.data_ptr(), targets.data_ptr(), nll.data_ptr(), count.data_ptr(), loss.data_ptr(), M, H, 1,
+                                             B._dtype_code(logits), B._stream()))
+            out += [h, grad_a, grad_b, logits, loss]
+        return out
+
+    try:
+        _lib.check(lib.mcb_set_option(_lib.MCB_OPT_PDL, 0))
+        want = chain()
+        torch.cuda.synchronize()
+    finally:
+        _lib.check(lib.mcb_set_option(_lib.MCB_OPT_PDL, 1))
+    for _ in range(5):
+        assert all(torch.equal(a, b) for a, b in zip(chain(), want))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = chain()
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(captured, want))
+    assert _lib.device_status() == 0
