@@ -23,7 +23,7 @@ struct DeviceState {
   int sm_count = 0;
   int* status_word = nullptr;  // device int: 0, or the code of a bounded wait that gave up
   long long* selftest_out = nullptr;  // three device words behind the status word (mcb_selftest_wait_timeout)
-  bool f32_tile_smem = false;  // the float32 tile kernel's shared-memory limit has been raised
+  int f32_tile_clusters[2][9] = {};  // clusters of the float32 tile kernel the device runs at once, by tile width and cluster size
   bool ce_smem[2] = {false, false};  // the same of the cross-entropy cluster kernel (bf16, float32)
   struct ResidentClusters {
     size_t smem = 0;  // shared memory of a CTA the answer holds for; 0 = no answer yet

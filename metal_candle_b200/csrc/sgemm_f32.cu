@@ -1,36 +1,27 @@
-// float32 path of the fused LoRA linear on CUDA cores with float32 FMA accumulation.  tcgen05 has no float32 MMA and a
-// single TF32 pass cannot hold the 1e-4 bound against the reference's f32 CPU arithmetic, so the contractions run on
-// the FMA pipes (148 SMs x 128 lanes = 74 TFLOP/s at the maximum clock), as four kinds of kernel:
+// float32 path of the fused LoRA linear.  tcgen05 has no float32 MMA and a single TF32 pass cannot hold the 1e-4 bound against
+// the reference's f32 CPU arithmetic; six bfloat16 products of operands cut into three parts each can, and hold float32's own
+// rounding (tile_kernel).  The kernels of kernel:
 //
-//   tile_kernel    C = A B (+ bias) (+ residual) with the rank-r update as extra reduction steps: 128 x 64 tiles,
-//                  the reduction split over the CTAs of a cluster when a shape has too few tiles for the chip
+//   tile_kernel    C = A B (+ bias) (+ residual) with the rank-r update as extra reduction steps, on the tensor cores: 128 x
+//                  128 (64) tiles, the reduction split over the CTAs of a cluster when a shape has too few tiles for the chip
+//   short_kernel   the same for reductions of at most 64, on the FMA pipes
 //   rank_kernel    the [M, r] intermediates scale * x A and scale * dy B^T
 //   grad_kernel    dA and dB, reductions over tokens
 //   lora_delta_cluster_kernel   scale * (x A) B of few tokens in one launch (also for bfloat16 x)
 #include <cooperative_groups.h>
 
 #include "lora_internal.cuh"
+#include "umma_ptx.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace mcb {
 namespace f32path {
+using namespace umma;
 namespace {
 
-// ---- asynchronous copies (0 source bytes: the destination is zero-filled) ------------------------------------------
-__device__ __forceinline__ void cp4(uint32_t dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp4_or_zero(uint32_t dst, const float* src, const float* any, bool in) {
-  const int n = in ? 4 : 0;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(in ? src : any), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 // ---- tile kernel -------------------------------------------------------------------------------------------------
-// An operand as the kernel reads it: element (row, k) at p[row * sr + k * sk].
+// An operand as the kernel reads it: element (row, k) at p[row * sr + k * sk]; one of the strides is 1.
 struct Operand {
   const float* p;
   int64_t sr, sk;
@@ -45,147 +36,256 @@ struct TileParams {
   int64_t cm, cn;
   int accumulate;
   int n_tiles, splits;
+  int* status;
 };
 
-constexpr int kTileM = 128, kTileN = 64, kStep = 32, kStages = 2, kTileThreads = 64;
-// A stage holds both tiles as [k][row]; the row pitches are 4 mod 32 words, so that the 8 k x 4 rows (or 32 rows) a warp
-// copies at a time fall into 32 different banks.
-constexpr int kPitchA = kTileM + 4, kPitchB = kTileN + 4;
-constexpr int kStageFloats = kStep * (kPitchA + kPitchB);
-constexpr int kOutPitch = kTileN + 4, kMaxSplits = 8;
-static_assert(kTileM * kOutPitch <= kStages * kStageFloats, "the output tile reuses the stage ring");
+// The tensor cores take bfloat16, whose eight significant bits are a third of float32's: x = h + m + l, each part the
+// upper half of the bits that the parts before it left over (cut off, not rounded, so that every remainder is exact); the
+// three hold all 24 bits.  Both operands are scaled by 2^24 first, so that the parts of the smallest normal numbers are
+// normal themselves; what overflows for it (operands beyond 2^103, products beyond 2^79) is computed again, see below.  Of the nine
+// products of the parts the six largest are taken; the other three are below 2^-23 of the product.
+constexpr int kTileM = 128, kStep = 64, kStages = 2, kParts = 3, kMaxSplits = 8;
+constexpr int kTileWarps = 16, kTileThreads = 32 * kTileWarps;
+constexpr float kPartScale = 16777216.0f, kPartUnscale = 1.0f / 16777216.0f / 16777216.0f;
 
-// Word copies serve every stride and alignment and transpose on the way; neighbouring lanes read neighbouring words
-// (8 k of a row where k is the contiguous index, else consecutive rows).  Whole tiles skip the bounds checks.
-template <int ROWS, int PITCH>
-__device__ __forceinline__ void load_tile(uint32_t dst, const Operand& o, int row0, int rows, int k0, int kend) {
-  const int t = threadIdx.x;
-  const bool whole = row0 + ROWS <= rows && k0 + kStep <= kend;
-  if (o.sk == 1) {
-    const int kk = t & 7, rr = t >> 3;   // 8 rows x 8 k per round of the CTA's two warps
-    const float* src = o.p + (row0 + rr) * o.sr + k0 + kk;
-    dst += (kk * PITCH + rr) * 4;
-    const int64_t jump = 8 * o.sr;
-    if (whole) {
-#pragma unroll 4
-      for (int i = 0; i < ROWS / 8; ++i, src += jump) {
+template <int BN>
+struct TileSmem {
+  static constexpr uint32_t kPlaneA = kTileM * kStep * 2, kPlaneB = BN * kStep * 2;
+  static constexpr uint32_t kStage = kParts * (kPlaneA + kPlaneB), kBars = kStages * kStage;
+  static constexpr size_t kBytes = kBars + 64 + 1024;
+  static constexpr int kOutPitch = BN + 4;   // the output tile reuses the stages; rows four banks apart
+  static_assert(kTileM * kOutPitch * 4 <= kBars, "output tile");
+};
+
+__device__ __forceinline__ uint32_t upper_halves(float a, float b) {
+  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+}
+__device__ __forceinline__ float cut(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
+// the three parts of eight values, 16 bytes each, `plane` bytes apart
+__device__ __forceinline__ void store_parts(uint8_t* dst, uint32_t plane, const float (&v)[8]) {
+  uint32_t w[kParts][4];
 #pragma unroll
-        for (int h = 0; h < kStep / 8; ++h) cp4(dst + (8 * h * PITCH + 8 * i) * 4, src + 8 * h);
-      }
-    } else {
-      for (int i = 0; i < ROWS / 8; ++i, src += jump) {
-        const bool row_in = row0 + rr + 8 * i < rows;
-#pragma unroll
-        for (int h = 0; h < kStep / 8; ++h)
-          cp4_or_zero(dst + (8 * h * PITCH + 8 * i) * 4, src + 8 * h, o.p, row_in && k0 + kk + 8 * h < kend);
-      }
-    }
-  } else {
-    const int r = t % ROWS, k = t / ROWS;   // 64 threads: half of A's rows, or all of B's, at one k
-    constexpr int kSub = ROWS > kTileThreads ? ROWS / kTileThreads : 1;
-    const float* src = o.p + (row0 + r) * o.sr + (k0 + k) * o.sk;
-    dst += (k * PITCH + r) * 4;
-    const int64_t hop = kTileThreads * o.sr;
-    for (int i = 0; i < kStep; ++i, src += o.sk)
-#pragma unroll
-      for (int h = 0; h < kSub; ++h) {
-        const uint32_t d = dst + (i * PITCH + h * kTileThreads) * 4;
-        if (whole) cp4(d, src + h * hop);
-        else cp4_or_zero(d, src + h * hop, o.p, row0 + r + h * kTileThreads < rows && k0 + i < kend);
-      }
+  for (int i = 0; i < 4; ++i) {
+    const float2 x = __fmul2_rn(make_float2(v[2 * i], v[2 * i + 1]), make_float2(kPartScale, kPartScale));
+    const float2 x1 = make_float2(x.x - cut(x.x), x.y - cut(x.y));
+    w[0][i] = upper_halves(x.x, x.y);
+    w[1][i] = upper_halves(x1.x, x1.y);
+    w[2][i] = upper_halves(x1.x - cut(x1.x), x1.y - cut(x1.y));
   }
+#pragma unroll
+  for (int s = 0; s < kParts; ++s) *reinterpret_cast<uint4*>(dst + s * plane) = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
 }
 
-// Bound: the FMA pipe, with shared-memory reads next.  A thread owns 16 x 8 outputs: 6 LDS.128 feed 128 FMAs, which keeps
-// the reads below the 128 bytes per cycle an SM has; the FMAs are packed pairs (fma.rn.f32x2), which leaves issue slots
-// for the copies.  2048 x 1536 x 1536: 262 us (37 TFLOP/s; 64 x 64 tiles of 4 x 4 outputs took 480), 512 x 768 x 768: 29
-// us (240).  A shape with few tiles (512 x 768 x 768: 48) leaves SMs idle, so up to 8 CTAs of a cluster share a tile's
-// reduction and add their partial tiles through distributed shared memory, in rank order: deterministic, no workspace.
-__global__ void __launch_bounds__(kTileThreads, 4) tile_kernel(const TileParams p) {
-  extern __shared__ __align__(16) float smem[];
-  const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+__device__ __forceinline__ bool is_k_major(const Operand& o) { return o.sk == 1; }
+__device__ __forceinline__ bool is_vec(const Operand& o) {
+  return (reinterpret_cast<uintptr_t>(o.p) & 15u) == 0 && ((o.sk == 1 ? o.sr : o.sk) & 3) == 0;
+}
+
+// One step's tile of an operand, ROWS x 64 reduction indices, as ROWS * 8 pieces of eight neighbouring values dealt out to
+// the threads.  In shared memory, per part: k contiguous: rows of 128 bytes (64 k); rows contiguous: blocks of 64 rows, each
+// 64 k of 128 bytes; the 16-byte pieces of a line in 128-byte swizzle order either way, and eight lanes write one line.
+template <int ROWS>
+struct Copy {
+  static constexpr int kPieces = ROWS * 8 / kTileThreads;
+  float v[kPieces][8];
+  __device__ __forceinline__ static void place(bool k_major, int i, int& row, int& k, uint32_t& at) {
+    const int u = threadIdx.x + i * kTileThreads;
+    if (k_major) {
+      row = u >> 3; k = (u & 7) * 8;
+      at = row * 128 + (((u & 7) ^ (row & 7)) << 4);
+    } else {
+      const int c = u % (ROWS / 8);
+      k = u / (ROWS / 8); row = c * 8;
+      at = (c >> 3) * (kStep * 128) + k * 128 + (((c & 7) ^ (k & 7)) << 4);
+    }
+  }
+  // rows [row0, row0 + ROWS) and indices [k0, k0 + 64); zeros beyond `rows` and `kend`
+  __device__ __forceinline__ void load(const Operand& o, int row0, int rows, int k0, int kend) {
+    const bool k_major = is_k_major(o);
+    const float* p = from_here(o.p) + (k_major ? row0 * o.sr + k0 : k0 * o.sk + row0);
+    const int64_t pitch = k_major ? o.sr : o.sk;
+    if (is_vec(o) && row0 + ROWS <= rows && k0 + kStep <= kend) {
+#pragma unroll
+      for (int i = 0; i < kPieces; ++i) {
+        int row, k;
+        uint32_t at;
+        place(k_major, i, row, k, at);
+        const float4* q = reinterpret_cast<const float4*>(p + (k_major ? row * pitch + k : k * pitch + row));
+        *reinterpret_cast<float4*>(v[i]) = __ldg(q);
+        *reinterpret_cast<float4*>(v[i] + 4) = __ldg(q + 1);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < kPieces; ++i) {
+        int row, k;
+        uint32_t at;
+        place(k_major, i, row, k, at);
+        const float* q = p + (k_major ? row * pitch + k : k * pitch + row);
+        const int left = (k_major ? row0 + row < rows : k0 + k < kend) ? (k_major ? kend - k0 - k : rows - row0 - row) : 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[i][j] = j < left ? __ldg(q + j) : 0.0f;
+      }
+    }
+  }
+  __device__ __forceinline__ void store(uint8_t* dst, uint32_t plane, bool k_major, int kn) const {
+#pragma unroll
+    for (int i = 0; i < kPieces; ++i) {
+      int row, k;
+      uint32_t at;
+      place(k_major, i, row, k, at);
+      if (k < kn) store_parts(dst + at, plane, v[i]);   // nobody reads beyond the step's last 16 indices
+    }
+  }
+};
+
+// One output in plain float32 arithmetic.  An operand that is infinite, or becomes so by the scaling, has no parts (inf - inf),
+// so an output that is not finite may be one the parts have spoilt: it is computed again, and is then what float32 gives.
+__device__ __noinline__ float plain_element(const TileParams& p, int m, int n) {
+  float s = 0.0f;
+  for (int k = 0; k < p.K; ++k) s = fmaf(p.a.p[m * p.a.sr + k * p.a.sk], p.b.p[n * p.b.sr + k * p.b.sk], s);
+  for (int k = 0; k < p.R; ++k) s = fmaf(p.ra.p[m * p.ra.sr + k * p.ra.sk], p.rb.p[n * p.rb.sr + k * p.rb.sk], s);
+  return s;
+}
+
+// A step of 64 reduction indices: the threads cut the values they loaded a step earlier into parts (two stages of shared
+// memory), one thread issues the six products, and meanwhile all add the step before's accumulator to float32 sums in
+// registers: the tensor core cuts its running sum off where float32 rounds to nearest, so a sum stays in it for one step only
+// (relative error to float64 of 512 x 768 x 768 1.4e-7, of the float32 FMAs before 1.9e-7; of 2048 x 1536 x 1536 1.5e-7, 2.6e-7).
+// Bound: the tensor pipe, 12 BN cycles a step, behind a CTA's start and the exchange of partial tiles.  A shape with few
+// tiles (512 x 768 x 768: 24) leaves SMs idle, so up to 8 CTAs of a cluster share a tile's reduction and add their
+// partial tiles through distributed shared memory, in rank order: deterministic, no workspace.
+template <int BN>
+__global__ void __launch_bounds__(kTileThreads, 1) tile_kernel(const __grid_constant__ TileParams p) {
+  using S = TileSmem<BN>;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t acc_full0 = base + S::kBars, tmem_slot = acc_full0 + 16;
+  volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(gen + (tmem_slot - base));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + (tmem_slot + 4 - base));
+
+  if (threadIdx.x == 0) {
+    for (int a = 0; a < 2; ++a) mbar_init(acc_full0 + 8 * a, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_proxy_async_smem();
+  }
+  constexpr uint32_t kCols = 2 * BN;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(kCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem_base = *tmem_slot_ptr;
+  grid_launch_dependents();
+  grid_dependency_wait();   // the set-up above ran under the tail of the kernel before
   const int split = blockIdx.x % p.splits, tile = blockIdx.x / p.splits;
-  const int m0 = (tile / p.n_tiles) * kTileM, n0 = (tile % p.n_tiles) * kTileN;
-  // main steps are shared out evenly; the rank steps go to the last CTA of the cluster
+  const int m0 = (tile / p.n_tiles) * kTileM, n0 = (tile % p.n_tiles) * BN;
+  // main steps are shared out evenly; the rank steps go to the first CTA of the cluster, which has the fewest
   const int ksteps = (p.K + kStep - 1) / kStep;
   const int s_begin = static_cast<int>(static_cast<int64_t>(ksteps) * split / p.splits);
   const int s_end = static_cast<int>(static_cast<int64_t>(ksteps) * (split + 1) / p.splits);
   const int main_steps = s_end - s_begin;
-  const int steps = main_steps + (split == p.splits - 1 ? (p.R + kStep - 1) / kStep : 0);
+  const int steps = main_steps + (split == 0 ? (p.R + kStep - 1) / kStep : 0);
+
+  Copy<kTileM> ca;
+  Copy<BN> cb;
   auto load_step = [&](int s) {
-    const uint32_t da = sbase + (s % kStages) * kStageFloats * 4, db = da + kStep * kPitchA * 4;
-    if (s < main_steps) {
-      const int k0 = (s_begin + s) * kStep;
-      load_tile<kTileM, kPitchA>(da, p.a, m0, p.M, k0, p.K);
-      load_tile<kTileN, kPitchB>(db, p.b, n0, p.N, k0, p.K);
-    } else if (s < steps) {
-      const int k0 = (s - main_steps) * kStep;
-      load_tile<kTileM, kPitchA>(da, p.ra, m0, p.M, k0, p.R);
-      load_tile<kTileN, kPitchB>(db, p.rb, n0, p.N, k0, p.R);
-    }
-    cp_commit();   // one group per step, empty or not
+    const bool main = s < main_steps;
+    const int k0 = (main ? s_begin + s : s - main_steps) * kStep, kend = main ? p.K : p.R;
+    ca.load(main ? p.a : p.ra, m0, p.M, k0, kend);
+    cb.load(main ? p.b : p.rb, n0, p.N, k0, kend);
   };
-  const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;   // rows 4 ty + 32 i + (0..3), columns 4 tx + 32 j + (0..3)
-  float2 acc[16][4];
+  // a thread's outputs: row 32 (warp % 4) + lane, BN / 4 columns from (warp / 4) BN / 4 on
+  const int quad = warp & 3, col0 = (warp >> 2) * (BN / 4);
+  float sum[BN / 4];
 #pragma unroll
-  for (int i = 0; i < 16; ++i)
+  for (int i = 0; i < BN / 4; ++i) sum[i] = 0.0f;
+  load_step(0);
+  for (int s = 0; s <= steps; ++s) {
+    if (s < steps) {
+      // Stage and accumulator s % 2 are free: every thread has waited for step s - 2's products and read their sums.
+      const bool main = s < main_steps, ak = is_k_major(main ? p.a : p.ra), bk = is_k_major(main ? p.b : p.rb);
+      const int left = main ? p.K - (s_begin + s) * kStep : p.R - (s - main_steps) * kStep;
+      const int k16 = (min(left, kStep) + 15) >> 4;   // the MMAs' reduction is 16 long
+      uint8_t* dst = gen + (s & 1) * S::kStage;
+      ca.store(dst, S::kPlaneA, ak, 16 * k16);
+      cb.store(dst + kParts * S::kPlaneA, S::kPlaneB, bk, 16 * k16);
+      fence_proxy_async_smem();
+      if (s + 1 < steps) load_step(s + 1);
+      tcgen05_fence_before();
+      __syncthreads();
+      if (threadIdx.x == 0 && *abort_flag == 0) {
+        tcgen05_fence_after();
+        const uint32_t idesc = make_idesc(BN) | (ak ? 0u : 1u << 15) | (bk ? 0u : 1u << 16);
+        const uint32_t pa = base + (s & 1) * S::kStage, pb = pa + kParts * S::kPlaneA, acc = tmem_base + (s & 1) * BN;
+        // 16 reduction indices further: 32 bytes along a line, or two groups of eight lines
+        const uint64_t da0 = ak ? desc_sw128(pa) : desc_sw128_mn(pa, kStep * 128, 1024);
+        const uint64_t db0 = bk ? desc_sw128(pb) : desc_sw128_mn(pb, kStep * 128, 1024);
+        const uint32_t ja = ak ? 32 : 2048, jb = bk ? 32 : 2048;
+        // smallest products first, so that what the running sum loses to them is small
+        constexpr int kA[6] = {2, 0, 1, 1, 0, 0}, kB[6] = {0, 2, 1, 0, 1, 0};
+        uint32_t add = 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
-  for (int s = 0; s < kStages - 1; ++s) load_step(s);
-  for (int s = 0; s < steps; ++s) {
-    cp_wait<kStages - 2>();
-    __syncthreads();            // step s has landed, and every thread is through with step s - 1
-    load_step(s + kStages - 1);
-    const float* sa = smem + (s % kStages) * kStageFloats + 4 * ty;
-    const float* sb = smem + (s % kStages) * kStageFloats + kStep * kPitchA + 4 * tx;
-    // a step's indices behind the end are zeros: a rank of 8 is a quarter of a step, and that step is the last CTA's fourth
-    // at 512 x 768 x 768 (forward 39.0 -> 34.9 us, 1024 x 768 -> 768 59.5 -> 55.4)
-    const int left = s < main_steps ? p.K - (s_begin + s) * kStep : p.R - (s - main_steps) * kStep;
-    const int kn = left < kStep ? left : kStep;
-#pragma unroll 2
-    for (int k = 0; k < kn; ++k) {
-      float a[16];
-      float4 b[2];
+        for (int q = 0; q < 6; ++q)
+          for (int k = 0; k < k16; ++k) {
+            umma_bf16(acc, desc_advance(da0, kA[q] * S::kPlaneA + k * ja), desc_advance(db0, kB[q] * S::kPlaneB + k * jb), idesc, add);
+            add = 1;
+          }
+        umma_commit(acc_full0 + 8 * (s & 1));
+      }
+      __syncwarp();
+    }
+    if (s > 0) {
+      const int d = s - 1;
+      if (__all_sync(0xffffffffu, mbar_wait(acc_full0 + 8 * (d & 1), (d >> 1) & 1, abort_flag, 100, p.status))) {
+        tcgen05_fence_after();
+        const uint32_t t = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + (d & 1) * BN + col0;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(a + 4 * i) = *reinterpret_cast<const float4*>(sa + k * kPitchA + 32 * i);
+        for (int c = 0; c < BN / 4; c += 16) {
+          uint32_t v[16];
+          tmem_ld_x16(t + c, v);
+          tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 2; ++j) b[j] = *reinterpret_cast<const float4*>(sb + k * kPitchB + 32 * j);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const float2 aa = make_float2(a[i], a[i]);
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          acc[i][2 * j] = __ffma2_rn(aa, make_float2(b[j].x, b[j].y), acc[i][2 * j]);
-          acc[i][2 * j + 1] = __ffma2_rn(aa, make_float2(b[j].z, b[j].w), acc[i][2 * j + 1]);
+          for (int i = 0; i < 16; ++i) sum[c + i] += __uint_as_float(v[i]);
         }
       }
     }
   }
-  cp_wait<0>();
+  // every product has been waited for: nothing reads the stages any more
   __syncthreads();
+  float* out = reinterpret_cast<float*>(gen) + (quad * 32 + lane) * S::kOutPitch + col0;
 #pragma unroll
-  for (int i = 0; i < 16; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-      *reinterpret_cast<float4*>(smem + (4 * ty + 32 * (i >> 2) + (i & 3)) * kOutPitch + 4 * tx + 32 * j) =
-          make_float4(acc[i][2 * j].x, acc[i][2 * j].y, acc[i][2 * j + 1].x, acc[i][2 * j + 1].y);
+  for (int i = 0; i < BN / 4; i += 4) *reinterpret_cast<float4*>(out + i) = make_float4(sum[i], sum[i + 1], sum[i + 2], sum[i + 3]);
+  if (*abort_flag != 0) {
+    for (int k = 0; k < 200; ++k) __nanosleep(1000);
+  }
+  tcgen05_fence_before();
   cg::cluster_group cl = cg::this_cluster();
   if (p.splits > 1) cl.sync();
   else __syncthreads();
+  if (warp == 0) {
+    tcgen05_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kCols) : "memory");
+  }
   // each CTA of the cluster finishes its share of the tile's rows
+  float* tile_out = reinterpret_cast<float*>(gen);
   const int row_begin = kTileM * split / p.splits, row_end = kTileM * (split + 1) / p.splits;
   const bool vec_out = p.cn == 1 && p.cm % 4 == 0 && p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15u) == 0;
-  for (int e = threadIdx.x; e < (row_end - row_begin) * (kTileN / 4); e += kTileThreads) {
-    const int r = row_begin + e / (kTileN / 4), c = (e % (kTileN / 4)) * 4;
+  for (int e = threadIdx.x; e < (row_end - row_begin) * (BN / 4); e += kTileThreads) {
+    const int r = row_begin + e / (BN / 4), c = (e % (BN / 4)) * 4;
     const int gm = m0 + r, gn = n0 + c;
     if (gm >= p.M || gn >= p.N) continue;
-    // all parts' loads in flight before the first sum: one after the other, a thread's 32 remote reads of 8 parts are 32
-    // trips through the cluster's network (64 x 256 -> 128 r8: forward 22.6 -> 20.6 us, backward 28.8 -> 26.8)
+    // all parts' loads in flight before the first sum: one after the other, a thread's remote reads are as many trips
+    // through the cluster's network
     float4 part[kMaxSplits];
 #pragma unroll
     for (int q = 0; q < kMaxSplits; ++q)
       if (q < p.splits)
-        part[q] = *reinterpret_cast<const float4*>((p.splits > 1 ? cl.map_shared_rank(smem, q) : smem) + r * kOutPitch + c);
+        part[q] = *reinterpret_cast<const float4*>((p.splits > 1 ? cl.map_shared_rank(tile_out, q) : tile_out) + r * S::kOutPitch + c);
     float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
     for (int q = 0; q < kMaxSplits; ++q)
@@ -195,6 +295,7 @@ __global__ void __launch_bounds__(kTileThreads, 4) tile_kernel(const TileParams 
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
       if (x >= live) break;
+      v[x] = fabsf(v[x]) < INFINITY ? v[x] * kPartUnscale : plain_element(p, gm, gn + x);
       v[x] *= p.alpha;
       if (p.bias != nullptr) v[x] += p.bias[gn + x];
       if (p.residual != nullptr) v[x] += p.residual[o + x * p.cn];
@@ -211,6 +312,62 @@ __global__ void __launch_bounds__(kTileThreads, 4) tile_kernel(const TileParams 
   if (p.splits > 1) cl.sync();   // nobody leaves while a peer still reads its tile
 }
 
+// ---- short reductions ----------------------------------------------------------------------------------------------
+// The same product where K and R are at most 64: with so few terms, plain float32 FMAs round less than the tensor cores' cut-off
+// sums (1024 x 8 x 512: 3e-8 of the result against 9e-8), and there is no reduction to speed up.
+// Bound: writing C.  A CTA holds both operands' 64 rows whole; a thread owns 8 x 4 outputs.
+constexpr int kShort = 64, kShortThreads = 128, kShortPitch = kShort + 4;
+__global__ void __launch_bounds__(kShortThreads) short_kernel(const __grid_constant__ TileParams p) {
+  __shared__ __align__(16) float sa[32][kShortPitch], sb[32][kShortPitch];   // [k][row], half of the reduction at a time
+  const int m0 = (blockIdx.x / p.n_tiles) * kShort, n0 = (blockIdx.x % p.n_tiles) * kShort;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // rows 8 ty.., columns 4 tx..
+  grid_launch_dependents();
+  grid_dependency_wait();
+  float acc[8][4] = {};
+  auto stage = [&](float (&dst)[32][kShortPitch], const Operand& o, int row0, int rows, int k0, int kend) {
+    const float* src = from_here(o.p);
+    const bool k_major = o.sk == 1;
+    for (int e = threadIdx.x; e < 32 * kShort; e += kShortThreads) {
+      const int k = k_major ? e & 31 : e >> 6, r = k_major ? e >> 5 : e & 63;
+      dst[k][r] = row0 + r < rows && k0 + k < kend ? src[(row0 + r) * o.sr + (k0 + k) * o.sk] : 0.0f;
+    }
+  };
+  auto run = [&](const Operand& a, const Operand& b, int len) {
+    for (int k0 = 0; k0 < len; k0 += 32) {
+      __syncthreads();
+      stage(sa, a, m0, p.M, k0, len);
+      stage(sb, b, n0, p.N, k0, len);
+      __syncthreads();
+      const int kn = min(32, len - k0);
+#pragma unroll 4
+      for (int k = 0; k < kn; ++k) {
+        const float4 a0 = *reinterpret_cast<const float4*>(&sa[k][8 * ty]), a1 = *reinterpret_cast<const float4*>(&sa[k][8 * ty + 4]);
+        const float4 b0 = *reinterpret_cast<const float4*>(&sb[k][4 * tx]);
+        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, bv[4] = {b0.x, b0.y, b0.z, b0.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+      }
+    }
+  };
+  run(p.a, p.b, p.K);
+  run(p.ra, p.rb, p.R);
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int gm = m0 + 8 * ty + i, gn = n0 + 4 * tx + j;
+      if (gm >= p.M || gn >= p.N) continue;
+      const int64_t o = gm * p.cm + gn * p.cn;
+      float v = acc[i][j] * p.alpha;
+      if (p.bias != nullptr) v += p.bias[gn];
+      if (p.residual != nullptr) v += p.residual[o];
+      if (p.accumulate) v += p.C[o];
+      p.C[o] = v;
+    }
+}
+
 // ---- rank intermediates ------------------------------------------------------------------------------------------
 // out(m, j) = scale * sum_k x[m, k] F(k, j), F(k, j) = F[k * fk + j * fj]; out(m, j) at out[m * om + j * oj].
 // Bound: latency (6 MFLOP at 512 x 768, r = 8).  A CTA takes 4 tokens and 8 rank columns; its 8 warps share the
@@ -225,6 +382,10 @@ rank_kernel(const float* __restrict__ x, const float* __restrict__ F, int64_t fk
   const int64_t m0 = static_cast<int64_t>(blockIdx.x) * kRankTokens;
   const int j0 = blockIdx.y * kRankCols;
   float acc[kRankTokens][kRankCols] = {};
+  grid_launch_dependents();
+  grid_dependency_wait();
+  x = from_here(x);
+  F = from_here(F);
   const bool vec_f = fj == 1 && (fk & 3) == 0 && j0 + kRankCols <= r && (reinterpret_cast<uintptr_t>(F) & 15u) == 0;
 #pragma unroll 2
   for (int k = warp * 32 + lane; k < K; k += kRankWarps * 32) {
@@ -292,12 +453,15 @@ grad_kernel(const GradProblemF32 qa, const GradProblemF32 qb, int M, int r, int 
   const int c = cb * 32 + lane, j0 = blockIdx.y * kGradCols;
   const int part = split * kGradWarps + warp, parts = splits * kGradWarps;
   float acc[kGradCols] = {};
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const float *X = from_here(q.X), *H = from_here(q.H);
 #pragma unroll 4
   for (int m = part; m < M; m += parts) {
-    const float xv = c < q.C ? q.X[static_cast<int64_t>(m) * q.C + c] : 0.0f;
+    const float xv = c < q.C ? X[static_cast<int64_t>(m) * q.C + c] : 0.0f;
 #pragma unroll
     for (int j = 0; j < kGradCols; ++j)
-      if (j0 + j < r) acc[j] = fmaf(xv, __ldg(q.H + m * q.hm + (j0 + j) * q.hj), acc[j]);
+      if (j0 + j < r) acc[j] = fmaf(xv, __ldg(H + m * q.hm + (j0 + j) * q.hj), acc[j]);
   }
 #pragma unroll
   for (int j = 0; j < kGradCols; ++j) red[warp][j][lane] = acc[j];
@@ -347,6 +511,11 @@ lora_delta_cluster_kernel(const T* __restrict__ x, const float* __restrict__ A, 
   const int groups = kDeltaThreads / r;
   const int j = t % r, g = t / r;
   float acc[TOK] = {};
+  grid_launch_dependents();
+  grid_dependency_wait();
+  x = from_here(x);
+  A = from_here(A);
+  B = from_here(B);
   for (int kc = k_begin; kc < k_end; kc += kDeltaChunk) {
     const int len = min(kDeltaChunk, k_end - kc);
     __syncthreads();
@@ -417,11 +586,13 @@ lora_delta_cluster_kernel(const T* __restrict__ x, const float* __restrict__ A, 
 cudaError_t launch_cluster(const void* kernel, dim3 grid, int threads, size_t smem, int cluster, cudaStream_t st, void** args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = dim3(static_cast<unsigned>(threads)); cfg.dynamicSmemBytes = smem; cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(cluster); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = chained_launch() ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(cluster); attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = cluster > 1 ? 1 : 0;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelExC(&cfg, kernel, args);
 }
 
@@ -442,19 +613,17 @@ int launch_delta(const LoraArgs& a) {
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------------
-constexpr size_t kTileSmem = static_cast<size_t>(kStages) * kStageFloats * sizeof(float);
-
-// CTAs that share a tile's reduction.  In cycles: a CTA-step of one reduction index is 64 cycles of an SM's FMA pipes, but
-// a CTA has two warps and so reaches only half of them alone; the tiles x splits units are dealt out to the SMs in whole
-// units; a partial tile's write and exchange costs 1000 per unit and 2000 for the cluster.
-int pick_splits(int64_t tiles, int64_t K, int sm_count) {
+// CTAs that share a tile's reduction (0: no cluster of that size fits the device).  In cycles: a step of 64 reduction
+// indices keeps the tensor pipe for 12 BN; a CTA's start, drain and write-out cost some four steps, and the exchange of the
+// partial tiles two more; tiles go over the resident clusters in whole rounds.
+int pick_splits(int64_t tiles, int64_t ksteps, const int (&resident)[kMaxSplits + 1]) {
   int best = 1;
   double best_cost = 0.0;
-  for (int s = 1; s <= kMaxSplits; s *= 2) {
-    if (s > 1 && K < static_cast<int64_t>(s) * 2 * kStep) break;
-    const double n = static_cast<double>((tiles * s + sm_count - 1) / sm_count);
-    const double cost = (n < 2.0 ? 2.0 : n) * 64.0 * static_cast<double>(K) / s + 1000.0 * n + (s > 1 ? 2000.0 : 0.0);
-    if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
+  for (int s = 1; s <= kMaxSplits && (s == 1 || s <= ksteps); ++s) {
+    if (resident[s] <= 0) continue;
+    const double rounds = static_cast<double>((tiles + resident[s] - 1) / resident[s]);
+    const double cost = rounds * (static_cast<double>((ksteps + s - 1) / s) + 4.0 + (s > 1 ? 2.0 : 0.0));
+    if (best_cost == 0.0 || cost < best_cost) { best = s; best_cost = cost; }
   }
   return best;
 }
@@ -469,24 +638,51 @@ TileParams product(const Operand& a, const Operand& b, float* C, int64_t M, int6
   return p;
 }
 
+template <int BN>
+int launch_tiles(DeviceState* ds, TileParams p, cudaStream_t st) {
+  const void* kernel = reinterpret_cast<const void*>(&tile_kernel<BN>);
+  constexpr size_t smem = TileSmem<BN>::kBytes;
+  int (&resident)[kMaxSplits + 1] = ds->f32_tile_clusters[BN == 64];
+  if (resident[1] == 0) {
+    MCB_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    for (int s = kMaxSplits; s >= 1; --s) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = static_cast<unsigned>(s); attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+      cfg.gridDim = dim3(static_cast<unsigned>(s)); cfg.blockDim = dim3(kTileThreads); cfg.dynamicSmemBytes = smem;
+      cfg.attrs = attr; cfg.numAttrs = 1;
+      int n = 0;
+      if (s == 1) n = ds->sm_count;
+      else if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) { cudaGetLastError(); n = -1; }
+      resident[s] = n > 0 ? n : -1;
+    }
+  }
+  p.n_tiles = (p.N + BN - 1) / BN;
+  const int64_t tiles = static_cast<int64_t>((p.M + kTileM - 1) / kTileM) * p.n_tiles;
+  p.splits = pick_splits(tiles, (p.K + kStep - 1) / kStep, resident);
+  if (tiles * p.splits > 0x7fffffffll) return fail(MCB_ERR_SHAPE, "f32 path: %d x %d outputs", p.M, p.N);
+  void* args[] = {&p};
+  const cudaError_t e = launch_cluster(kernel, dim3(static_cast<unsigned>(tiles * p.splits)), kTileThreads, smem, p.splits, st, args);
+  if (e != cudaSuccess) return cuda_fail(e, "f32 tile_kernel launch");
+  MCB_CHECK_LAUNCH("f32 tile_kernel");
+  return MCB_OK;
+}
+
 int gemm(cudaStream_t st, TileParams p) {
   DeviceState* ds = current_device_state();
   if (!ds) return MCB_ERR_NOT_INIT;
   if (p.residual != nullptr && p.residual == p.C) return fail(MCB_ERR_UNSUPPORTED, "f32 path: residual must not alias the output");
-  p.n_tiles = (p.N + kTileN - 1) / kTileN;
-  const int64_t tiles = static_cast<int64_t>((p.M + kTileM - 1) / kTileM) * p.n_tiles;
-  p.splits = pick_splits(tiles, p.K, ds->sm_count);
-  if (tiles * p.splits > 0x7fffffffll) return fail(MCB_ERR_SHAPE, "f32 path: %d x %d outputs", p.M, p.N);
-  if (!ds->f32_tile_smem) {
-    MCB_CHECK_CUDA(cudaFuncSetAttribute(tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTileSmem)));
-    ds->f32_tile_smem = true;
+  p.status = ds->status_word;
+  if (p.K <= kShort && p.R <= kShort) {
+    p.n_tiles = (p.N + kShort - 1) / kShort;
+    const int64_t tiles = static_cast<int64_t>((p.M + kShort - 1) / kShort) * p.n_tiles;
+    if (tiles > 0x7fffffffll) return fail(MCB_ERR_SHAPE, "f32 path: %d x %d outputs", p.M, p.N);
+    MCB_CHECK_CUDA(launch_kernel(short_kernel, dim3(static_cast<unsigned>(tiles)), dim3(kShortThreads), 0, st, chained_launch(), p));
+    MCB_CHECK_LAUNCH("f32 short_kernel");
+    return MCB_OK;
   }
-  void* args[] = {&p};
-  const cudaError_t e = launch_cluster(reinterpret_cast<const void*>(&tile_kernel), dim3(static_cast<unsigned>(tiles * p.splits)),
-                                       kTileThreads, kTileSmem, p.splits, st, args);
-  if (e != cudaSuccess) return cuda_fail(e, "f32 tile_kernel launch");
-  MCB_CHECK_LAUNCH("f32 tile_kernel");
-  return MCB_OK;
+  return p.N <= 64 ? launch_tiles<64>(ds, p, st) : launch_tiles<128>(ds, p, st);
 }
 
 // From here on a rank fills enough of a 64-wide tile that the tile kernel's reuse beats the lean kernels' short start.
@@ -500,7 +696,8 @@ int rank_product(cudaStream_t st, const float* x, const float* F, int64_t fk, in
     return gemm(st, p);
   }
   const dim3 grid(static_cast<unsigned>((M + kRankTokens - 1) / kRankTokens), static_cast<unsigned>((r + kRankCols - 1) / kRankCols));
-  rank_kernel<<<grid, kRankWarps * 32, 0, st>>>(x, F, fk, fj, out, om, oj, static_cast<int>(M), static_cast<int>(K), static_cast<int>(r), scale);
+  MCB_CHECK_CUDA(launch_kernel(rank_kernel, grid, dim3(kRankWarps * 32), 0, st, chained_launch(), x, F, fk, fj, out, om, oj, static_cast<int>(M),
+                               static_cast<int>(K), static_cast<int>(r), scale));
   MCB_CHECK_LAUNCH("f32 rank_kernel");
   return MCB_OK;
 }

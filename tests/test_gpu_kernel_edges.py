@@ -28,7 +28,7 @@ def rounded(a, dtype):
     return a if dtype == torch.float32 else S.bf16_round(a)
 
 
-# float32: 128 x 64 tiles, reductions split in 2 to 8, rank columns through the lean kernels (below 24) and the tile
+# float32: 128 x 128 and 128 x 64 tiles, reductions split in up to 8, rank columns through the lean kernels (below 24) and the tile
 # kernel, odd strides
 @pytest.mark.parametrize("M,K,N,r", [(1, 3, 5, 1), (127, 33, 65, 3), (129, 511, 63, 23), (512, 768, 768, 24), (1030, 129, 257, 40),
                                      (2000, 1500, 1, 1), (64, 1500, 300, 65)])
@@ -430,6 +430,48 @@ def test_bf16_delta_is_recorded_by_the_profile(cuda_device, M):
     finally:
         _lib.profile_enable(False)
     assert launches == 1 and ms > 0 and flops == 2.0 * M * r * (K + N)
+
+
+# float32 products on the tensor cores: rows and indices around the 128 x 128 (64) tile and the 64-index step, the last reduction
+# of the short kernel (64) and the first beyond, both orders of either operand, reductions shared by 1 to 8 CTAs
+@pytest.mark.parametrize("M,K,N", [(128, 64, 128), (129, 65, 129), (127, 128, 64), (1, 127, 1), (300, 1024, 65), (1200, 200, 1100)])
+def test_f32_product_rounds_like_float32(cuda_device, M, K, N):
+    """Against float64, relative to the sum of magnitudes: a float32 sum of K terms, whatever its order, errs by up to K 2^-24;
+    what the parts' products leave out is at most 2^-20 of each product, the worst for any of them and not for their sum."""
+    from metal_candle_b200 import backend as B
+    from metal_candle_b200._lib import MCB_W_OUT_IN
+
+    g = torch.Generator(device=cuda_device).manual_seed(M + K)
+    x, w, dy = (torch.randn(*s, device=cuda_device, generator=g) for s in ((M, K), (N, K), (M, N)))
+    wt = w.t().contiguous()
+    bound = 2.0 ** -20
+    for got, p, q in ((B.lora_linear_forward(x, w, None, None, None, 1.0)[0], x, w.t()), (B.matmul(x, wt), x, w.t()),
+                      (B.lora_linear_backward(None, wt, None, None, 1.0, dy)[0], dy, w),
+                      (B.lora_linear_backward(None, w, None, None, 1.0, dy, weight_layout=MCB_W_OUT_IN)[0], dy, w)):
+        err = (got.double() - p.double() @ q.double()).abs() / (p.double().abs() @ q.double().abs())
+        assert err.max().item() <= bound
+
+
+def test_f32_product_of_extreme_values(cuda_device):
+    """Infinities, NaN, the largest and the smallest numbers come out as float32 arithmetic has them (each output is one product:
+    one term per row is not zero)."""
+    from metal_candle_b200 import backend as B
+
+    K = 200
+    a = torch.tensor([3.4e38, -3.4e38, 1e31, 1e38, 1.2e-38, 1e-38, 3e-42, 1e-45, 0.0, 1.7, -2.3e-20, float("inf"), float("nan")], device=cuda_device)
+    b = torch.tensor([1.0, -0.25, 3.3e-39, 1e-30, 1e25, 3.4e38, 1e-3], device=cuda_device)
+    x = torch.zeros(len(a), K, device=cuda_device)
+    x[:, 77] = a
+    w = torch.zeros(len(b), K, device=cuda_device)
+    w[:, 77] = b
+    y, _ = B.lora_linear_forward(x, w, None, None, None, 1.0)
+    want = (a.double()[:, None] * b.double()[None, :]).float()
+    assert torch.equal(y.isnan(), want.isnan())
+    ok = ~want.isnan()
+    # the products of the smaller parts that are left out (2^-20), and the spacing of the smallest numbers
+    assert torch.equal(y[ok].isinf(), want[ok].isinf())
+    fin = ok & want.isfinite()
+    assert ((y[fin].double() - want[fin].double()).abs() <= want[fin].double().abs() * 2.0 ** -20 + 2.0 ** -149).all()
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
