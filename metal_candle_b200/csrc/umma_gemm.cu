@@ -62,6 +62,7 @@ struct GemmParams {
   int M, N, K;
   int BN, rp, has_w, stages;
   int num_m_tiles, num_n_tiles, num_tiles, num_k_blocks, group_m;
+  int k1_blocks;      // k-blocks of the first operand pair; those behind them come from the second (maps in P's and Q's places)
   float scale;
   __nv_bfloat16* Y;
   const __nv_bfloat16* bias;
@@ -175,8 +176,10 @@ lora_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
           const uint32_t fb = b.full0 + 8 * stage;
           const uint32_t sb = base + stage * p.stage_bytes;
           mbar_expect_tx(fb, p.stage_bytes);
-          tma_load_2d(sb, &tmX, fb, kb * BK, m0);
-          if (p.has_w) tma_load_2d(sb + p.w_off, &tmW, fb, kb * BK, n0);
+          const bool first = kb < p.k1_blocks;
+          const int k0 = (first ? kb : kb - p.k1_blocks) * BK;
+          tma_load_2d(sb, first ? &tmX : &tmP, fb, k0, m0);
+          if (p.has_w) tma_load_2d(sb + p.w_off, first ? &tmW : &tmQ, fb, k0, n0);
           if (p.rp > 0) tma_load_2d(sb + p.p_off, &tmP, fb, kb * BK, 0);
           if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
@@ -599,11 +602,17 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
   if (c.K % 8 != 0 || c.N % 8 != 0)
     return fail(MCB_ERR_ALIGN, "bf16 path needs in/out features that are multiples of 8 (got reduction %lld, output %lld)",
                 (long long)c.K, (long long)c.N);
+  if (c.X2 != nullptr) {
+    if (c.rp != 0 || c.W == nullptr || c.W2 == nullptr || c.K2 <= 0 || c.K2 > 0x3fffff00ll || c.K > 0x3fffff00ll)
+      return fail(MCB_ERR_UNSUPPORTED, "bf16 GEMM: second operand pair of %lld features", (long long)c.K2);
+    if (c.K2 % 8 != 0 || !aligned16(c.X2) || !aligned16(c.W2))
+      return fail(MCB_ERR_ALIGN, "bf16 path needs features that are multiples of 8 and 16-byte aligned matrices");
+  }
   if (!aligned16(c.X) || (c.W && !aligned16(c.W)) || (c.Y && !aligned16(c.Y)) || (c.H && !aligned16(c.H)) || (c.R && !aligned16(c.R)))
     return fail(MCB_ERR_ALIGN, "bf16 path needs 16-byte aligned matrices");
   // shapes with too few tiles to fill the chip: narrower tiles, reduction in parts (umma_split.cu)
   if (c.W != nullptr && c.Y != nullptr && c.swiglu_up == nullptr) {
-    const SplitPlan sp = split_plan(c.M, c.N, c.K, c.rp, gemm2_eligible(c), ds);
+    const SplitPlan sp = split_plan(c.M, c.N, c.K + c.K2, c.rp, gemm2_eligible(c), ds);
     if (sp.bn > 0) {
       if (int rc = launch_split(sp, c, nullptr, nullptr, ds, st)) return rc;
       if (c.grads == nullptr) return MCB_OK;
@@ -623,7 +632,8 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
   p.num_m_tiles = (p.M + BM - 1) / BM;
   p.num_n_tiles = (p.N + p.BN - 1) / p.BN;
   p.num_tiles = p.num_m_tiles * p.num_n_tiles;
-  p.num_k_blocks = (p.K + BK - 1) / BK;
+  p.k1_blocks = (p.K + BK - 1) / BK;
+  p.num_k_blocks = p.k1_blocks + static_cast<int>((c.K2 + BK - 1) / BK);
   p.group_m = p.num_m_tiles < 16 ? p.num_m_tiles : 16;
   p.scale = c.scale;
   p.Y = c.Y; p.bias = c.bias; p.R = c.R; p.H = c.H; p.h_pitch = c.h_pitch; p.status = ds->status_word;
@@ -663,6 +673,9 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
   if (p.rp > 0) {
     if (int rc = make_map(ds, &tmP, c.P, c.K, p.rp, BK, p.rp, 128, "P")) return rc;
     if (int rc = make_map(ds, &tmQ, c.Q, p.rp, c.N, 8, p.BN, 0, "Q")) return rc;
+  } else if (c.X2 != nullptr) {
+    if (int rc = make_map(ds, &tmP, c.X2, c.K2, c.M, BK, BM, 128, "X2")) return rc;
+    if (int rc = make_map(ds, &tmQ, c.W2, c.K2, c.N, BK, p.BN, 128, "W2")) return rc;
   } else { tmP = tmX; tmQ = tmX; }
   const int grid = p.num_tiles < ds->sm_count ? p.num_tiles : ds->sm_count;
   // the weight gradients as a tail phase: the same CTAs, the stage ring re-cut for token rows
@@ -698,7 +711,7 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
   }
   const bool prof = profile_on();
   if (prof) {
-    const double m = static_cast<double>(c.M), n = static_cast<double>(c.N), k = static_cast<double>(c.K);
+    const double m = static_cast<double>(c.M), n = static_cast<double>(c.N), k = static_cast<double>(c.K + c.K2);
     double flops = (p.has_w ? 2.0 * m * n * k : 0.0) + 2.0 * m * c.r_true * (k + n);
     double bytes = 2.0 * (m * k + (p.has_w ? n * k : 0.0) + (c.Y ? m * n : 0.0)) + 2.0 * p.rp * (k + n);
     if (tail_on) {
@@ -1074,6 +1087,18 @@ int matmul_nt(const void* a, const void* bt, void* out, int64_t M, int64_t K, in
   c.W = static_cast<const __nv_bfloat16*>(bt);
   c.Y = static_cast<__nv_bfloat16*>(out);
   c.M = M; c.N = N; c.K = K;
+  return launch_gemm(c, ds, st);
+}
+
+int matmul_nt_sum(const void* a1, const void* bt1, int64_t K1, const void* a2, const void* bt2, int64_t K2, void* out, int64_t M, int64_t N,
+                  const DeviceState* ds, cudaStream_t st) {
+  GemmCall c;
+  c.X = static_cast<const __nv_bfloat16*>(a1);
+  c.W = static_cast<const __nv_bfloat16*>(bt1);
+  c.X2 = static_cast<const __nv_bfloat16*>(a2);
+  c.W2 = static_cast<const __nv_bfloat16*>(bt2);
+  c.Y = static_cast<__nv_bfloat16*>(out);
+  c.M = M; c.N = N; c.K = K1; c.K2 = K2;
   return launch_gemm(c, ds, st);
 }
 

@@ -56,6 +56,7 @@ struct Gemm2Params {
   int epi_bufs; // 2-KB staging buffers per 32 rows of the tile (kEpiBufs; 12 in the SwiGLU-backward form)
   int sw_pairs, sw_ahead;  // SwiGLU backward: buffer pairs per 32 rows, jobs loaded ahead
   int num_m_tiles, num_n_tiles, num_tiles, num_k_blocks, group_m;  // m tiles of 256 rows
+  int k1_blocks;  // k-blocks of the first operand pair; those behind them come from the second, whose maps take P's and Q's places
   float scale;
   __nv_bfloat16* Y;
   __nv_bfloat16* U;  // swiglu == 2: Y holds gate and U holds up [M,N] on entry, d gate and d up on return
@@ -234,8 +235,10 @@ lora_gemm2_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
           const uint32_t fb = map_to_cta(full0 + 8 * stage, 0);  // the leader's barrier
           const uint32_t sb = base + stage * p.stage_bytes;
           if (rank == 0) mbar_expect_tx(full0 + 8 * stage, 2 * p.stage_bytes);
-          tma_load_2d_pair(sb, &tmX, fb, kb * BK2, m0);
-          tma_load_2d_pair(sb + p.w_off, &tmW, fb, kb * BK2, n0);
+          const bool first = kb < p.k1_blocks;
+          const int k0 = (first ? kb : kb - p.k1_blocks) * BK2;
+          tma_load_2d_pair(sb, first ? &tmX : &tmP, fb, k0, m0);
+          tma_load_2d_pair(sb + p.w_off, first ? &tmW : &tmQ, fb, k0, n0);
           if (p.rp > 0) tma_load_2d_pair(sb + p.p_off, &tmP, fb, kb * BK2, static_cast<int>(rank) * half_r);
           if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
@@ -638,7 +641,8 @@ int launch_gemm2(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
   p.num_m_tiles = static_cast<int>((M + 255) / 256);
   p.num_n_tiles = static_cast<int>((N + bn - 1) / bn);
   p.num_tiles = p.num_m_tiles * p.num_n_tiles;
-  p.num_k_blocks = static_cast<int>((K + BK2 - 1) / BK2);
+  p.k1_blocks = static_cast<int>((K + BK2 - 1) / BK2);
+  p.num_k_blocks = p.k1_blocks + static_cast<int>((c.K2 + BK2 - 1) / BK2);
   p.group_m = p.num_m_tiles < 8 ? p.num_m_tiles : 8;
   p.Y = c.Y; p.bias = c.bias; p.R = c.R; p.H = c.H; p.h_pitch = c.h_pitch; p.status = ds->status_word;
   p.epi_bufs = kEpiBufs;
@@ -683,12 +687,15 @@ int launch_gemm2(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
   if (c.rp > 0) {
     if (int rc = make_map2(ds, &tmP, c.P, K, c.rp, BK2, c.rp / 2, 128, "P (pair)")) return rc;
     if (int rc = make_map2(ds, &tmQ, c.Q, c.rp, N, 8, bn / 4, 0, "Q (pair)")) return rc;
+  } else if (c.X2 != nullptr) {
+    if (int rc = make_map2(ds, &tmP, c.X2, c.K2, M, BK2, 128, 128, "X2 (pair)")) return rc;
+    if (int rc = make_map2(ds, &tmQ, c.W2, c.K2, N, BK2, bn / 2, 128, "W2 (pair)")) return rc;
   } else { tmP = tmX; tmQ = tmX; }
   int pairs = ds->sm_count / 2;
   if (pairs > p.num_tiles) pairs = p.num_tiles;
   const bool prof = profile_on();
   if (prof) {
-    const double m = static_cast<double>(M), n = static_cast<double>(N), k = static_cast<double>(K);
+    const double m = static_cast<double>(M), n = static_cast<double>(N), k = static_cast<double>(K + c.K2);
     profile_begin(c.swiglu_up != nullptr ? kProfGemmSwigluBwd : c.rp > 0 ? kProfGemmLora : kProfGemm,
                   2.0 * m * n * k + 2.0 * m * c.r_true * (k + n),
                   2.0 * (m * k + n * k + (c.swiglu_up != nullptr ? 4.0 : 1.0) * m * n) + 2.0 * c.rp * (k + n), st);
@@ -728,7 +735,7 @@ int launch_gemm2_swiglu(const __nv_bfloat16* X, const __nv_bfloat16* Wgu, __nv_b
   p.num_m_tiles = static_cast<int>((M + 255) / 256);
   p.num_n_tiles = static_cast<int>(F / 128);
   p.num_tiles = p.num_m_tiles * p.num_n_tiles;
-  p.num_k_blocks = static_cast<int>((K + BK2 - 1) / BK2);
+  p.num_k_blocks = p.k1_blocks = static_cast<int>((K + BK2 - 1) / BK2);
   p.group_m = p.num_m_tiles < 8 ? p.num_m_tiles : 8;
   p.Y = G; p.status = ds->status_word;
   const uint32_t x_bytes = 128 * BK2 * 2, w_bytes = 128u * BK2 * 2;
