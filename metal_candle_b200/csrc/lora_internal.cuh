@@ -97,6 +97,10 @@ SplitPlan split_plan(int64_t M, int64_t N, int64_t K, int rp, bool pair_kernel, 
 // Runs the call with that plan; with act != null its columns are blocks of 128 gate and 128 up features (bn 256) and c.Y,
 // up, act receive gate, up and silu(gate) * up.
 int launch_split(const SplitPlan& plan, const GemmCall& c, __nv_bfloat16* up, __nv_bfloat16* act, const DeviceState* ds, cudaStream_t st);
+// Tiles of 256 x up to 512 on CTA pairs (umma_wide.cu): their width for a call without a rank path, or 0 (the other kernels run),
+// and the better one's estimated cycles.
+int wide_bn(int64_t M, int64_t N, int64_t nkb, bool swiglu, const DeviceState* ds, double* cycles = nullptr);
+int launch_wide(int bn, const GemmCall& c, __nv_bfloat16* up, __nv_bfloat16* act, const DeviceState* ds, cudaStream_t st);
 size_t workspace_bytes(int64_t M, int64_t K, int64_t N, int64_t r);
 int delta_fwd(const LoraArgs& a, const DeviceState* ds);
 int linear_fwd(const LoraArgs& a, const DeviceState* ds);

@@ -42,6 +42,7 @@ using namespace umma;
 int init_grad_kernel();
 int init_gemm2_kernel();
 int init_split_kernel(DeviceState* ds);
+int init_wide_kernel();
 bool gemm2_eligible(const GemmCall& c);
 int launch_gemm2(const GemmCall& c, const DeviceState* ds, cudaStream_t st);
 size_t grad_partial_bytes(int64_t M, int64_t K, int64_t N, int rp);
@@ -621,6 +622,8 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
                           q.h_pitch, q.part, c.M, q.r, c.rp, q.accumulate, ds, st);
     }
   }
+  if (c.rp == 0 && c.swiglu_up == nullptr && gemm2_eligible(c))
+    if (const int bn = wide_bn(c.M, c.N, (c.K + BK - 1) / BK + (c.K2 + BK - 1) / BK, false, ds)) return launch_wide(bn, c, nullptr, nullptr, ds, st);
   // linears of useful size (with or without the rank path) run on CTA pairs (umma_gemm2.cu)
   if (gemm2_eligible(c)) return launch_gemm2(c, ds, st);
   GemmParams p;
@@ -794,6 +797,7 @@ int init_kernels(DeviceState* ds) {
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(lora_gemm_kernel)");
   if (int rc = init_gemm2_kernel()) return rc;
   if (int rc = init_split_kernel(ds)) return rc;
+  if (int rc = init_wide_kernel()) return rc;
   return init_grad_kernel();
 }
 

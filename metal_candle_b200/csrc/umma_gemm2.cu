@@ -70,54 +70,6 @@ struct Gemm2Params {
   uint32_t q_off, q_bytes, hs_off, hs_bytes;  // per CTA and accumulator buffer; q_bytes covers both halves' quarter-tiles
 };
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// shared::cluster address of the same shared-memory offset in CTA `cta` of the cluster
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t cta) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(cta));
-  return r;
-}
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar, uint32_t cta) {
-  asm volatile(
-      "{\n\t.reg .b32 ra;\n\t"
-      "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
-      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}"
-      ::"r"(bar), "r"(cta) : "memory");
-}
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t leader_bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(leader_bar), "r"(c0), "r"(c1)
-      : "memory");
-}
-__device__ __forceinline__ void umma2_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
-      : "memory");
-}
-__device__ __forceinline__ void umma2_commit_both(uint32_t bar) {
-  asm volatile(
-      "{\n\t.reg .b16 m;\n\t"
-      "mov.b16 m, 3;\n\t"
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}"
-      ::"r"(bar) : "memory");
-}
-// kind::f16, D=f32, A=B=bf16 K-major, M=256 (the pair), N=n
-__host__ __device__ constexpr uint32_t make_idesc2(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(256 >> 4) << 24);
-}
-
 // Two neighbouring elements of the SwiGLU backward: d gate = d u s (1 + g (1 - s)), d up = d g s with s = sigmoid(g).
 // The epilogue warps are bound by their instruction count, so: the two approximate special functions flush
 // denormals (the compiler then adds no range handling around them; relative error of s about 2^-22 from the functions and
@@ -719,13 +671,14 @@ int launch_gemm2_swiglu(const __nv_bfloat16* X, const __nv_bfloat16* Wgu, __nv_b
   // Up to one round of 128-token tiles over the SMs, one-CTA tiles (umma_split.cu) end earlier than 256-token pairs: pairs /
   // one-CTA tiles in us, 896 -> 4864 at 64 tokens 12.5 / 10.6, at 384 (114 tiles) 18.8 / 12.3; 2048 -> 5632 at 256 20.1 /
   // 19.3, at 384 (132 tiles) 31.7 / 19.5; 4096 -> 14336 at 128 (112 tiles) 58 / 46.  Beyond one round the pairs run.
+  GemmCall c;
+  c.X = X; c.W = Wgu; c.Y = G; c.M = M; c.N = 2 * F; c.K = K;
   if ((M + 127) / 128 * (F / 128) <= ds->sm_count) {
-    GemmCall c;
-    c.X = X; c.W = Wgu; c.Y = G; c.M = M; c.N = 2 * F; c.K = K;
     SplitPlan sp;
     sp.bn = 256;
     return launch_split(sp, c, U, Act, ds, st);
   }
+  if (const int bn = wide_bn(M, 2 * F, (K + BK2 - 1) / BK2, true, ds)) return launch_wide(bn, c, U, Act, ds, st);
   Gemm2Params p;
   memset(&p, 0, sizeof(p));
   p.M = static_cast<int>(M); p.N = static_cast<int>(2 * F); p.K = static_cast<int>(K);

@@ -512,3 +512,30 @@ def test_linear_pair_backward(cuda_device, M, K, N):
     d1, d2, w1, w2 = ((torch.randn(*s, device=cuda_device, generator=g) * f).bfloat16() for s, f in (((M, N), 1.0), ((M, N), 1.0), ((K, N), N ** -0.5), ((K, N), N ** -0.5)))
     want = d1.double() @ w1.double().t() + d2.double() @ w2.double().t()
     _close_bf16(B.linear_pair_backward(d1, w1, d2, w2), want, 2.0 ** -8)
+
+
+# 256-token tiles of more than 256 columns (18 to 19 row tiles x 2 to 4 wide column tiles fill the 74 CTA pairs once where narrow ones
+# need two rounds): widths of 320 to 512, ragged last rows, columns and k-blocks
+@pytest.mark.parametrize("M,K,N", [(4865, 2048, 896), (4608, 2040, 2040), (4700, 3000, 1000), (4801, 2504, 1272), (9400, 4864, 896)])
+def test_bf16_linear_wide_tiles(cuda_device, M, K, N):
+    from metal_candle_b200 import backend as B
+
+    g = torch.Generator(device=cuda_device).manual_seed(M)
+    x, w, bias, res = ((torch.randn(*s, device=cuda_device, generator=g) * f).bfloat16() for s, f in (((M, K), 1.0), ((N, K), K ** -0.5), ((N,), 1.0), ((M, N), 1.0)))
+    want = x.double() @ w.double().t()
+    _close_bf16(B.lora_linear_forward(x, w, None, None, None, 1.0)[0], want)
+    _close_bf16(B.lora_linear_forward(x, w, bias, None, None, 1.0, residual=res)[0], want + bias.double() + res.double())
+
+
+@pytest.mark.parametrize("M,K,F", [(4600, 2048, 1024), (4500, 2504, 1152), (9300, 4096, 896)])
+def test_gate_up_swiglu_wide_tiles(cuda_device, M, K, F):
+    """An even and an odd number of 128-feature blocks; against float64 of the same bf16 inputs."""
+    from metal_candle_b200 import backend as B
+
+    g = torch.Generator(device=cuda_device).manual_seed(M)
+    x, wg, wu = ((torch.randn(*s, device=cuda_device, generator=g) * f).bfloat16() for s, f in (((M, K), 1.0), ((F, K), K ** -0.5), ((F, K), K ** -0.5)))
+    gate, up, act = B.linear_swiglu_forward(x, B.interleave_gate_up(wg, wu))
+    want_g, want_u = x.double() @ wg.double().t(), x.double() @ wu.double().t()
+    _close_bf16(gate, want_g)
+    _close_bf16(up, want_u)
+    _close_bf16(act, torch.nn.functional.silu(want_g) * want_u)
