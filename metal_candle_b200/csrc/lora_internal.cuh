@@ -79,6 +79,8 @@ struct GemmCall {
   const __nv_bfloat16* X2 = nullptr;
   const __nv_bfloat16* W2 = nullptr;
   int64_t K2 = 0;
+  // Scratch [M, rp] for a rank intermediate that is computed apart (launch_gemm decides), or null: always in the product's own tiles.
+  __nv_bfloat16* Hr = nullptr;
   int rp = 0;
   int r_true = 0;  // unpadded rank, for the algorithmic flop count
   float scale = 1.0f;

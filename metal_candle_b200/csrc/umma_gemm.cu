@@ -69,6 +69,7 @@ struct GemmParams {
   const __nv_bfloat16* bias;
   const __nv_bfloat16* R;   // [M,N] added to the output (residual / gradient accumulation), or null
   __nv_bfloat16* H;   // [rp, h_pitch]: scale * X P^T, transposed (token index contiguous), or null
+  __nv_bfloat16* Hr;  // [M, rp]: the same as it lies, or null
   int64_t h_pitch;
   int* h_flags;       // per m-tile count of epilogue warps that have stored their H rows (tail phase), or null
   int* status;
@@ -163,7 +164,7 @@ lora_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         tile_coords(p, t, mt, nt);
         const int m0 = mt * BM, n0 = nt * p.BN;
         const int a = i & 1;
-        if (p.rp > 0) {
+        if (p.rp > 0 && p.Y != nullptr) {   // without an output there is no rank update: H is all this launch computes
           if (i >= 2) ok = mbar_wait(b.d1_full0 + 8 * a, ((i - 2) >> 1) & 1, abort_flag, 11, p.status);
           if (!ok) break;
           const uint32_t qbar = b.q_full0 + 8 * a;
@@ -254,6 +255,7 @@ lora_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         if (!ok) break;
         if (p.rp > 0) {
           umma_commit(b.d2_full0 + 8 * a);
+          if (p.Y == nullptr) continue;
           if (pend_a >= 0) {         // the previous tile's update has still not been issued: wait for it now
             ok = finish_pending();
             if (!ok) break;
@@ -301,6 +303,11 @@ lora_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
           // no-swizzle K-major operand: 16-byte K chunk j of row m lives at j*(128*16) + m*16
           *reinterpret_cast<uint4*>(hs_gen + (c / 8) * (BM * 16) + row_in_tile * 16) = lo;
           *reinterpret_cast<uint4*>(hs_gen + (c / 8 + 1) * (BM * 16) + row_in_tile * 16) = hi;
+          if (p.Hr != nullptr && grow < p.M) {
+            uint4* hp = reinterpret_cast<uint4*>(p.Hr + grow * p.rp + c);
+            hp[0] = lo;
+            hp[1] = hi;
+          }
           if (p.H != nullptr && nt == 0 && grow < p.M) {
             // transposed copy for the weight-gradient kernel: lanes hold consecutive tokens, so each of
             // these 2-byte stores is a contiguous 64-byte run across the warp
@@ -326,9 +333,11 @@ lora_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
             asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(p.h_flags + mt) : "memory");
         }
       }
-      ok = __all_sync(0xffffffffu, mbar_wait(b.d1_full0 + 8 * a, u & 1, abort_flag, 32, p.status));
-      if (!ok) break;
-      tcgen05_fence_after();
+      if (p.Y != nullptr) {
+        ok = __all_sync(0xffffffffu, mbar_wait(b.d1_full0 + 8 * a, u & 1, abort_flag, 32, p.status));
+        if (!ok) break;
+        tcgen05_fence_after();
+      }
       if (p.Y != nullptr && p.epi_bufs > 0) {
         // Output leaves in chunks of 32 columns: each thread rounds its row's 64 bytes into this warp's staging
         // buffer (64-byte swizzle, conflict-free) and one tiled store per chunk writes 32 rows x 64 bytes,
@@ -597,6 +606,29 @@ int pick_bn(int64_t N, int rp) {
   return bn;
 }
 
+// Whether the rank intermediate of a call is better computed ahead, by a launch of its own that reads X once more, and its update
+// added as one more k-block of the main product.  In the main product's own tiles the rank columns ride along in every n-tile:
+// at rank 16 they take the place of 32 of 256 output columns (19 tiles instead of 16 at N = 4096), at rank 64 of 64, and an n-tile of
+// few columns pays them in full.  Both ways in cycles: what a CTA pulls from L2 for its k-blocks at 42 bytes per cycle (the
+// rate of either kernel, 896 x 896 to 4096 x 14336), the launch ahead X at 23 (HBM) and 9000 for its start.
+// 32768 x 4096 -> 4096 r16 forward, in the tiles / apart: 916 / 778 us (with the wide tiles that the main product then takes).
+bool rank_apart(const GemmCall& c, const DeviceState* ds) {
+  if (c.rp == 0 || c.Hr == nullptr || c.W == nullptr || c.Y == nullptr || c.swiglu_up != nullptr || c.X2 != nullptr) return false;
+  GemmCall plain = c;
+  plain.rp = 0;
+  if (!gemm2_eligible(plain)) return false;
+  const double nkb = static_cast<double>((c.K + BK - 1) / BK);
+  const bool pair = gemm2_eligible(c);
+  const int bn = pick_bn(c.N, c.rp);
+  const int64_t rows = pair ? 256 : BM, slots = pair ? ds->sm_count / 2 : ds->sm_count;
+  const int64_t rounds = ((c.M + rows - 1) / rows * ((c.N + bn - 1) / bn) + slots - 1) / slots;
+  const double now = static_cast<double>(rounds) * nkb * (BM + (bn + c.rp) / (pair ? 2.0 : 1.0)) * 128.0 / 42.0;
+  double product = 0.0;
+  wide_bn(c.M, c.N, (c.K + BK - 1) / BK + 1, false, ds, &product);
+  const int64_t ahead_rounds = ((c.M + BM - 1) / BM + ds->sm_count - 1) / ds->sm_count;
+  return product + static_cast<double>(ahead_rounds) * nkb * (BM + c.rp) * 128.0 / 23.0 + 9000.0 < now;
+}
+
 int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
   if (c.M > 0x7fffff00ll || c.N > 0x7fffff00ll || c.K > 0x7fffff00ll)
     return fail(MCB_ERR_SHAPE, "bf16 GEMM: dimension exceeds 2^31");
@@ -622,6 +654,19 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
                           q.h_pitch, q.part, c.M, q.r, c.rp, q.accumulate, ds, st);
     }
   }
+  if (rank_apart(c, ds)) {
+    GemmCall h = c;
+    h.W = nullptr; h.Y = nullptr; h.bias = nullptr; h.R = nullptr; h.grads = nullptr;
+    if (int rc = launch_gemm(h, ds, st)) return rc;
+    GemmCall y = c;
+    y.P = nullptr; y.Q = nullptr; y.H = nullptr; y.Hr = nullptr; y.rp = 0; y.grads = nullptr;
+    y.X2 = c.Hr; y.W2 = c.Q; y.K2 = c.rp;
+    if (int rc = launch_gemm(y, ds, st)) return rc;
+    if (c.grads == nullptr) return MCB_OK;
+    const GradRequest& q = *c.grads;
+    return launch_grad2(q.X[0], q.Ht[0], q.C[0], q.out[0], q.transposed[0], q.X[1], q.Ht[1], q.C[1], q.out[1], q.transposed[1],
+                        q.h_pitch, q.part, c.M, q.r, c.rp, q.accumulate, ds, st);
+  }
   if (c.rp == 0 && c.swiglu_up == nullptr && gemm2_eligible(c))
     if (const int bn = wide_bn(c.M, c.N, (c.K + BK - 1) / BK + (c.K2 + BK - 1) / BK, false, ds)) return launch_wide(bn, c, nullptr, nullptr, ds, st);
   // linears of useful size (with or without the rank path) run on CTA pairs (umma_gemm2.cu)
@@ -631,15 +676,15 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
   p.M = static_cast<int>(c.M); p.N = static_cast<int>(c.N); p.K = static_cast<int>(c.K);
   p.rp = c.rp;
   p.has_w = c.W != nullptr ? 1 : 0;
-  p.BN = pick_bn(c.N, c.rp);
+  p.BN = c.Y != nullptr ? pick_bn(c.N, c.rp) : 32;
   p.num_m_tiles = (p.M + BM - 1) / BM;
-  p.num_n_tiles = (p.N + p.BN - 1) / p.BN;
+  p.num_n_tiles = c.Y != nullptr ? (p.N + p.BN - 1) / p.BN : 1;
   p.num_tiles = p.num_m_tiles * p.num_n_tiles;
   p.k1_blocks = (p.K + BK - 1) / BK;
   p.num_k_blocks = p.k1_blocks + static_cast<int>((c.K2 + BK - 1) / BK);
   p.group_m = p.num_m_tiles < 16 ? p.num_m_tiles : 16;
   p.scale = c.scale;
-  p.Y = c.Y; p.bias = c.bias; p.R = c.R; p.H = c.H; p.h_pitch = c.h_pitch; p.status = ds->status_word;
+  p.Y = c.Y; p.bias = c.bias; p.R = c.R; p.H = c.H; p.Hr = c.Hr; p.h_pitch = c.h_pitch; p.status = ds->status_word;
   const uint32_t x_bytes = BM * BK * 2;
   const uint32_t w_bytes = p.has_w ? p.BN * BK * 2 : 0;
   const uint32_t p_bytes = p.rp * BK * 2;
@@ -740,7 +785,7 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
 }
 
 struct Workspace {
-  __nv_bfloat16 *P, *Q, *H1, *H2;
+  __nv_bfloat16 *P, *Q, *H1, *H2, *Hr;
   float* part;
   int* flags;   // one counter per 128-token tile
   size_t total;
@@ -756,6 +801,7 @@ Workspace carve(void* ws, int64_t M, int64_t K, int64_t N, int64_t r) {
   w.Q = reinterpret_cast<__nv_bfloat16*>(take(static_cast<size_t>(rp) * big * 2));
   w.H1 = reinterpret_cast<__nv_bfloat16*>(take(static_cast<size_t>(h_pitch(M)) * rp * 2));
   w.H2 = reinterpret_cast<__nv_bfloat16*>(take(static_cast<size_t>(h_pitch(M)) * rp * 2));
+  w.Hr = reinterpret_cast<__nv_bfloat16*>(take(static_cast<size_t>(M) * rp * 2));
   w.part = reinterpret_cast<float*>(take(grad_partial_bytes(M, K, N, static_cast<int>(rp))));
   w.flags = reinterpret_cast<int*>(take(static_cast<size_t>((M + BM - 1) / BM) * sizeof(int)));
   w.total = off;
@@ -850,6 +896,7 @@ int linear_fwd(const LoraArgs& a, const DeviceState* ds) {
     if (int rc = pack(a, w, 0)) return rc;
     c.P = w.P; c.Q = w.Q;
     c.H = static_cast<__nv_bfloat16*>(a.h_save);
+    c.Hr = w.Hr;
     c.h_pitch = h_pitch(a.M);
     c.rp = static_cast<int>(rank_padded(a.r));
   c.r_true = static_cast<int>(a.r);
@@ -898,6 +945,7 @@ int linear_bwd(const LoraArgs& a, const DeviceState* ds) {
     if (a.r > 0) {
       c.P = w.P; c.Q = w.Q;
       c.H = (a.dA != nullptr) ? w.H1 : nullptr;
+      c.Hr = w.Hr;
       c.h_pitch = h_pitch(a.M);
       c.rp = rp;
       c.r_true = static_cast<int>(a.r);
@@ -1027,6 +1075,7 @@ int linear_fused_fwd(const LoraArgs& a, const LoraSegments& sg, const DeviceStat
   c.M = a.M; c.N = a.N; c.K = a.K;
   c.P = f.w.P; c.Q = f.w.Q;
   c.H = static_cast<__nv_bfloat16*>(a.h_save);
+  c.Hr = f.w.Hr;
   c.h_pitch = h_pitch(a.M);
   c.rp = rp;
   c.r_true = static_cast<int>(r_tot);
@@ -1056,6 +1105,7 @@ int linear_fused_bwd(const LoraArgs& a, const LoraSegments& sg, const DeviceStat
   c.M = a.M; c.N = a.K; c.K = a.N;
   c.P = f.w.P; c.Q = f.w.Q;
   c.H = want_grads ? f.w.H1 : nullptr;
+  c.Hr = f.w.Hr;
   c.h_pitch = h_pitch(a.M);
   c.rp = rp;
   c.r_true = static_cast<int>(r_tot);

@@ -539,3 +539,26 @@ def test_gate_up_swiglu_wide_tiles(cuda_device, M, K, F):
     _close_bf16(gate, want_g)
     _close_bf16(up, want_u)
     _close_bf16(act, torch.nn.functional.silu(want_g) * want_u)
+
+
+# ranks of one and several 16-column groups; reductions on either side of the pair kernel's line (1536), rows off the tiles
+@pytest.mark.parametrize("M,K,N,r", [(4700, 2048, 2048, 64), (5000, 896, 4864, 16), (4100, 1544, 4096, 16), (20000, 896, 896, 64), (3000, 896, 1160, 40)])
+def test_bf16_linear_rank_apart(cuda_device, M, K, N, r):
+    """Where the rank intermediate gets a launch of its own: forward, saved intermediate and all gradients against float64, with the
+    bounds of the other bf16 parity tests."""
+    from metal_candle_b200 import backend as B
+
+    g = torch.Generator(device=cuda_device).manual_seed(M)
+    R_ = lambda *s, f=1.0: torch.randn(*s, device=cuda_device, generator=g) * f  # noqa: E731
+    x, w, dy = R_(M, K).bfloat16(), R_(N, K, f=K ** -0.5).bfloat16(), R_(M, N).bfloat16()
+    a, b = R_(K, r, f=K ** -0.5), R_(r, N, f=0.1)
+    y, h = B.lora_linear_forward(x, w, None, a, b, 2.0)
+    dx, da, db = B.lora_linear_backward(x, B.transpose_2d(w), a, b, 2.0, dy, h_save=h)
+    X, W, D, A, Bm = (t.double() for t in (x, w, dy, a, b))
+    H, G = 2.0 * X @ A, 2.0 * D @ Bm.t()
+    _close_bf16(y, X @ W.t() + H @ Bm)
+    _close_bf16(h[:r, :M].t(), H)
+    assert bool((h[r:, :M] == 0).all())
+    _close_bf16(dx, D @ W + G @ A.t())
+    _close_bf16(da, X.t() @ G)
+    _close_bf16(db, H.t() @ D)
