@@ -209,11 +209,6 @@ int64_t mcb_lora_h_pitch(int64_t M);
 /* dst[cols,rows] = src[rows,cols]^T; makes the [K,N] copy of a frozen weight for the backward. */
 int mcb_transpose_2d(const void* src, void* dst, int64_t rows, int64_t cols, int dtype, void* stream);
 
-/* The input gradient of two frozen linears of the same input, dx [M,K] = dy1 [M,N] W1 + dy2 [M,N] W2 with W1, W2 as [in, out]
- * = [K,N] (the gate and up projections, src/models/transformer.rs:389-395): one product over both, summed before it is
- * rounded.  bfloat16. */
-int mcb_linear_pair_bwd(const void* dy1, const void* W1, const void* dy2, const void* W2, void* dx, int64_t M, int64_t K, int64_t N,
-                        int dtype, void* stream);
 /* The MLP's first half in one kernel: gate = x Wg^T, up = x Wu^T, act = silu(gate) * up  (MLP::forward,
  * src/models/transformer.rs:389-395: two candle_nn::Linear calls, silu, mul).  w_gate_up is [2F, K]: the gate and up
  * weights (each [F, K]) interleaved in blocks of 128 rows - gate rows 0..127, up rows 0..127, gate rows 128..255,

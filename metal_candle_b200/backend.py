@@ -398,21 +398,6 @@ def linear_swiglu_forward(x: torch.Tensor, w_gate_up: torch.Tensor):
     return gate, up, act
 
 
-def linear_pair_backward(dy1, weight1_t, dy2, weight2_t):
-    """dx of two frozen linears of the same input in one product: `dy1 W1 + dy2 W2` with the [in, out] copies of the weights
-    (bfloat16 only)."""
-    _require_cuda(dy1, weight1_t, dy2, weight2_t)
-    K, N = weight1_t.shape
-    if weight2_t.shape != weight1_t.shape or dy1.shape[-1] != N or dy2.shape != dy1.shape:
-        raise TrainingError(f"linear_pair_backward: {list(dy1.shape)} / {list(dy2.shape)} and weights {list(weight1_t.shape)} / {list(weight2_t.shape)}")
-    if len({t.dtype for t in (dy1, dy2, weight1_t, weight2_t)}) != 1:
-        raise TrainingError("linear_pair_backward: tensors of different types")
-    dx = torch.empty(*dy1.shape[:-1], K, dtype=dy1.dtype, device=dy1.device)
-    _lib.check(_lib_for(dy1).mcb_linear_pair_bwd(_ptr(dy1), _ptr(weight1_t), _ptr(dy2), _ptr(weight2_t), _ptr(dx), dy1.numel() // N, K, N,
-                                                 _dtype_code(dy1), _stream()))
-    return dx
-
-
 # ---------------------------------------------------------------------------------------------
 # fused causal attention
 # ---------------------------------------------------------------------------------------------

@@ -143,17 +143,6 @@ extern "C" int mcb_matmul(const void* a, const void* b, void* out, int64_t M, in
   return bf16path::matmul_nt(a, workspace, out, M, K, N, ds, st);
 }
 
-extern "C" int mcb_linear_pair_bwd(const void* dy1, const void* W1, const void* dy2, const void* W2, void* dx, int64_t M, int64_t K, int64_t N,
-                                   int dtype, void* stream) {
-  MCB_NVTX_RANGE("mcb_linear_pair_bwd");
-  if (!dy1 || !W1 || !dy2 || !W2 || !dx) return fail(MCB_ERR_NULL, "linear_pair_bwd: null pointer");
-  if (M <= 0 || K <= 0 || N <= 0) return fail(MCB_ERR_SHAPE, "linear_pair_bwd: empty dimension (M=%lld K=%lld N=%lld)", (long long)M, (long long)K, (long long)N);
-  if (dtype != MCB_BF16) return fail(MCB_ERR_UNSUPPORTED, "linear_pair_bwd: dtype %d (bfloat16 only)", dtype);
-  DeviceState* ds = current_device_state();
-  if (!ds) return MCB_ERR_NOT_INIT;
-  return bf16path::matmul_nt_sum(dy1, W1, N, dy2, W2, N, dx, M, K, ds, static_cast<cudaStream_t>(stream));
-}
-
 extern "C" int mcb_linear_swiglu_fwd(const void* x, const void* w_gate_up, void* gate, void* up, void* act, int64_t M,
                                      int64_t K, int64_t F, int dtype, void* stream) {
   MCB_NVTX_RANGE("mcb_linear_swiglu_fwd");

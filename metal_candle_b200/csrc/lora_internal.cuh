@@ -116,9 +116,6 @@ int linear_fused_bwd(const LoraArgs& a, const LoraSegments& sg, const DeviceStat
 // out[M,N] = a[M,K] bt[N,K]^T (bt is b transposed, both operands K-major)
 int matmul_nt(const void* a, const void* bt, void* out, int64_t M, int64_t K, int64_t N, const DeviceState* ds,
               cudaStream_t st);
-// out[M,N] = a1[M,K1] bt1[N,K1]^T + a2[M,K2] bt2[N,K2]^T, summed before it is rounded
-int matmul_nt_sum(const void* a1, const void* bt1, int64_t K1, const void* a2, const void* bt2, int64_t K2, void* out, int64_t M, int64_t N,
-                  const DeviceState* ds, cudaStream_t st);
 // gate, up [M,F] = x w_gu^T (w_gu: gate and up rows interleaved in blocks of 128), act = silu(gate) * up
 int launch_gemm2_swiglu(const __nv_bfloat16* X, const __nv_bfloat16* Wgu, __nv_bfloat16* G, __nv_bfloat16* U,
                         __nv_bfloat16* Act, int64_t M, int64_t K, int64_t F, const DeviceState* ds, cudaStream_t st);

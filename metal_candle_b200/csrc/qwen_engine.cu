@@ -334,12 +334,8 @@ int layer_backward(const Dims* q, const StepPlan& p, const LayerState& L, const 
     }
   }
   __nv_bfloat16 *dn2a = p.t_MH[1], *dn2 = p.t_MH[2];
-  if (!has(L, kGate) && !has(L, kUp)) {
-    QCHECK(mcb_linear_pair_bwd(s.gate, L.wt[kGate], s.up, L.wt[kUp], dn2, M, H, I, MCB_BF16, st));
-  } else {
-    QCHECK(lin_bwd(q, p, s.n2, L.wt[kGate], L.ad[kGate], s.gate, s.hg, nullptr, dn2a, accumulate, M, H, I, st));
-    QCHECK(lin_bwd(q, p, s.n2, L.wt[kUp], L.ad[kUp], s.up, s.hu, dn2a, dn2, accumulate, M, H, I, st));
-  }
+  QCHECK(lin_bwd(q, p, s.n2, L.wt[kGate], L.ad[kGate], s.gate, s.hg, nullptr, dn2a, accumulate, M, H, I, st));
+  QCHECK(lin_bwd(q, p, s.n2, L.wt[kUp], L.ad[kUp], s.up, s.hu, dn2a, dn2, accumulate, M, H, I, st));
   __nv_bfloat16* dh2 = p.t_MH[3];
   QCHECK(mcb_rmsnorm_bwd_ex(s.h2, L.ln2, dn2, dh3, dh2, nullptr, 0, M, H, eps, MCB_BF16, nullptr, 0, st));
   // attention

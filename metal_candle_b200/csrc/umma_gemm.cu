@@ -63,7 +63,6 @@ struct GemmParams {
   int M, N, K;
   int BN, rp, has_w, stages;
   int num_m_tiles, num_n_tiles, num_tiles, num_k_blocks, group_m;
-  int k1_blocks;      // k-blocks of the first operand pair; those behind them come from the second (maps in P's and Q's places)
   float scale;
   __nv_bfloat16* Y;
   const __nv_bfloat16* bias;
@@ -178,10 +177,8 @@ lora_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
           const uint32_t fb = b.full0 + 8 * stage;
           const uint32_t sb = base + stage * p.stage_bytes;
           mbar_expect_tx(fb, p.stage_bytes);
-          const bool first = kb < p.k1_blocks;
-          const int k0 = (first ? kb : kb - p.k1_blocks) * BK;
-          tma_load_2d(sb, first ? &tmX : &tmP, fb, k0, m0);
-          if (p.has_w) tma_load_2d(sb + p.w_off, first ? &tmW : &tmQ, fb, k0, n0);
+          tma_load_2d(sb, &tmX, fb, kb * BK, m0);
+          if (p.has_w) tma_load_2d(sb + p.w_off, &tmW, fb, kb * BK, n0);
           if (p.rp > 0) tma_load_2d(sb + p.p_off, &tmP, fb, kb * BK, 0);
           if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
@@ -613,7 +610,7 @@ int pick_bn(int64_t N, int rp) {
 // rate of either kernel, 896 x 896 to 4096 x 14336), the launch ahead X at 23 (HBM) and 9000 for its start.
 // 32768 x 4096 -> 4096 r16 forward, in the tiles / apart: 916 / 778 us (with the wide tiles that the main product then takes).
 bool rank_apart(const GemmCall& c, const DeviceState* ds) {
-  if (c.rp == 0 || c.Hr == nullptr || c.W == nullptr || c.Y == nullptr || c.swiglu_up != nullptr || c.X2 != nullptr) return false;
+  if (c.rp == 0 || c.Hr == nullptr || c.W == nullptr || c.Y == nullptr || c.swiglu_up != nullptr) return false;
   GemmCall plain = c;
   plain.rp = 0;
   if (!gemm2_eligible(plain)) return false;
@@ -629,23 +626,23 @@ bool rank_apart(const GemmCall& c, const DeviceState* ds) {
   return product + static_cast<double>(ahead_rounds) * nkb * (BM + c.rp) * 128.0 / 23.0 + 9000.0 < now;
 }
 
+// A product without a rank path of its own (a second operand pair at most) on CTA pairs, by wide tiles or narrower ones.
+int launch_plain(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
+  if (const int bn = wide_bn(c.M, c.N, (c.K + BK - 1) / BK + (c.K2 + BK - 1) / BK, false, ds)) return launch_wide(bn, c, nullptr, nullptr, ds, st);
+  return launch_gemm2(c, ds, st);
+}
+
 int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
   if (c.M > 0x7fffff00ll || c.N > 0x7fffff00ll || c.K > 0x7fffff00ll)
     return fail(MCB_ERR_SHAPE, "bf16 GEMM: dimension exceeds 2^31");
   if (c.K % 8 != 0 || c.N % 8 != 0)
     return fail(MCB_ERR_ALIGN, "bf16 path needs in/out features that are multiples of 8 (got reduction %lld, output %lld)",
                 (long long)c.K, (long long)c.N);
-  if (c.X2 != nullptr) {
-    if (c.rp != 0 || c.W == nullptr || c.W2 == nullptr || c.K2 <= 0 || c.K2 > 0x3fffff00ll || c.K > 0x3fffff00ll)
-      return fail(MCB_ERR_UNSUPPORTED, "bf16 GEMM: second operand pair of %lld features", (long long)c.K2);
-    if (c.K2 % 8 != 0 || !aligned16(c.X2) || !aligned16(c.W2))
-      return fail(MCB_ERR_ALIGN, "bf16 path needs features that are multiples of 8 and 16-byte aligned matrices");
-  }
   if (!aligned16(c.X) || (c.W && !aligned16(c.W)) || (c.Y && !aligned16(c.Y)) || (c.H && !aligned16(c.H)) || (c.R && !aligned16(c.R)))
     return fail(MCB_ERR_ALIGN, "bf16 path needs 16-byte aligned matrices");
   // shapes with too few tiles to fill the chip: narrower tiles, reduction in parts (umma_split.cu)
   if (c.W != nullptr && c.Y != nullptr && c.swiglu_up == nullptr) {
-    const SplitPlan sp = split_plan(c.M, c.N, c.K + c.K2, c.rp, gemm2_eligible(c), ds);
+    const SplitPlan sp = split_plan(c.M, c.N, c.K, c.rp, gemm2_eligible(c), ds);
     if (sp.bn > 0) {
       if (int rc = launch_split(sp, c, nullptr, nullptr, ds, st)) return rc;
       if (c.grads == nullptr) return MCB_OK;
@@ -661,15 +658,14 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
     GemmCall y = c;
     y.P = nullptr; y.Q = nullptr; y.H = nullptr; y.Hr = nullptr; y.rp = 0; y.grads = nullptr;
     y.X2 = c.Hr; y.W2 = c.Q; y.K2 = c.rp;
-    if (int rc = launch_gemm(y, ds, st)) return rc;
+    if (int rc = launch_plain(y, ds, st)) return rc;
     if (c.grads == nullptr) return MCB_OK;
     const GradRequest& q = *c.grads;
     return launch_grad2(q.X[0], q.Ht[0], q.C[0], q.out[0], q.transposed[0], q.X[1], q.Ht[1], q.C[1], q.out[1], q.transposed[1],
                         q.h_pitch, q.part, c.M, q.r, c.rp, q.accumulate, ds, st);
   }
-  if (c.rp == 0 && c.swiglu_up == nullptr && gemm2_eligible(c))
-    if (const int bn = wide_bn(c.M, c.N, (c.K + BK - 1) / BK + (c.K2 + BK - 1) / BK, false, ds)) return launch_wide(bn, c, nullptr, nullptr, ds, st);
-  // linears of useful size (with or without the rank path) run on CTA pairs (umma_gemm2.cu)
+  // linears of useful size (with or without the rank path) run on CTA pairs (umma_wide.cu, umma_gemm2.cu)
+  if (c.rp == 0 && c.swiglu_up == nullptr && gemm2_eligible(c)) return launch_plain(c, ds, st);
   if (gemm2_eligible(c)) return launch_gemm2(c, ds, st);
   GemmParams p;
   memset(&p, 0, sizeof(p));
@@ -680,8 +676,7 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
   p.num_m_tiles = (p.M + BM - 1) / BM;
   p.num_n_tiles = c.Y != nullptr ? (p.N + p.BN - 1) / p.BN : 1;
   p.num_tiles = p.num_m_tiles * p.num_n_tiles;
-  p.k1_blocks = (p.K + BK - 1) / BK;
-  p.num_k_blocks = p.k1_blocks + static_cast<int>((c.K2 + BK - 1) / BK);
+  p.num_k_blocks = (p.K + BK - 1) / BK;
   p.group_m = p.num_m_tiles < 16 ? p.num_m_tiles : 16;
   p.scale = c.scale;
   p.Y = c.Y; p.bias = c.bias; p.R = c.R; p.H = c.H; p.Hr = c.Hr; p.h_pitch = c.h_pitch; p.status = ds->status_word;
@@ -721,9 +716,6 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
   if (p.rp > 0) {
     if (int rc = make_map(ds, &tmP, c.P, c.K, p.rp, BK, p.rp, 128, "P")) return rc;
     if (int rc = make_map(ds, &tmQ, c.Q, p.rp, c.N, 8, p.BN, 0, "Q")) return rc;
-  } else if (c.X2 != nullptr) {
-    if (int rc = make_map(ds, &tmP, c.X2, c.K2, c.M, BK, BM, 128, "X2")) return rc;
-    if (int rc = make_map(ds, &tmQ, c.W2, c.K2, c.N, BK, p.BN, 128, "W2")) return rc;
   } else { tmP = tmX; tmQ = tmX; }
   const int grid = p.num_tiles < ds->sm_count ? p.num_tiles : ds->sm_count;
   // the weight gradients as a tail phase: the same CTAs, the stage ring re-cut for token rows
@@ -759,7 +751,7 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
   }
   const bool prof = profile_on();
   if (prof) {
-    const double m = static_cast<double>(c.M), n = static_cast<double>(c.N), k = static_cast<double>(c.K + c.K2);
+    const double m = static_cast<double>(c.M), n = static_cast<double>(c.N), k = static_cast<double>(c.K);
     double flops = (p.has_w ? 2.0 * m * n * k : 0.0) + 2.0 * m * c.r_true * (k + n);
     double bytes = 2.0 * (m * k + (p.has_w ? n * k : 0.0) + (c.Y ? m * n : 0.0)) + 2.0 * p.rp * (k + n);
     if (tail_on) {
@@ -1141,18 +1133,6 @@ int matmul_nt(const void* a, const void* bt, void* out, int64_t M, int64_t K, in
   c.W = static_cast<const __nv_bfloat16*>(bt);
   c.Y = static_cast<__nv_bfloat16*>(out);
   c.M = M; c.N = N; c.K = K;
-  return launch_gemm(c, ds, st);
-}
-
-int matmul_nt_sum(const void* a1, const void* bt1, int64_t K1, const void* a2, const void* bt2, int64_t K2, void* out, int64_t M, int64_t N,
-                  const DeviceState* ds, cudaStream_t st) {
-  GemmCall c;
-  c.X = static_cast<const __nv_bfloat16*>(a1);
-  c.W = static_cast<const __nv_bfloat16*>(bt1);
-  c.X2 = static_cast<const __nv_bfloat16*>(a2);
-  c.W2 = static_cast<const __nv_bfloat16*>(bt2);
-  c.Y = static_cast<__nv_bfloat16*>(out);
-  c.M = M; c.N = N; c.K = K1; c.K2 = K2;
   return launch_gemm(c, ds, st);
 }
 

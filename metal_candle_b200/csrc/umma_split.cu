@@ -32,7 +32,6 @@ constexpr uint32_t kSplitSmemMax = 227 * 1024 - 1024;
 struct SplitParams {
   int M, N, K;
   int BN, rp, stages, splits, nkb, m_tiles;
-  int k1_blocks;     // k-blocks of the first operand pair; those behind them come from the second
   int swiglu;        // 1: columns [0, 128) of a tile are gate features, [128, 256) the same features of up
   float scale;
   __nv_bfloat16* Y;  // swiglu: gate [M, F]
@@ -63,8 +62,7 @@ __device__ __forceinline__ float2 ld_peer2(uint32_t addr) {
 template <int S>
 __global__ void __launch_bounds__(kSplitThreads, 1)
 lora_gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
-                       const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmX2,
-                       const __grid_constant__ CUtensorMap tmW2, const SplitParams p) {
+                       const __grid_constant__ CUtensorMap tmP, const SplitParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen_base = smem_raw + (base - smem_u32(smem_raw));
@@ -110,11 +108,9 @@ lora_gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
         if (!mbar_wait(empty0 + 8 * stage, phase ^ 1, abort_flag, 13, p.status)) break;
         const uint32_t fb = full0 + 8 * stage, sb = base + stage * p.stage_bytes;
         mbar_expect_tx(fb, p.stage_bytes);
-        const bool first = kb < p.k1_blocks;
-        const int k0 = (first ? kb : kb - p.k1_blocks) * kSplitBK;
-        tma_load_2d(sb, first ? &tmX : &tmX2, fb, k0, m0);
-        tma_load_2d(sb + p.w_off, first ? &tmW : &tmW2, fb, k0, n0);
-        if (p.rp > 0) tma_load_2d(sb + p.p_off, &tmP, fb, k0, 0);
+        tma_load_2d(sb, &tmX, fb, kb * kSplitBK, m0);
+        tma_load_2d(sb + p.w_off, &tmW, fb, kb * kSplitBK, n0);
+        if (p.rp > 0) tma_load_2d(sb + p.p_off, &tmP, fb, kb * kSplitBK, 0);
         if (++stage == p.stages) { stage = 0; phase ^= 1; }
       }
     }
@@ -296,7 +292,7 @@ double kblock_cycles(double rows, double cols, double bytes_per_cycle) {
   return feed > cols ? feed : cols;
 }
 
-typedef void (*SplitKernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const SplitParams);
+typedef void (*SplitKernel)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const SplitParams);
 SplitKernel split_kernel(int s) {
   return s == 8 ? lora_gemm_split_kernel<8> : s == 4 ? lora_gemm_split_kernel<4> : s == 2 ? lora_gemm_split_kernel<2> : lora_gemm_split_kernel<1>;
 }
@@ -364,8 +360,7 @@ int launch_split(const SplitPlan& plan, const GemmCall& c, __nv_bfloat16* up, __
   memset(&p, 0, sizeof(p));
   p.M = static_cast<int>(c.M); p.N = static_cast<int>(c.N); p.K = static_cast<int>(c.K);
   p.BN = plan.bn; p.splits = plan.splits; p.rp = c.rp;
-  p.k1_blocks = (p.K + kSplitBK - 1) / kSplitBK;
-  p.nkb = p.k1_blocks + static_cast<int>((c.K2 + kSplitBK - 1) / kSplitBK);
+  p.nkb = (p.K + kSplitBK - 1) / kSplitBK;
   p.m_tiles = (p.M + BM - 1) / BM;
   p.swiglu = act != nullptr ? 1 : 0;
   p.scale = c.scale;
@@ -393,15 +388,10 @@ int launch_split(const SplitPlan& plan, const GemmCall& c, __nv_bfloat16* up, __
   if (int rc = split_map(ds, &tmW, c.W, c.K, c.N, p.BN, "W")) return rc;
   if (p.rp > 0) { if (int rc = split_map(ds, &tmP, c.P, c.K, p.rp, p.rp, "P")) return rc; }
   else tmP = tmX;
-  CUtensorMap tmX2 = tmX, tmW2 = tmW;
-  if (c.X2 != nullptr) {
-    if (int rc = split_map(ds, &tmX2, c.X2, c.K2, c.M, BM, "X2")) return rc;
-    if (int rc = split_map(ds, &tmW2, c.W2, c.K2, c.N, p.BN, "W2")) return rc;
-  }
   const int64_t n_tiles = (c.N + p.BN - 1) / p.BN;
   const bool prof = profile_on();
   if (prof) {
-    const double m = static_cast<double>(c.M), n = static_cast<double>(c.N), k = static_cast<double>(c.K + c.K2);
+    const double m = static_cast<double>(c.M), n = static_cast<double>(c.N), k = static_cast<double>(c.K);
     profile_begin(c.rp > 0 ? kProfGemmLora : kProfGemm, 2.0 * m * n * k + 2.0 * m * c.r_true * (k + n),
                   2.0 * (m * k + n * k + (act ? 1.5 : 1.0) * m * n) + 2.0 * c.rp * (k + n), st);
   }
@@ -421,7 +411,7 @@ int launch_split(const SplitPlan& plan, const GemmCall& c, __nv_bfloat16* up, __
     ++na;
   }
   cfg.attrs = attr; cfg.numAttrs = na;
-  const cudaError_t le = cudaLaunchKernelEx(&cfg, split_kernel(p.splits), tmX, tmW, tmP, tmX2, tmW2, p);
+  const cudaError_t le = cudaLaunchKernelEx(&cfg, split_kernel(p.splits), tmX, tmW, tmP, p);
   if (le != cudaSuccess) return cuda_fail(le, "lora_gemm_split_kernel launch");
   if (prof) profile_end(st);
   MCB_CHECK_LAUNCH("lora_gemm_split_kernel");

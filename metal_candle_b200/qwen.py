@@ -582,11 +582,8 @@ class Qwen:
             _lib.check(self.lib.mcb_swiglu_bwd(_ptr(gt), _ptr(up), _ptr(dact), _ptr(gt), _ptr(up), gt.numel(), self.dt,
                                                _stream()))  # in place: gate <- d gate, up <- d up
             del dact
-        if self.dtype == torch.bfloat16 and L["gate_proj"].lora is None and L["up_proj"].lora is None:
-            dn2 = backend.linear_pair_backward(gt, L["gate_proj"].weight_t, up, L["up_proj"].weight_t)
-        else:
-            dn2 = self._lin_bwd(sv["n2"], L["gate_proj"], gt, sv["hg"], key("gate_proj"), accumulate)
-            dn2 = self._lin_bwd(sv["n2"], L["up_proj"], up, sv["hu"], key("up_proj"), accumulate, dx_residual=dn2)
+        dn2 = self._lin_bwd(sv["n2"], L["gate_proj"], gt, sv["hg"], key("gate_proj"), accumulate)
+        dn2 = self._lin_bwd(sv["n2"], L["up_proj"], up, sv["hu"], key("up_proj"), accumulate, dx_residual=dn2)
         # gradient through the norm plus the one along the residual connection, added inside the norm's kernel
         dh2, _ = backend.rms_norm_backward(sv["h2"], L["post_attention_layernorm"], dn2, c.rms_norm_eps, need_dw=False,
                                            dx_residual=dh3)

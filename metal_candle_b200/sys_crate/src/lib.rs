@@ -171,7 +171,6 @@ extern "C" {
     pub fn mcb_lora_rank_padded(r: i64) -> i64;
     pub fn mcb_lora_h_pitch(M: i64) -> i64;
     pub fn mcb_transpose_2d(src: *const c_void, dst: *mut c_void, rows: i64, cols: i64, dtype: c_int, stream: *mut c_void) -> c_int;
-    pub fn mcb_linear_pair_bwd(dy1: *const c_void, W1: *const c_void, dy2: *const c_void, W2: *const c_void, dx: *mut c_void, M: i64, K: i64, N: i64, dtype: c_int, stream: *mut c_void) -> c_int;
     pub fn mcb_linear_swiglu_fwd(x: *const c_void, w_gate_up: *const c_void, gate: *mut c_void, up: *mut c_void, act: *mut c_void, M: i64, K: i64, F: i64, dtype: c_int, stream: *mut c_void) -> c_int;
     pub fn mcb_matmul_workspace_bytes(K: i64, N: i64, dtype: c_int) -> usize;
     pub fn mcb_matmul(a: *const c_void, b: *const c_void, out: *mut c_void, M: i64, K: i64, N: i64, dtype: c_int, workspace: *mut c_void, workspace_bytes: usize, stream: *mut c_void) -> c_int;
