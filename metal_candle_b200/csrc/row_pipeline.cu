@@ -15,6 +15,8 @@
 // part of the scores is never read from HBM.
 //
 // Every mbarrier wait is bounded; on expiry the CTA records a code in the device status word and leaves.
+#include <algorithm>
+
 #include "common.cuh"
 #include "umma_ptx.cuh"
 
@@ -130,7 +132,8 @@ __device__ __forceinline__ uint32_t causal_bytes(int q, int elem_bytes, int row_
 
 // Two CTAs per SM wherever the registers allow it without heavy spilling (a 9-warp CTA pair needs <= 96
 // registers per thread, a 17-warp pair <= 56); the wide register-resident forms run one CTA per SM.
-__host__ __device__ constexpr int rowpipe_min_blocks(int op, int w, int elems_per_lane) {
+__host__ __device__ constexpr int rowpipe_min_blocks(int op, int w, int elems_per_lane, bool two) {
+  if (two) return 3;
   if (op == kRmsFwd) return elems_per_lane > 0 ? 2 : 1;
   if (op == kSmFwd) return (elems_per_lane > 0 && (elems_per_lane <= 32 || w <= 8)) ? 2 : 1;
   if (op == kRmsBwd) return (w <= 8 && elems_per_lane <= 32) ? 2 : 1;
@@ -144,8 +147,17 @@ __host__ __device__ constexpr int rowpipe_min_blocks(int op, int w, int elems_pe
 // KMAX > 0: a lane owns vectors lane, lane+32, ... (KMAX of them) of every row and keeps them in registers —
 // the row itself (forward ops) or the dw sums (rmsnorm backward with dw).  KMAX == 0: rows of any width,
 // streamed from shared memory twice.
-template <typename T, int OP, int W, int KMAX, bool RAG>
-__global__ void __launch_bounds__((W + 1) * 32, rowpipe_min_blocks(OP, W, KMAX * Vec16<T>::N))
+//
+// TWO (RMSNorm backward without dw, rows of 17 to 128 vectors): two rows share a warp, 16 lanes each.  A warp's fixed work per row
+// (waits, two reductions, square root and division: some 300 instructions) is as much as its work on the three or four vectors a
+// lane has of 896 columns, and is done once for both; three CTAs of four such warps sit on an SM.  A lane keeps the sums of its even
+// and its odd vectors apart and adds them last, which is the order of the additions over 32 lanes: the results are the same bits.
+// One row / two rows per warp, us (bf16; with a residual in brackets): 32768 x 896 37.7 / 31.4 (39.1 / 32.7), 114688 x 896 113 / 104
+// (119 / 98), 8192 x 896 12.7 / 10.7, 2400 x 896 6.9 / 6.0, 100000 x 256 50.1 / 35.0, 20000 x 1000 26.6 / 24.1; float32 512 34.8 / 34.0.
+// The other operations are slower with two rows per warp: with dw (32 more accumulators a lane) 44.6 / 49.2, softmax 87024 x 777
+// forward 50.0 / 55.1 and backward 65.6 / 72.7; the RMSNorm forward gains at 32768 x 896 (17.6 / 16.2) and loses at 100000 x 256 (18.4 / 22.0).
+template <typename T, int OP, int W, int KMAX, bool RAG, bool TWO>
+__global__ void __launch_bounds__((W + 1) * 32, rowpipe_min_blocks(OP, W, KMAX * Vec16<T>::N, TWO))
 rowpipe_kernel(const Params p) {
   using V = Vec16<T>;
   constexpr int N = V::N;
@@ -183,7 +195,7 @@ rowpipe_kernel(const Params p) {
   }
   __syncthreads();
 
-  const int R = W / p.wpr;   // rows per tile
+  const int R = TWO ? 2 * W : W / p.wpr;   // rows per tile
   const int64_t n_tiles = (p.rows + R - 1) / R;
   const uint32_t stream_bytes = p.stream_bytes;
 
@@ -242,30 +254,34 @@ rowpipe_kernel(const Params p) {
       if (++stage == p.stages) { stage = 0; phase ^= 1; }
     }
   } else {
-    // ---------------- consumers: warp `warp` owns row `warp` of every tile ----------------
+    // ---------------- consumers: warp `warp` owns row `warp` of every tile (TWO: rows 2 `warp` and 2 `warp` + 1) ----------------
     constexpr bool kEarlyRes = OP == kRmsBwd && KMAX == 0;
-    constexpr int kEarly = kEarlyRes ? 4 : 1;
+    constexpr int kLanes = TWO ? 16 : 32;            // lanes per row
+    constexpr int kEarly = kEarlyRes ? (TWO ? 8 : 4) : 1;
+    const int l = TWO ? lane & 15 : lane;            // this lane's place in its row
     int stage = 0;
     uint32_t phase = 0;
     const float inv_d = 1.0f / static_cast<float>(p.D);
     int nvec = p.nvec;
     for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-      const int rit = warp / p.wpr, seg = warp - rit * p.wpr;   // row of the tile, segment of the row
+      const int rit = TWO ? 2 * warp + lane / 16 : warp / p.wpr, seg = TWO ? 0 : warp - rit * p.wpr;   // row of the tile, segment of the row
       const int64_t row = t * R + rit;
       // RMSNorm backward: the first vectors of the residual row are requested before the wait for x and dy, so that their
       // way from global memory passes under it and under the first pass (32768 x 896: 53.4 -> 43.7 us, 131072 x 896 185 -> 148, float32 117 -> 95)
       V early[kEarly];
       if constexpr (kEarlyRes) {
         if (p.res != nullptr && row < p.rows) {
-          const int vseg = nvec / p.wpr, v0 = seg * vseg + lane;
+          const int vseg = nvec / p.wpr, v0 = seg * vseg + l;
           const T* rrow = static_cast<const T*>(p.res) + row * p.D;
 #pragma unroll
           for (int k = 0; k < kEarly; ++k)
-            if (v0 + 32 * k < seg * vseg + vseg) early[k].raw = __ldcs(reinterpret_cast<const decltype(early[k].raw)*>(rrow) + v0 + 32 * k);
+            if (v0 + kLanes * k < seg * vseg + vseg) early[k].raw = __ldcs(reinterpret_cast<const decltype(early[k].raw)*>(rrow) + v0 + kLanes * k);
         }
       }
       if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * stage, phase, abort_flag, 52, p.status))) break;
-      if (row < p.rows) {
+      // (TWO: where the last row has no neighbour, the lanes that would have it go through the sums, whose shuffles are the whole
+      // warp's, over whatever their place in the stage holds, and write nothing)
+      if (TWO || row < p.rows) {
         const uint8_t* s0 = gen_base + stage * p.stage_bytes + rit * p.row_bytes;
         T* orow = static_cast<T*>(p.out) + row * p.D;
         // ragged rows: elements [lo, end) of the covering granules, whole granules [fa, nvec); the first 2N lanes each take
@@ -351,9 +367,10 @@ rowpipe_kernel(const Params p) {
           // pass 1: sum x^2 and sum (dy*w)*x, two lanes of float32 at a time
           // (a row may be shared by p.wpr warps, each with a contiguous segment of its vectors)
           const int vseg = nvec / p.wpr, v_begin = seg * vseg, v_end = v_begin + vseg;
-          float2 ss2 = f2(0.0f, 0.0f), gx2 = f2(0.0f, 0.0f);
-#pragma unroll 4
-          for (int vi = v_begin + lane; vi < v_end; vi += 32) {
+          float2 ss2[TWO ? 2 : 1], gx2[TWO ? 2 : 1];
+#pragma unroll
+          for (int h = 0; h < (TWO ? 2 : 1); ++h) ss2[h] = gx2[h] = f2(0.0f, 0.0f);
+          auto sums = [&](int vi, float2& sq, float2& gxq) {
             V a, b; a.raw = reinterpret_cast<const decltype(a.raw)*>(s0)[vi];
             b.raw = reinterpret_cast<const decltype(b.raw)*>(s1)[vi];
             float x[N], g[N]; a.to_float(x); b.to_float(g);
@@ -366,14 +383,33 @@ rowpipe_kernel(const Params p) {
                 g1 = __fmul2_rn(g1, f2(ww.z, ww.w));
               }
               const float2 x0 = f2(x[j], x[j + 1]), x1 = f2(x[j + 2], x[j + 3]);
-              ss2 = __ffma2_rn(x0, x0, ss2);
-              ss2 = __ffma2_rn(x1, x1, ss2);
-              gx2 = __ffma2_rn(g0, x0, gx2);
-              gx2 = __ffma2_rn(g1, x1, gx2);
+              sq = __ffma2_rn(x0, x0, sq);
+              sq = __ffma2_rn(x1, x1, sq);
+              gxq = __ffma2_rn(g0, x0, gxq);
+              gxq = __ffma2_rn(g1, x1, gxq);
             }
+          };
+          float ss, gx;
+          if constexpr (TWO) {
+#pragma unroll 2
+            for (int vi = l; vi < nvec; vi += 32) {
+              sums(vi, ss2[0], gx2[0]);
+              if (vi + 16 < nvec) sums(vi + 16, ss2[1], gx2[1]);
+            }
+            ss = (ss2[0].x + ss2[0].y) + (ss2[1].x + ss2[1].y);
+            gx = (gx2[0].x + gx2[0].y) + (gx2[1].x + gx2[1].y);
+            __syncwarp();
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) {
+              ss += __shfl_xor_sync(0xffffffffu, ss, o);
+              gx += __shfl_xor_sync(0xffffffffu, gx, o);
+            }
+          } else {
+#pragma unroll 4
+            for (int vi = v_begin + lane; vi < v_end; vi += 32) sums(vi, ss2[0], gx2[0]);
+            ss = warp_sum(ss2[0].x + ss2[0].y);
+            gx = warp_sum(gx2[0].x + gx2[0].y);
           }
-          float ss = warp_sum(ss2.x + ss2.y);
-          float gx = warp_sum(gx2.x + gx2.y);
           if (p.wpr > 1) {
             // the row's warps exchange their sums through shared memory and add them in segment order
             if (lane == 0) xch[rit][seg] = f2(ss, gx);
@@ -437,7 +473,9 @@ rowpipe_kernel(const Params p) {
             a.from_float(o);
             __stcs(reinterpret_cast<decltype(a.raw)*>(orow) + vi, a.raw);
           };
-          if constexpr (kDw) {
+          if (TWO && row >= p.rows) {
+            // no second row
+          } else if constexpr (kDw) {
 #pragma unroll
             for (int k = 0; k < KMAX; ++k) {
               const int vi = v_begin + lane + 32 * k;
@@ -448,18 +486,18 @@ rowpipe_kernel(const Params p) {
             constexpr int kRes = 2;
 #pragma unroll
             for (int k = 0; k < kEarly; ++k)
-              if (v_begin + lane + 32 * k < v_end) body_res(v_begin + lane + 32 * k, early[k]);
-            for (int v0 = v_begin + lane + 32 * kEarly; v0 < v_end; v0 += 32 * kRes) {
+              if (v_begin + l + kLanes * k < v_end) body_res(v_begin + l + kLanes * k, early[k]);
+            for (int v0 = v_begin + l + kLanes * kEarly; v0 < v_end; v0 += kLanes * kRes) {
               V rr[kRes];
 #pragma unroll
               for (int k = 0; k < kRes; ++k)
-                if (v0 + 32 * k < v_end) rr[k].raw = __ldcs(reinterpret_cast<const decltype(rr[k].raw)*>(rrow) + v0 + 32 * k);
+                if (v0 + kLanes * k < v_end) rr[k].raw = __ldcs(reinterpret_cast<const decltype(rr[k].raw)*>(rrow) + v0 + kLanes * k);
 #pragma unroll
               for (int k = 0; k < kRes; ++k)
-                if (v0 + 32 * k < v_end) body_res(v0 + 32 * k, rr[k]);
+                if (v0 + kLanes * k < v_end) body_res(v0 + kLanes * k, rr[k]);
             }
           } else {
-            for (int vi = v_begin + lane; vi < v_end; vi += 32) body(vi, nullptr);
+            for (int vi = v_begin + l; vi < v_end; vi += kLanes) body(vi, nullptr);
           }
         } else if constexpr (OP == kSmFwd && KMAX > 0) {
           const bool causal = p.causal_seq > 0;
@@ -742,22 +780,22 @@ rowpipe_kernel(const Params p) {
   }
 }
 
-template <typename T, int OP, int W, int KMAX, bool RAG>
+template <typename T, int OP, int W, int KMAX, bool RAG, bool TWO = false>
 int launch_one(const Params& p, int grid, size_t smem, cudaStream_t st) {
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(rowpipe_kernel<T, OP, W, KMAX, RAG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(rowpipe_kernel<T, OP, W, KMAX, RAG, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (227 * 1024) / 2 - 1024);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(rowpipe_kernel)");
-    // ask for the largest shared-memory carve-out so that two CTAs of ~100 KB fit an SM
-    e = cudaFuncSetAttribute(rowpipe_kernel<T, OP, W, KMAX, RAG>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    // ask for the largest shared-memory carve-out so that two CTAs of ~100 KB (three of ~70 KB) fit an SM
+    e = cudaFuncSetAttribute(rowpipe_kernel<T, OP, W, KMAX, RAG, TWO>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(rowpipe_kernel carve-out)");
     attr_set[dev] = true;
   }
-  const cudaError_t le = launch_kernel(rowpipe_kernel<T, OP, W, KMAX, RAG>, dim3(grid), dim3((W + 1) * 32), smem, st, chained_launch(), p);
+  const cudaError_t le = launch_kernel(rowpipe_kernel<T, OP, W, KMAX, RAG, TWO>, dim3(grid), dim3((W + 1) * 32), smem, st, chained_launch(), p);
   if (le != cudaSuccess) return cuda_fail(le, "rowpipe_kernel launch");
   MCB_CHECK_LAUNCH("rowpipe_kernel");
   return MCB_OK;
@@ -837,6 +875,16 @@ int try_launch(int op, const void* in0, const void* in1, const void* w, void* ou
     }
   }
   if (op != kRmsBwd) R = W;
+  // Two rows per warp (see the kernel): enough of them for every SM to have several tiles, and two stages or more in a third of an SM
+  constexpr int kTwoWarps = 4, kTwoCtas = 3;
+  const int two_stages = static_cast<int>(std::min<int64_t>(kMaxStages, (227 * 1024 / kTwoCtas - 1024 - 1024 - w_bytes) / (2 * kTwoWarps * row_bytes * n_streams)));
+  const bool two = op == kRmsBwd && dw_part == nullptr && nvec > 16 && nvec <= 128 && two_stages >= 2 && rows >= 4ll * kTwoWarps * ds->sm_count;
+  if (two) {
+    W = kTwoWarps;
+    R = 2 * kTwoWarps;
+    wpr = 1;
+    stages = two_stages;
+  }
   if (dw_part != nullptr) {
     const int need = (nvec / wpr + 31) / 32;
     kmax = need <= 1 ? 1 : need <= 2 ? 2 : need <= 4 ? 4 : need <= 8 ? 8 : need <= 16 ? 16 : 0;
@@ -859,9 +907,10 @@ int try_launch(int op, const void* in0, const void* in1, const void* w, void* ou
     smem = p.w_off + static_cast<size_t>(D) * 4 + 128;
   }
   const int64_t n_tiles = (rows + R - 1) / R;
-  int grid = 2 * ds->sm_count;
+  int grid = (two ? kTwoCtas : 2) * ds->sm_count;
   if (grid > n_tiles) grid = static_cast<int>(n_tiles);
   if (dw_blocks) *dw_blocks = grid;
+  if (two) return launch_one<T, kRmsBwd, kTwoWarps, 0, false, true>(p, grid, smem, st);
   if (rag) {
     if (op == kSmBwd) {
       switch (kmax) {

@@ -78,6 +78,27 @@ def test_rmsnorm_bwd_with_residual(cuda_device, dtype, rows, D, need_dw):
         assert dw is None
 
 
+# two rows per warp: 17 vectors (one lane with two), 112, 125, 128; an odd last row, a last tile of one row
+@pytest.mark.parametrize("dtype,rows,D", [(torch.bfloat16, 2401, 136), (torch.bfloat16, 2375, 896), (torch.bfloat16, 7107, 1000),
+                                          (torch.bfloat16, 2368, 1024), (torch.float32, 4737, 260), (torch.float32, 2369, 512)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_rmsnorm_bwd_two_rows_per_warp(cuda_device, dtype, rows, D, weighted):
+    """Against the oracle; and, where no residual is added, against the 32-lane form that also sums dw: the same additions in the same
+    order, so the same bits."""
+    from metal_candle_b200 import backend as B
+
+    c = S.rmsnorm_case(77, rows, D)
+    x, w, dy = (as_input(c[k], dtype) for k in ("x", "w", "dy"))
+    res = as_input(S.rmsnorm_case(78, rows, D)["dy"], dtype)
+    xd, dyd, resd = (to_dev(t, dtype, cuda_device) for t in (x, dy, res))
+    wd = to_dev(w, dtype, cuda_device) if weighted else None
+    wdx, _ = R.rms_norm_backward(x, w if weighted else None, 1e-6, dy)
+    dx = B.rms_norm_backward(xd, wd, dyd, 1e-6, need_dw=False)[0]
+    assert R.max_abs_normalised(back(dx), wdx) <= TOL[dtype]
+    assert torch.equal(dx, B.rms_norm_backward(xd, wd, dyd, 1e-6, need_dw=True)[0])
+    assert R.max_abs_normalised(back(B.rms_norm_backward(xd, wd, dyd, 1e-6, need_dw=False, dx_residual=resd)[0]), wdx + res) <= TOL[dtype]
+
+
 def test_rmsnorm_known_answers(cuda_device):
     """The reference's own known-answer values (tests/executor_direct.rs:480-496,
     src/backend/tensor.rs:321-336,382-397)."""
