@@ -83,7 +83,8 @@ int mcb_selftest_wait_timeout(int64_t limit_cycles, int64_t* waited_cycles_out, 
  * SMs, should set it to 0: the gradients then take their own launch, which waits for nothing. */
 #define MCB_OPT_GRAD_TAIL 0
 /* Smallest reduction length (in features) from which a linear WITH a rank path runs on CTA pairs instead of the
- * one-CTA kernel (default 1536; linears without a rank path always take the pair kernel when large enough). */
+ * one-CTA kernel (default 1536; from 16384 tokens on 13/24 of it, 832; linears without a rank path always take the pair
+ * kernel when large enough). */
 #define MCB_OPT_PAIR_MIN_K 1
 /* 1 (default): the library's kernels are launched as programmatic dependents of the kernel before them in their stream, so that
  * a kernel's launch and set-up run under its predecessor's tail (it touches no memory before that has finished); 0: plain

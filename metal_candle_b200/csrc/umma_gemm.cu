@@ -607,7 +607,8 @@ int pick_bn(int64_t N, int rp) {
 // added as one more k-block of the main product.  In the main product's own tiles the rank columns ride along in every n-tile:
 // at rank 16 they take the place of 32 of 256 output columns (19 tiles instead of 16 at N = 4096), at rank 64 of 64, and an n-tile of
 // few columns pays them in full.  Both ways in cycles: what a CTA pulls from L2 for its k-blocks at 42 bytes per cycle (the
-// rate of either kernel, 896 x 896 to 4096 x 14336), the launch ahead X at 23 (HBM) and 9000 for its start.
+// rate of either kernel, 896 x 896 to 4096 x 14336) and, on pairs, 3000 per tile that the rank update holds it up (32768 x 896 -> 896
+// r64: 78.8 in the tiles against 72.7 us apart), the launch ahead X at 23 (HBM) and 9000 for its start.
 // 32768 x 4096 -> 4096 r16 forward, in the tiles / apart: 916 / 778 us (with the wide tiles that the main product then takes).
 bool rank_apart(const GemmCall& c, const DeviceState* ds) {
   if (c.rp == 0 || c.Hr == nullptr || c.W == nullptr || c.Y == nullptr || c.swiglu_up != nullptr) return false;
@@ -619,7 +620,7 @@ bool rank_apart(const GemmCall& c, const DeviceState* ds) {
   const int bn = pick_bn(c.N, c.rp);
   const int64_t rows = pair ? 256 : BM, slots = pair ? ds->sm_count / 2 : ds->sm_count;
   const int64_t rounds = ((c.M + rows - 1) / rows * ((c.N + bn - 1) / bn) + slots - 1) / slots;
-  const double now = static_cast<double>(rounds) * nkb * (BM + (bn + c.rp) / (pair ? 2.0 : 1.0)) * 128.0 / 42.0;
+  const double now = static_cast<double>(rounds) * (nkb * (BM + (bn + c.rp) / (pair ? 2.0 : 1.0)) * 128.0 / 42.0 + (pair ? 3000.0 : 0.0));
   double product = 0.0;
   wide_bn(c.M, c.N, (c.K + BK - 1) / BK + 1, false, ds, &product);
   const int64_t ahead_rounds = ((c.M + BM - 1) / BM + ds->sm_count - 1) / ds->sm_count;
@@ -901,6 +902,7 @@ bool swiglu_bwd_supported(int64_t M, int64_t K, int64_t N, int64_t r) {
   if (M <= 0 || K <= 0 || N <= 0 || r < 0 || K % 8 != 0 || N % 8 != 0) return false;
   GemmCall c;   // the input-gradient product: [M,N] . [K,N]^T, rank path over N
   c.X = c.W = c.Y = reinterpret_cast<__nv_bfloat16*>(16);   // placeholders: only their presence is looked at
+  c.swiglu_up = c.Y;
   c.M = M; c.N = K; c.K = N;
   c.rp = static_cast<int>(rank_padded(r));
   return gemm2_eligible(c);

@@ -564,15 +564,21 @@ int init_gemm2_kernel() {
 
 // Whether the pair kernel takes this call (everything else stays on the one-CTA kernel): a main product
 // with an output, large enough to fill CTA pairs; with a rank path, rank padded to a multiple of 16 and at
-// most 64 and a long enough reduction.
+// most 64 and a long enough reduction (MCB_OPT_PAIR_MIN_K; many tokens: 13/24 of it, 832 by default).
 bool gemm2_eligible(const GemmCall& c) {
   if (c.W == nullptr || c.Y == nullptr || c.M < 1024 || c.N < 128 || c.K < 64) return false;
   if (c.rp == 0) return true;
-  // Short reductions stay on the one-CTA kernel.  Alone, the pair is a little ahead even there once the rank
-  // update is issued between the next tile's k-blocks (32768x896x896 r16 forward 953 against 922 TFLOP/s), but
-  // inside the training step, with its k/v projections of 128 outputs and its backward calls, the one-CTA kernel
-  // measured 1-2 % faster per step on the same box (116.1-118.5 against 118.4-119.5 ms).
-  return c.rp % 16 == 0 && c.rp <= 64 && c.K >= option(MCB_OPT_PAIR_MIN_K);
+  if (c.rp % 16 != 0 || c.rp > 64) return false;
+  const int64_t min_k = option(MCB_OPT_PAIR_MIN_K);
+  if (c.K >= min_k) return true;
+  // Shorter reductions only of many tokens: a pair's k-blocks cost an SM less, its start and (in a backward) the gradients' own launch
+  // cost more, and below 13 k-blocks the tile's epilogue hides the difference.  One CTA / pairs, us, forward and backward r16:
+  // 16384 x 896 -> 896 42.0 / 36.2 and 60.6 / 53.7, 32768 tokens 70.7 / 59.2 and 99.9 / 90.3, 131072 r8 236 / 214 and 322 / 298,
+  // 16384 x 1152 -> 896 45.4 / 42.0 and 68.7 / 68.8, 24576 x 1000 -> 1000 76.4 / 70.6 and 112 / 106, 16384 x 832 -> 832 r32 40.7 / 36.4 and
+  // 64.0 / 59.6; but 4096 x 896 -> 896 15.1 / 14.9 and 23.9 / 26.1, 32768 x 640 -> 640 40.7 / 44.3 and 61.6 / 66.6, and where one narrow
+  // column tile makes the call HBM-bound 131072 x 896 -> 128 58.8 / 63.6.
+  // (The SwiGLU form keeps to the long reductions that mcb_lora_linear_bwd_swiglu_supported has always named.)
+  return c.swiglu_up == nullptr && c.N >= 256 && c.M >= 16384 && c.K * 24 >= min_k * 13;
 }
 
 int launch_gemm2(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {

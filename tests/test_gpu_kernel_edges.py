@@ -534,6 +534,16 @@ def test_gate_up_swiglu_wide_tiles(cuda_device, M, K, F):
 def test_bf16_linear_rank_apart(cuda_device, M, K, N, r):
     """Where the rank intermediate gets a launch of its own: forward, saved intermediate and all gradients against float64, with the
     bounds of the other bf16 parity tests."""
+    _linear_with_rank_path(cuda_device, M, K, N, r)
+
+
+# short reductions of 16384 tokens and more on CTA pairs: from 832 features on, ragged last rows, columns and k-blocks
+@pytest.mark.parametrize("M,K,N,r", [(16384, 832, 264, 16), (16390, 896, 896, 16), (17001, 1000, 840, 8), (16384, 840, 904, 40)])
+def test_bf16_linear_short_reduction_on_pairs(cuda_device, M, K, N, r):
+    _linear_with_rank_path(cuda_device, M, K, N, r)
+
+
+def _linear_with_rank_path(cuda_device, M, K, N, r):
     from metal_candle_b200 import backend as B
 
     g = torch.Generator(device=cuda_device).manual_seed(M)
