@@ -72,8 +72,8 @@ void note_launch();
 
 // Whether kernels are launched as programmatic dependents of the kernel before them in their stream (MCB_OPT_PDL; not while
 // launches are timed one by one): the launch and the kernel's set-up then pass under the tail of that kernel.  Every kernel
-// launched so lets its own dependents start at once and waits (grid_dependency_wait) before it touches memory: the wait ends
-// when the kernel before it, which has waited likewise, is complete.
+// launched so lets its own dependents start at once and waits (grid_dependency_wait) before it reads or writes memory: the wait
+// ends when the kernel before it, which has waited likewise, is complete.  (Before the wait it may ask for lines to be in L2.)
 inline bool chained_launch() { return !profile_on() && option(MCB_OPT_PDL) != 0; }
 
 // Kernel launch with or without the programmatic-serialization attribute.
@@ -100,6 +100,9 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // start early (it has no effect otherwise).  Both are no-ops for kernels launched the ordinary way.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Asks for the line of `p` to be brought into L2.  Nothing is read: whatever is written to the line later is what a later load gets,
+// so a kernel may ask for operands before its grid_dependency_wait even if the kernel before it should be writing them.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // The pointer again, as a value that is not known before this point: a load that may be taken for one of constant memory
 // (const __restrict__, __ldg) cannot be moved up over the wait before it.
 template <typename T>

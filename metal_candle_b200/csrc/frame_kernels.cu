@@ -102,24 +102,16 @@ __global__ void rope_relayout_qkv_kernel(T* __restrict__ fused, RopeSegment<T> s
   using V = Vec16<T>;
   constexpr int N = V::N;
   grid_launch_dependents();
-  grid_dependency_wait();
-  fused = from_here(fused);
-  s0.head_major = from_here(s0.head_major);
-  s1.head_major = from_here(s1.head_major);
-  s2.head_major = from_here(s2.head_major);
   const int half = d / 2;
   const int chunks = half / N;
   const int64_t total = static_cast<int64_t>(B) * S * chunks;
   const int heads = s0.H + s1.H + s2.H;
   const int h_begin = static_cast<int>(static_cast<int64_t>(heads) * blockIdx.y / gridDim.y);
   const int h_end = static_cast<int>(static_cast<int64_t>(heads) * (blockIdx.y + 1) / gridDim.y);
-  for (int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-       idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int c = static_cast<int>(idx % chunks);
-    const int64_t bs = idx / chunks;
-    const int s = static_cast<int>(bs % S);
-    const int b = static_cast<int>(bs / S);
-    float cs[N], sn[N];
+  const int64_t first_idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  float cs[N], sn[N];
+  auto angles = [&](int64_t idx) {
+    const int c = static_cast<int>(idx % chunks), s = static_cast<int>(idx / chunks % S);
 #pragma unroll
     for (int j = 0; j < N; ++j) {
       const int i = c * N + j;
@@ -127,6 +119,20 @@ __global__ void rope_relayout_qkv_kernel(T* __restrict__ fused, RopeSegment<T> s
       sincosf(static_cast<float>(s) * inv_freq, &sn[j], &cs[j]);
       if (inverse) sn[j] = -sn[j];
     }
+  };
+  // The first (with few tokens the only) sines and cosines, some 1500 instructions, under the tail of the kernel before.
+  if (first_idx < total) angles(first_idx);
+  grid_dependency_wait();
+  fused = from_here(fused);
+  s0.head_major = from_here(s0.head_major);
+  s1.head_major = from_here(s1.head_major);
+  s2.head_major = from_here(s2.head_major);
+  for (int64_t idx = first_idx; idx < total; idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int c = static_cast<int>(idx % chunks);
+    const int64_t bs = idx / chunks;
+    const int s = static_cast<int>(bs % S);
+    const int b = static_cast<int>(bs / S);
+    if (idx != first_idx) angles(idx);
 #pragma unroll
     for (int g = 0; g < 3; ++g) {
       const RopeSegment<T>& sg = g == 0 ? s0 : g == 1 ? s1 : s2;

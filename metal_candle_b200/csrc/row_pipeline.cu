@@ -177,6 +177,8 @@ rowpipe_kernel(const Params p) {
     fence_proxy_async_smem();
   }
   grid_launch_dependents();
+  if constexpr (OP == kRmsFwd || OP == kRmsBwd)
+    if (p.w != nullptr && threadIdx.x * 128 < p.D * static_cast<int>(sizeof(T))) prefetch_l2(static_cast<const char*>(p.w) + threadIdx.x * 128);
   grid_dependency_wait();
   // The weight as float32, in planes of four columns per vector: column vi * N + j is at (j / 4) * w_plane + vi * 4 + j % 4,
   // so that the lanes of a warp, one vector each, read 16 bytes next to each other.  Column after column a bf16 vector's

@@ -464,10 +464,12 @@ __global__ void pack_lora_kernel(const float* __restrict__ A, const float* __res
                                  __nv_bfloat16* __restrict__ P, __nv_bfloat16* __restrict__ Q, int K, int N, int r,
                                  int rp, int mode, int* __restrict__ flags, int n_flags) {
   grid_launch_dependents();   // the GEMM chained behind this kernel may start its set-up; it waits before it loads P / Q
+  const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (tid * 32 < static_cast<int64_t>(K) * r) prefetch_l2(A + tid * 32);
+  if (tid * 32 < static_cast<int64_t>(N) * r) prefetch_l2(B + tid * 32);
   grid_dependency_wait();     // P, Q and the counters may still be in use, A and B in the making
   A = from_here(A);
   B = from_here(B);
-  const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   // the per-tile counters of the backward kernel's tail phase start from zero in every call
   for (int64_t i = tid; i < n_flags; i += static_cast<int64_t>(gridDim.x) * blockDim.x) flags[i] = 0;
   const int64_t nP = static_cast<int64_t>(rp) * (mode == 0 ? K : N);
@@ -504,8 +506,12 @@ struct SegTable {
 __global__ void pack_lora_fused_kernel(const SegTable t, __nv_bfloat16* __restrict__ P, __nv_bfloat16* __restrict__ Q, int K,
                                        int N, int r, int rp, int mode, int* __restrict__ flags, int n_flags) {
   grid_launch_dependents();
-  grid_dependency_wait();
   const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  for (int sg = 0; sg < t.count; ++sg) {
+    if (tid * 32 < static_cast<int64_t>(K) * r) prefetch_l2(t.A[sg] + tid * 32);
+    if (tid * 32 < static_cast<int64_t>(t.n[sg]) * r) prefetch_l2(t.B[sg] + tid * 32);
+  }
+  grid_dependency_wait();
   for (int64_t i = tid; i < n_flags; i += static_cast<int64_t>(gridDim.x) * blockDim.x) flags[i] = 0;
   const int64_t nP = static_cast<int64_t>(rp) * (mode == 0 ? K : N);
   const int64_t nQ = static_cast<int64_t>(rp) * (mode == 0 ? N : K);

@@ -27,6 +27,7 @@ using namespace umma;
 namespace {
 
 constexpr int kSplitThreads = 320, kSplitMaxStages = 8, kSplitBK = 64;
+constexpr int kSplitAhead = 16;   // k-blocks of the weight that a CTA asks for ahead: at most 148 x 16 x 32 KB, within L2
 constexpr uint32_t kSplitSmemMax = 227 * 1024 - 1024;
 
 struct SplitParams {
@@ -95,7 +96,20 @@ lora_gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
   grid_launch_dependents();
-  grid_dependency_wait();   // the set-up above ran under the tail of the kernel before
+  // The set-up above runs under the tail of the kernel before, and so does the weight's way from HBM to L2: a model's weights are
+  // more than L2 holds, so with 333 tokens every launch finds them cold and its first k-blocks waited for HBM.  The CTAs of the
+  // m-tiles that share a weight tile ask for its k-blocks in turn.  With the like of it in the pack, RMSNorm and rotary kernels: forward of
+  // 24 layers with 333 tokens 1817 -> 1665 us, with 128 tokens and four adapters a layer 1865 -> 1677, training pass of 6 layers with 512
+  // tokens 1673 -> 1610.  (Two CTAs per SM, so that the next launch's could ask even earlier, cost the ring its depth: 1809 and 1735.)
+  if (warp == 0 && lane == 0) {
+    prefetch_map(&tmX);
+    if (p.rp > 0) prefetch_map(&tmP);
+    const int kb_ahead = min(kb_end, kb_begin + kSplitAhead * p.m_tiles);
+    for (int kb = kb_begin + tile % p.m_tiles; kb < kb_ahead; kb += p.m_tiles) tma_prefetch_l2_2d(&tmW, kb * kSplitBK, n0);
+  } else if (warp == 2 && p.bias != nullptr && !p.swiglu) {
+    for (int c = lane * 64; c < p.BN && n0 + c < p.N; c += 32 * 64) prefetch_l2(p.bias + n0 + c);
+  }
+  grid_dependency_wait();
   float* part = reinterpret_cast<float*>(gen_base);                    // [128][pitch], over the stage ring
   uint32_t* qs = reinterpret_cast<uint32_t*>(gen_base + p.qs_off);     // [rp / 2][BN]: pairs of rank columns of Q
   uint32_t* hs = reinterpret_cast<uint32_t*>(gen_base + p.hs_off);     // [128 rows][rp / 2]
