@@ -249,29 +249,29 @@ rmsnorm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __
   }
 }
 
-// dw[c] (+)= sum over blocks of dw_partial[b][c] (deterministic: fixed order).  A CTA owns 32 columns; its 8
-// warps each sum every 8th partial row (independent loads, unrolled), then warp 0 adds the 8 sums in warp order.
-__global__ void __launch_bounds__(256)
+// dw[c] (+)= sum over blocks of dw_partial[b][c] (deterministic: fixed order).  A CTA owns 32 columns; its 32 warps each sum every
+// 32nd partial row, then warp w adds the 32 sums of column w.  Bound: latency (the partials, 1 MB at D = 896, are in L2), so all the
+// loads of a warp are in flight at once.  Backward with dw with 8 warps / 32: 32768 x 512 float32 41.7 / 39.6 us, 100000 x 256 48.4 / 46.4,
+// 32768 x 896 44.7 / 44.4.
+constexpr int kColsumWarps = 32;
+__global__ void __launch_bounds__(kColsumWarps * 32)
 colsum_partials_kernel(const float* __restrict__ partial, float* __restrict__ dw, int nblocks, int D, int accumulate) {
-  __shared__ float red[8][32];
+  __shared__ float red[kColsumWarps][33];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = blockIdx.x * 32 + lane;
+  const int c = blockIdx.x * 32 + lane, cw = blockIdx.x * 32 + warp;
   float s = 0.0f;
   grid_launch_dependents();
   grid_dependency_wait();
   partial = from_here(partial);
+  const float before = accumulate && lane == 0 && cw < D ? from_here(dw)[cw] : 0.0f;
   if (c < D) {
-#pragma unroll 8
-    for (int b = warp; b < nblocks; b += 8) s += partial[static_cast<int64_t>(b) * D + c];
+#pragma unroll 10
+    for (int b = warp; b < nblocks; b += kColsumWarps) s += partial[static_cast<int64_t>(b) * D + c];
   }
   red[warp][lane] = s;
   __syncthreads();
-  if (warp == 0 && c < D) {
-    float t = 0.0f;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) t += red[w][lane];
-    dw[c] = accumulate ? dw[c] + t : t;
-  }
+  const float t = warp_sum(red[lane][warp]);
+  if (lane == 0 && cw < D) dw[cw] = before + t;
 }
 
 // ---- softmax forward --------------------------------------------------------------------------
@@ -586,7 +586,7 @@ int rmsnorm_bwd_t(const void* x, const void* w, const void* dy, void* dx, float*
     const int rc = rowpipe::try_launch<T>(rowpipe::kRmsBwd, x, dy, w, dx, nullptr, dw ? (float*)ws : nullptr, &blocks, rows, D,
                                           eps, 0, 1.0f, ds, st, res);
     if (rc == MCB_OK && dw != nullptr) {
-      const cudaError_t le = launch_kernel(colsum_partials_kernel, dim3((unsigned)((D + 31) / 32)), dim3(256), 0, st, chained_launch(),
+      const cudaError_t le = launch_kernel(colsum_partials_kernel, dim3((unsigned)((D + 31) / 32)), dim3(kColsumWarps * 32), 0, st, chained_launch(),
                                            (const float*)ws, dw, blocks, (int)D, accumulate);
       if (le != cudaSuccess) return cuda_fail(le, "rmsnorm_dw_reduce launch");
       MCB_CHECK_LAUNCH("rmsnorm_dw_reduce");
@@ -630,7 +630,7 @@ int rmsnorm_bwd_t(const void* x, const void* w, const void* dy, void* dx, float*
   }
   MCB_CHECK_LAUNCH("rmsnorm_bwd");
   if (dw != nullptr) {
-    colsum_partials_kernel<<<(unsigned)((D + 31) / 32), 256, 0, st>>>((const float*)ws, dw, nblocks, (int)D,
+    colsum_partials_kernel<<<(unsigned)((D + 31) / 32), kColsumWarps * 32, 0, st>>>((const float*)ws, dw, nblocks, (int)D,
                                                                         accumulate);
     MCB_CHECK_LAUNCH("rmsnorm_dw_reduce");
   }
@@ -742,7 +742,7 @@ extern "C" int mcb_rmsnorm_bwd_ex(const void* x, const void* w, const void* dy, 
         : rowpipe::try_launch<__nv_bfloat16>(rowpipe::kRmsBwd, x, dy, w, dx, nullptr, dw ? (float*)workspace : nullptr,
                                              &blocks, rows, D, eps, 0, 1.0f, ds, st, dx_residual);
     if (rc == MCB_OK && dw != nullptr) {
-      colsum_partials_kernel<<<(unsigned)((D + 31) / 32), 256, 0, st>>>((const float*)workspace, dw, blocks, (int)D, accumulate);
+      colsum_partials_kernel<<<(unsigned)((D + 31) / 32), kColsumWarps * 32, 0, st>>>((const float*)workspace, dw, blocks, (int)D, accumulate);
       MCB_CHECK_LAUNCH("rmsnorm_dw_reduce");
     }
     if (rc != 1) return rc;
@@ -857,7 +857,7 @@ int rmsnorm_bwd_noalloc_t(const void* x, const void* w, const void* dy, void* dx
   MCB_CHECK_LAUNCH("rmsnorm_bwd_noalloc");
   if (dw != nullptr) {
     // every block wrote its whole row of partials above, so nothing stale from an earlier call is read
-    colsum_partials_kernel<<<(unsigned)((D + 31) / 32), 256, 0, st>>>(scratch, dw, nblocks, (int)D, accumulate);
+    colsum_partials_kernel<<<(unsigned)((D + 31) / 32), kColsumWarps * 32, 0, st>>>(scratch, dw, nblocks, (int)D, accumulate);
     MCB_CHECK_LAUNCH("rmsnorm_dw_reduce_noalloc");
   }
   return MCB_OK;
