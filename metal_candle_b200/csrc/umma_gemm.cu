@@ -617,7 +617,7 @@ int pick_bn(int64_t N, int rp) {
 // r64: 78.8 in the tiles against 72.7 us apart), the launch ahead X at 23 (HBM) and 9000 for its start.
 // 32768 x 4096 -> 4096 r16 forward, in the tiles / apart: 916 / 778 us (with the wide tiles that the main product then takes).
 bool rank_apart(const GemmCall& c, const DeviceState* ds) {
-  if (c.rp == 0 || c.Hr == nullptr || c.W == nullptr || c.Y == nullptr || c.swiglu_up != nullptr) return false;
+  if (c.rp == 0 || c.Hr == nullptr || c.W == nullptr || c.Y == nullptr || c.swiglu_up != nullptr || c.M < 1024) return false;
   GemmCall plain = c;
   plain.rp = 0;
   if (!gemm2_eligible(plain)) return false;

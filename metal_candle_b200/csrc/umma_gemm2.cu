@@ -566,7 +566,15 @@ int init_gemm2_kernel() {
 // with an output, large enough to fill CTA pairs; with a rank path, rank padded to a multiple of 16 and at
 // most 64 and a long enough reduction (MCB_OPT_PAIR_MIN_K; many tokens: 13/24 of it, 832 by default).
 bool gemm2_eligible(const GemmCall& c) {
-  if (c.W == nullptr || c.Y == nullptr || c.M < 1024 || c.N < 128 || c.K < 64) return false;
+  if (c.W == nullptr || c.Y == nullptr || c.N < 128 || c.K < 64) return false;
+  if (c.M < 1024) {
+    // Fewer tokens: only a plain product whose 128-token tiles pair up and take every CTA pair twice or more (the lm_head).  Its time is
+    // what an SM pulls from L2, a third less per tile on pairs.  One CTA / pairs, us: 512 x 896 -> 151936 136 / 120, 200 tokens 75 / 65, 400
+    // 132 / 115, 700 192 / 171, 900 251 / 222; 512 x 2048 -> 32000 69 / 54, 256 x 4096 -> 50264 110 / 95; but five tiles in three pairs, 640
+    // tokens, 166 / 168.
+    const int64_t tiles = (c.M + 127) / 128;
+    return c.rp == 0 && c.swiglu_up == nullptr && tiles % 2 == 0 && tiles / 2 * ((c.N + 255) / 256) >= 148;
+  }
   if (c.rp == 0) return true;
   if (c.rp % 16 != 0 || c.rp > 64) return false;
   const int64_t min_k = option(MCB_OPT_PAIR_MIN_K);

@@ -543,6 +543,17 @@ def test_bf16_linear_short_reduction_on_pairs(cuda_device, M, K, N, r):
     _linear_with_rank_path(cuda_device, M, K, N, r)
 
 
+# fewer than 1024 tokens and many outputs: CTA pairs from 148 tiles of 256 x 256 on where the 128-token tiles pair up (two, not three)
+@pytest.mark.parametrize("M,K,N", [(130, 72, 148 * 256), (256, 896, 148 * 256 - 248), (257, 200, 148 * 256), (1000, 136, 37 * 256)])
+def test_bf16_linear_few_tokens_many_outputs(cuda_device, M, K, N):
+    from metal_candle_b200 import backend as B
+
+    g = torch.Generator(device=cuda_device).manual_seed(M)
+    x, w, bias = ((torch.randn(*s, device=cuda_device, generator=g) * f).bfloat16() for s, f in (((M, K), 1.0), ((N, K), K ** -0.5), ((N,), 1.0)))
+    # one rounding to bf16 of sums whose operands are exact
+    _close_bf16(B.lora_linear_forward(x, w, bias, None, None, 1.0)[0], x.double() @ w.double().t() + bias.double(), 2.0 ** -8)
+
+
 def _linear_with_rank_path(cuda_device, M, K, N, r):
     from metal_candle_b200 import backend as B
 
