@@ -133,7 +133,7 @@ __device__ __forceinline__ uint32_t causal_bytes(int q, int elem_bytes, int row_
 // Two CTAs per SM wherever the registers allow it without heavy spilling (a 9-warp CTA pair needs <= 96
 // registers per thread, a 17-warp pair <= 56); the wide register-resident forms run one CTA per SM.
 __host__ __device__ constexpr int rowpipe_min_blocks(int op, int w, int elems_per_lane, bool two) {
-  if (two) return 3;
+  if (two) return elems_per_lane > 0 ? 2 : 3;
   if (op == kRmsFwd) return elems_per_lane > 0 ? 2 : 1;
   if (op == kSmFwd) return (elems_per_lane > 0 && (elems_per_lane <= 32 || w <= 8)) ? 2 : 1;
   if (op == kRmsBwd) return (w <= 8 && elems_per_lane <= 32) ? 2 : 1;
@@ -148,13 +148,15 @@ __host__ __device__ constexpr int rowpipe_min_blocks(int op, int w, int elems_pe
 // the row itself (forward ops) or the dw sums (rmsnorm backward with dw).  KMAX == 0: rows of any width,
 // streamed from shared memory twice.
 //
-// TWO (RMSNorm backward without dw, rows of 17 to 128 vectors): two rows share a warp, 16 lanes each.  A warp's fixed work per row
+// TWO (RMSNorm backward, rows of 17 to 128 vectors): two rows share a warp, 16 lanes each.  A warp's fixed work per row
 // (waits, two reductions, square root and division: some 300 instructions) is as much as its work on the three or four vectors a
 // lane has of 896 columns, and is done once for both; three CTAs of four such warps sit on an SM.  A lane keeps the sums of its even
 // and its odd vectors apart and adds them last, which is the order of the additions over 32 lanes: the results are the same bits.
 // One row / two rows per warp, us (bf16; with a residual in brackets): 32768 x 896 37.7 / 31.4 (39.1 / 32.7), 114688 x 896 113 / 104
 // (119 / 98), 8192 x 896 12.7 / 10.7, 2400 x 896 6.9 / 6.0, 100000 x 256 50.1 / 35.0, 20000 x 1000 26.6 / 24.1; float32 512 34.8 / 34.0.
-// The other operations are slower with two rows per warp: with dw (32 more accumulators a lane) 44.6 / 49.2, softmax 87024 x 777
+// With dw a lane has 64 accumulators instead of 32, and two CTAs fit an SM: worth it where the 32-lane form leaves its last round of
+// vectors part empty, 32768 x 896 44.8 / 41.4, 500000 x 896 478 / 419, 8192 x 896 19.4 / 17.7, 65536 x 1024 75.9 / 73.7; not at 768 columns (35.4 / 37.5),
+// with a residual (32768 x 896 50.7 / 56.4) or in float32 (512 columns 39.4 / 39.8).  Softmax is slower with two rows per warp, 87024 x 777
 // forward 50.0 / 55.1 and backward 65.6 / 72.7; the RMSNorm forward gains at 32768 x 896 (17.6 / 16.2) and loses at 100000 x 256 (18.4 / 22.0).
 template <typename T, int OP, int W, int KMAX, bool RAG, bool TWO>
 __global__ void __launch_bounds__((W + 1) * 32, rowpipe_min_blocks(OP, W, KMAX * Vec16<T>::N, TWO))
@@ -480,7 +482,7 @@ rowpipe_kernel(const Params p) {
           } else if constexpr (kDw) {
 #pragma unroll
             for (int k = 0; k < KMAX; ++k) {
-              const int vi = v_begin + lane + 32 * k;
+              const int vi = v_begin + l + kLanes * k;
               if (vi < v_end) body(vi, dwa[k]);
             }
           } else if (rrow != nullptr) {
@@ -759,11 +761,11 @@ rowpipe_kernel(const Params p) {
     __syncthreads();
     float* red = reinterpret_cast<float*>(gen_base);
     if (warp < W) {
-      const int rit = warp / p.wpr, seg = warp - rit * p.wpr;
+      const int rit = TWO ? 2 * warp + lane / 16 : warp / p.wpr, seg = TWO ? 0 : warp - rit * p.wpr;
       const int vseg = p.nvec / p.wpr, v_begin = seg * vseg, v_end = v_begin + vseg;
 #pragma unroll
       for (int k = 0; k < KMAX; ++k) {
-        const int vi = v_begin + lane + 32 * k;
+        const int vi = v_begin + (TWO ? lane & 15 : lane) + (TWO ? 16 : 32) * k;
         if (vi < v_end) {
 #pragma unroll
           for (int j = 0; j < N; ++j) red[rit * p.D + vi * N + j] = dwa[k][j];
@@ -878,21 +880,26 @@ int try_launch(int op, const void* in0, const void* in1, const void* w, void* ou
   }
   if (op != kRmsBwd) R = W;
   // Two rows per warp (see the kernel): enough of them for every SM to have several tiles, and two stages or more in a third of an SM
-  constexpr int kTwoWarps = 4, kTwoCtas = 3;
-  const int two_stages = static_cast<int>(std::min<int64_t>(kMaxStages, (227 * 1024 / kTwoCtas - 1024 - 1024 - w_bytes) / (2 * kTwoWarps * row_bytes * n_streams)));
-  const bool two = op == kRmsBwd && dw_part == nullptr && nvec > 16 && nvec <= 128 && two_stages >= 2 && rows >= 4ll * kTwoWarps * ds->sm_count;
+  constexpr int kTwoWarps = 4;
+  const int two_ctas = dw_part != nullptr ? 2 : 3;
+  const int two_stages = static_cast<int>(std::min<int64_t>(kMaxStages, (227 * 1024 / two_ctas - 1024 - 1024 - w_bytes) / (2 * kTwoWarps * row_bytes * n_streams)));
+  // with dw only wide bfloat16 rows without a residual (see the kernel)
+  const bool two = op == kRmsBwd && nvec > (dw_part != nullptr ? 96 : 16) && nvec <= 128 && two_stages >= 2 &&
+                   rows >= 4ll * kTwoWarps * ds->sm_count && (dw_part == nullptr || (sizeof(T) == 2 && res == nullptr));
   if (two) {
     W = kTwoWarps;
     R = 2 * kTwoWarps;
     wpr = 1;
     stages = two_stages;
   }
-  if (dw_part != nullptr) {
+  if (dw_part != nullptr && two) {
+    kmax = 8;
+  } else if (dw_part != nullptr) {
     const int need = (nvec / wpr + 31) / 32;
     kmax = need <= 1 ? 1 : need <= 2 ? 2 : need <= 4 ? 4 : need <= 8 ? 8 : need <= 16 ? 16 : 0;
     if (kmax == 0) return 1;
-    if (static_cast<int64_t>(R) * D * 4 > static_cast<int64_t>(stages) * R * row_bytes * n_streams) return 1;
   }
+  if (dw_part != nullptr && static_cast<int64_t>(R) * D * 4 > static_cast<int64_t>(stages) * R * row_bytes * n_streams) return 1;
   Params p;
   p.in0 = in0; p.in1 = in1; p.w = w; p.out = out; p.res = res; p.rstd = rstd; p.dw_part = dw_part;
   p.rows = rows; p.D = static_cast<int>(D); p.nvec = nvec; p.row_bytes = static_cast<int>(row_bytes);
@@ -909,9 +916,12 @@ int try_launch(int op, const void* in0, const void* in1, const void* w, void* ou
     smem = p.w_off + static_cast<size_t>(D) * 4 + 128;
   }
   const int64_t n_tiles = (rows + R - 1) / R;
-  int grid = (two ? kTwoCtas : 2) * ds->sm_count;
+  int grid = (two ? two_ctas : 2) * ds->sm_count;
   if (grid > n_tiles) grid = static_cast<int>(n_tiles);
   if (dw_blocks) *dw_blocks = grid;
+  if constexpr (sizeof(T) == 2) {
+    if (two && kmax == 8) return launch_one<T, kRmsBwd, kTwoWarps, 8, false, true>(p, grid, smem, st);
+  }
   if (two) return launch_one<T, kRmsBwd, kTwoWarps, 0, false, true>(p, grid, smem, st);
   if (rag) {
     if (op == kSmBwd) {
