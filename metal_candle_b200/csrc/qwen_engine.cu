@@ -470,6 +470,7 @@ extern "C" int mcb_qwen_set_exchange(mcb_qwen* q, mcb_comm* comm, void* side_str
 // time is how many WAVES of tiles the CTA pairs need.  Among the chunk sizes of 4096..12288 tokens (multiples of
 // 256) this returns the one with the fewest waves over all `tokens` (the smallest of those): 9472 for 32768 tokens
 // of width 896 on 148 SMs (37 x 4 = 148 tiles = two full waves; 8192 gives 128 tiles, a wave and three quarters).
+// (Wide tiles, 256 x 448 there, are half as many and as long: the same sizes fill their waves.)
 extern "C" int64_t mcb_ce_chunk_tokens(int64_t tokens, int64_t hidden) {
   if (tokens <= 0 || hidden <= 0) return 0;
   const DeviceState* ds = current_device_state();
