@@ -107,22 +107,33 @@ class _LayerCalls:
         # what the library's layer takes; other models and settings run kernel by kernel
         self.usable = (model.dtype == torch.bfloat16 and c.head_dim == 64 and c.intermediate_size % 8 == 0 and c.vocab_size % 8 == 0
                        and model.fuse_swiglu_bwd)
+        H, I = c.hidden_size, c.intermediate_size
+        self.norm_shape, self.qkv_width, self.qkv_offsets = (H,), H + 2 * c.kv_size, [0, H, H + c.kv_size]
+        self.shapes = {"q_proj": (H, H), "k_proj": (c.kv_size, H), "v_proj": (c.kv_size, H), "o_proj": (H, H), "gate_proj": (I, H),
+                       "up_proj": (I, H), "down_proj": (H, I)}   # [out, in]
         self.sizes: Dict[Tuple[int, int], Tuple[int, int]] = {}
         self.scratch = None
         self.shared = None    # without a backward to come, every layer uses the same block
 
-    def _tensors_ok(self, L, names) -> bool:
-        """The shapes and layouts the library's layer assumes (the call per kernel checks its own and reports)."""
-        c, dt = self.model.config, self.model.dtype
-        for name in ("input_layernorm", "post_attention_layernorm"):
-            if L[name].shape != (c.hidden_size,) or L[name].dtype != dt or not L[name].is_contiguous():
+    def _tensors_ok(self, L, fq) -> bool:
+        """Whether every tensor of the layer is where and what the library's layer assumes, whose sizes are the model's own: it
+        gets addresses and cannot look.  (Where not, the call per kernel checks its own and reports.)"""
+        dt = self.model.dtype
+        if fq["offsets"] != self.qkv_offsets:
+            return False
+        for w in (L["input_layernorm"], L["post_attention_layernorm"]):
+            if w.shape != self.norm_shape or w.dtype != dt or not w.is_contiguous() or not w.is_cuda:
                 return False
-        for name in names:
-            lin = L[name]
-            for w, shape in ((lin.weight, (lin.out_f, lin.in_f)), (lin.weight_t, (lin.in_f, lin.out_f))):
-                if w.shape != shape or w.dtype != dt or not w.is_contiguous() or not w.is_cuda:
+        for w, shape in ((fq["w"], (self.qkv_width, *self.norm_shape)), (fq["wt"], (*self.norm_shape, self.qkv_width)),
+                         (fq["bias"], (self.qkv_width,))):
+            if w.shape != shape or w.dtype != dt or not w.is_cuda:
+                return False
+        for name in self.model.MODULES[3:]:   # q, k and v are read from the stacked weight
+            lin, shape = L[name], self.shapes[name]
+            for w, want in ((lin.weight, shape), (lin.weight_t, shape[::-1])):
+                if w.shape != want or w.dtype != dt or not w.is_contiguous() or not w.is_cuda:
                     return False
-            if lin.bias is not None and name not in ("q_proj", "k_proj", "v_proj"):
+            if lin.bias is not None:
                 return False
         return True
 
@@ -135,9 +146,9 @@ class _LayerCalls:
         if fq is None:
             return None
         rank = next(l.lora for l in fq["lins"] if l.lora is not None).config.rank
-        w_gu = m._gate_up_weight(L)
-        if rank * 3 > 64 or not self._tensors_ok(L, ("o_proj", "gate_proj", "up_proj", "down_proj")):
+        if rank * 3 > 64 or not self._tensors_ok(L, fq):
             return None
+        w_gu = m._gate_up_weight(L)
         call = _lib.QwenLayerCall()
         mask = 0
         for i, name in enumerate(m.MODULES):
@@ -148,7 +159,8 @@ class _LayerCalls:
             if lora is None:
                 continue
             a, b = lora.lora_a, lora.lora_b
-            if (lora.config.scaling() != fq["scale"] or a.shape != (lin.in_f, rank) or b.shape != (rank, lin.out_f)
+            out_f, in_f = self.shapes[name]
+            if (lora.config.scaling() != fq["scale"] or a.shape != (in_f, rank) or b.shape != (rank, out_f)
                     or a.dtype != torch.float32 or b.dtype != torch.float32 or not (a.is_cuda and b.is_cuda)
                     or not (a.is_contiguous() and b.is_contiguous())):
                 return None

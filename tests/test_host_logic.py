@@ -262,3 +262,91 @@ def test_adamw_state_is_not_inherited_through_a_reused_address(launch_log):
     assert len(opt.state) == 50
     opt.zero_state()
     assert opt.state == {} and opt._held == {}
+
+
+class _OnDevice(torch.Tensor):
+    """A CPU tensor that says it is on the GPU."""
+
+    is_cuda = property(lambda self: True)
+
+
+def _layer_model():
+    """One layer with q and v adapters and nothing behind it but shapes: `prepare` launches nothing."""
+    from types import SimpleNamespace
+
+    from metal_candle_b200 import _lib
+    from metal_candle_b200.qwen import ModelConfig, Qwen
+
+    def dev(*shape, dtype=torch.bfloat16):
+        return torch.zeros(*shape, dtype=dtype).as_subclass(_OnDevice)
+
+    cfg = ModelConfig(vocab_size=320, hidden_size=256, intermediate_size=384, num_hidden_layers=1, num_attention_heads=4,
+                      num_key_value_heads=2, max_position_embeddings=256, rms_norm_eps=1e-6, rope_theta=1.0e6)
+    m = Qwen.__new__(Qwen)
+    m.config, m.dtype, m.device, m.lib = cfg, torch.bfloat16, torch.device("cpu"), _lib.load()
+    m.fuse_qkv = m.fuse_swiglu_bwd = True
+    L = {"input_layernorm": dev(256), "post_attention_layernorm": dev(256)}
+    for name, out, inp in (("q_proj", 256, 256), ("k_proj", 128, 256), ("v_proj", 128, 256), ("o_proj", 256, 256), ("gate_proj", 384, 256),
+                           ("up_proj", 384, 256), ("down_proj", 256, 384)):
+        lora = None
+        if name in ("q_proj", "v_proj"):
+            lora = SimpleNamespace(lora_a=dev(inp, 4, dtype=torch.float32), lora_b=dev(4, out, dtype=torch.float32), config=LoRAConfig(rank=4))
+        L[name] = SimpleNamespace(weight=dev(out, inp), weight_t=dev(inp, out), bias=dev(out) if name in ("q_proj", "k_proj", "v_proj") else None,
+                                  lora=lora, in_f=inp, out_f=out)
+    m.layers, m._on_device = [L], dev
+    return m, L
+
+
+def _wrong_norm(m, L):
+    L["input_layernorm"] = torch.ones(256, dtype=torch.bfloat16)
+
+
+def _wrong_second_norm(m, L):
+    L["post_attention_layernorm"] = torch.ones(256, dtype=torch.bfloat16)
+
+
+def _wrong_biases(m, L):
+    for name in ("q_proj", "k_proj", "v_proj"):
+        L[name].bias = torch.zeros(L[name].out_f, dtype=torch.bfloat16)
+
+
+def _float32_biases(m, L):
+    for name in ("q_proj", "k_proj", "v_proj"):
+        L[name].bias = m._on_device(L[name].out_f, dtype=torch.float32)
+
+
+def _short_bias(m, L):
+    L["q_proj"].bias = m._on_device(8)
+
+
+def _narrow_qkv(m, L):
+    for name in ("q_proj", "k_proj", "v_proj"):
+        L[name].weight = m._on_device(L[name].out_f, 128)
+
+
+def _shifted_qkv(m, L):
+    for name, out in (("q_proj", 128), ("k_proj", 256)):
+        L[name].weight, L[name].out_f = m._on_device(out, 256), out
+    L["q_proj"].lora.lora_b = m._on_device(4, 128, dtype=torch.float32)
+
+
+def _narrow_mlp(m, L):
+    for name in ("gate_proj", "up_proj"):
+        L[name].weight, L[name].weight_t, L[name].out_f = m._on_device(256, 256), m._on_device(256, 256), 256
+
+
+# A layer goes to the library as addresses: whatever the calls per kernel refuse or read by its own shape has to stay with them.
+@pytest.mark.parametrize("spoil", [None, _wrong_norm, _wrong_second_norm, _wrong_biases, _float32_biases, _short_bias, _narrow_qkv, _shifted_qkv,
+                                   _narrow_mlp], ids=lambda f: f.__name__ if f else "sound")
+def test_layer_call_takes_only_tensors_of_the_layers_own_shape_and_device(monkeypatch, spoil):
+    from metal_candle_b200 import backend
+    from metal_candle_b200.qwen import _LayerCalls
+
+    monkeypatch.setattr(backend, "transpose_2d", lambda w: w.t().contiguous())
+    monkeypatch.setattr(backend, "interleave_gate_up", lambda g, u: torch.cat([g, u], 0))
+    m, L = _layer_model()
+    if spoil is not None:
+        spoil(m, L)
+    calls = _LayerCalls(m, 1, 16, backward=False)
+    prepared = calls.prepare(0)
+    assert (prepared is None) == (spoil is not None)
