@@ -1,10 +1,10 @@
 // float32 path of the fused LoRA linear.  tcgen05 has no float32 MMA and a single TF32 pass cannot hold the 1e-4 bound against
-// the reference's f32 CPU arithmetic; six bfloat16 products of operands cut into three parts each can, and hold float32's own
-// rounding (tile_kernel).  The kernels of kernel:
+// the reference's f32 CPU arithmetic; eight bfloat16 products of operands taken apart into three parts each can, with a smaller error
+// than a chain of float32 FMAs (tile_kernel).  The kinds of kernel:
 //
 //   tile_kernel    C = A B (+ bias) (+ residual) with the rank-r update as extra reduction steps, on the tensor cores: 128 x
 //                  128 (64) tiles, the reduction split over the CTAs of a cluster when a shape has too few tiles for the chip
-//   short_kernel   the same for reductions of at most 64, on the FMA pipes
+//   short_kernel   the same for reductions of at most 32, on the FMA pipes
 //   rank_kernel    the [M, r] intermediates scale * x A and scale * dy B^T
 //   grad_kernel    dA and dB, reductions over tokens
 //   lora_delta_cluster_kernel   scale * (x A) B of few tokens in one launch (also for bfloat16 x)
@@ -39,41 +39,41 @@ struct TileParams {
   int* status;
 };
 
-// The tensor cores take bfloat16, whose eight significant bits are a third of float32's: x = h + m + l, each part the
-// upper half of the bits that the parts before it left over (cut off, not rounded, so that every remainder is exact); the
-// three hold all 24 bits.  Both operands are scaled by 2^24 first, so that the parts of the smallest normal numbers are
-// normal themselves; what overflows for it (operands beyond 2^103, products beyond 2^79) is computed again, see below.  Of the nine
-// products of the parts the six largest are taken; the other three are below 2^-23 of the product.
+// The tensor cores take bfloat16, whose eight significant bits are a third of float32's: x = h + m + l, each part what is left
+// of x rounded to nearest bfloat16.  A remainder is at most half a unit of the part before it, so the three hold all 24 bits,
+// and it has either sign, so that nothing that is left out of a product adds up over many of them.  Both operands are scaled by 2^24
+// first, so that the parts of the smallest normal numbers are normal themselves; what overflows for it (operands beyond 2^103,
+// products beyond 2^79) is computed again, see plain_element.  Of the nine products of the parts l x l alone is left out: below 2^-33 of
+// the product, where one float32 rounding is up to 2^-24.
 constexpr int kTileM = 128, kStep = 64, kStages = 2, kParts = 3, kMaxSplits = 8;
-constexpr int kTileWarps = 16, kTileThreads = 32 * kTileWarps;
+constexpr int kSumWarps = 8, kCopyWarps = 7, kCopyThreads = 32 * kCopyWarps, kTileThreads = 32 * kSumWarps + kCopyThreads + 32;
 constexpr float kPartScale = 16777216.0f, kPartUnscale = 1.0f / 16777216.0f / 16777216.0f;
 
 template <int BN>
 struct TileSmem {
   static constexpr uint32_t kPlaneA = kTileM * kStep * 2, kPlaneB = BN * kStep * 2;
   static constexpr uint32_t kStage = kParts * (kPlaneA + kPlaneB), kBars = kStages * kStage;
-  static constexpr size_t kBytes = kBars + 64 + 1024;
+  static constexpr size_t kBytes = kBars + 128 + 1024;
   static constexpr int kOutPitch = BN + 4;   // the output tile reuses the stages; rows four banks apart
   static_assert(kTileM * kOutPitch * 4 <= kBars, "output tile");
 };
 
-__device__ __forceinline__ uint32_t upper_halves(float a, float b) {
-  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+// two values rounded to bfloat16 (the first in the lower half), and what the rounding left of them
+__device__ __forceinline__ uint32_t take_part(float2& x) {
+  const __nv_bfloat162 r = __float22bfloat162_rn(x);
+  const uint32_t w = *reinterpret_cast<const uint32_t*>(&r);
+  x = __ffma2_rn(make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)), make_float2(-1.0f, -1.0f), x);
+  return w;
 }
-__device__ __forceinline__ float cut(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
-// the three parts of eight values, 16 bytes each, `plane` bytes apart
-__device__ __forceinline__ void store_parts(uint8_t* dst, uint32_t plane, const float (&v)[8]) {
-  uint32_t w[kParts][4];
+// the three parts of four values, 8 bytes each, `plane` bytes apart
+__device__ __forceinline__ void store_parts(uint8_t* dst, uint32_t plane, const float4& v) {
+  const float2 scale = make_float2(kPartScale, kPartScale);
+  float2 x = __fmul2_rn(make_float2(v.x, v.y), scale), y = __fmul2_rn(make_float2(v.z, v.w), scale);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 x = __fmul2_rn(make_float2(v[2 * i], v[2 * i + 1]), make_float2(kPartScale, kPartScale));
-    const float2 x1 = make_float2(x.x - cut(x.x), x.y - cut(x.y));
-    w[0][i] = upper_halves(x.x, x.y);
-    w[1][i] = upper_halves(x1.x, x1.y);
-    w[2][i] = upper_halves(x1.x - cut(x1.x), x1.y - cut(x1.y));
+  for (int s = 0; s < kParts; ++s) {
+    const uint32_t lo = take_part(x), hi = take_part(y);
+    *reinterpret_cast<uint2*>(dst + s * plane) = make_uint2(lo, hi);
   }
-#pragma unroll
-  for (int s = 0; s < kParts; ++s) *reinterpret_cast<uint4*>(dst + s * plane) = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
 }
 
 __device__ __forceinline__ bool is_k_major(const Operand& o) { return o.sk == 1; }
@@ -81,59 +81,61 @@ __device__ __forceinline__ bool is_vec(const Operand& o) {
   return (reinterpret_cast<uintptr_t>(o.p) & 15u) == 0 && ((o.sk == 1 ? o.sr : o.sk) & 3) == 0;
 }
 
-// One step's tile of an operand, ROWS x 64 reduction indices, as ROWS * 8 pieces of eight neighbouring values dealt out to
-// the threads.  In shared memory, per part: k contiguous: rows of 128 bytes (64 k); rows contiguous: blocks of 64 rows, each
-// 64 k of 128 bytes; the 16-byte pieces of a line in 128-byte swizzle order either way, and eight lanes write one line.
-template <int ROWS>
+// One step's tile of an operand, ROWS x 64 reduction indices, as ROWS * 16 pieces of four neighbouring values dealt out to THREADS
+// threads.  In shared memory, per part: k contiguous: rows of 128 bytes (64 k); rows contiguous: blocks of 64 rows, each
+// 64 k of 128 bytes; the 16-byte groups of a line in 128-byte swizzle order either way.  Half a warp reads 256 neighbouring bytes and
+// writes a line.
+template <int ROWS, int THREADS>
 struct Copy {
-  static constexpr int kPieces = ROWS * 8 / kTileThreads;
-  float v[kPieces][8];
-  __device__ __forceinline__ static void place(bool k_major, int i, int& row, int& k, uint32_t& at) {
-    const int u = threadIdx.x + i * kTileThreads;
-    if (k_major) {
-      row = u >> 3; k = (u & 7) * 8;
-      at = row * 128 + (((u & 7) ^ (row & 7)) << 4);
-    } else {
-      const int c = u % (ROWS / 8);
-      k = u / (ROWS / 8); row = c * 8;
-      at = (c >> 3) * (kStep * 128) + k * 128 + (((c & 7) ^ (k & 7)) << 4);
-    }
-  }
+  static constexpr int kTotal = ROWS * 16, kPieces = (kTotal + THREADS - 1) / THREADS;
+  static constexpr int kHop = THREADS / 16, kHopAcross = THREADS / (ROWS / 4);   // lines from a thread's piece to its next
+  static_assert(THREADS % 16 == 0 && THREADS % (ROWS / 4) == 0, "a thread keeps its place in the line");
+  float4 v[kPieces];
+  // line (row, or index k if the rows are contiguous) of piece i of thread t, and its place in it, in values
+  __device__ __forceinline__ static int line_of(bool k_major, int t, int i) { return k_major ? (t >> 4) + i * kHop : t / (ROWS / 4) + i * kHopAcross; }
+  __device__ __forceinline__ static int at_of(bool k_major, int t) { return (k_major ? t & 15 : t % (ROWS / 4)) * 4; }
+  __device__ __forceinline__ static bool has(int t, int i) { return (i + 1) * THREADS <= kTotal || t + i * THREADS < kTotal; }
   // rows [row0, row0 + ROWS) and indices [k0, k0 + 64); zeros beyond `rows` and `kend`
-  __device__ __forceinline__ void load(const Operand& o, int row0, int rows, int k0, int kend) {
+  __device__ __forceinline__ void load(const Operand& o, int t, int row0, int rows, int k0, int kend) {
     const bool k_major = is_k_major(o);
-    const float* p = from_here(o.p) + (k_major ? row0 * o.sr + k0 : k0 * o.sk + row0);
     const int64_t pitch = k_major ? o.sr : o.sk;
+    const int line0 = k_major ? row0 : k0, lines = k_major ? rows : kend, at = (k_major ? k0 : row0) + at_of(k_major, t), end = k_major ? kend : rows;
+    const float* q = from_here(o.p) + (line0 + line_of(k_major, t, 0)) * pitch + at;
+    const int64_t hop = (k_major ? kHop : kHopAcross) * pitch;
     if (is_vec(o) && row0 + ROWS <= rows && k0 + kStep <= kend) {
 #pragma unroll
-      for (int i = 0; i < kPieces; ++i) {
-        int row, k;
-        uint32_t at;
-        place(k_major, i, row, k, at);
-        const float4* q = reinterpret_cast<const float4*>(p + (k_major ? row * pitch + k : k * pitch + row));
-        *reinterpret_cast<float4*>(v[i]) = __ldg(q);
-        *reinterpret_cast<float4*>(v[i] + 4) = __ldg(q + 1);
-      }
+      for (int i = 0; i < kPieces; ++i, q += hop)
+        if (has(t, i)) v[i] = __ldg(reinterpret_cast<const float4*>(q));
     } else {
 #pragma unroll
-      for (int i = 0; i < kPieces; ++i) {
-        int row, k;
-        uint32_t at;
-        place(k_major, i, row, k, at);
-        const float* q = p + (k_major ? row * pitch + k : k * pitch + row);
-        const int left = (k_major ? row0 + row < rows : k0 + k < kend) ? (k_major ? kend - k0 - k : rows - row0 - row) : 0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[i][j] = j < left ? __ldg(q + j) : 0.0f;
+      for (int i = 0; i < kPieces; ++i, q += hop) {
+        const int left = has(t, i) && line0 + line_of(k_major, t, i) < lines ? end - at : 0;
+        v[i].x = left > 0 ? __ldg(q) : 0.0f;
+        v[i].y = left > 1 ? __ldg(q + 1) : 0.0f;
+        v[i].z = left > 2 ? __ldg(q + 2) : 0.0f;
+        v[i].w = left > 3 ? __ldg(q + 3) : 0.0f;
       }
     }
   }
-  __device__ __forceinline__ void store(uint8_t* dst, uint32_t plane, bool k_major, int kn) const {
+  // the parts of the indices below kn (nobody reads beyond the step's last 16); a whole step without a branch, so that the pieces'
+  // dependent instructions run side by side (2048 x 1536 x 1536 111 -> 102 us)
+  template <bool K_MAJOR, bool WHOLE>
+  __device__ __forceinline__ void store_as(uint8_t* dst, uint32_t plane, int t, int kn) const {
+    const int at = at_of(K_MAJOR, t), group = (at & 63) >> 3;
+    dst += (K_MAJOR ? 0 : (at >> 6) * (kStep * 128)) + (at & 4) * 2;
 #pragma unroll
     for (int i = 0; i < kPieces; ++i) {
-      int row, k;
-      uint32_t at;
-      place(k_major, i, row, k, at);
-      if (k < kn) store_parts(dst + at, plane, v[i]);   // nobody reads beyond the step's last 16 indices
+      const int line = line_of(K_MAJOR, t, i);
+      if (has(t, i) && (WHOLE || (K_MAJOR ? at : line) < kn)) store_parts(dst + line * 128 + ((group ^ (line & 7)) << 4), plane, v[i]);
+    }
+  }
+  __device__ __forceinline__ void store(uint8_t* dst, uint32_t plane, bool k_major, int t, int kn) const {
+    if (kn == kStep) {
+      if (k_major) store_as<true, true>(dst, plane, t, kn);
+      else store_as<false, true>(dst, plane, t, kn);
+    } else {
+      if (k_major) store_as<true, false>(dst, plane, t, kn);
+      else store_as<false, false>(dst, plane, t, kn);
     }
   }
 };
@@ -147,12 +149,22 @@ __device__ __noinline__ float plain_element(const TileParams& p, int m, int n) {
   return s;
 }
 
-// A step of 64 reduction indices: the threads cut the values they loaded a step earlier into parts (two stages of shared
-// memory), one thread issues the six products, and meanwhile all add the step before's accumulator to float32 sums in
-// registers: the tensor core cuts its running sum off where float32 rounds to nearest, so a sum stays in it for one step only
-// (relative error to float64 of 512 x 768 x 768 1.4e-7, of the float32 FMAs before 1.9e-7; of 2048 x 1536 x 1536 1.5e-7, 2.6e-7).
-// Bound: the tensor pipe, 12 BN cycles a step, behind a CTA's start and the exchange of partial tiles.  A shape with few
-// tiles (512 x 768 x 768: 24) leaves SMs idle, so up to 8 CTAs of a cluster share a tile's reduction and add their
+// A step of 64 reduction indices: seven warps take the values they loaded a step earlier apart (two stages of shared memory), one issues
+// the products, and eight add the step before's accumulators to float32 sums in registers (having taken their half of the first step).
+// The tensor core adds an MMA's 16 products and its accumulator exactly down to 2^-25 of the largest of them and cuts the rest off, always
+// towards zero, where float32 rounds to nearest: terms of one sign lose half a unit of the sum with every MMA that adds to it.
+// So the h x h products, which make the sum, get an accumulator for every 16 indices (16 products of eight bits by eight fit the 24 bits
+// of a sum but for their smallest terms); the seven small ones, whose cut-off is 2^-8 of that, share one.
+// Relative error to float64, in brackets that of float32 FMAs split likewise and of six products of cut parts in one accumulator per step:
+//   512 x 768 x 768      normal 7.3e-8 (1.9e-7, 1.3e-7)   uniform(0, 1) 4.8e-8 (7.0e-8, 1.2e-7)   uniform(1, 2) 4.1e-8 (6.7e-8, 9.7e-8)
+//   300 x 65 x 200              5.5e-8 (1.4e-7, 1.2e-7)                 5.1e-8 (1.2e-7, 1.2e-7)                 4.6e-8 (1.2e-7, 9.8e-8)
+//   2048 x 1536 x 1536          8.8e-8 (2.5e-7, 1.4e-7)                 5.3e-8 (8.7e-8, 1.2e-7)                 4.7e-8 (8.3e-8, 9.9e-8)
+// and the mean deviation of positive terms is -1e-8 to -2e-8 (0, -1e-7).  Larger than the FMAs' where one term of a short sum dwarfs the
+// others, whose last bits it pushes out: exp(2 normal), 65 indices 1.8e-7 (1.0e-7, 7.4e-7), 768 indices 1.4e-7 (1.5e-7, 4.8e-7).
+// Bound: taking the values apart (about 4800 cycles a step of seven warps; the products are 16 BN), then a CTA's start and the exchange of
+// partial tiles.  us, FMAs / six products / this: 512 x 768 x 768 29 / 14.5 / 14.9, 2048 x 1536 x 1536 254 / 105 / 97, 64 x 256 x 128
+// 14.7 / 12.0 / 11.6.  (All 16 warps at everything, a barrier a half step: 18.5 and 151; one warp issuing beside its other work: 16.9 and 133.)
+// A shape with few tiles (512 x 768 x 768: 24) leaves SMs idle, so up to 8 CTAs of a cluster share a tile's reduction and add their
 // partial tiles through distributed shared memory, in rank order: deterministic, no workspace.
 template <int BN>
 __global__ void __launch_bounds__(kTileThreads, 1) tile_kernel(const __grid_constant__ TileParams p) {
@@ -160,18 +172,28 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_kernel(const __grid_cons
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t acc_full0 = base + S::kBars, tmem_slot = acc_full0 + 16;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (known to be the warp's, not a lane's)
+  const uint32_t stage_free0 = base + S::kBars, parts_ready0 = stage_free0 + 8 * kStages, high_full = parts_ready0 + 8 * kStages, high_read = high_full + 8;
+  const uint32_t all_full = high_read + 8, low_read = all_full + 8, first_ready = low_read + 8, tmem_slot = first_ready + 8;
   volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(gen + (tmem_slot - base));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + (tmem_slot + 4 - base));
 
   if (threadIdx.x == 0) {
-    for (int a = 0; a < 2; ++a) mbar_init(acc_full0 + 8 * a, 1);
+    // a barrier per stage where one side can be a stage ahead of the other: a wait tells a phase from the next one only
+    for (int a = 0; a < kStages; ++a) {
+      mbar_init(stage_free0 + 8 * a, 1);
+      mbar_init(parts_ready0 + 8 * a, kCopyWarps);
+    }
+    mbar_init(high_full, 1);
+    mbar_init(all_full, 1);
+    mbar_init(high_read, kSumWarps);
+    mbar_init(low_read, kSumWarps);
+    mbar_init(first_ready, kSumWarps);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async_smem();
   }
-  constexpr uint32_t kCols = 2 * BN;
+  constexpr uint32_t kCols = 4 * BN;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(kCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -191,75 +213,152 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_kernel(const __grid_cons
   const int main_steps = s_end - s_begin;
   const int steps = main_steps + (split == 0 ? (p.R + kStep - 1) / kStep : 0);
 
-  Copy<kTileM> ca;
-  Copy<BN> cb;
-  auto load_step = [&](int s) {
-    const bool main = s < main_steps;
-    const int k0 = (main ? s_begin + s : s - main_steps) * kStep, kend = main ? p.K : p.R;
-    ca.load(main ? p.a : p.ra, m0, p.M, k0, kend);
-    cb.load(main ? p.b : p.rb, n0, p.N, k0, kend);
-  };
-  // a thread's outputs: row 32 (warp % 4) + lane, BN / 4 columns from (warp / 4) BN / 4 on
-  const int quad = warp & 3, col0 = (warp >> 2) * (BN / 4);
-  float sum[BN / 4];
-#pragma unroll
-  for (int i = 0; i < BN / 4; ++i) sum[i] = 0.0f;
-  load_step(0);
-  for (int s = 0; s <= steps; ++s) {
-    if (s < steps) {
-      // Stage and accumulator s % 2 are free: every thread has waited for step s - 2's products and read their sums.
-      const bool main = s < main_steps, ak = is_k_major(main ? p.a : p.ra), bk = is_k_major(main ? p.b : p.rb);
-      const int left = main ? p.K - (s_begin + s) * kStep : p.R - (s - main_steps) * kStep;
-      const int k16 = (min(left, kStep) + 15) >> 4;   // the MMAs' reduction is 16 long
+  // Four accumulators take turns: step s has number s % 4 for all small products, the next three for the h x h products of its second to
+  // last 16 indices; the first 16 go to the last of the three where it is free (a short step, as of a rank), else to the small products.
+  // The three are filled between the small products' halves: they are read under the second half, the first accumulator under the next
+  // step's first half, and either is free when its turn comes without the tensor pipe having waited.
+  auto indices = [&](int s) { return min(kStep, s < main_steps ? p.K - (s_begin + s) * kStep : p.R - (s - main_steps) * kStep); };
+  auto wait = [&](uint32_t bar, int n, int code) { return __all_sync(0xffffffffu, mbar_wait(bar, n & 1, abort_flag, code, p.status)) != 0; };
+  if (warp >= kSumWarps && warp < kSumWarps + kCopyWarps) {
+    // ---------------- copy ----------------
+    // (tb: what is left over of either operand goes to another warp)
+    const int t = threadIdx.x - 32 * kSumWarps, tb = t >= 96 ? t - 96 : t + kCopyThreads - 96;
+    Copy<kTileM, kCopyThreads> ca;
+    Copy<BN, kCopyThreads> cb;
+    auto load_a = [&](int s) {
+      const bool main = s < main_steps;
+      ca.load(main ? p.a : p.ra, t, m0, p.M, (main ? s_begin + s : s - main_steps) * kStep, main ? p.K : p.R);
+    };
+    auto load_b = [&](int s) {
+      const bool main = s < main_steps;
+      cb.load(main ? p.b : p.rb, tb, n0, p.N, (main ? s_begin + s : s - main_steps) * kStep, main ? p.K : p.R);
+    };
+    load_a(0);
+    if (steps > 1) load_b(1);   // step 0's is the sum warps', which have nothing to add yet
+    for (int s = 0; s < steps; ++s) {
+      const bool main = s < main_steps;
+      const int kn = (indices(s) + 15) & ~15;   // the MMAs' reduction is 16 long
       uint8_t* dst = gen + (s & 1) * S::kStage;
-      ca.store(dst, S::kPlaneA, ak, 16 * k16);
-      cb.store(dst + kParts * S::kPlaneA, S::kPlaneB, bk, 16 * k16);
+      if (s >= kStages && !wait(stage_free0 + 8 * (s & 1), (s >> 1) - 1, 100)) break;
+      ca.store(dst, S::kPlaneA, is_k_major(main ? p.a : p.ra), t, kn);
+      if (s > 0) cb.store(dst + kParts * S::kPlaneA, S::kPlaneB, is_k_major(main ? p.b : p.rb), tb, kn);
       fence_proxy_async_smem();
-      if (s + 1 < steps) load_step(s + 1);
-      tcgen05_fence_before();
-      __syncthreads();
-      if (threadIdx.x == 0 && *abort_flag == 0) {
-        tcgen05_fence_after();
-        const uint32_t idesc = make_idesc(BN) | (ak ? 0u : 1u << 15) | (bk ? 0u : 1u << 16);
-        const uint32_t pa = base + (s & 1) * S::kStage, pb = pa + kParts * S::kPlaneA, acc = tmem_base + (s & 1) * BN;
-        // 16 reduction indices further: 32 bytes along a line, or two groups of eight lines
-        const uint64_t da0 = ak ? desc_sw128(pa) : desc_sw128_mn(pa, kStep * 128, 1024);
-        const uint64_t db0 = bk ? desc_sw128(pb) : desc_sw128_mn(pb, kStep * 128, 1024);
-        const uint32_t ja = ak ? 32 : 2048, jb = bk ? 32 : 2048;
-        // smallest products first, so that what the running sum loses to them is small
-        constexpr int kA[6] = {2, 0, 1, 1, 0, 0}, kB[6] = {0, 2, 1, 0, 1, 0};
-        uint32_t add = 0;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(parts_ready0 + 8 * (s & 1));
+      if (s + 1 < steps) {
+        load_a(s + 1);
+        if (s > 0) load_b(s + 1);
+      }
+    }
+  } else if (warp >= kSumWarps) {
+    // ---------------- MMA issuer ----------------
+    // Smallest products first, so that what the running sum loses to them is small.
+    for (int s = 0; s < steps; ++s) {
+      constexpr int kA[7] = {2, 1, 2, 0, 1, 1, 0}, kB[7] = {1, 2, 0, 2, 1, 0, 1};
+      const bool main = s < main_steps, ak = is_k_major(main ? p.a : p.ra), bk = is_k_major(main ? p.b : p.rb);
+      const uint32_t idesc = make_idesc(BN) | (ak ? 0u : 1u << 15) | (bk ? 0u : 1u << 16);
+      const uint32_t pa = base + (s & 1) * S::kStage, pb = pa + kParts * S::kPlaneA, acc = tmem_base + (s & 3) * BN;
+      // 16 reduction indices further: 32 bytes along a line, or two groups of eight lines
+      const uint64_t da0 = ak ? desc_sw128(pa) : desc_sw128_mn(pa, kStep * 128, 1024);
+      const uint64_t db0 = bk ? desc_sw128(pb) : desc_sw128_mn(pb, kStep * 128, 1024);
+      const uint32_t ja = ak ? 32 : 2048, jb = bk ? 32 : 2048;
+      const int k16 = (indices(s) + 15) >> 4;   // the MMAs' reduction is 16 long
+      auto product = [&](uint32_t d, int qa, int qb, int k, uint32_t add) {
+        umma_bf16(d, desc_advance(da0, qa * S::kPlaneA + k * ja), desc_advance(db0, qb * S::kPlaneB + k * jb), idesc, add);
+      };
+      if (!wait(parts_ready0 + 8 * (s & 1), s >> 1, 101) || !(s > 0 ? wait(high_read, s - 1, 102) : wait(first_ready, 0, 102))) break;
+      tcgen05_fence_after();
+      if (elect_one()) {
 #pragma unroll
-        for (int q = 0; q < 6; ++q)
-          for (int k = 0; k < k16; ++k) {
-            umma_bf16(acc, desc_advance(da0, kA[q] * S::kPlaneA + k * ja), desc_advance(db0, kB[q] * S::kPlaneB + k * jb), idesc, add);
-            add = 1;
-          }
-        umma_commit(acc_full0 + 8 * (s & 1));
+        for (int k = 0; k < 4; ++k) {
+          if (k >= k16) break;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) product(acc, kA[q], kB[q], k, q + k > 0);
+        }
+      }
+      __syncwarp();
+      if (s > 0 && !wait(low_read, s - 1, 103)) break;
+      tcgen05_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 1; k < 4; ++k)
+          if (k < k16) product(tmem_base + ((s + k) & 3) * BN, 0, 0, k, 0);
+        if (k16 < 4) product(tmem_base + ((s + 3) & 3) * BN, 0, 0, 0, 0);
+        umma_commit(high_full);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (k >= k16) break;
+#pragma unroll
+          for (int q = 4; q < 7; ++q) product(acc, kA[q], kB[q], k, 1);
+        }
+        if (k16 == 4) product(acc, 0, 0, 0, 1);
+        umma_commit(all_full);
+        umma_commit(stage_free0 + 8 * (s & 1));
       }
       __syncwarp();
     }
-    if (s > 0) {
-      const int d = s - 1;
-      if (__all_sync(0xffffffffu, mbar_wait(acc_full0 + 8 * (d & 1), (d >> 1) & 1, abort_flag, 100, p.status))) {
-        tcgen05_fence_after();
-        const uint32_t t = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + (d & 1) * BN + col0;
+  }
+  // the sums: row 32 (warp % 4) + lane, BN / 2 columns from (warp / 4) BN / 2 on
+  const int quad = warp & 3, col0 = (warp >> 2) * (BN / 2);
+  if (warp < kSumWarps) {
+    const uint32_t own = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + col0;
+    {
+      Copy<BN, 32 * kSumWarps> first;
+      first.load(p.b, threadIdx.x, n0, p.N, s_begin * kStep, p.K);
+      first.store(gen + kParts * S::kPlaneA, S::kPlaneB, is_k_major(p.b), threadIdx.x, (indices(0) + 15) & ~15);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(first_ready);
+    }
+    float sum[BN / 2];
 #pragma unroll
-        for (int c = 0; c < BN / 4; c += 16) {
-          uint32_t v[16];
-          tmem_ld_x16(t + c, v);
-          tmem_ld_wait();
+    for (int i = 0; i < BN / 2; ++i) sum[i] = 0.0f;
+    auto arrive = [&](uint32_t bar) {
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    for (int s = 0; s < steps; ++s) {
+      const int k16 = (indices(s) + 15) >> 4;
+      if (!wait(high_full, s, 104)) break;
+      tcgen05_fence_after();
 #pragma unroll
-          for (int i = 0; i < 16; ++i) sum[c + i] += __uint_as_float(v[i]);
+      for (int c = 0; c < BN / 2; c += 16) {
+        uint32_t x[16], y[16], z[16];
+        tmem_ld_x16(own + ((s + 3) & 3) * BN + c, z);
+        if (k16 > 1) tmem_ld_x16(own + ((s + 1) & 3) * BN + c, x);
+        if (k16 > 2) tmem_ld_x16(own + ((s + 2) & 3) * BN + c, y);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+          float2 t = make_float2(__uint_as_float(z[i]), __uint_as_float(z[i + 1]));
+          if (k16 > 1) t = __fadd2_rn(t, make_float2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])));
+          if (k16 > 2) t = __fadd2_rn(t, make_float2(__uint_as_float(y[i]), __uint_as_float(y[i + 1])));
+          t = __fadd2_rn(t, make_float2(sum[c + i], sum[c + i + 1]));
+          sum[c + i] = t.x;
+          sum[c + i + 1] = t.y;
         }
       }
-    }
-  }
-  // every product has been waited for: nothing reads the stages any more
-  __syncthreads();
-  float* out = reinterpret_cast<float*>(gen) + (quad * 32 + lane) * S::kOutPitch + col0;
+      arrive(high_read);
+      if (!wait(all_full, s, 105)) break;
+      tcgen05_fence_after();
 #pragma unroll
-  for (int i = 0; i < BN / 4; i += 4) *reinterpret_cast<float4*>(out + i) = make_float4(sum[i], sum[i + 1], sum[i + 2], sum[i + 3]);
+      for (int c = 0; c < BN / 2; c += 32) {
+        uint32_t x[32];
+        tmem_ld_x16(own + (s & 3) * BN + c, *reinterpret_cast<uint32_t(*)[16]>(&x[0]));
+        tmem_ld_x16(own + (s & 3) * BN + c + 16, *reinterpret_cast<uint32_t(*)[16]>(&x[16]));
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) sum[c + i] += __uint_as_float(x[i]);
+      }
+      arrive(low_read);
+    }
+    // every product has been waited for: nothing reads the stages any more
+    float* out = reinterpret_cast<float*>(gen) + (quad * 32 + lane) * S::kOutPitch + col0;
+#pragma unroll
+    for (int i = 0; i < BN / 2; i += 4) *reinterpret_cast<float4*>(out + i) = make_float4(sum[i], sum[i + 1], sum[i + 2], sum[i + 3]);
+  }
+  __syncwarp();
   if (*abort_flag != 0) {
     for (int k = 0; k < 200; ++k) __nanosleep(1000);
   }
@@ -286,10 +385,14 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_kernel(const __grid_cons
     for (int q = 0; q < kMaxSplits; ++q)
       if (q < p.splits)
         part[q] = *reinterpret_cast<const float4*>((p.splits > 1 ? cl.map_shared_rank(tile_out, q) : tile_out) + r * S::kOutPitch + c);
+    // the rank update, which can be most of the output, comes with the first part: added last, it is rounded once
     float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-    for (int q = 0; q < kMaxSplits; ++q)
-      if (q < p.splits) { v[0] += part[q].x; v[1] += part[q].y; v[2] += part[q].z; v[3] += part[q].w; }
+    for (int q = 1; q <= kMaxSplits; ++q)
+      if (q < p.splits || q == kMaxSplits) {
+        const float4 t = part[q % kMaxSplits];
+        v[0] += t.x; v[1] += t.y; v[2] += t.z; v[3] += t.w;
+      }
     const int64_t o = gm * p.cm + gn * p.cn;
     const int live = min(4, p.N - gn);
 #pragma unroll
@@ -313,10 +416,10 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_kernel(const __grid_cons
 }
 
 // ---- short reductions ----------------------------------------------------------------------------------------------
-// The same product where K and R are at most 64: with so few terms, plain float32 FMAs round less than the tensor cores' cut-off
-// sums (1024 x 8 x 512: 3e-8 of the result against 9e-8), and there is no reduction to speed up.
+// The same product where K and R are at most 32, with float32 FMAs: there is no reduction to speed up.  (With 64 terms they err by 1.4e-7
+// and tile_kernel by 4.9e-8, in 112 and 65 us at 4096 x 64 x 4096.)
 // Bound: writing C.  A CTA holds both operands' 64 rows whole; a thread owns 8 x 4 outputs.
-constexpr int kShort = 64, kShortThreads = 128, kShortPitch = kShort + 4;
+constexpr int kShort = 64, kShortTerms = 32, kShortThreads = 128, kShortPitch = kShort + 4;
 __global__ void __launch_bounds__(kShortThreads) short_kernel(const __grid_constant__ TileParams p) {
   __shared__ __align__(16) float sa[32][kShortPitch], sb[32][kShortPitch];   // [k][row], half of the reduction at a time
   const int m0 = (blockIdx.x / p.n_tiles) * kShort, n0 = (blockIdx.x % p.n_tiles) * kShort;
@@ -613,9 +716,9 @@ int launch_delta(const LoraArgs& a) {
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------------
-// CTAs that share a tile's reduction (0: no cluster of that size fits the device).  In cycles: a step of 64 reduction
-// indices keeps the tensor pipe for 12 BN; a CTA's start, drain and write-out cost some four steps, and the exchange of the
-// partial tiles two more; tiles go over the resident clusters in whole rounds.
+// CTAs that share a tile's reduction (0: no cluster of that size fits the device).  In steps of 64 reduction indices: a CTA's
+// start, drain and write-out cost some four steps, and the exchange of the partial tiles two more; tiles go over the resident clusters
+// in whole rounds.
 int pick_splits(int64_t tiles, int64_t ksteps, const int (&resident)[kMaxSplits + 1]) {
   int best = 1;
   double best_cost = 0.0;
@@ -674,7 +777,7 @@ int gemm(cudaStream_t st, TileParams p) {
   if (!ds) return MCB_ERR_NOT_INIT;
   if (p.residual != nullptr && p.residual == p.C) return fail(MCB_ERR_UNSUPPORTED, "f32 path: residual must not alias the output");
   p.status = ds->status_word;
-  if (p.K <= kShort && p.R <= kShort) {
+  if (p.K <= kShortTerms && p.R <= kShortTerms) {
     p.n_tiles = (p.N + kShort - 1) / kShort;
     const int64_t tiles = static_cast<int64_t>((p.M + kShort - 1) / kShort) * p.n_tiles;
     if (tiles > 0x7fffffffll) return fail(MCB_ERR_SHAPE, "f32 path: %d x %d outputs", p.M, p.N);

@@ -452,6 +452,44 @@ def test_f32_product_rounds_like_float32(cuda_device, M, K, N):
         assert err.max().item() <= bound
 
 
+# operands of one sign and of both: what is left out of a product or cut off a sum must not add up
+@pytest.mark.parametrize("M,K,N", [(512, 768, 768), (300, 65, 200), (257, 1024, 129), (300, 1000, 64)])
+@pytest.mark.parametrize("values", ["normal", "uniform01", "uniform12", "shifted"])
+def test_f32_product_error_has_no_sign(cuda_device, values, M, K, N):
+    """Against float64.  A float32 result is rounded to 2^-24 of itself; sums of rounded terms wander about it, so the error of the
+    whole result stays below one unit in the last place, 2^-23, and its mean below half of one."""
+    from metal_candle_b200 import backend as B
+    from metal_candle_b200._lib import MCB_W_OUT_IN
+
+    g = torch.Generator(device=cuda_device).manual_seed(M * N + K)
+    make = {"normal": lambda *s: torch.randn(*s, device=cuda_device, generator=g), "uniform01": lambda *s: torch.rand(*s, device=cuda_device, generator=g),
+            "uniform12": lambda *s: torch.rand(*s, device=cuda_device, generator=g) + 1.0,
+            "shifted": lambda *s: torch.randn(*s, device=cuda_device, generator=g) + 3.0}[values]
+    x, w, dy = make(M, K), make(N, K), make(M, N)
+    wt = w.t().contiguous()
+    for got, p, q in ((B.lora_linear_forward(x, w, None, None, None, 1.0)[0], x, w.t()), (B.matmul(x, wt), x, w.t()),
+                      (B.lora_linear_backward(None, w, None, None, 1.0, dy, weight_layout=MCB_W_OUT_IN)[0], dy, w)):
+        want = p.double() @ q.double()
+        err = got.double() - want
+        assert (err.norm() / want.norm()).item() <= 2.0 ** -23
+        assert abs((err.sum() / want.abs().sum()).item()) <= 2.0 ** -24
+
+
+def test_f32_product_of_equal_operands_keeps_every_bit(cuda_device):
+    """x = 1 + 2^-7 - 2^-23: products whose smaller parts are as large as they get.  A row of one such term is the product rounded once
+    (2^-24), one of K terms a sum of K / 16 + 1 roundings."""
+    from metal_candle_b200 import backend as B
+
+    v = 1.0 + 2.0 ** -7 - 2.0 ** -23
+    for K, terms in ((128, 1), (128, 128), (1024, 1024)):
+        x, w = torch.zeros(130, K, device=cuda_device), torch.zeros(70, K, device=cuda_device)
+        x[:, :terms] = v
+        w[:, :terms] = -v
+        y = B.lora_linear_forward(x, w, None, None, None, 1.0)[0].double()
+        want = -terms * v * v
+        assert ((y - want).abs().max().item()) <= abs(want) * 2.0 ** -24 * (1 if terms == 1 else terms // 16 + 1)
+
+
 def test_f32_product_of_extreme_values(cuda_device):
     """Infinities, NaN, the largest and the smallest numbers come out as float32 arithmetic has them (each output is one product:
     one term per row is not zero)."""
