@@ -416,59 +416,74 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_kernel(const __grid_cons
 }
 
 // ---- short reductions ----------------------------------------------------------------------------------------------
-// The same product where K and R are at most 32, with float32 FMAs: there is no reduction to speed up.  (With 64 terms they err by 1.4e-7
-// and tile_kernel by 4.9e-8, in 112 and 65 us at 4096 x 64 x 4096.)
-// Bound: writing C.  A CTA holds both operands' 64 rows whole; a thread owns 8 x 4 outputs.
-constexpr int kShort = 64, kShortTerms = 32, kShortThreads = 128, kShortPitch = kShort + 4;
+// The same product where K and R are at most 32, with float32 FMAs: there is no reduction to speed up, and taking a step's values
+// apart costs more than multiplying them.  Bound: writing C, 16 bytes a thread and row, 256 next to each other.  A CTA holds both
+// operands' 64 rows whole; a thread owns 8 x 4 outputs.  us, copies of 64-wide FMA tiles / single words stored and staged in 32 / this:
+// 4096 x 8 x 4096 41.0 / 50.8 / 25.5, 4096 x 16 x 4096 45.1 / 56.4 / 35.5, 4096 x 32 x 4096 53.4 / 70.5 / 54.3, 8192 x 16 x 896 26.7 / 31.1 / 17.2,
+// delta of 4096 tokens 4096 -> 4096 r8 74.9 / 84.7 / 59.4.  Beyond 32 tile_kernel, which errs less (64 terms 4.9e-8 against 1.4e-7):
+// 4096 x 40 x 4096 62.8 / 78.0 / 69.1, 2048 x 40 x 2048 21.5 / 27.5 / 20.1, 4096 x 64 x 4096 75.8 / 112 / 65.6.
+constexpr int kShort = 32, kShortRows = 64, kShortThreads = 128, kShortPitch = kShortRows + 4;
 __global__ void __launch_bounds__(kShortThreads) short_kernel(const __grid_constant__ TileParams p) {
-  __shared__ __align__(16) float sa[32][kShortPitch], sb[32][kShortPitch];   // [k][row], half of the reduction at a time
-  const int m0 = (blockIdx.x / p.n_tiles) * kShort, n0 = (blockIdx.x % p.n_tiles) * kShort;
+  __shared__ __align__(16) float sa[kShort][kShortPitch], sb[kShort][kShortPitch];   // [k][row]
+  const int m0 = (blockIdx.x / p.n_tiles) * kShortRows, n0 = (blockIdx.x % p.n_tiles) * kShortRows;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // rows 8 ty.., columns 4 tx..
   grid_launch_dependents();
   grid_dependency_wait();
-  float acc[8][4] = {};
-  auto stage = [&](float (&dst)[32][kShortPitch], const Operand& o, int row0, int rows, int k0, int kend) {
+  float2 sum[8][2] = {};
+  auto stage = [&](float (&dst)[kShort][kShortPitch], const Operand& o, int row0, int rows, int len) {
     const float* src = from_here(o.p);
-    const bool k_major = o.sk == 1;
-    for (int e = threadIdx.x; e < 32 * kShort; e += kShortThreads) {
-      const int k = k_major ? e & 31 : e >> 6, r = k_major ? e >> 5 : e & 63;
-      dst[k][r] = row0 + r < rows && k0 + k < kend ? src[(row0 + r) * o.sr + (k0 + k) * o.sk] : 0.0f;
+    if (is_k_major(o)) {
+      for (int e = threadIdx.x; e < len * kShortRows; e += kShortThreads) {   // neighbouring threads, neighbouring words
+        const int r = e / len, k = e - r * len;
+        dst[k][r] = row0 + r < rows ? src[(row0 + r) * o.sr + k] : 0.0f;
+      }
+    } else {
+      for (int e = threadIdx.x; e < len * kShortRows; e += kShortThreads) {
+        const int k = e / kShortRows, r = e % kShortRows;
+        dst[k][r] = row0 + r < rows ? src[row0 + r + k * o.sk] : 0.0f;
+      }
     }
   };
   auto run = [&](const Operand& a, const Operand& b, int len) {
-    for (int k0 = 0; k0 < len; k0 += 32) {
-      __syncthreads();
-      stage(sa, a, m0, p.M, k0, len);
-      stage(sb, b, n0, p.N, k0, len);
-      __syncthreads();
-      const int kn = min(32, len - k0);
+    stage(sa, a, m0, p.M, len);
+    stage(sb, b, n0, p.N, len);
+    __syncthreads();
 #pragma unroll 4
-      for (int k = 0; k < kn; ++k) {
-        const float4 a0 = *reinterpret_cast<const float4*>(&sa[k][8 * ty]), a1 = *reinterpret_cast<const float4*>(&sa[k][8 * ty + 4]);
-        const float4 b0 = *reinterpret_cast<const float4*>(&sb[k][4 * tx]);
-        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, bv[4] = {b0.x, b0.y, b0.z, b0.w};
+    for (int k = 0; k < len; ++k) {
+      const float4 a0 = *reinterpret_cast<const float4*>(&sa[k][8 * ty]), a1 = *reinterpret_cast<const float4*>(&sa[k][8 * ty + 4]);
+      const float4 b0 = *reinterpret_cast<const float4*>(&sb[k][4 * tx]);
+      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+      for (int i = 0; i < 8; ++i) {
+        sum[i][0] = __ffma2_rn(make_float2(av[i], av[i]), make_float2(b0.x, b0.y), sum[i][0]);
+        sum[i][1] = __ffma2_rn(make_float2(av[i], av[i]), make_float2(b0.z, b0.w), sum[i][1]);
       }
     }
   };
   run(p.a, p.b, p.K);
-  run(p.ra, p.rb, p.R);
+  if (p.R > 0) {
+    __syncthreads();
+    run(p.ra, p.rb, p.R);
+  }
+  const bool vec = p.cn == 1 && p.cm % 4 == 0 && p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15u) == 0;
+  const int gn0 = n0 + 4 * tx;
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < 8; ++i) {
+    const int gm = m0 + 8 * ty + i;
+    if (gm >= p.M || gn0 >= p.N) continue;
+    const int64_t o = gm * p.cm + gn0 * p.cn;
+    float v[4] = {sum[i][0].x, sum[i][0].y, sum[i][1].x, sum[i][1].y};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int gm = m0 + 8 * ty + i, gn = n0 + 4 * tx + j;
-      if (gm >= p.M || gn >= p.N) continue;
-      const int64_t o = gm * p.cm + gn * p.cn;
-      float v = acc[i][j] * p.alpha;
-      if (p.bias != nullptr) v += p.bias[gn];
-      if (p.residual != nullptr) v += p.residual[o];
-      if (p.accumulate) v += p.C[o];
-      p.C[o] = v;
+      if (gn0 + j >= p.N) break;
+      v[j] *= p.alpha;
+      if (p.bias != nullptr) v[j] += p.bias[gn0 + j];
+      if (p.residual != nullptr) v[j] += p.residual[o + j * p.cn];
+      if (p.accumulate) v[j] += p.C[o + j * p.cn];
+      if (!vec) p.C[o + j * p.cn] = v[j];
     }
+    if (vec) *reinterpret_cast<float4*>(p.C + o) = make_float4(v[0], v[1], v[2], v[3]);
+  }
 }
 
 // ---- rank intermediates ------------------------------------------------------------------------------------------
@@ -777,9 +792,9 @@ int gemm(cudaStream_t st, TileParams p) {
   if (!ds) return MCB_ERR_NOT_INIT;
   if (p.residual != nullptr && p.residual == p.C) return fail(MCB_ERR_UNSUPPORTED, "f32 path: residual must not alias the output");
   p.status = ds->status_word;
-  if (p.K <= kShortTerms && p.R <= kShortTerms) {
-    p.n_tiles = (p.N + kShort - 1) / kShort;
-    const int64_t tiles = static_cast<int64_t>((p.M + kShort - 1) / kShort) * p.n_tiles;
+  if (p.K <= kShort && p.R <= kShort) {
+    p.n_tiles = (p.N + kShortRows - 1) / kShortRows;
+    const int64_t tiles = static_cast<int64_t>((p.M + kShortRows - 1) / kShortRows) * p.n_tiles;
     if (tiles > 0x7fffffffll) return fail(MCB_ERR_SHAPE, "f32 path: %d x %d outputs", p.M, p.N);
     MCB_CHECK_CUDA(launch_kernel(short_kernel, dim3(static_cast<unsigned>(tiles)), dim3(kShortThreads), 0, st, chained_launch(), p));
     MCB_CHECK_LAUNCH("f32 short_kernel");

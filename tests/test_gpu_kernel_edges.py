@@ -490,6 +490,33 @@ def test_f32_product_of_equal_operands_keeps_every_bit(cuda_device):
         assert ((y - want).abs().max().item()) <= abs(want) * 2.0 ** -24 * (1 if terms == 1 else terms // 16 + 1)
 
 
+# short reductions: the first and the last of the short kernel, the first of the tile kernel behind it; widths with and without whole
+# 16-byte stores, rows beyond a block of 64
+@pytest.mark.parametrize("M,K,N,r", [(1, 1, 1, 1), (65, 5, 63, 3), (64, 31, 64, 8), (130, 32, 132, 32), (200, 32, 66, 16), (97, 33, 130, 30)])
+def test_f32_short_reduction_edges(cuda_device, M, K, N, r):
+    """With bias, residual and adapter, against float64: a chain of n float32 operations errs by at most n 2^-24 of the sum of
+    magnitudes; the adapter's h has K + 1 of its own, and an output K + r + 4."""
+    from metal_candle_b200 import backend as B
+    from metal_candle_b200._lib import MCB_W_OUT_IN
+
+    g = torch.Generator(device=cuda_device).manual_seed(M * K + N)
+    rnd = lambda *s: torch.randn(*s, device=cuda_device, generator=g)  # noqa: E731
+    x, w, bias, a, b, res, dy = rnd(M, K), rnd(N, K), rnd(N), rnd(K, r), rnd(r, N), rnd(M, N), rnd(M, N)
+    d = lambda t: t.double()  # noqa: E731
+    got = B.lora_linear_forward(x, w, bias, a, b, 2.0, residual=res)[0]
+    want = d(x) @ d(w).t() + d(bias) + 2 * (d(x) @ d(a)) @ d(b) + d(res)
+    size = d(x).abs() @ d(w).abs().t() + d(bias).abs() + 2 * (d(x).abs() @ d(a).abs()) @ d(b).abs() + d(res).abs()
+    assert ((d(got) - want).abs() <= size * 2.0 ** -24 * (2 * K + r + 5)).all()
+    for wt, kw in ((w.t().contiguous(), {}), (w, dict(weight_layout=MCB_W_OUT_IN))):
+        dx = rnd(M, K)
+        got = B.lora_linear_backward(x, wt, a, b, 2.0, dy, dx_residual=dx, **kw)[0]
+        want = d(dy) @ d(w) + 2 * (d(dy) @ d(b).t()) @ d(a).t() + d(dx)
+        size = d(dy).abs() @ d(w).abs() + 2 * (d(dy).abs() @ d(b).abs().t()) @ d(a).abs().t() + d(dx).abs()
+        assert ((d(got) - want).abs() <= size * 2.0 ** -24 * (2 * N + r + 5)).all()
+    got = B.matmul(x, w.t().contiguous())
+    assert ((d(got) - d(x) @ d(w).t()).abs() <= d(x).abs() @ d(w).abs().t() * 2.0 ** -24 * (K + 1)).all()
+
+
 def test_f32_product_of_extreme_values(cuda_device):
     """Infinities, NaN, the largest and the smallest numbers come out as float32 arithmetic has them (each output is one product:
     one term per row is not zero)."""
