@@ -43,7 +43,7 @@ struct TileParams {
 // of x rounded to nearest bfloat16.  A remainder is at most half a unit of the part before it, so the three hold all 24 bits,
 // and it has either sign, so that nothing that is left out of a product adds up over many of them.  Both operands are scaled by 2^24
 // first, so that the parts of the smallest normal numbers are normal themselves; what overflows for it (operands beyond 2^103,
-// products beyond 2^79) is computed again, see plain_element.  Of the nine products of the parts l x l alone is left out: below 2^-33 of
+// products beyond 2^79) is computed again, see redo_outputs.  Of the nine products of the parts l x l alone is left out: below 2^-33 of
 // the product, where one float32 rounding is up to 2^-24.
 constexpr int kTileM = 128, kStep = 64, kStages = 2, kParts = 3, kMaxSplits = 8;
 constexpr int kSumWarps = 8, kCopyWarps = 7, kCopyThreads = 32 * kCopyWarps, kTileThreads = 32 * kSumWarps + kCopyThreads + 32;
@@ -55,7 +55,8 @@ struct TileSmem {
   static constexpr uint32_t kStage = kParts * (kPlaneA + kPlaneB), kBars = kStages * kStage;
   static constexpr size_t kBytes = kBars + 128 + 1024;
   static constexpr int kOutPitch = BN + 4;   // the output tile reuses the stages; rows four banks apart
-  static_assert(kTileM * kOutPitch * 4 <= kBars, "output tile");
+  static_assert((kTileM * kOutPitch + kTileM * 36 + 32 * (BN + 4)) * 4 <= kBars, "output tile, and what redo_outputs stages behind it");
+  static_assert(kTileM * (BN / 4) <= 8 * kTileThreads, "32 bits say which of a thread's outputs are spoilt");
 };
 
 // two values rounded to bfloat16 (the first in the lower half), and what the rounding left of them
@@ -140,13 +141,108 @@ struct Copy {
   }
 };
 
-// One output in plain float32 arithmetic.  An operand that is infinite, or becomes so by the scaling, has no parts (inf - inf),
-// so an output that is not finite may be one the parts have spoilt: it is computed again, and is then what float32 gives.
-__device__ __noinline__ float plain_element(const TileParams& p, int m, int n) {
-  float s = 0.0f;
-  for (int k = 0; k < p.K; ++k) s = fmaf(p.a.p[m * p.a.sr + k * p.a.sk], p.b.p[n * p.b.sr + k * p.b.sk], s);
-  for (int k = 0; k < p.R; ++k) s = fmaf(p.ra.p[m * p.ra.sr + k * p.ra.sk], p.rb.p[n * p.rb.sr + k * p.rb.sk], s);
-  return s;
+// What a CTA has to do to an output besides the sum.
+__device__ __forceinline__ float finish_output(const TileParams& p, float v, int gn, int64_t at) {
+  v *= p.alpha;
+  if (p.bias != nullptr) v += p.bias[gn];
+  if (p.residual != nullptr) v += p.residual[at];
+  if (p.accumulate) v += p.C[at];
+  return v;
+}
+
+// The outputs of `bad` (bit 4 i + x: column x of the four that the thread has of its i-th row) in plain float32 arithmetic, a chain of FMAs
+// over K and R.  An operand that is infinite, or becomes so by the scaling, has no parts (inf - inf), so an output that is not finite
+// may be one the parts have spoilt: it is computed again, and is then what float32 gives.  Rare, or a run that has diverged, which should
+// not take a hundred times as long either: the CTA goes over the reduction together, 32 indices at a time.  us, a serial sum
+// by the thread that has the output / this (all clean): 512 x 768 x 768 all NaN 1703 / 101 (21), a row with an infinity 253 / 73;
+// 2048 x 1536 x 1536 20313 / 643 (113), 522 / 161; 4096^3 249700 / 5450 (1075), 1737 / 1175.  (FMA tiles took 33, 259 and 2834 for any values.)
+template <int BN>
+struct Redo {
+  static constexpr int kTerms = 32, kPitchA = kTerms + 4, kPitchB = BN + 4;
+  static constexpr int kHop = kTileThreads / (BN / 4), kRows = kTileM / kHop;   // rows from one of a thread's to the next, and how many it has
+  static constexpr int kFloats = kTileM * kPitchA + kTerms * kPitchB;
+};
+// 32 indices of an operand's ROWS rows, a word a thread at a time, neighbours next to each other
+template <int ROWS>
+struct RedoCopy {
+  static constexpr int kWords = ROWS * 32 / kTileThreads;
+  float v[kWords];
+  __device__ __forceinline__ void load(const Operand& o, int row0, int first, int last, int rows, int k0, int kend) {
+#pragma unroll
+    for (int j = 0; j < kWords; ++j) {
+      const int e = threadIdx.x + j * kTileThreads, r = is_k_major(o) ? e >> 5 : e % ROWS, k = k0 + (is_k_major(o) ? e & 31 : e / ROWS);
+      v[j] = r >= first && r < last && row0 + r < rows && k < kend ? o.p[(row0 + r) * o.sr + k * o.sk] : 0.0f;
+    }
+  }
+  // element (row, k) to dst[row * sr + k * sk]
+  __device__ __forceinline__ void store(float* dst, int sr, int sk, bool k_major) const {
+#pragma unroll
+    for (int j = 0; j < kWords; ++j) {
+      const int e = threadIdx.x + j * kTileThreads;
+      dst[(k_major ? e >> 5 : e % ROWS) * sr + (k_major ? e & 31 : e / ROWS) * sk] = v[j];
+    }
+  }
+};
+// NR: of how many of its rows a thread has outputs
+template <int BN, int NR>
+__device__ __noinline__ void redo_rows(const TileParams& p, float* sa, int m0, int n0, int row_begin, int row_end, uint32_t bad) {
+  using D = Redo<BN>;
+  float* sb = sa + kTileM * D::kPitchA;
+  const int c = (threadIdx.x % (BN / 4)) * 4, r0 = row_begin + threadIdx.x / (BN / 4);
+  const bool any = __any_sync(0xffffffffu, bad != 0);
+  float2 acc[NR][2] = {};
+  RedoCopy<kTileM> ca;
+  RedoCopy<BN> cb;
+  auto add = [&](const Operand& a, const Operand& b, int len) {
+    auto load = [&](int k0) {
+      ca.load(a, m0, row_begin, row_end, p.M, k0, len);
+      cb.load(b, n0, 0, BN, p.N, k0, len);
+    };
+    if (len > 0) load(0);
+    for (int k0 = 0; k0 < len; k0 += D::kTerms) {
+      __syncthreads();   // the terms before have been read
+      ca.store(sa, D::kPitchA, 1, is_k_major(a));
+      cb.store(sb, 1, D::kPitchB, is_k_major(b));
+      __syncthreads();
+      if (k0 + D::kTerms < len) load(k0 + D::kTerms);
+      if (!any) continue;
+#pragma unroll 2
+      for (int k = 0; k < D::kTerms; k += 4) {   // behind the end both are zeros
+        float4 x[NR], y[4];
+#pragma unroll
+        for (int i = 0; i < NR; ++i) x[i] = *reinterpret_cast<const float4*>(sa + min(r0 + i * D::kHop, kTileM - 1) * D::kPitchA + k);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) y[t] = *reinterpret_cast<const float4*>(sb + (k + t) * D::kPitchB + c);
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+          for (int i = 0; i < NR; ++i) {
+            const float v = t == 0 ? x[i].x : t == 1 ? x[i].y : t == 2 ? x[i].z : x[i].w;
+            acc[i][0] = __ffma2_rn(make_float2(v, v), make_float2(y[t].x, y[t].y), acc[i][0]);
+            acc[i][1] = __ffma2_rn(make_float2(v, v), make_float2(y[t].z, y[t].w), acc[i][1]);
+          }
+      }
+    }
+  };
+  add(p.a, p.b, p.K);
+  add(p.ra, p.rb, p.R);
+#pragma unroll
+  for (int i = 0; i < NR; ++i)
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+      if (bad >> (4 * i + x) & 1u) {
+        const int gm = m0 + r0 + i * D::kHop, gn = n0 + c + x;
+        const int64_t at = gm * p.cm + gn * p.cn;
+        p.C[at] = finish_output(p, x == 0 ? acc[i][0].x : x == 1 ? acc[i][0].y : x == 2 ? acc[i][1].x : acc[i][1].y, gn, at);
+      }
+}
+template <int BN>
+__device__ __forceinline__ void redo_outputs(const TileParams& p, float* stage, int m0, int n0, int row_begin, int row_end, uint32_t bad) {
+  const int nr = (row_end - row_begin + Redo<BN>::kHop - 1) / Redo<BN>::kHop;
+  if (nr <= 1) redo_rows<BN, 1>(p, stage, m0, n0, row_begin, row_end, bad);
+  else if (nr <= 2) redo_rows<BN, 2>(p, stage, m0, n0, row_begin, row_end, bad);
+  else if (nr <= 4) redo_rows<BN, 4>(p, stage, m0, n0, row_begin, row_end, bad);
+  else redo_rows<BN, 8>(p, stage, m0, n0, row_begin, row_end, bad);
 }
 
 // A step of 64 reduction indices: seven warps take the values they loaded a step earlier apart (two stages of shared memory), one issues
@@ -374,10 +470,13 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_kernel(const __grid_cons
   float* tile_out = reinterpret_cast<float*>(gen);
   const int row_begin = kTileM * split / p.splits, row_end = kTileM * (split + 1) / p.splits;
   const bool vec_out = p.cn == 1 && p.cm % 4 == 0 && p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15u) == 0;
-  for (int e = threadIdx.x; e < (row_end - row_begin) * (BN / 4); e += kTileThreads) {
-    const int r = row_begin + e / (BN / 4), c = (e % (BN / 4)) * 4;
+  uint32_t bad = 0;   // see redo_outputs
+#pragma unroll 2
+  for (int i = 0; i < Redo<BN>::kRows; ++i) {
+    const int r = row_begin + threadIdx.x / (BN / 4) + i * Redo<BN>::kHop, c = (threadIdx.x % (BN / 4)) * 4;
     const int gm = m0 + r, gn = n0 + c;
-    if (gm >= p.M || gn >= p.N) continue;
+    if (r >= row_end || gm >= p.M) break;
+    if (gn >= p.N) continue;
     // all parts' loads in flight before the first sum: one after the other, a thread's remote reads are as many trips
     // through the cluster's network
     float4 part[kMaxSplits];
@@ -395,23 +494,25 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_kernel(const __grid_cons
       }
     const int64_t o = gm * p.cm + gn * p.cn;
     const int live = min(4, p.N - gn);
+    // (no branch: with one around each output's arithmetic 4096 x 64 x 4096 took 74.7 us instead of 65.9)
+    uint32_t spoilt = 0;
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
       if (x >= live) break;
-      v[x] = fabsf(v[x]) < INFINITY ? v[x] * kPartUnscale : plain_element(p, gm, gn + x);
-      v[x] *= p.alpha;
-      if (p.bias != nullptr) v[x] += p.bias[gn + x];
-      if (p.residual != nullptr) v[x] += p.residual[o + x * p.cn];
-      if (p.accumulate) v[x] += p.C[o + x * p.cn];
+      spoilt |= fabsf(v[x]) < INFINITY ? 0u : 1u << x;
+      v[x] = finish_output(p, v[x] * kPartUnscale, gn + x, o + x * p.cn);
     }
-    if (vec_out) {
+    bad |= spoilt << (4 * i);
+    // what is computed again may be stored here first, unless C is one of its terms
+    if (vec_out && (spoilt == 0 || !p.accumulate)) {
       *reinterpret_cast<float4*>(p.C + o) = make_float4(v[0], v[1], v[2], v[3]);
     } else {
 #pragma unroll
       for (int x = 0; x < 4; ++x)
-        if (x < live) p.C[o + x * p.cn] = v[x];
+        if (x < live && (spoilt >> x & 1u) == 0) p.C[o + x * p.cn] = v[x];
     }
   }
+  if (__syncthreads_or(bad != 0)) redo_outputs<BN>(p, tile_out + kTileM * S::kOutPitch, m0, n0, row_begin, row_end, bad);
   if (p.splits > 1) cl.sync();   // nobody leaves while a peer still reads its tile
 }
 

@@ -539,6 +539,67 @@ def test_f32_product_of_extreme_values(cuda_device):
     assert ((y[fin].double() - want[fin].double()).abs() <= want[fin].double().abs() * 2.0 ** -20 + 2.0 ** -149).all()
 
 
+# outputs that the parts spoil, among others: whole tiles and ragged ones, reductions of one CTA and shared by up to 8, 64-wide tiles
+@pytest.mark.parametrize("M,K,N,r", [(512, 768, 768, 8), (300, 200, 132, 40), (257, 1024, 63, 3), (1200, 100, 1101, 16)])
+def test_f32_outputs_that_are_computed_again(cuda_device, M, K, N, r):
+    """A NaN, an infinity and a number too large for the parts in x and W touch their rows and columns and nothing else: the other
+    outputs keep their bits, those of the large numbers are a float32 chain of FMAs (its error: a unit per term of the magnitudes)."""
+    from metal_candle_b200 import backend as B
+
+    g = torch.Generator(device=cuda_device).manual_seed(M + N)
+    rnd = lambda *s: torch.randn(*s, device=cuda_device, generator=g)  # noqa: E731
+    x, w, bias, a, b, res = rnd(M, K), rnd(N, K), rnd(N), rnd(K, r), rnd(r, N), rnd(M, N)
+    clean = B.lora_linear_forward(x, w, bias, a, b, 2.0, residual=res)[0]
+    xs, ws = x.clone(), w.clone()
+    xs[1, 3], xs[M // 2, K - 1], xs[M - 1, 0] = float("nan"), float("inf"), 3e33
+    ws[2, 5], ws[N - 1, K // 2] = float("nan"), -2e34
+    got = B.lora_linear_forward(xs, ws, bias, a, b, 2.0, residual=res)[0]
+    rows, cols = [1, M // 2, M - 1], [2, N - 1]
+    kept = torch.ones(M, N, dtype=torch.bool, device=cuda_device)
+    kept[rows] = False
+    kept[:, cols] = False
+    assert torch.equal(got[kept], clean[kept])
+    want = xs.double() @ ws.double().t() + bias.double() + 2 * (xs.double() @ a.double()) @ b.double() + res.double()
+    size = xs.double().abs() @ ws.double().abs().t() + bias.double().abs() + 2 * (xs.double().abs() @ a.double().abs()) @ b.double().abs() + res.double().abs()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    fin = want.isfinite() & ~kept
+    assert ((got.double() - want)[fin].abs() <= size[fin] * 2.0 ** -24 * (2 * K + r + 5)).all()
+    # gradients that are added to what is there, an infinity among the terms (rank 24: products of the tile kernel)
+    a, b, dy = rnd(K, 24), rnd(24, N), rnd(M, N)
+    xs = x.clone()
+    xs[M // 2, 1] = float("inf")
+    start = rnd(K, 24)
+    grads = [start.clone(), rnd(24, N)]
+    B.lora_linear_backward(xs, w.t().contiguous(), a, b, 1.0, dy, grad_a=grads[0], grad_b=grads[1], accumulate=True)
+    h = dy.double() @ b.double().t()
+    want = start.double() + xs.double().t() @ h
+    size = start.double().abs() + x.double().abs().t() @ (dy.double().abs() @ b.double().abs().t())
+    assert torch.equal(grads[0].isinf(), want.isinf())
+    ok = want.isfinite()
+    assert ((grads[0].double() - want)[ok].abs() <= size[ok] * 2.0 ** -24 * (M + N + 3)).all()
+
+
+def test_f32_product_of_nan_costs_no_multiple(cuda_device):
+    """A run that has diverged goes on at the pace of float32 FMAs, not at that of a serial sum per output (86 times the clean call
+    where that was done): eight times the clean call at most."""
+    from metal_candle_b200 import backend as B
+
+    def us(x, w):
+        best = float("inf")
+        for _ in range(6):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            B.lora_linear_forward(x, w, None, None, None, 1.0)
+            e[1].record()
+            e[1].synchronize()
+            best = min(best, e[0].elapsed_time(e[1]))
+        return best
+
+    x, w = torch.randn(2048, 1536, device=cuda_device), torch.randn(1536, 1536, device=cuda_device)
+    clean = us(x, w)
+    assert us(torch.full_like(x, float("nan")), w) <= 8 * clean
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("seq", [32, 64, 255, 256, 512, 777, 1024, 1100])
 def test_causal_softmax_backward_in_registers(cuda_device, dtype, seq):
