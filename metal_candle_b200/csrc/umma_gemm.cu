@@ -639,41 +639,8 @@ int launch_plain(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
   return launch_gemm2(c, ds, st);
 }
 
-int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
-  if (c.M > 0x7fffff00ll || c.N > 0x7fffff00ll || c.K > 0x7fffff00ll)
-    return fail(MCB_ERR_SHAPE, "bf16 GEMM: dimension exceeds 2^31");
-  if (c.K % 8 != 0 || c.N % 8 != 0)
-    return fail(MCB_ERR_ALIGN, "bf16 path needs in/out features that are multiples of 8 (got reduction %lld, output %lld)",
-                (long long)c.K, (long long)c.N);
-  if (!aligned16(c.X) || (c.W && !aligned16(c.W)) || (c.Y && !aligned16(c.Y)) || (c.H && !aligned16(c.H)) || (c.R && !aligned16(c.R)))
-    return fail(MCB_ERR_ALIGN, "bf16 path needs 16-byte aligned matrices");
-  // shapes with too few tiles to fill the chip: narrower tiles, reduction in parts (umma_split.cu)
-  if (c.W != nullptr && c.Y != nullptr && c.swiglu_up == nullptr) {
-    const SplitPlan sp = split_plan(c.M, c.N, c.K, c.rp, gemm2_eligible(c), ds);
-    if (sp.bn > 0) {
-      if (int rc = launch_split(sp, c, nullptr, nullptr, ds, st)) return rc;
-      if (c.grads == nullptr) return MCB_OK;
-      const GradRequest& q = *c.grads;
-      return launch_grad2(q.X[0], q.Ht[0], q.C[0], q.out[0], q.transposed[0], q.X[1], q.Ht[1], q.C[1], q.out[1], q.transposed[1],
-                          q.h_pitch, q.part, c.M, q.r, c.rp, q.accumulate, ds, st);
-    }
-  }
-  if (rank_apart(c, ds)) {
-    GemmCall h = c;
-    h.W = nullptr; h.Y = nullptr; h.bias = nullptr; h.R = nullptr; h.grads = nullptr;
-    if (int rc = launch_gemm(h, ds, st)) return rc;
-    GemmCall y = c;
-    y.P = nullptr; y.Q = nullptr; y.H = nullptr; y.Hr = nullptr; y.rp = 0; y.grads = nullptr;
-    y.X2 = c.Hr; y.W2 = c.Q; y.K2 = c.rp;
-    if (int rc = launch_plain(y, ds, st)) return rc;
-    if (c.grads == nullptr) return MCB_OK;
-    const GradRequest& q = *c.grads;
-    return launch_grad2(q.X[0], q.Ht[0], q.C[0], q.out[0], q.transposed[0], q.X[1], q.Ht[1], q.C[1], q.out[1], q.transposed[1],
-                        q.h_pitch, q.part, c.M, q.r, c.rp, q.accumulate, ds, st);
-  }
-  // linears of useful size (with or without the rank path) run on CTA pairs (umma_wide.cu, umma_gemm2.cu)
-  if (c.rp == 0 && c.swiglu_up == nullptr && gemm2_eligible(c)) return launch_plain(c, ds, st);
-  if (gemm2_eligible(c)) return launch_gemm2(c, ds, st);
+// The call on the one-CTA kernel.  hr: [M, rp] for the rank intermediate as a product's operand, where that is all the call computes, or null.
+int launch_one_cta(const GemmCall& c, __nv_bfloat16* hr, const DeviceState* ds, cudaStream_t st) {
   GemmParams p;
   memset(&p, 0, sizeof(p));
   p.M = static_cast<int>(c.M); p.N = static_cast<int>(c.N); p.K = static_cast<int>(c.K);
@@ -686,7 +653,7 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
   p.num_k_blocks = (p.K + BK - 1) / BK;
   p.group_m = p.num_m_tiles < 16 ? p.num_m_tiles : 16;
   p.scale = c.scale;
-  p.Y = c.Y; p.bias = c.bias; p.R = c.R; p.H = c.H; p.Hr = c.Hr; p.h_pitch = c.h_pitch; p.status = ds->status_word;
+  p.Y = c.Y; p.bias = c.bias; p.R = c.R; p.H = c.H; p.Hr = hr; p.h_pitch = c.h_pitch; p.status = ds->status_word;
   const uint32_t x_bytes = BM * BK * 2;
   const uint32_t w_bytes = p.has_w ? p.BN * BK * 2 : 0;
   const uint32_t p_bytes = p.rp * BK * 2;
@@ -781,6 +748,44 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
                         q.h_pitch, q.part, c.M, q.r, c.rp, q.accumulate, ds, st);
   }
   return MCB_OK;
+}
+
+int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
+  if (c.M > 0x7fffff00ll || c.N > 0x7fffff00ll || c.K > 0x7fffff00ll)
+    return fail(MCB_ERR_SHAPE, "bf16 GEMM: dimension exceeds 2^31");
+  if (c.K % 8 != 0 || c.N % 8 != 0)
+    return fail(MCB_ERR_ALIGN, "bf16 path needs in/out features that are multiples of 8 (got reduction %lld, output %lld)",
+                (long long)c.K, (long long)c.N);
+  if (!aligned16(c.X) || (c.W && !aligned16(c.W)) || (c.Y && !aligned16(c.Y)) || (c.H && !aligned16(c.H)) || (c.R && !aligned16(c.R)))
+    return fail(MCB_ERR_ALIGN, "bf16 path needs 16-byte aligned matrices");
+  // shapes with too few tiles to fill the chip: narrower tiles, reduction in parts (umma_split.cu)
+  if (c.W != nullptr && c.Y != nullptr && c.swiglu_up == nullptr) {
+    const SplitPlan sp = split_plan(c.M, c.N, c.K, c.rp, gemm2_eligible(c), ds);
+    if (sp.bn > 0) {
+      if (int rc = launch_split(sp, c, nullptr, nullptr, ds, st)) return rc;
+      if (c.grads == nullptr) return MCB_OK;
+      const GradRequest& q = *c.grads;
+      return launch_grad2(q.X[0], q.Ht[0], q.C[0], q.out[0], q.transposed[0], q.X[1], q.Ht[1], q.C[1], q.out[1], q.transposed[1],
+                          q.h_pitch, q.part, c.M, q.r, c.rp, q.accumulate, ds, st);
+    }
+  }
+  if (rank_apart(c, ds)) {
+    GemmCall h = c;
+    h.W = nullptr; h.Y = nullptr; h.bias = nullptr; h.R = nullptr; h.grads = nullptr;
+    if (int rc = launch_one_cta(h, c.Hr, ds, st)) return rc;
+    GemmCall y = c;
+    y.P = nullptr; y.Q = nullptr; y.H = nullptr; y.Hr = nullptr; y.rp = 0; y.grads = nullptr;
+    y.X2 = c.Hr; y.W2 = c.Q; y.K2 = c.rp;
+    if (int rc = launch_plain(y, ds, st)) return rc;
+    if (c.grads == nullptr) return MCB_OK;
+    const GradRequest& q = *c.grads;
+    return launch_grad2(q.X[0], q.Ht[0], q.C[0], q.out[0], q.transposed[0], q.X[1], q.Ht[1], q.C[1], q.out[1], q.transposed[1],
+                        q.h_pitch, q.part, c.M, q.r, c.rp, q.accumulate, ds, st);
+  }
+  // linears of useful size (with or without the rank path) run on CTA pairs (umma_wide.cu, umma_gemm2.cu)
+  if (c.rp == 0 && c.swiglu_up == nullptr && gemm2_eligible(c)) return launch_plain(c, ds, st);
+  if (gemm2_eligible(c)) return launch_gemm2(c, ds, st);
+  return launch_one_cta(c, nullptr, ds, st);
 }
 
 struct Workspace {

@@ -697,3 +697,27 @@ def _linear_with_rank_path(cuda_device, M, K, N, r):
     _close_bf16(dx, D @ W + G @ A.t())
     _close_bf16(da, X.t() @ G)
     _close_bf16(db, H.t() @ D)
+
+
+@pytest.mark.parametrize("M,K,N,r", [(4096, 896, 896, 16), (1030, 640, 1536, 8), (20000, 896, 128, 16)])
+def test_bf16_linear_stores_nothing_that_nobody_reads(cuda_device, M, K, N, r):
+    """A call whose rank path stays in its own tiles writes its packed operands into the workspace and nothing else: the rank
+    intermediate leaves the kernel only where a launch of its own computes it for the product behind."""
+    from metal_candle_b200 import _lib, backend as B
+
+    g = torch.Generator(device=cuda_device).manual_seed(M)
+    x, w = (torch.randn(*s, device=cuda_device, generator=g).bfloat16() for s in ((M, K), (N, K)))
+    a, b = torch.randn(K, r, device=cuda_device, generator=g), torch.randn(r, N, device=cuda_device, generator=g)
+    y = torch.empty(M, N, dtype=torch.bfloat16, device=cuda_device)
+    lib, code = _lib.load(), B._dtype_code(x)
+    rp = lib.mcb_lora_rank_padded(r)
+    h = torch.empty(rp, lib.mcb_lora_h_pitch(M), dtype=torch.bfloat16, device=cuda_device)
+    ws = B.aligned_block(cuda_device, lib.mcb_lora_workspace_bytes(M, K, N, r, code)).fill_(0x5a)
+    before = lib.mcb_launch_count()
+    _lib.check(lib.mcb_lora_linear_fwd(x.data_ptr(), w.data_ptr(), None, a.data_ptr(), b.data_ptr(), y.data_ptr(), h.data_ptr(), M, K, N, r, 2.0,
+                                       code, 0, ws.data_ptr(), ws.numel(), B._stream()))
+    assert lib.mcb_launch_count() - before == 2   # the pack and the product
+    packed = 2 * ((rp * max(K, N) * 2 + 1023) // 1024 * 1024)
+    assert (ws[packed:] == 0x5a).all()
+    want = x.double() @ w.double().t() + 2 * (x.double() @ a.bfloat16().double()) @ b.bfloat16().double()
+    assert ((y.double() - want).abs().max() / want.abs().max()).item() <= 2e-2
