@@ -75,7 +75,8 @@ struct GemmCall {
   __nv_bfloat16* H = nullptr;         // [rp,h_pitch] or null
   int64_t h_pitch = 0;
   int64_t M = 0, N = 0, K = 0;
-  // A second pair of operands whose product is added in the same accumulators, X2 [M,K2] . W2 [N,K2]^T, or null (rp = 0 only).
+  // A second pair of operands whose product is added in the same accumulators, X2 [M,K2] . W2 [N,K2]^T, or null (rp = 0 only): a
+  // rank update whose intermediate a launch ahead has computed.
   const __nv_bfloat16* X2 = nullptr;
   const __nv_bfloat16* W2 = nullptr;
   int64_t K2 = 0;
@@ -91,6 +92,12 @@ struct GemmCall {
   // up by d gate and d up instead of storing it (pair kernel only).
   __nv_bfloat16* swiglu_up = nullptr;
 };
+// What the per-kernel profile records of a product on its own: an update from a second operand pair counts with the unpadded rank.
+inline double gemm_flops(const GemmCall& c) {
+  const double m = static_cast<double>(c.M), n = static_cast<double>(c.N), k = static_cast<double>(c.K), r = c.r_true;
+  return 2.0 * m * n * k + (c.rp > 0 ? 2.0 * m * r * (k + n) : c.X2 != nullptr ? 2.0 * m * r * n : 0.0);
+}
+inline int gemm_kind(const GemmCall& c) { return c.rp > 0 || c.X2 != nullptr ? kProfGemmLora : kProfGemm; }
 // Tile width and reduction parts of the split-reduction kernel (umma_split.cu); bn == 0: the persistent kernels run.
 struct SplitPlan {
   int bn = 0, splits = 1;

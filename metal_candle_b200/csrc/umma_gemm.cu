@@ -726,8 +726,9 @@ int launch_one_cta(const GemmCall& c, __nv_bfloat16* hr, const DeviceState* ds, 
   const bool prof = profile_on();
   if (prof) {
     const double m = static_cast<double>(c.M), n = static_cast<double>(c.N), k = static_cast<double>(c.K);
-    double flops = (p.has_w ? 2.0 * m * n * k : 0.0) + 2.0 * m * c.r_true * (k + n);
-    double bytes = 2.0 * (m * k + (p.has_w ? n * k : 0.0) + (c.Y ? m * n : 0.0)) + 2.0 * p.rp * (k + n);
+    const double rank_n = c.Y ? n : 0.0;   // without an output there is no update
+    double flops = (p.has_w ? 2.0 * m * n * k : 0.0) + 2.0 * m * c.r_true * (k + rank_n);
+    double bytes = 2.0 * (m * k + (p.has_w ? n * k : 0.0) + (c.Y ? m * n : 0.0)) + 2.0 * p.rp * (k + rank_n);
     if (tail_on) {
       flops += 2.0 * m * (c.grads->C[0] + c.grads->C[1]) * c.r_true;
       bytes += 2.0 * m * (c.grads->C[0] + c.grads->C[1]) + 4.0 * m * c.rp;

@@ -662,8 +662,7 @@ int launch_gemm2(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
   const bool prof = profile_on();
   if (prof) {
     const double m = static_cast<double>(M), n = static_cast<double>(N), k = static_cast<double>(K + c.K2);
-    profile_begin(c.swiglu_up != nullptr ? kProfGemmSwigluBwd : c.rp > 0 ? kProfGemmLora : kProfGemm,
-                  2.0 * m * n * k + 2.0 * m * c.r_true * (k + n),
+    profile_begin(c.swiglu_up != nullptr ? kProfGemmSwigluBwd : gemm_kind(c), gemm_flops(c),
                   2.0 * (m * k + n * k + (c.swiglu_up != nullptr ? 4.0 : 1.0) * m * n) + 2.0 * c.rp * (k + n), st);
   }
   {

@@ -363,7 +363,7 @@ int launch_wide(int bn, const GemmCall& c, __nv_bfloat16* up, __nv_bfloat16* act
   const bool prof = profile_on();
   if (prof) {
     const double m = static_cast<double>(c.M), n = static_cast<double>(c.N), k = static_cast<double>(c.K + c.K2);
-    profile_begin(kProfGemm, 2.0 * m * n * k, 2.0 * (m * k + n * k + (act ? 1.5 : 1.0) * m * n), st);
+    profile_begin(gemm_kind(c), gemm_flops(c), 2.0 * (m * k + n * k + (act ? 1.5 : 1.0) * m * n), st);
   }
   const cudaError_t le = launch_kernel(gemm_wide_kernel, dim3(2 * pairs), dim3(kWideThreads), kWideSmem + 1024, st, chained_launch(), tmX, tmW, tmX2,
                                        tmW2, tmY, tmU, tmA, p);

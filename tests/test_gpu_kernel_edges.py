@@ -721,3 +721,28 @@ def test_bf16_linear_stores_nothing_that_nobody_reads(cuda_device, M, K, N, r):
     assert (ws[packed:] == 0x5a).all()
     want = x.double() @ w.double().t() + 2 * (x.double() @ a.bfloat16().double()) @ b.bfloat16().double()
     assert ((y.double() - want).abs().max() / want.abs().max()).item() <= 2e-2
+
+
+@pytest.mark.parametrize("M,K,N,r", [(2048, 4096, 4096, 16), (2048, 1024, 4096, 40), (4096, 896, 896, 16), (512, 896, 896, 8), (16384, 896, 896, 16)])
+def test_profile_counts_a_linear_with_an_adapter_once(cuda_device, M, K, N, r):
+    """However many launches a call takes (a rank intermediate of its own, wide tiles or pairs behind it; one kernel; parts of the
+    reduction), they are recorded as a linear with a rank path, with 2 M N K + 2 M r (K + N) operations between them."""
+    from metal_candle_b200 import _lib, backend as B
+
+    x, w = (torch.zeros(*s, dtype=torch.bfloat16, device=cuda_device) for s in ((M, K), (N, K)))
+    a, b = torch.zeros(K, r, device=cuda_device), torch.zeros(r, N, device=cuda_device)
+    dy = torch.zeros(M, N, dtype=torch.bfloat16, device=cuda_device)
+    _lib.profile_enable(True)
+    try:
+        for kind in range(4):
+            _lib.profile_summary(kind)
+        B.lora_linear_forward(x, w, None, a, b, 2.0)
+        plain, lora = _lib.profile_summary(0), _lib.profile_summary(2)
+        assert plain[0] == 0 and lora[0] >= 1 and lora[2] == 2.0 * M * N * K + 2.0 * M * r * (K + N)
+        # a backward without an input gradient computes the rank intermediate alone, and the gradients
+        h = torch.zeros(_lib.load().mcb_lora_rank_padded(r), _lib.load().mcb_lora_h_pitch(M), dtype=torch.bfloat16, device=cuda_device)
+        B.lora_linear_backward(x, w.t().contiguous(), a, b, 2.0, dy, h_save=h, need_dx=False)
+        lora, grad = _lib.profile_summary(2), _lib.profile_summary(1)
+        assert lora[2] + grad[2] == 2.0 * M * r * N + 2.0 * M * r * (K + N)
+    finally:
+        _lib.profile_enable(False)
