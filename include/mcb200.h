@@ -84,7 +84,9 @@ int mcb_selftest_wait_timeout(int64_t limit_cycles, int64_t* waited_cycles_out, 
 #define MCB_OPT_GRAD_TAIL 0
 /* Smallest reduction length (in features) from which a linear WITH a rank path runs on CTA pairs instead of the
  * one-CTA kernel (default 1536; from 16384 tokens on 13/24 of it, 832; linears without a rank path always take the pair
- * kernel when large enough). */
+ * kernel when large enough).  A linear whose rank intermediate is quicker by a launch of its own runs the product
+ * behind that on CTA pairs whatever its length, unless the option is raised: with a value above the default, linears of
+ * shorter reductions than it keep their rank path in one launch, on the kernel that the rule above names. */
 #define MCB_OPT_PAIR_MIN_K 1
 /* 1 (default): the library's kernels are launched as programmatic dependents of the kernel before them in their stream, so that
  * a kernel's launch and set-up run under its predecessor's tail (it touches no memory before that has finished); 0: plain

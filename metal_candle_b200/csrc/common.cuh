@@ -43,6 +43,7 @@ void profile_begin(int kind, double flops, double bytes, cudaStream_t st);
 void profile_end(cudaStream_t st);
 
 // Library switches (mcb_set_option).
+constexpr int kPairMinK = 1536;   // MCB_OPT_PAIR_MIN_K unless set
 int option(int which);
 
 // An NVTX range around the body of an entry point: shows each call (and the kernels it enqueues) by name on a

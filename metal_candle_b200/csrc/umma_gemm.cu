@@ -618,6 +618,9 @@ int pick_bn(int64_t N, int rp) {
 // 32768 x 4096 -> 4096 r16 forward, in the tiles / apart: 916 / 778 us (with the wide tiles that the main product then takes).
 bool rank_apart(const GemmCall& c, const DeviceState* ds) {
   if (c.rp == 0 || c.Hr == nullptr || c.W == nullptr || c.Y == nullptr || c.swiglu_up != nullptr || c.M < 1024) return false;
+  // the product apart runs on pairs: a caller that has raised the option does not want that below it
+  const int64_t min_k = option(MCB_OPT_PAIR_MIN_K);
+  if (min_k > kPairMinK && c.K < min_k) return false;
   GemmCall plain = c;
   plain.rp = 0;
   if (!gemm2_eligible(plain)) return false;

@@ -746,3 +746,30 @@ def test_profile_counts_a_linear_with_an_adapter_once(cuda_device, M, K, N, r):
         assert lora[2] + grad[2] == 2.0 * M * r * N + 2.0 * M * r * (K + N)
     finally:
         _lib.profile_enable(False)
+
+
+@pytest.mark.parametrize("M,K,N,r", [(1024, 1024, 4096, 16), (4096, 512, 8192, 64)])
+def test_raised_pair_option_keeps_linears_in_one_launch(cuda_device, M, K, N, r):
+    """MCB_OPT_PAIR_MIN_K above the reduction: no product on CTA pairs behind a launch of its own for the rank intermediate, as by
+    default; the results agree to the rounding of either."""
+    from metal_candle_b200 import _lib, backend as B
+
+    g = torch.Generator(device=cuda_device).manual_seed(K)
+    x, w = (torch.randn(*s, device=cuda_device, generator=g).bfloat16() for s in ((M, K), (N, K)))
+    a, b = torch.randn(K, r, device=cuda_device, generator=g), torch.randn(r, N, device=cuda_device, generator=g)
+    lib = _lib.load()
+
+    def launches():
+        before = lib.mcb_launch_count()
+        y = B.lora_linear_forward(x, w, None, a, b, 2.0, save_hidden=False)[0]
+        return lib.mcb_launch_count() - before, y
+
+    apart, y = launches()
+    assert apart == 3   # the pack, the rank intermediate, the product
+    try:
+        _lib.check(lib.mcb_set_option(_lib.MCB_OPT_PAIR_MIN_K, 1 << 20))
+        n, z = launches()
+        assert n == 2
+    finally:
+        _lib.check(lib.mcb_set_option(_lib.MCB_OPT_PAIR_MIN_K, 1536))
+    assert ((y.double() - z.double()).abs().max() / y.double().abs().max()).item() <= 2e-2
