@@ -43,7 +43,7 @@ int init_grad_kernel();
 int init_gemm2_kernel();
 int init_split_kernel(DeviceState* ds);
 int init_wide_kernel();
-bool gemm2_eligible(const GemmCall& c);
+bool gemm2_eligible(const GemmCall& c, int sm_count);
 int launch_gemm2(const GemmCall& c, const DeviceState* ds, cudaStream_t st);
 size_t grad_partial_bytes(int64_t M, int64_t K, int64_t N, int rp);
 int launch_grad2(const __nv_bfloat16* X0, const __nv_bfloat16* Ht0, int64_t C0, float* out0, int transposed0,
@@ -623,9 +623,9 @@ bool rank_apart(const GemmCall& c, const DeviceState* ds) {
   if (min_k > kPairMinK && c.K < min_k) return false;
   GemmCall plain = c;
   plain.rp = 0;
-  if (!gemm2_eligible(plain)) return false;
+  if (!gemm2_eligible(plain, ds->sm_count)) return false;
   const double nkb = static_cast<double>((c.K + BK - 1) / BK);
-  const bool pair = gemm2_eligible(c);
+  const bool pair = gemm2_eligible(c, ds->sm_count);
   const int bn = pick_bn(c.N, c.rp);
   const int64_t rows = pair ? 256 : BM, slots = pair ? ds->sm_count / 2 : ds->sm_count;
   const int64_t rounds = ((c.M + rows - 1) / rows * ((c.N + bn - 1) / bn) + slots - 1) / slots;
@@ -764,7 +764,7 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
     return fail(MCB_ERR_ALIGN, "bf16 path needs 16-byte aligned matrices");
   // shapes with too few tiles to fill the chip: narrower tiles, reduction in parts (umma_split.cu)
   if (c.W != nullptr && c.Y != nullptr && c.swiglu_up == nullptr) {
-    const SplitPlan sp = split_plan(c.M, c.N, c.K, c.rp, gemm2_eligible(c), ds);
+    const SplitPlan sp = split_plan(c.M, c.N, c.K, c.rp, gemm2_eligible(c, ds->sm_count), ds);
     if (sp.bn > 0) {
       if (int rc = launch_split(sp, c, nullptr, nullptr, ds, st)) return rc;
       if (c.grads == nullptr) return MCB_OK;
@@ -787,8 +787,8 @@ int launch_gemm(const GemmCall& c, const DeviceState* ds, cudaStream_t st) {
                         q.h_pitch, q.part, c.M, q.r, c.rp, q.accumulate, ds, st);
   }
   // linears of useful size (with or without the rank path) run on CTA pairs (umma_wide.cu, umma_gemm2.cu)
-  if (c.rp == 0 && c.swiglu_up == nullptr && gemm2_eligible(c)) return launch_plain(c, ds, st);
-  if (gemm2_eligible(c)) return launch_gemm2(c, ds, st);
+  if (c.rp == 0 && c.swiglu_up == nullptr && gemm2_eligible(c, ds->sm_count)) return launch_plain(c, ds, st);
+  if (gemm2_eligible(c, ds->sm_count)) return launch_gemm2(c, ds, st);
   return launch_one_cta(c, nullptr, ds, st);
 }
 
@@ -920,7 +920,7 @@ bool swiglu_bwd_supported(int64_t M, int64_t K, int64_t N, int64_t r) {
   c.swiglu_up = c.Y;
   c.M = M; c.N = K; c.K = N;
   c.rp = static_cast<int>(rank_padded(r));
-  return gemm2_eligible(c);
+  return gemm2_eligible(c, 0);   // (a SwiGLU's rule does not ask for the SMs)
 }
 
 int linear_bwd(const LoraArgs& a, const DeviceState* ds) {
@@ -960,7 +960,7 @@ int linear_bwd(const LoraArgs& a, const DeviceState* ds) {
       c.r_true = static_cast<int>(a.r);
       c.scale = a.scale;
     }
-    if (a.dA != nullptr && a.dB != nullptr && a.h_save != nullptr && !gemm2_eligible(c) &&
+    if (a.dA != nullptr && a.dB != nullptr && a.h_save != nullptr && !gemm2_eligible(c, ds->sm_count) &&
         grad_tail_possible(a.K, a.N, rp)) {
       rq.X[0] = static_cast<const __nv_bfloat16*>(a.x);  rq.Ht[0] = w.H1; rq.C[0] = a.K; rq.out[0] = a.dA; rq.transposed[0] = 0;
       rq.X[1] = static_cast<const __nv_bfloat16*>(a.dy); rq.Ht[1] = static_cast<const __nv_bfloat16*>(a.h_save);

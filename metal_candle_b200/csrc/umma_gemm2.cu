@@ -565,7 +565,7 @@ int init_gemm2_kernel() {
 // Whether the pair kernel takes this call (everything else stays on the one-CTA kernel): a main product
 // with an output, large enough to fill CTA pairs; with a rank path, rank padded to a multiple of 16 and at
 // most 64 and a long enough reduction (MCB_OPT_PAIR_MIN_K; many tokens: 13/24 of it, 832 by default).
-bool gemm2_eligible(const GemmCall& c) {
+bool gemm2_eligible(const GemmCall& c, int sm_count) {
   if (c.W == nullptr || c.Y == nullptr || c.N < 128 || c.K < 64) return false;
   if (c.M < 1024) {
     // Fewer tokens: only a plain product whose 128-token tiles pair up and take every CTA pair twice or more (the lm_head).  Its time is
@@ -573,7 +573,7 @@ bool gemm2_eligible(const GemmCall& c) {
     // 132 / 115, 700 192 / 171, 900 251 / 222; 512 x 2048 -> 32000 69 / 54, 256 x 4096 -> 50264 110 / 95; but five tiles in three pairs, 640
     // tokens, 166 / 168.
     const int64_t tiles = (c.M + 127) / 128;
-    return c.rp == 0 && c.swiglu_up == nullptr && tiles % 2 == 0 && tiles / 2 * ((c.N + 255) / 256) >= 148;
+    return c.rp == 0 && c.swiglu_up == nullptr && tiles % 2 == 0 && tiles / 2 * ((c.N + 255) / 256) >= 2 * (sm_count / 2);
   }
   if (c.rp == 0) return true;
   if (c.rp % 16 != 0 || c.rp > 64) return false;
