@@ -108,9 +108,13 @@ class _LayerCalls:
         self.usable = (model.dtype == torch.bfloat16 and c.head_dim == 64 and c.intermediate_size % 8 == 0 and c.vocab_size % 8 == 0
                        and model.fuse_swiglu_bwd)
         H, I = c.hidden_size, c.intermediate_size
-        self.norm_shape, self.qkv_width, self.qkv_offsets = (H,), H + 2 * c.kv_size, [0, H, H + c.kv_size]
+        W3 = H + 2 * c.kv_size
+        self.norm_shape, self.qkv_offsets = (H,), [0, H, H + c.kv_size]
+        self.qkv_shapes = (("w", (W3, H)), ("wt", (H, W3)), ("bias", (W3,)))
         self.shapes = {"q_proj": (H, H), "k_proj": (c.kv_size, H), "v_proj": (c.kv_size, H), "o_proj": (H, H), "gate_proj": (I, H),
                        "up_proj": (I, H), "down_proj": (H, I)}   # [out, in]
+        # q, k and v are read from the stacked weight
+        self.own_weights = tuple((name, self.shapes[name], self.shapes[name][::-1]) for name in model.MODULES[3:])
         self.sizes: Dict[Tuple[int, int], Tuple[int, int]] = {}
         self.scratch = None
         self.shared = None    # without a backward to come, every layer uses the same block
@@ -124,16 +128,15 @@ class _LayerCalls:
         for w in (L["input_layernorm"], L["post_attention_layernorm"]):
             if w.shape != self.norm_shape or w.dtype != dt or not w.is_contiguous() or not w.is_cuda:
                 return False
-        for w, shape in ((fq["w"], (self.qkv_width, *self.norm_shape)), (fq["wt"], (*self.norm_shape, self.qkv_width)),
-                         (fq["bias"], (self.qkv_width,))):
+        for name, shape in self.qkv_shapes:
+            w = fq[name]
             if w.shape != shape or w.dtype != dt or not w.is_cuda:
                 return False
-        for name in self.model.MODULES[3:]:   # q, k and v are read from the stacked weight
-            lin, shape = L[name], self.shapes[name]
-            for w, want in ((lin.weight, shape), (lin.weight_t, shape[::-1])):
-                if w.shape != want or w.dtype != dt or not w.is_contiguous() or not w.is_cuda:
-                    return False
-            if lin.bias is not None:
+        for name, shape, shape_t in self.own_weights:
+            lin = L[name]
+            w, wt = lin.weight, lin.weight_t
+            if (w.shape != shape or wt.shape != shape_t or w.dtype != dt or wt.dtype != dt or not (w.is_contiguous() and wt.is_contiguous())
+                    or not (w.is_cuda and wt.is_cuda) or lin.bias is not None):
                 return False
         return True
 
