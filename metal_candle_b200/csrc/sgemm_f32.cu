@@ -258,8 +258,9 @@ __device__ __forceinline__ void redo_outputs(const TileParams& p, float* stage, 
 // and the mean deviation of positive terms is -1e-8 to -2e-8 (0, -1e-7).  Larger than the FMAs' where one term of a short sum dwarfs the
 // others, whose last bits it pushes out: exp(2 normal), 65 indices 1.8e-7 (1.0e-7, 7.4e-7), 768 indices 1.4e-7 (1.5e-7, 4.8e-7).
 // Bound: taking the values apart (about 4800 cycles a step of seven warps; the products are 16 BN), then a CTA's start and the exchange of
-// partial tiles.  us, FMAs / six products / this: 512 x 768 x 768 29 / 14.5 / 14.9, 2048 x 1536 x 1536 254 / 105 / 97, 64 x 256 x 128
-// 14.7 / 12.0 / 11.6.  (All 16 warps at everything, a barrier a half step: 18.5 and 151; one warp issuing beside its other work: 16.9 and 133.)
+// partial tiles.  us, FMAs / six products / this: 512 x 768 x 768 28.8 / 14.3 / 14.7, 2048 x 1536 x 1536 253 / 105 / 99, 256 x 1536 x 128
+// 28.8 / 14.3 / 14.4, 1200 x 200 x 1100 34.1 / 17.1 / 17.5, 1000^3 70.3 / 32.3 / 31.1, 300 x 1001 x 130 22.7 / 13.6 / 13.6.
+// (All 16 warps at everything, a barrier a half step: 18.5 and 151 for the first two; one warp issuing beside its other work: 16.9 and 133.)
 // A shape with few tiles (512 x 768 x 768: 24) leaves SMs idle, so up to 8 CTAs of a cluster share a tile's reduction and add their
 // partial tiles through distributed shared memory, in rank order: deterministic, no workspace.
 template <int BN>
